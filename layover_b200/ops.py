@@ -74,15 +74,25 @@ def _need_rows(t: torch.Tensor, dtype: torch.dtype | None, name: str) -> None:
 _signatures_done: set[str] = set()
 
 
-def _fn(lib_name: str, fn_name: str, argtypes):
+def _fn(lib_name: str, fn_name: str, argtypes, restype=c_int):
     lib = build.load(lib_name)
     fn = getattr(lib, fn_name)
     key = lib_name + "." + fn_name
     if key not in _signatures_done:
         fn.argtypes = argtypes
-        fn.restype = c_int
+        fn.restype = restype
         _signatures_done.add(key)
     return fn
+
+
+_sm_counts: dict[int, int] = {}
+
+
+def sm_count(device: torch.device) -> int:
+    index = torch.cuda.current_device() if device.index is None else device.index
+    if index not in _sm_counts:
+        _sm_counts[index] = torch.cuda.get_device_properties(index).multi_processor_count
+    return _sm_counts[index]
 
 
 # ------------------------------------------------------------------ elementwise
@@ -1091,10 +1101,17 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tens
         raise ValueError(f"gemm: shapes do not agree: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
     if a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
         raise ValueError("gemm: innermost dimension must be contiguous")
+    scratch = None
+    if a.dtype == torch.float32 and min(m, n, k) > 0:      # partial sums of this call alone, on its own stream
+        wanted = _fn("gemm_simt", "lb_gemm_simt_scratch", [c_int] * 4, c_long)(m, n, k, sm_count(a.device))
+        scratch = torch.empty(wanted, dtype=torch.float32, device=a.device) if wanted else None
     fn = _fn("gemm_simt", "lb_gemm_simt",
-             [c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_long, c_long, c_long, c_void_p])
+             [c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_long, c_long, c_long, c_void_p, c_int, c_void_p])
     _check(fn(dtype_code(a.dtype), dtype_code(out.dtype), _ptr(a), _ptr(w), _ptr(out), m, n, k, a.stride(0),
-              w.stride(0), out.stride(0), _stream()), "gemm_simt")
+              w.stride(0), out.stride(0), _ptr(scratch), sm_count(a.device), _stream()), "gemm_simt")
+    if scratch is not None:
+        global LAUNCHES
+        LAUNCHES += 1          # the ranges' sums are added by a kernel of their own
     return out
 
 
@@ -1202,7 +1219,8 @@ def sample(logits: torch.Tensor, tokens: torch.Tensor, records: torch.Tensor | N
 # `reset_after_error` puts back what such a block may have left behind (counters that a launch
 # normally returns to zero).
 _STATUS_LIBRARIES = (("gemm_tcgen05", "lb_gemm_tcgen05_status_address", "lb_gemm_tcgen05_status"),
-                     ("attention_tcgen05", "lb_attention_tcgen05_status_address", "lb_attention_tcgen05_status"))
+                     ("attention_tcgen05", "lb_attention_tcgen05_status_address", "lb_attention_tcgen05_status"),
+                     ("gemm_simt", "lb_gemm_simt_status_address", "lb_gemm_simt_status"))
 _status_words: dict[tuple[int, tuple[str, ...]], tuple[torch.Tensor, tuple[str, ...]]] = {}
 
 

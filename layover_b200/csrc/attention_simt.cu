@@ -13,26 +13,33 @@
 // denominator, o = sum_j exp(s_j) V_j / (exp(sink_h) + sum_j exp(s_j)); and a gate per (token,
 // head), a 32-bit factor on the head's output. Two more: a soft cap, s_j <- cap * tanh(s_j / cap), and a factor
 // `out_scale` on every output. Keys are walked in tiles of 32 aligned to absolute
-// positions (tile i holds keys [32 i, 32 i + 32)), each score is one sequential dot product and
-// the running maximum / sum follow the same recurrence for every row, so a row's result does
-// not depend on how the tokens were cut into steps or on which other rows share its block.
+// positions (tile i holds keys [32 i, 32 i + 32)), four tiles are a chunk. Within a chunk each score is a dot product
+// of four interleaved chains and the running maximum / sum / output follow the same recurrence for every row, starting
+// anew with the chunk; then the chunks' results are merged in their order. So a row's result does not depend on how the
+// tokens were cut into steps, on which other rows share its block, or on how many blocks share its keys.
 // Keys outside [first needed key, context length) are never used: their scores are replaced,
 // not multiplied, and their values are read as zero, so stale or non-finite contents of a page
 // cannot leak.
 //
 // Work is a list of tiles made on the host: tile w covers queries [tile_q0[w], +BQ) of sequence
-// tile_seq[w]. Grid = (tiles, query heads). Query t of sequence s is row cu_q[s] + t of q and
-// out, at absolute position ctx_len[s] - q_len(s) + t.
+// tile_seq[w]. Query t of sequence s is row cu_q[s] + t of q and out, at absolute position ctx_len[s] - q_len(s) + t. A
+// row is one query of one query head; the rows of a tile that share a key/value head share every load of its keys and
+// values: a block takes 4 R of them (R a warp), and with few blocks (a decode step) the chunks of a row are dealt to
+// `splits` blocks, which leave each chunk's maximum, sum and output in scratch memory for a second kernel to merge.
+// What bounds it: a decode step the latency of a tile (scores, softmax, output: about a thousand cycles for its 32 KB), which
+// more blocks hide; a prompt the reads of shared memory, one of 16 bytes per 4 R fused multiply-adds.
+// Measured (one B200, 32 query heads of 128 over 8, per layer): four decoding requests of 900 keys 386 -> 24.5 us and 3.6 for the
+// merge, a prompt of 261 tokens 205 -> 114 and 18 us (against a block per 16 queries of one head, a chain per score).
 #include <math.h>
 
 #include "common.cuh"
 
 namespace {
-constexpr int BQ = 16;      // queries per block
+constexpr int BQ = 16;      // queries per tile
 constexpr int BKEYS = 32;   // keys per tile (one per lane)
+constexpr int CHUNK_TILES = 4;
 constexpr int WARPS = 4;
-constexpr int ROWS_PER_WARP = BQ / WARPS;
-constexpr int MAX_DIM = 640;      // head sizes up to 256 keep 8 accumulators a lane, larger ones 20
+constexpr int MAX_DIM = 640;      // value sizes up to 128 keep one quad of the output a lane, the largest five
 
 // four neighbouring elements with one load (the head size is a multiple of 4 and rows are 16-byte aligned)
 template <typename T> struct Quad;
@@ -46,170 +53,398 @@ template <> struct Quad<bf16> {
     return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
   }
 };
+// a quad of a page into shared memory, or zeros: asynchronously where no conversion is needed
+__device__ __forceinline__ void fetch_quad(float* dst, const float* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(valid ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void fetch_quad(float* dst, const bf16* src, bool valid) {
+  *reinterpret_cast<float4*>(dst) = valid ? Quad<bf16>::load(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
 
-template <typename T, int ACC_PER_LANE>
+template <typename T> struct Attention {
+  const T *q, *k_pool, *v_pool;
+  T* out;
+  const int *block_table, *cu_q, *ctx_len, *tile_seq, *tile_q0;
+  const float *sinks, *gates;
+  float* partials;            // [item][row of the item][chunk][2 + vdim]; null: a block walks all of its rows' chunks
+  int chunk_room;             // chunks there is room for: all that a block table can hold
+  int table_width, q_heads, kv_heads, dim, key_pitch, vdim, page_tokens, window, mask_chunk, keep_first, row_groups, stages;
+  float scale, cap, out_scale;
+  long out_stride;
+};
+
+// What a block works on: rows first_row .. of a tile (row = query * group + query head of the group).
+struct Item {
+  int seq, row0, start, n_rows, group, kv_head, first_row;      // row0: the tile's first query in q; start: its position
+  template <typename T, int ROWS> static __device__ __forceinline__ Item at(const Attention<T>& a) {
+    Item item;
+    item.seq = a.tile_seq[blockIdx.x];
+    const int q0 = a.tile_q0[blockIdx.x], begin = a.cu_q[item.seq], q_len = a.cu_q[item.seq + 1] - begin;
+    item.group = a.q_heads / a.kv_heads;
+    item.row0 = begin + q0;
+    item.start = a.ctx_len[item.seq] - q_len + q0;
+    item.n_rows = min(BQ, q_len - q0) * item.group;
+    item.kv_head = blockIdx.y / a.row_groups;
+    item.first_row = blockIdx.y % a.row_groups * ROWS;
+    return item;
+  }
+  __device__ __forceinline__ int position(int row) const { return start + row / group; }
+};
+
+// One chunk's result joins those of the chunks before it; explicit roundings, the same bits wherever it happens.
+__device__ __forceinline__ float merge_scale(float& m, float& l, float chunk_m, float chunk_l, float& chunk_scale) {
+  const float top = fmaxf(m, chunk_m), keep = m == -INFINITY ? 0.f : expf(m - top);
+  chunk_scale = expf(chunk_m - top);
+  l = fmaf(chunk_l, chunk_scale, __fmul_rn(l, keep));
+  m = top;
+  return keep;
+}
+__device__ __forceinline__ void merge_quad(float4& total, const float4& chunk, float keep, float chunk_scale) {
+  total.x = fmaf(chunk.x, chunk_scale, __fmul_rn(total.x, keep));
+  total.y = fmaf(chunk.y, chunk_scale, __fmul_rn(total.y, keep));
+  total.z = fmaf(chunk.z, chunk_scale, __fmul_rn(total.z, keep));
+  total.w = fmaf(chunk.w, chunk_scale, __fmul_rn(total.w, keep));
+}
+
+template <typename T, int NV>
+__device__ __forceinline__ void store_row(const Attention<T>& a, const Item& item, int row, float m, float l, const float4 (&total)[NV], int lane) {
+  const int token = item.row0 + row / item.group, head = item.kv_head * item.group + row % item.group;
+  float denominator = l, keep = 1.f;
+  if (a.sinks) {                                   // the sink joins the denominator only; m is finite (a row sees itself)
+    const float sink = a.sinks[head], top = fmaxf(m, sink);
+    keep = expf(m - top);
+    denominator = l * keep + expf(sink - top);
+  }
+  const float gate = a.gates ? a.gates[(size_t)token * a.q_heads + head] : 1.f;
+  T* o = a.out + (size_t)token * a.out_stride + head * a.vdim;
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    const int d = 4 * (lane + 32 * n);
+    if (d >= a.vdim) continue;
+    const float v[4] = {total[n].x, total[n].y, total[n].z, total[n].w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float value = a.sinks ? v[e] * keep / denominator : v[e] / l;
+      if (a.gates) value *= gate;
+      value *= a.out_scale;
+      Elem<T>::store(o + d + e, value);
+    }
+  }
+}
+
+// NV: quads of a value that a lane accumulates. Row i of a warp is row 4 i + warp of the block's, so that few rows spread
+// over the warps.
+template <typename T, int NV, int R>
 __global__ void __launch_bounds__(WARPS * 32)
-paged_attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const T* __restrict__ v_pool,
-                            T* __restrict__ out, const int* __restrict__ block_table, int table_width,
-                            const int* __restrict__ cu_q, const int* __restrict__ ctx_len,
-                            const int* __restrict__ tile_seq, const int* __restrict__ tile_q0, int q_heads,
-                            int kv_heads, int dim, int page_tokens, float scale, int window, int vdim,
-                            const float* __restrict__ sinks, const float* __restrict__ gates, int mask_chunk,
-                            int keep_first, float cap, float out_scale, long out_stride) {
+attention_rows_kernel(const Attention<T> a) {
   extern __shared__ __align__(16) float smem[];
+  constexpr int ROWS = WARPS * R;
   pdl_launch_dependents();
   pdl_wait();
-  float* q_s = smem;                               // [BQ][dim]
-  float* k_s = q_s + BQ * dim;                     // [BKEYS][dim + 1]
-  float* v_s = k_s + BKEYS * (dim + 1);            // [BKEYS][vdim]
-
-  const int seq = tile_seq[blockIdx.x], q0 = tile_q0[blockIdx.x];
-  const int head = blockIdx.y, kv_head = head / (q_heads / kv_heads);
-  const int row0 = cu_q[seq], q_len = cu_q[seq + 1] - row0, ctx = ctx_len[seq];
-  const int start = ctx - q_len;                   // absolute position of the sequence's first query here
-  const int n_q = min(BQ, q_len - q0);
+  const Item item = Item::at<T, ROWS>(a);
+  if (item.first_row >= item.n_rows) return;
+  const int dim = a.dim, vdim = a.vdim, pitch = a.key_pitch;
+  float* q_s = smem;                                             // [ROWS][dim]
+  float* p_s = q_s + ROWS * dim;                                 // [WARPS][R][BKEYS]
+  float* k_s = p_s + ROWS * BKEYS;                               // [stages][BKEYS][pitch]
+  float* v_s = k_s + a.stages * BKEYS * pitch;                   // [stages][BKEYS][vdim]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int* table = block_table + (size_t)seq * table_width;
+  const int rows = min(ROWS, item.n_rows - item.first_row);      // live rows of the block
+  const int mine = rows > warp ? (rows - warp + WARPS - 1) / WARPS : 0;       // and of the warp
+  const int* table = a.block_table + (size_t)item.seq * a.table_width;
 
-  for (int i = threadIdx.x; i < n_q * dim; i += blockDim.x) {
-    const int r = i / dim, c = i % dim;
-    q_s[r * dim + c] = Elem<T>::load(q + ((size_t)(row0 + q0 + r) * q_heads + head) * dim + c);
+  for (int r = warp; r < rows; r += WARPS) {
+    const int row = item.first_row + r;
+    const T* src = a.q + ((size_t)(item.row0 + row / item.group) * a.q_heads + item.kv_head * item.group + row % item.group) * dim;
+    for (int c = 4 * lane; c < dim; c += 128) *reinterpret_cast<float4*>(q_s + r * dim + c) = Quad<T>::load(src + c);
   }
-
-  const int p_first = start + q0, p_last = start + q0 + n_q - 1;
-  int key_lo = window > 0 ? max(0, p_first - window + 1) : 0;        // first key any row here may see
-  if (mask_chunk > 0) key_lo = max(key_lo, p_first / mask_chunk * mask_chunk);
+  const int p_first = item.position(item.first_row), p_last = item.position(item.first_row + rows - 1);
+  int key_lo = a.window > 0 ? max(0, p_first - a.window + 1) : 0;            // first key any row here may see
+  if (a.mask_chunk > 0) key_lo = max(key_lo, p_first / a.mask_chunk * a.mask_chunk);
   const int tile_lo = key_lo / BKEYS, tile_hi = p_last / BKEYS;
   // the tiles of the kept first keys come first, then the window's; tiles between the two are skipped
-  const int kept_keys = window > 0 ? min(keep_first, key_lo) : 0;        // kept keys that lie before the window
-  const int kept_tiles = min((kept_keys + BKEYS - 1) / BKEYS, tile_lo), skipped = tile_lo - kept_tiles;
-
-  float m[ROWS_PER_WARP], l[ROWS_PER_WARP], acc[ROWS_PER_WARP][ACC_PER_LANE];
-#pragma unroll
-  for (int r = 0; r < ROWS_PER_WARP; ++r) {
-    m[r] = -INFINITY;
-    l[r] = 0.f;
-#pragma unroll
-    for (int c = 0; c < ACC_PER_LANE; ++c) acc[r][c] = 0.f;
+  const int kept_keys = a.window > 0 ? min(a.keep_first, key_lo) : 0;        // kept keys that lie before the window
+  const int kept_tiles = min((kept_keys + BKEYS - 1) / BKEYS, tile_lo);
+  const int chunks = tile_hi / CHUNK_TILES + 1, per_block = (chunks + gridDim.z - 1) / gridDim.z;
+  const int chunk_begin = blockIdx.z * per_block, chunk_end = min(chunks, chunk_begin + per_block);
+  if (chunk_begin >= chunk_end) return;
+  const int tile_end = min(tile_hi + 1, chunk_end * CHUNK_TILES);
+  auto seen_tile = [&](int tile) { return tile >= kept_tiles && tile < tile_lo ? tile_lo : tile; };
+  float* left = nullptr;                                         // where the warp's rows leave their chunks' results
+  if (a.partials) {
+    left = a.partials + ((size_t)(blockIdx.x * gridDim.y + blockIdx.y) * ROWS + warp) * a.chunk_room * (vdim + 2);
+    if (lane == 0)
+      for (int r = 0; r < mine; ++r)
+        for (int c = chunk_begin; c < chunk_end; ++c) left[((size_t)r * WARPS * a.chunk_room + c) * (vdim + 2)] = -INFINITY;
   }
 
-  for (int walk = 0; walk <= tile_hi - skipped; ++walk) {
-    const int tile = walk < kept_tiles ? walk : walk + skipped;
-    __syncthreads();  // the previous tile is no longer read (and q_s is complete)
-    const int quads = dim >> 2;
-    for (int i = threadIdx.x; i < BKEYS * quads; i += blockDim.x) {
-      const int j = i / quads, c = (i - j * quads) << 2;
-      const int key = tile * BKEYS + j;
-      float4 kv = make_float4(0.f, 0.f, 0.f, 0.f);
-      if ((key >= key_lo || key < kept_keys) && key <= p_last) {
-        const size_t page = (size_t)table[key / page_tokens];
-        kv = Quad<T>::load(k_pool + ((page * kv_heads + kv_head) * page_tokens + key % page_tokens) * dim + c);
-      }
-      float* kd = k_s + j * (dim + 1) + c;
-      kd[0] = kv.x; kd[1] = kv.y; kd[2] = kv.z; kd[3] = kv.w;
+  auto fetch = [&](int tile, int stage) {
+    // the pages of the warp's keys in one load, a lane each: a copy that waits for its own page every time takes as many trips
+    // to memory as the warp has keys
+    constexpr int EACH = BKEYS / WARPS;
+    const int my_key = tile * BKEYS + warp + (lane % EACH) * WARPS;
+    const bool my_valid = (my_key >= key_lo || my_key < kept_keys) && my_key <= p_last;
+    const int my_page = my_valid ? table[my_key / a.page_tokens] : -1;
+#pragma unroll 2
+    for (int i = 0; i < EACH; ++i) {
+      const int j = warp + i * WARPS, key = tile * BKEYS + j, page = __shfl_sync(0xffffffffu, my_page, i);
+      const bool valid = page >= 0;
+      const size_t at = valid ? ((size_t)page * a.kv_heads + item.kv_head) * a.page_tokens + key % a.page_tokens : 0;
+      for (int c = 4 * lane; c < dim; c += 128) fetch_quad(k_s + (stage * BKEYS + j) * pitch + c, a.k_pool + at * dim + c, valid);
+      for (int c = 4 * lane; c < vdim; c += 128) fetch_quad(v_s + (stage * BKEYS + j) * vdim + c, a.v_pool + at * vdim + c, valid);
     }
-    const int vquads = vdim >> 2;
-    for (int i = threadIdx.x; i < BKEYS * vquads; i += blockDim.x) {
-      const int j = i / vquads, c = (i - j * vquads) << 2;
-      const int key = tile * BKEYS + j;
-      float4 vv = make_float4(0.f, 0.f, 0.f, 0.f);
-      if ((key >= key_lo || key < kept_keys) && key <= p_last) {
-        const size_t page = (size_t)table[key / page_tokens];
-        vv = Quad<T>::load(v_pool + ((page * kv_heads + kv_head) * page_tokens + key % page_tokens) * vdim + c);
-      }
-      *reinterpret_cast<float4*>(v_s + j * vdim + c) = vv;
-    }
-    __syncthreads();
-    const int key = tile * BKEYS + lane;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  float m[R], l[R], total_m[R], total_l[R];
+  float4 acc[R][NV], total[R][NV];
 #pragma unroll
-    for (int r = 0; r < ROWS_PER_WARP; ++r) {
-      const int row = warp * ROWS_PER_WARP + r;
-      if (row >= n_q) continue;  // uniform over the warp
-      const int p = p_first + row;
-      const bool seen = key <= p && (window <= 0 || p - key < window || key < keep_first) &&
-                        (mask_chunk <= 0 || key >= p / mask_chunk * mask_chunk);
-      float s = 0.f;
-      const float* qr = q_s + row * dim;
-      const float* kr = k_s + lane * (dim + 1);
-      for (int c = 0; c < dim; ++c) s = fmaf(qr[c], kr[c], s);
-      s *= scale;
-      if (cap > 0.f) s = cap * tanhf(s / cap);
+  for (int r = 0; r < R; ++r) {
+    m[r] = total_m[r] = -INFINITY;
+    l[r] = total_l[r] = 0.f;
+#pragma unroll
+    for (int n = 0; n < NV; ++n) acc[r][n] = total[r][n] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+
+  int tile = seen_tile(chunk_begin * CHUNK_TILES), stage = 0;
+  if (tile < tile_end) fetch(tile, 0);
+  while (tile < tile_end) {
+    const int next = seen_tile(tile + 1);
+    if (a.stages > 1 && next < tile_end) {
+      fetch(next, stage ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();                                             // the tile (and q_s) is complete
+    const float* k_row = k_s + (stage * BKEYS + lane) * pitch;
+    float4 s4[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) s4[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int c = 0; c < dim; c += 4) {
+      const float4 k = *reinterpret_cast<const float4*>(k_row + c);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        if (R > 1 && r >= mine) break;
+        const float4 qv = *reinterpret_cast<const float4*>(q_s + (WARPS * r + warp) * dim + c);
+        s4[r].x = fmaf(qv.x, k.x, s4[r].x);
+        s4[r].y = fmaf(qv.y, k.y, s4[r].y);
+        s4[r].z = fmaf(qv.z, k.z, s4[r].z);
+        s4[r].w = fmaf(qv.w, k.w, s4[r].w);
+      }
+    }
+    const int key = tile * BKEYS + lane;
+    float* p_row = p_s + warp * R * BKEYS;
+    unsigned active = 0;                                         // rows that see something of this tile
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (r >= mine) break;                                      // uniform over the warp
+      const int p = item.position(item.first_row + WARPS * r + warp);
+      const bool seen = key <= p && (a.window <= 0 || p - key < a.window || key < a.keep_first) &&
+                        (a.mask_chunk <= 0 || key >= p / a.mask_chunk * a.mask_chunk);
+      float s = __fadd_rn(__fadd_rn(s4[r].x, s4[r].y), __fadd_rn(s4[r].z, s4[r].w));
+      s = __fmul_rn(s, a.scale);
+      if (a.cap > 0.f) s = a.cap * tanhf(s / a.cap);
       s = seen ? s : -INFINITY;
       const float tile_max = warp_max(s);
-      if (tile_max == -INFINITY) continue;  // nothing of this tile is seen by this row
-      const float m_new = fmaxf(m[r], tile_max);
-      const float prob = seen ? expf(s - m_new) : 0.f;
-      const float alpha = m[r] == -INFINITY ? 0.f : expf(m[r] - m_new);
-      l[r] = l[r] * alpha + warp_sum(prob);
-      m[r] = m_new;
+      if (tile_max == -INFINITY) continue;
+      active |= 1u << r;
+      const float top = fmaxf(m[r], tile_max), prob = seen ? expf(s - top) : 0.f;
+      const float alpha = m[r] == -INFINITY ? 0.f : expf(m[r] - top);
+      l[r] = __fadd_rn(__fmul_rn(l[r], alpha), warp_sum(prob));
+      m[r] = top;
+      p_row[r * BKEYS + lane] = prob;
 #pragma unroll
-      for (int c = 0; c < ACC_PER_LANE; ++c) acc[r][c] *= alpha;
-      for (int j = 0; j < BKEYS; ++j) {
-        const float pj = __shfl_sync(0xffffffffu, prob, j);
+      for (int n = 0; n < NV; ++n) {
+        acc[r][n].x *= alpha; acc[r][n].y *= alpha; acc[r][n].z *= alpha; acc[r][n].w *= alpha;
+      }
+    }
+    __syncwarp();
+#pragma unroll 2
+    for (int j = 0; j < BKEYS; j += 4) {
+      float4 p4[R];
 #pragma unroll
-        for (int c = 0; c < ACC_PER_LANE; ++c) {
-          const int d = lane + 32 * c;
-          if (d < vdim) acc[r][c] = fmaf(pj, v_s[j * vdim + d], acc[r][c]);
+      for (int r = 0; r < R; ++r)
+        if (active >> r & 1) p4[r] = *reinterpret_cast<const float4*>(p_row + r * BKEYS + j);
+#pragma unroll
+      for (int n = 0; n < NV; ++n) {
+        const int d = 4 * (lane + 32 * n);
+        if (d >= vdim) break;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float4 v = *reinterpret_cast<const float4*>(v_s + (stage * BKEYS + j + e) * vdim + d);
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            if (!(active >> r & 1)) continue;
+            const float p = e == 0 ? p4[r].x : e == 1 ? p4[r].y : e == 2 ? p4[r].z : p4[r].w;
+            acc[r][n].x = fmaf(p, v.x, acc[r][n].x);
+            acc[r][n].y = fmaf(p, v.y, acc[r][n].y);
+            acc[r][n].z = fmaf(p, v.z, acc[r][n].z);
+            acc[r][n].w = fmaf(p, v.w, acc[r][n].w);
+          }
         }
       }
     }
-  }
+    if (next >= tile_end || next / CHUNK_TILES != tile / CHUNK_TILES) {        // the chunk is done
 #pragma unroll
-  for (int r = 0; r < ROWS_PER_WARP; ++r) {
-    const int row = warp * ROWS_PER_WARP + r;
-    if (row >= n_q) continue;
-    T* o = out + (size_t)(row0 + q0 + row) * out_stride + head * vdim;
-    float denominator = l[r], keep = 1.f;
-    if (sinks) {                                   // the sink joins the denominator only; m is finite (a row sees itself)
-      const float sink = sinks[head], top = fmaxf(m[r], sink);
-      keep = expf(m[r] - top);
-      denominator = l[r] * keep + expf(sink - top);
-    }
-    const float gate = gates ? gates[(size_t)(row0 + q0 + row) * q_heads + head] : 1.f;
+      for (int r = 0; r < R; ++r) {
+        if (r >= mine) break;
+        if (m[r] == -INFINITY) continue;                         // nothing of it is seen by this row
+        if (left) {
+          float* at = left + ((size_t)r * WARPS * a.chunk_room + tile / CHUNK_TILES) * (vdim + 2);
+          if (lane == 0) { at[0] = m[r]; at[1] = l[r]; }
 #pragma unroll
-    for (int c = 0; c < ACC_PER_LANE; ++c) {
-      const int d = lane + 32 * c;
-      if (d < vdim) {
-        float value = sinks ? acc[r][c] * keep / denominator : acc[r][c] / l[r];
-        if (gates) value *= gate;
-        value *= out_scale;
-        Elem<T>::store(o + d, value);
+          for (int n = 0; n < NV; ++n) {
+            const int d = 4 * (lane + 32 * n);
+            if (d < vdim) {
+              reinterpret_cast<float2*>(at + 2 + d)[0] = make_float2(acc[r][n].x, acc[r][n].y);
+              reinterpret_cast<float2*>(at + 2 + d)[1] = make_float2(acc[r][n].z, acc[r][n].w);
+            }
+          }
+        } else {
+          float chunk_scale;
+          const float keep = merge_scale(total_m[r], total_l[r], m[r], l[r], chunk_scale);
+#pragma unroll
+          for (int n = 0; n < NV; ++n) merge_quad(total[r][n], acc[r][n], keep, chunk_scale);
+        }
+        m[r] = -INFINITY;
+        l[r] = 0.f;
+#pragma unroll
+        for (int n = 0; n < NV; ++n) acc[r][n] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
+    __syncthreads();                                             // the tile is read
+    if (a.stages == 1 && next < tile_end) fetch(next, 0);
+    if (a.stages > 1) stage ^= 1;
+    tile = next;
   }
+  if (!left) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (r < mine) store_row<T, NV>(a, item, item.first_row + WARPS * r + warp, total_m[r], total_l[r], total[r], lane);
+  }
+}
+
+// Merges the chunks' results of every row in their order: a warp per row, four chunks' loads on their way at once.
+template <typename T, int NV, int R>
+__global__ void __launch_bounds__(WARPS * 32)
+merge_chunks_kernel(const Attention<T> a) {
+  constexpr int ROWS = WARPS * R;
+  pdl_launch_dependents();
+  pdl_wait();
+  const Item item = Item::at<T, ROWS>(a);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rows = min(ROWS, item.n_rows - item.first_row);
+  if (rows <= 0) return;
+  const int chunks = item.position(item.first_row + rows - 1) / BKEYS / CHUNK_TILES + 1;
+  for (int row = warp; row < rows; row += WARPS) {
+    const float* left = a.partials + ((size_t)(blockIdx.x * gridDim.y + blockIdx.y) * ROWS + row) * a.chunk_room * (a.vdim + 2);
+    float m = -INFINITY, l = 0.f;
+    float4 total[NV];
+#pragma unroll
+    for (int n = 0; n < NV; ++n) total[n] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int c0 = 0; c0 < chunks; c0 += 4) {
+      float2 ml[4];
+      float4 part[4][NV];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float* at = left + (size_t)(c0 + c) * (a.vdim + 2);
+        ml[c] = c0 + c < chunks ? make_float2(at[0], at[1]) : make_float2(-INFINITY, 0.f);
+#pragma unroll
+        for (int n = 0; n < NV; ++n) {
+          const int d = 4 * (lane + 32 * n);
+          part[c][n] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (c0 + c < chunks && d < a.vdim) {
+            const float2 lo = reinterpret_cast<const float2*>(at + 2 + d)[0], hi = reinterpret_cast<const float2*>(at + 2 + d)[1];
+            part[c][n] = make_float4(lo.x, lo.y, hi.x, hi.y);
+          }
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        if (ml[c].x == -INFINITY) continue;
+        float chunk_scale;
+        const float keep = merge_scale(m, l, ml[c].x, ml[c].y, chunk_scale);
+#pragma unroll
+        for (int n = 0; n < NV; ++n) merge_quad(total[n], part[c][n], keep, chunk_scale);
+      }
+    }
+    store_row<T, NV>(a, item, item.first_row + row, m, l, total, lane);
+  }
+}
+
+template <typename T, int NV, int R>
+int launch_rows(Attention<T> a, int n_tiles, int max_rows, int splits, cudaStream_t stream) {
+  constexpr int ROWS = WARPS * R;
+  static LbPerDeviceOnce configured;
+  if (configured.first() &&
+      cudaFuncSetAttribute(attention_rows_kernel<T, NV, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
+    return lb_last_error();
+  a.row_groups = (max_rows + ROWS - 1) / ROWS;
+  auto smem = [&](int stages) { return (size_t)(ROWS * (a.dim + BKEYS) + stages * BKEYS * (a.key_pitch + a.vdim)) * sizeof(float); };
+  a.stages = smem(2) <= 227 * 1024 ? 2 : 1;
+  if (smem(a.stages) > 227 * 1024 || (long)a.kv_heads * a.row_groups > 65535) return LB_ERR_SIZE;
+  const dim3 grid(n_tiles, a.kv_heads * a.row_groups, a.partials ? splits : 1);
+  lb_launch(attention_rows_kernel<T, NV, R>, grid, dim3(WARPS * 32), smem(a.stages), stream, a);
+  if (a.partials) lb_launch(merge_chunks_kernel<T, NV, R>, dim3(grid.x, grid.y), dim3(WARPS * 32), 0, stream, a);
+  return lb_last_error();
+}
+
+// Rows of a warp: enough for a block to hold a tile's rows of a key/value head at once, as far as registers go.
+int rows_per_warp(int max_rows, int vdim) {
+  if (max_rows <= WARPS) return 1;
+  return vdim <= 128 ? (max_rows <= 4 * WARPS ? 4 : 8) : (vdim <= 256 ? 4 : 2);
+}
+
+template <typename T>
+int launch_attention(const Attention<T>& a, int n_tiles, int max_rows, int splits, cudaStream_t stream) {
+  const int r = rows_per_warp(max_rows, a.vdim);
+  if (a.vdim <= 128) {
+    if (r == 1) return launch_rows<T, 1, 1>(a, n_tiles, max_rows, splits, stream);
+    return r == 4 ? launch_rows<T, 1, 4>(a, n_tiles, max_rows, splits, stream) : launch_rows<T, 1, 8>(a, n_tiles, max_rows, splits, stream);
+  }
+  if (a.vdim <= 256) return r == 1 ? launch_rows<T, 2, 1>(a, n_tiles, max_rows, splits, stream) : launch_rows<T, 2, 4>(a, n_tiles, max_rows, splits, stream);
+  return r == 1 ? launch_rows<T, 5, 1>(a, n_tiles, max_rows, splits, stream) : launch_rows<T, 5, 2>(a, n_tiles, max_rows, splits, stream);
 }
 }  // namespace
 
 LB_EXPORT int lb_attention_simt_block_queries() { return BQ; }
 
+// Blocks that a launch has without a split, and the rows that each leaves results for: what a caller needs to size the
+// scratch (blocks * rows * chunks a block table can hold * (vdim + 2) floats) and to choose `splits`.
+LB_EXPORT int lb_attention_simt_plan(int n_tiles, int q_heads, int kv_heads, int vdim, int max_q_len, int* rows_of_block) {
+  if (kv_heads <= 0 || q_heads % kv_heads) return 0;
+  const int max_rows = (max_q_len < BQ ? max_q_len : BQ) * (q_heads / kv_heads);
+  *rows_of_block = WARPS * rows_per_warp(max_rows, vdim);
+  return n_tiles * kv_heads * ((max_rows + *rows_of_block - 1) / *rows_of_block);
+}
+LB_EXPORT int lb_attention_simt_chunk() { return BKEYS * CHUNK_TILES; }
+
+// `max_q_len`: no sequence has more queries in this step (BQ or more: any number). `splits` > 1: the keys of a row are dealt to
+// that many blocks, `partials` has the room that `lb_attention_simt_plan` speaks of, `chunk_room` chunks a row.
 LB_EXPORT int lb_attention_simt(int dtype, const void* q, const void* k_pool, const void* v_pool, void* out,
                                 const int* block_table, int table_width, const int* cu_q, const int* ctx_len,
                                 const int* tile_seq, const int* tile_q0, int n_tiles, int q_heads, int kv_heads,
                                 int dim, int page_tokens, float scale, int window, int vdim, const float* sinks,
                                 const float* gates, int mask_chunk, int keep_first, float softcap, float out_scale,
-                                long out_stride, cudaStream_t stream) {
+                                long out_stride, int max_q_len, int splits, float* partials, int chunk_room, cudaStream_t stream) {
   if (n_tiles <= 0) return 0;
   if (dim <= 0 || dim > MAX_DIM || dim % 4 || kv_heads <= 0 || q_heads % kv_heads || q_heads > 65535) return LB_ERR_SIZE;
   if (vdim <= 0 || vdim > MAX_DIM || vdim % 4 || keep_first < 0 || (keep_first && mask_chunk)) return LB_ERR_SIZE;
-  if (!(softcap >= 0.f) || out_stride < (long)q_heads * vdim) return LB_ERR_SIZE;
-  // q rows, key rows padded by one float, value rows (16-byte aligned: both sizes are multiples of 4)
-  const size_t smem = (size_t)(BQ * dim + BKEYS * (dim + 1) + BKEYS * vdim) * sizeof(float);
-  dim3 grid(n_tiles, q_heads);
-  if (smem > 227 * 1024) return LB_ERR_SIZE;
-#define LB_SIMT(T, ACC)                                                                                                      \
+  if (!(softcap >= 0.f) || out_stride < (long)q_heads * vdim || max_q_len < 1 || (splits > 1 && !partials)) return LB_ERR_SIZE;
+  const int max_rows = (max_q_len < BQ ? max_q_len : BQ) * (q_heads / kv_heads);
+  // rows of a key tile: a pitch of 4 floats beyond a multiple of 32 keeps the 16-byte reads of 32 keys free of bank conflicts
+  const int key_pitch = dim + (36 - dim % 32) % 32;
+#define LB_SIMT(T)                                                                                                           \
   do {                                                                                                                       \
-    if (smem > 48 * 1024)                                                                                                    \
-      cudaFuncSetAttribute(paged_attention_simt_kernel<T, ACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
-    lb_launch(paged_attention_simt_kernel<T, ACC>, grid, WARPS * 32, smem, stream, (const T*)q, (const T*)k_pool,            \
-              (const T*)v_pool, (T*)out, block_table, table_width, cu_q, ctx_len, tile_seq, tile_q0, q_heads, kv_heads, dim, \
-              page_tokens, scale, window, vdim, sinks, gates, mask_chunk, keep_first, softcap, out_scale, out_stride);       \
+    Attention<T> a{(const T*)q, (const T*)k_pool, (const T*)v_pool, (T*)out, block_table, cu_q, ctx_len, tile_seq, tile_q0,   \
+                   sinks, gates, splits > 1 ? partials : nullptr, chunk_room, table_width, q_heads, kv_heads, dim, key_pitch, \
+                   vdim, page_tokens, window, mask_chunk, keep_first, 0, 0, scale, softcap, out_scale, out_stride};           \
+    return launch_attention<T>(a, n_tiles, max_rows, splits, stream);                                                        \
   } while (0)
-  if (dtype == LB_F32) {
-    if (vdim <= 256) LB_SIMT(float, 8); else LB_SIMT(float, 20);
-  } else if (dtype == LB_BF16) {
-    if (vdim <= 256) LB_SIMT(bf16, 8); else LB_SIMT(bf16, 20);
-  } else
-    return LB_ERR_DTYPE;
+  if (dtype == LB_F32) LB_SIMT(float);
+  if (dtype == LB_BF16) LB_SIMT(bf16);
 #undef LB_SIMT
-  return lb_last_error();
+  return LB_ERR_DTYPE;
 }

@@ -1130,7 +1130,7 @@ def attention_simt(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, 
                    tile_q0: torch.Tensor, n_tiles: int, q_heads: int, kv_heads: int, dim: int, page_tokens: int,
                    scale: float, window: int = 0, vdim: int | None = None, sinks: torch.Tensor | None = None,
                    gates: torch.Tensor | None = None, chunk: int = 0, keep_first: int = 0, softcap: float = 0.0,
-                   out_scale: float = 1.0) -> torch.Tensor:
+                   out_scale: float = 1.0, max_q_len: int | None = None, max_ctx: int = 0) -> torch.Tensor:
     """Paged causal attention in 32-bit arithmetic for any mix of segment lengths.
 
     q [T, q_heads * dim]; out [T, q_heads * vdim] (vdim defaults to dim); pools [pages, kv_heads, page_tokens,
@@ -1139,7 +1139,9 @@ def attention_simt(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, 
     denominator only; `gates` float32 [T, q_heads]: a factor on each head's output. `chunk` > 0: a query sees
     only the keys of its own chunk of that many positions (counted from position 0 of its sequence). `keep_first` > 0:
     behind a window the first `keep_first` keys of the sequence stay visible. `softcap` > 0: a score s becomes softcap *
-    tanh(s / softcap). `out_scale` multiplies the outputs; `out` may be a view into wider rows."""
+    tanh(s / softcap). `out_scale` multiplies the outputs; `out` may be a view into wider rows. `max_q_len`: no sequence has
+    more queries in this step (None: unknown). `max_ctx`: about the longest context (0: unknown); steps of few blocks deal
+    its keys to several. Neither changes a bit of the result."""
     vdim = dim if vdim is None else int(vdim)
     _need(q, None, "q"); _need_rows(out, q.dtype, "out"); _need(k_pool, q.dtype, "k_pool"); _need(v_pool, q.dtype, "v_pool")
     if tuple(out.shape) != (q.shape[0], q_heads * vdim) or k_pool.shape[-1] != dim or v_pool.shape[-1] != vdim:
@@ -1155,15 +1157,48 @@ def attention_simt(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, 
     for name, t in (("block_table", block_table), ("cu_q", cu_q), ("ctx_len", ctx_len), ("tile_seq", tile_seq),
                     ("tile_q0", tile_q0)):
         _need(t, torch.int32, name)
+    max_q_len = 1 << 30 if max_q_len is None else int(max_q_len)
+    splits, chunk_room = _simt_splits(n_tiles, q_heads, kv_heads, vdim, max_q_len, max_ctx, block_table.shape[1] * page_tokens, q.device)
+    partials = None
+    if splits > 1:          # of this call alone, on its own stream
+        partials = torch.empty(_simt_rows(n_tiles, q_heads, kv_heads, vdim, max_q_len)[1] * chunk_room * (vdim + 2),
+                               dtype=torch.float32, device=q.device)
     fn = _fn("attention_simt", "lb_attention_simt",
              [c_int] + [c_void_p] * 5 + [c_int] + [c_void_p] * 4 + [c_int] * 5 + [c_float, c_int, c_int, c_void_p,
-                                                                                c_void_p, c_int, c_int, c_float, c_float, c_long, c_void_p])
+              c_void_p, c_int, c_int, c_float, c_float, c_long, c_int, c_int, c_void_p, c_int, c_void_p])
     _check(fn(dtype_code(q.dtype), _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(out), _ptr(block_table),
               block_table.shape[1], _ptr(cu_q), _ptr(ctx_len), _ptr(tile_seq), _ptr(tile_q0), n_tiles, q_heads,
               kv_heads, dim, page_tokens, float(scale), int(window), vdim, _ptr(sinks), _ptr(gates), int(chunk), int(keep_first),
-              float(softcap), float(out_scale), out.stride(0), _stream()),
+              float(softcap), float(out_scale), out.stride(0), max_q_len, splits, _ptr(partials), chunk_room, _stream()),
            "attention_simt")
+    if splits > 1:
+        global LAUNCHES
+        LAUNCHES += 1          # the chunks' results are merged by a kernel of their own
     return out
+
+
+def _simt_rows(n_tiles: int, q_heads: int, kv_heads: int, vdim: int, max_q_len: int) -> tuple[int, int]:
+    """(blocks, rows over all blocks) of the 32-bit attention kernel without a split."""
+    rows = c_int(0)
+    blocks = _fn("attention_simt", "lb_attention_simt_plan", [c_int] * 5 + [c_void_p])(n_tiles, q_heads, kv_heads, vdim, max_q_len,
+                                                                                       ctypes.addressof(rows))
+    return blocks, blocks * rows.value
+
+
+_SIMT_SCRATCH_FLOATS = 64 << 20     # the most that the chunks' results may take (256 MiB)
+
+
+def _simt_splits(n_tiles: int, q_heads: int, kv_heads: int, vdim: int, max_q_len: int, max_ctx: int, room_tokens: int,
+                 device: torch.device) -> tuple[int, int]:
+    """(blocks that share a row's keys, chunks there must be room for): three blocks an SM where the rows alone do not give
+    them, as far as there are chunks to share."""
+    keys = _fn("attention_simt", "lb_attention_simt_chunk", [])()
+    blocks, rows = _simt_rows(n_tiles, q_heads, kv_heads, vdim, max_q_len)
+    room = -(-room_tokens // keys)
+    splits = min(-(-max_ctx // keys), -(-3 * sm_count(device) // max(blocks, 1)), room)
+    if splits <= 1 or rows * room * (vdim + 2) > _SIMT_SCRATCH_FLOATS:
+        return 1, 0
+    return splits, room
 
 
 def attention_f32(q, cache, out, block_table, batch, q_heads, kv_heads, dim, page_tokens, scale, window, vdim=None,
@@ -1173,7 +1208,7 @@ def attention_f32(q, cache, out, block_table, batch, q_heads, kv_heads, dim, pag
     tiles = batch.tiles[attention_simt_block_queries()]
     attention_simt(q, cache.k_pool, cache.v_pool, out, block_table, batch.cu_q, batch.ctx_len, tiles.tile_seq, tiles.tile_q0,
                    tiles.count, q_heads, kv_heads, dim, page_tokens, scale, window, vdim, sinks, gates, chunk, keep_first,
-                   softcap, out_scale)
+                   softcap, out_scale, batch.max_q_len, max(batch.max_ctx, batch.plan_max_ctx))
 
 
 # ------------------------------------------------------------------ sampling

@@ -1,13 +1,13 @@
-"""The 32-bit path's products at the edges of their tiles, ranges, groups and splits.
+"""The 32-bit path's products and attention at the edges of their tiles, ranges, groups and splits.
 
-They promise the same bits for a row however the work is cut; the values are checked against float64."""
+Both promise the same bits for a row however the work is cut; the values are checked against float64."""
 
 import math
 
 import pytest
 import torch
 
-from test_gpu_kernels import ops
+from test_gpu_kernels import ops, paged_setup
 
 pytestmark = pytest.mark.gpu
 
@@ -27,3 +27,45 @@ def test_f32_product_has_the_same_bits_in_every_batch(n, k):
         part = torch.empty(hi - lo, n, device="cuda")
         ops().gemm_simt(a[lo:hi], w, part)
         assert torch.equal(part, full[lo:hi]), (lo, hi)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("q_heads, kv_heads, dim, vdim", [(4, 1, 16, 16), (4, 2, 128, 128), (6, 2, 64, 132), (9, 1, 28, 256), (5, 1, 300, 260)])
+@pytest.mark.parametrize("mask", [{}, {"window": 100}, {"window": 40, "keep_first": 5}, {"chunk": 96}])
+def test_f32_attention_split_over_blocks_has_the_bits_of_one_block(dtype, q_heads, kv_heads, dim, vdim, mask):
+    """Contexts at the edges of a tile of 32 and a chunk of 128 keys; decoded tokens alone, and beside portions."""
+    o, page = ops(), 16
+    for lengths, q_lens in (([1, 127, 128, 129, 700], [1] * 5), ([31, 300, 260, 513], [31, 1, 40, 2])):
+        k_pool, _, table, ks, _ = paged_setup(dtype, lengths, kv_heads, dim, page, 5)
+        _, v_pool, _, _, vs = paged_setup(dtype, lengths, kv_heads, vdim, page, 5)      # the same pages, from the same seed
+        tokens = sum(q_lens)
+        gen = torch.Generator().manual_seed(6)
+        q = torch.randn(tokens, q_heads * dim, generator=gen).to(dtype).cuda()
+        starts = [sum(q_lens[:s]) for s in range(len(q_lens) + 1)]
+        bq = o.attention_simt_block_queries()
+        tiles = [(s, q0) for s, n in enumerate(q_lens) for q0 in range(0, n, bq)]
+        ints = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+        tile_seq, tile_q0 = ints([t[0] for t in tiles]), ints([t[1] for t in tiles])
+        outs = []
+        for hints in ({}, {"max_q_len": max(q_lens)}, {"max_q_len": max(q_lens), "max_ctx": max(lengths)}, {"max_ctx": 200}):
+            out = torch.full((tokens, q_heads * vdim), float("nan"), dtype=dtype, device="cuda")
+            o.attention_simt(q, k_pool, v_pool, out, table, ints(starts), ints(lengths), tile_seq, tile_q0, len(tiles), q_heads, kv_heads,
+                             dim, page, dim ** -0.5, vdim=vdim, **mask, **hints)
+            outs.append(out)
+        assert all(torch.equal(outs[0], other) for other in outs[1:])
+        for s, (length, n) in enumerate(zip(lengths, q_lens)):
+            i, j = torch.arange(length - n, length)[:, None], torch.arange(length)[None]
+            seen = j <= i
+            if "window" in mask:
+                seen &= (i - j < mask["window"]) | (j < mask.get("keep_first", 0))
+            if "chunk" in mask:
+                seen &= i // mask["chunk"] == j // mask["chunk"]
+            for h in range(q_heads):
+                g = h // (q_heads // kv_heads)
+                rows = q[starts[s]: starts[s + 1]].view(n, q_heads, dim)[:, h].double().cpu()
+                scores = (rows @ ks[s][:, g].double().T * dim ** -0.5).masked_fill(~seen, -math.inf)
+                expected = torch.softmax(scores, -1) @ vs[s][:, g].double()
+                got = outs[0][starts[s]: starts[s + 1]].view(n, q_heads, vdim)[:, h].double().cpu()
+                # scores of dim / 4 + 4 sums of terms below 12 in all, weights and their sums within as much, values below 6
+                tolerance = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -24 * (dim / 4 + 16) * 12
+                assert ((got - expected).abs() <= 6 * tolerance).all()

@@ -29,3 +29,33 @@ def test_few_token_gated_product_split_over_a_cluster(m, inter, k):
             want = g * torch.sigmoid(1.7 * g) * (u + 1)
         # gate, up, activation and product each round to bfloat16 where the value is below 8
         assert ((out.double() - want).abs() <= 4 * 2.0 ** -8 * (want.abs() + u.abs() + 0.1)).all()
+
+
+@pytest.mark.parametrize("flags", [{}, {"neighbours": True}, {"whole_norm": True, "norms": True}, {"norms": True, "blend": 2}, {"values_from_keys": True}])
+def test_heads_of_a_projection_row_four_channels_at_a_time(flags):
+    """Rows on 16-byte boundaries (four channels a thread) give the bits that rows off them (one a thread) give."""
+    o, gen = ops(), torch.Generator().manual_seed(9)
+    tokens, q_heads, kv_heads, dim, page, room = 5, 6, 2, 24, 16, 32
+    vdim = dim if flags.get("values_from_keys") else 20
+    width = q_heads * dim + kv_heads * dim + (0 if flags.get("values_from_keys") else kv_heads * vdim)
+    values = torch.randn(tokens, width, generator=gen).cuda()
+    bias = {n: torch.randn(s, generator=gen).cuda() for n, s in (("q", q_heads * dim), ("k", kv_heads * dim), ("v", kv_heads * vdim))}
+    size = q_heads * dim, kv_heads * dim
+    norms = [1 + 0.1 * torch.randn(n if flags.get("whole_norm") else dim, generator=gen).cuda() for n in size] if flags.get("norms") else [None, None]
+    table = torch.randn(tokens, 2, 8, generator=gen).cuda()
+    slots = torch.tensor([0, 17, 5, 40, 31], dtype=torch.int32, device="cuda")
+    kept, lam = torch.randn(tokens, kv_heads * vdim, generator=gen).cuda(), torch.tensor([0.3], device="cuda")
+    results = []
+    for shift in (0, 1):
+        wide = torch.zeros(tokens, width + 4, device="cuda")
+        wide[:, shift: shift + width] = values
+        proj = wide[:, shift: shift + width]
+        q = torch.full((tokens, q_heads * room), float("nan"), dtype=torch.bfloat16, device="cuda")
+        k_pool, v_pool = (torch.full((3, kv_heads, page, room), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        o.heads_bias_rope_kv(proj, q, k_pool, v_pool, bias["q"], bias["k"], None if flags.get("values_from_keys") else bias["v"], table, slots,
+                             kept.clone(), flags.get("blend", 0), lam if flags.get("blend") else None, q_heads, kv_heads, dim, vdim, page, norms[0],
+                             norms[1], 1e-6, neighbours=flags.get("neighbours", False), values_from_keys=flags.get("values_from_keys", False),
+                             whole_norm=flags.get("whole_norm", False))
+        results.append((q, k_pool, v_pool))
+    for a, b in zip(*results):
+        assert not torch.isnan(a).any() and torch.equal(a, b)

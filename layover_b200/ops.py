@@ -1629,20 +1629,38 @@ def attention_tcgen05_status() -> int:
 
 
 def attention_tcgen05_prefill(q, pool, layer, out, block_table, cu_q, ctx_len, tile_seq, tile_q0, n_tiles, q_heads,
-                              kv_heads, dim, page_tokens, scale, window=0):
-    """Prompt portions on tcgen05: tiles of 128 queries; pool is the cache group's whole pool."""
+                              kv_heads, dim, page_tokens, scale, window=0, splits=1):
+    """Prompt portions on tcgen05: tiles of 128 queries; pool is the cache group's whole pool. `splits` > 1 (where an even
+    number of query heads shares a key/value head): the keys of a row are dealt to that many blocks."""
     for name, t in (("q", q), ("out", out)):
         _need(t, torch.bfloat16, name)
     for name, t in (("block_table", block_table), ("cu_q", cu_q), ("ctx_len", ctx_len), ("tile_seq", tile_seq),
                     ("tile_q0", tile_q0)):
         _need(t, torch.int32, name)
+    partials = None
+    if splits > 1:          # of this call alone, on its own stream
+        partials = torch.empty(n_tiles * q_heads * splits * TCGEN05_TILE * (dim + 2), dtype=torch.float32, device=q.device)
     fn = _fn("attention_tcgen05", "lb_attention_tcgen05_prefill",
              [c_void_p, c_long, c_void_p, c_int, c_void_p, c_void_p, c_int] + [c_void_p] * 4 + [c_int] * 5 +
-             [c_float, c_int, c_void_p])
+             [c_float, c_int, c_int, c_void_p, c_void_p])
     _check(fn(_ptr(q), q.shape[0], ctypes.addressof(_pool_map(pool)), int(layer), _ptr(out), _ptr(block_table),
               block_table.shape[1], _ptr(cu_q), _ptr(ctx_len), _ptr(tile_seq), _ptr(tile_q0), n_tiles, q_heads, kv_heads,
-              dim, page_tokens, float(scale), int(window), _stream()), "attention_tcgen05_prefill")
+              dim, page_tokens, float(scale), int(window), int(splits), _ptr(partials), _stream()), "attention_tcgen05_prefill")
+    if splits > 1:
+        global LAUNCHES
+        LAUNCHES += 1          # the blocks' results are merged by a kernel of their own
     return out
+
+
+def portion_splits(n_tiles: int, q_heads: int, kv_heads: int, keys: int, sms: int) -> int:
+    """How many blocks share the keys of a prompt portion's rows: the number that ends first when a block holds an SM,
+    takes its key tiles and two tiles' time to start and end, and a split costs four tiles' time (the partial results'
+    way through the L2, and their merge)."""
+    blocks, tiles = n_tiles * q_heads // 2, -(-keys // TCGEN05_TILE)
+    if (q_heads // kv_heads) % 2 or blocks >= 2 * sms:
+        return 1
+    cost = lambda s: -(-blocks * s // sms) * (-(-tiles // s) + 2) + (4 + s if s > 1 else 0)
+    return min(range(1, max(2, min(9, tiles // 4 + 1))), key=cost)
 
 
 def attention_bf16(q, cache, out, block_table, batch, q_heads, kv_heads, dim, page_tokens, scale, window, sinks=None,
@@ -1688,7 +1706,8 @@ def attention_bf16(q, cache, out, block_table, batch, q_heads, kv_heads, dim, pa
     if plain and cache.pool is not None and attention_tcgen05_supports(q_heads, kv_heads, dim, page_tokens):
         tiles = tiles_of[TCGEN05_TILE]
         attention_tcgen05_prefill(q, cache.pool, cache.layer, out, block_table, batch.cu_q, batch.ctx_len, tiles.tile_seq,
-                                  tiles.tile_q0, tiles.count, q_heads, kv_heads, dim, page_tokens, scale, window)
+                                  tiles.tile_q0, tiles.count, q_heads, kv_heads, dim, page_tokens, scale, window,
+                                  portion_splits(tiles.count, q_heads, kv_heads, seen(batch.max_ctx), sm_count(q.device)))
         return
     tiles = tiles_of[attention_mma_block_queries()]
     attention_prefill_bf16(q, cache.k_pool, cache.v_pool, out, block_table, batch.cu_q, batch.ctx_len, tiles.tile_seq,

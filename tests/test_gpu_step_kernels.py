@@ -5,7 +5,7 @@ import math
 import pytest
 import torch
 
-from test_gpu_kernels import ops
+from test_gpu_kernels import ops, paged_setup
 
 pytestmark = pytest.mark.gpu
 
@@ -29,6 +29,40 @@ def test_few_token_gated_product_split_over_a_cluster(m, inter, k):
             want = g * torch.sigmoid(1.7 * g) * (u + 1)
         # gate, up, activation and product each round to bfloat16 where the value is below 8
         assert ((out.double() - want).abs() <= 4 * 2.0 ** -8 * (want.abs() + u.abs() + 0.1)).all()
+
+
+@pytest.mark.parametrize("q_heads, kv_heads", [(4, 2), (32, 8)])
+@pytest.mark.parametrize("window", [0, 200])
+def test_prompt_attention_with_keys_dealt_to_several_blocks(q_heads, kv_heads, window):
+    """Fewer key tiles than blocks, whole ranges under the mask, rows that end within a tile."""
+    o, dim, page = ops(), 128, 16
+    lengths, q_lens = [5, 129, 700, 1300, 513], [5, 129, 130, 1, 512]
+    k_pool, v_pool, table, ks, vs = paged_setup(torch.bfloat16, lengths, kv_heads, dim, page, 3)
+    pool = torch.stack((k_pool, v_pool))[None].contiguous()
+    q = torch.randn(sum(q_lens), q_heads * dim, generator=torch.Generator().manual_seed(4)).to(torch.bfloat16).cuda()
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    starts = [sum(q_lens[:s]) for s in range(len(q_lens) + 1)]
+    tiles = [(s, q0) for s, n in enumerate(q_lens) for q0 in range(0, n, 128)]
+    outs = []
+    for splits in (1, 2, 3, 8, 32):
+        out = torch.full_like(q, float("nan"))
+        o.attention_tcgen05_prefill(q, pool, 0, out, table, ints(starts), ints(lengths), ints([t[0] for t in tiles]), ints([t[1] for t in tiles]),
+                                    len(tiles), q_heads, kv_heads, dim, page, dim ** -0.5, window, splits)
+        assert o.attention_tcgen05_status() == 0
+        outs.append(out)
+    for s, (length, n) in enumerate(zip(lengths, q_lens)):
+        i, j = torch.arange(length - n, length)[:, None], torch.arange(length)[None]
+        seen = (j <= i) & ((i - j < window) if window else (j >= 0))
+        for h in range(q_heads):
+            g = h // (q_heads // kv_heads)
+            rows = q[starts[s]: starts[s + 1]].view(n, q_heads, dim)[:, h].double().cpu()
+            scores = (rows @ ks[s][:, g].double().T * dim ** -0.5).masked_fill(~seen, -math.inf)
+            p = torch.softmax(scores, -1)
+            want, spread = p @ vs[s][:, g].double(), p @ vs[s][:, g].double().abs()
+            for out in outs:
+                got = out[starts[s]: starts[s + 1]].view(n, q_heads, dim)[:, h].double().cpu()
+                # weights and output round to bfloat16 (2^-9 of their own each)
+                assert ((got - want).abs() <= 2.0 ** -8 * (spread + want.abs()) + 1e-6).all()
 
 
 @pytest.mark.parametrize("flags", [{}, {"neighbours": True}, {"whole_norm": True, "norms": True}, {"norms": True, "blend": 2}, {"values_from_keys": True}])

@@ -215,6 +215,11 @@ struct Args {
   int layer2;               // 2 * layer: the K plane of this layer in the pool's last dimension
   float scale_log2;
   float* partials;          // pairs of heads, keys dealt to gridDim.z blocks: [tile][head][block][128 rows][128 + 2], else null
+  // the variant with exact weights alone: a score per query head that joins the denominator only, a factor per (token, head) on
+  // the output (either may be null), a factor on every output, and output rows that may be part of wider ones
+  const float *sinks, *gates;
+  float out_scale;
+  long out_stride;
 };
 
 // The producer warp's loop. K and V tiles are requested independently, each as soon as its own
@@ -557,9 +562,16 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid
 // (gridDim.z), each of which leaves its maximum, sum and output for `attention_merge_kernel`. Measured (one B200, 32 heads
 // over 8, 512 tokens after 8,209, 64 blocks on 148 SMs): the attention
 // of a layer 177 -> 105 us (two blocks a tile) and 6 us for the merge
+// EXACT: the variant for attention with weights that keep 16 bits of mantissa in the second product (and sinks, gates, a
+// factor on the outputs; a negative window is a chunked mask: a query sees the keys of its own chunk of -window positions). A
+// weight is the sum of two bfloat16 numbers, its rounded value and the rounded rest; the rests take the upper half of the
+// columns that the scores leave free, and the second product runs over them as well. Measured (one B200, 1,500 tokens of 32
+// heads over 8 behind a window of 1,024; two prompts of 611, 16 over 4): 224 -> 96 us and 87 -> 35 us
+// (on mma.sync before)
 constexpr int PAIR_THREADS = 320;   // warp 0 producer, warp 1 MMA issuer, warps 2-5 and 6-9 the softmax warpgroups
 constexpr int PAIR_SMEM = TILE_BYTES * (2 + 2 * KV_STAGES) + 1024 + 512 + TABLE_CACHE * 4;   // Q x2, K and V stages, slack, barriers, table
 
+template <bool EXACT>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map,
                               const Args args) {
@@ -590,7 +602,8 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
   const int row0 = args.cu_q[seq], q_len = args.cu_q[seq + 1] - row0, ctx = args.ctx_len[seq];
   const int n_rows = min(ROWS, q_len - q0);
   const int p_first = ctx - q_len + q0, p_last = p_first + n_rows - 1;
-  const int key_lo = args.window > 0 ? max(0, p_first - args.window + 1) : 0;
+  const int chunk = EXACT && args.window < 0 ? -args.window : 0;
+  const int key_lo = args.window > 0 ? max(0, p_first - args.window + 1) : (chunk ? p_first / chunk * chunk : 0);
   const int first_tile = key_lo / KEYS, all_tiles = max(0, p_last / KEYS + 1 - first_tile);
   const int q_row = row0 + q0;
   // this block's share of the key tiles: all of them, or one of gridDim.z ranges (empty where there are fewer tiles)
@@ -668,6 +681,11 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
           for (int ks = 0; ks < KEYS / 16; ++ks)       // 16 keys: 8 columns of packed probabilities, 16 rows of V
             umma_bf16_ts(tmem_o + u * 128, tmem_s + u * 128 + ks * 8, desc_mn_major(v_addr + ks * 16 * 128), idesc_o,
                          (i > 0 || ks > 0) ? 1u : 0u);
+          if (EXACT) {
+#pragma unroll
+            for (int ks = 0; ks < KEYS / 16; ++ks)
+              umma_bf16_ts(tmem_o + u * 128, tmem_s + u * 128 + 64 + ks * 8, desc_mn_major(v_addr + ks * 16 * 128), idesc_o, 1u);
+          }
           umma_commit(&pv_done[u]);
           if (u == 1) umma_commit(&v_empty[stage]);
           if (i + 1 < n_tiles) {
@@ -687,6 +705,7 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const uint32_t my_s = tmem_s + u * 128 + lane_addr, my_o = tmem_o + u * 128 + lane_addr;
     const int p_row = p_first + row;                          // rows past n_rows are ballast
+    const int chunk_lo = chunk ? p_row / chunk * chunk : 0, last_chunk = chunk ? p_last / chunk * chunk : 0;
     const float c = args.scale_log2;
     float m_ref = -INFINITY, l_sum = 0.f;
     bool ok = true;
@@ -695,7 +714,7 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
       const int key0 = tile * KEYS;
       if (!mbar_wait(&s_full[u], i & 1)) { atomicCAS(&g_attn_error, 0, 26); flag[0] = 1; ok = false; break; }
       fence_after_sync();
-      const bool masked = key0 + KEYS - 1 > p_first || key0 < key_lo || args.window > 0;
+      const bool masked = key0 + KEYS - 1 > p_first || key0 < key_lo || args.window > 0 || (chunk && key0 < last_chunk);
       float s[KEYS];
       {
         uint32_t raw[64];
@@ -712,7 +731,7 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
 #pragma unroll
         for (int e = 0; e < KEYS; ++e) {
           const int key = key0 + e;
-          const bool seen = key <= p_row && key >= key_lo && (args.window <= 0 || p_row - key < args.window);
+          const bool seen = key <= p_row && key >= key_lo && (args.window <= 0 || p_row - key < args.window) && (!chunk || key >= chunk_lo);
           if (!seen) s[e] = -INFINITY;
         }
       }
@@ -727,7 +746,7 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
       // exponentials, 32 scores at a time: 16 columns of packed probabilities over the row's own scores
 #pragma unroll
       for (int ch = 0; ch < KEYS / 32; ++ch) {
-        uint32_t w[16];
+        uint32_t w[16], rest[EXACT ? 16 : 1];
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
           const float a = fast_exp2(fmaf(s[ch * 32 + 2 * e], c, neg_base));
@@ -735,8 +754,13 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
           part_sum[e & 3] += a + b;
           const __nv_bfloat162 pair = __floats2bfloat162_rn(a, b);
           w[e] = *reinterpret_cast<const uint32_t*>(&pair);
+          if (EXACT) {
+            const __nv_bfloat162 left = __floats2bfloat162_rn(a - __low2float(pair), b - __high2float(pair));
+            rest[e] = *reinterpret_cast<const uint32_t*>(&left);
+          }
         }
         tmem_st16_nowait(my_s + ch * 16, w);
+        if constexpr (EXACT) tmem_st16_nowait(my_s + 64 + ch * 16, rest);
       }
       const float tile_sum = (part_sum[0] + part_sum[1]) + (part_sum[2] + part_sum[3]);
       l_sum = l_sum * factor + tile_sum;
@@ -784,12 +808,18 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
     if (ok) {
       // tensor-memory loads are warp-wide: every lane reads its row, rows of the tile only are stored
       const bool valid = row < n_rows;
-      bf16* dst = args.out + ((size_t)(q_row + (valid ? row : 0)) * args.q_heads + head0 + u) * DIM;
+      const size_t token = (size_t)(q_row + (valid ? row : 0));
+      bf16* dst = EXACT ? args.out + token * args.out_stride + (head0 + u) * DIM : args.out + (token * args.q_heads + head0 + u) * DIM;
       // with the keys dealt to several blocks: maximum, sum and unnormalised output, for the merge kernel
       float* left = args.partials ? args.partials + ((((size_t)tile_index * args.q_heads + head0 + u) * gridDim.z + blockIdx.z) * ROWS + row) * (DIM + 2)
                                   : nullptr;
       if (left) reinterpret_cast<float2*>(left + DIM)[0] = make_float2(m_ref, l_sum);
-      const float inv = left ? 1.0f : 1.0f / l_sum;
+      float inv = left ? 1.0f : 1.0f / l_sum;
+      if (EXACT) {       // the row's maximum is finite (a query sees itself); scores are unscaled, the sink is not to be scaled
+        if (args.sinks) inv = 1.0f / (l_sum + fast_exp2(args.sinks[head0 + u] * 1.4426950408889634f - m_ref * c));
+        if (args.gates) inv *= args.gates[token * args.q_heads + head0 + u];
+        inv *= args.out_scale;
+      }
 #pragma unroll
       for (int ch = 0; ch < DIM / 16; ++ch) {
         float v[16];
@@ -877,7 +907,8 @@ void configure_once() {      // once per device: the attribute belongs to the de
   static LbPerDeviceOnce once;
   if (!once.first()) return;
   cudaFuncSetAttribute(attention_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-  cudaFuncSetAttribute(attention_tcgen05_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
+  cudaFuncSetAttribute(attention_tcgen05_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
+  cudaFuncSetAttribute(attention_tcgen05_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
 }
 
 // q as a 2-D bf16 matrix [rows, cols] with rows `stride` elements apart: box 64 columns x 128 rows
@@ -939,25 +970,32 @@ LB_EXPORT int lb_attention_tcgen05_status() {
 
 // Prompt portions: tiles of 128 queries (tile_seq, tile_q0), grid (query heads, tiles). `splits` > 1 (up to 32, only where pairs of
 // heads share a KV head): the keys of a row are dealt to that many blocks; `partials` holds n_tiles * q_heads * splits * 128 * 130
-// floats for this call alone.
+// floats for this call alone. `exact`: the variant with exact weights, which takes `sinks`, `gates`, `out_scale`, `out_stride` and a
+// negative window (see the kernel), and no split; the others take none of them.
 LB_EXPORT int lb_attention_tcgen05_prefill(const void* q, long q_rows, const void* pool_map, int layer, void* out,
                                            const int* block_table, int table_width, const int* cu_q, const int* ctx_len,
                                            const int* tile_seq, const int* tile_q0, int n_tiles, int q_heads, int kv_heads,
                                            int dim, int page_tokens, float scale, int window, int splits, float* partials,
+                                           int exact, const float* sinks, const float* gates, float out_scale, long out_stride,
                                            cudaStream_t stream) {
   if (n_tiles <= 0) return 0;
   if (!lb_attention_tcgen05_supports(q_heads, kv_heads, dim, page_tokens) || n_tiles > 65535) return LB_ERR_SIZE;
-  if (splits < 1 || splits > 32 || (splits > 1 && (!partials || (q_heads / kv_heads) % 2))) return LB_ERR_SIZE;
+  if (splits < 1 || splits > 32 || (splits > 1 && (!partials || exact || (q_heads / kv_heads) % 2))) return LB_ERR_SIZE;
+  if (exact ? (q_heads / kv_heads) % 2 || out_stride < (long)q_heads * dim : sinks || gates || window < 0 || out_scale != 1.f) return LB_ERR_SIZE;
+  if (exact && (out_stride % 8 || (uintptr_t)out % 16)) return LB_ERR_ALIGN;
   if ((uintptr_t)q % 16) return LB_ERR_ALIGN;
   configure_once();
   CUtensorMap q_map, kv_map;
   if (!make_q_map(&q_map, q, q_rows, (long)q_heads * dim, (long)q_heads * dim)) return LB_ERR_ALIGN;
   memcpy(&kv_map, pool_map, sizeof(kv_map));
   Args args{(bf16*)out, block_table, table_width, cu_q, ctx_len, tile_seq, tile_q0, q_heads, kv_heads, page_tokens, window,
-            2 * layer, scale * 1.4426950408889634f, splits > 1 ? partials : nullptr};
+            2 * layer, scale * 1.4426950408889634f, splits > 1 ? partials : nullptr, sinks, gates, out_scale, out_stride};
   int code;
-  if ((q_heads / kv_heads) % 2 == 0)    // two heads of a KV head per block
-    code = lb_launch(attention_tcgen05_pair_kernel, dim3(q_heads / 2, n_tiles, splits), dim3(PAIR_THREADS), (size_t)PAIR_SMEM, stream,
+  if (exact)
+    code = lb_launch(attention_tcgen05_pair_kernel<true>, dim3(q_heads / 2, n_tiles), dim3(PAIR_THREADS), (size_t)PAIR_SMEM, stream,
+                     q_map, kv_map, args);
+  else if ((q_heads / kv_heads) % 2 == 0)    // two heads of a KV head per block
+    code = lb_launch(attention_tcgen05_pair_kernel<false>, dim3(q_heads / 2, n_tiles, splits), dim3(PAIR_THREADS), (size_t)PAIR_SMEM, stream,
                      q_map, kv_map, args);
   else
     code = lb_launch(attention_tcgen05_kernel, dim3(q_heads, n_tiles), dim3(THREADS), (size_t)SMEM_BYTES, stream,

@@ -1599,6 +1599,11 @@ def attention_tcgen05_takes_heads(q_heads: int, kv_heads: int, dim: int) -> bool
     return dim == 128 and kv_heads > 0 and q_heads % kv_heads == 0 and q_heads // kv_heads <= 128
 
 
+def attention_tcgen05_exact_takes(q_heads: int, kv_heads: int, dim: int) -> bool:
+    """Whether the tcgen05 kernel has a variant with exact weights for these heads: pairs of query heads share a key/value head."""
+    return attention_tcgen05_takes_heads(q_heads, kv_heads, dim) and (q_heads // kv_heads) % 2 == 0
+
+
 def attention_tcgen05_supports(q_heads: int, kv_heads: int, dim: int, page_tokens: int) -> bool:
     return (attention_tcgen05_takes_heads(q_heads, kv_heads, dim)
             and page_tokens >= 8 and page_tokens % 8 == 0 and 128 % page_tokens == 0)
@@ -1629,11 +1634,18 @@ def attention_tcgen05_status() -> int:
 
 
 def attention_tcgen05_prefill(q, pool, layer, out, block_table, cu_q, ctx_len, tile_seq, tile_q0, n_tiles, q_heads,
-                              kv_heads, dim, page_tokens, scale, window=0, splits=1):
+                              kv_heads, dim, page_tokens, scale, window=0, splits=1, exact_weights=False, sinks=None,
+                              gates=None, out_scale=1.0):
     """Prompt portions on tcgen05: tiles of 128 queries; pool is the cache group's whole pool. `splits` > 1 (where an even
-    number of query heads shares a key/value head): the keys of a row are dealt to that many blocks."""
-    for name, t in (("q", q), ("out", out)):
-        _need(t, torch.bfloat16, name)
+    number of query heads shares a key/value head): the keys of a row are dealt to that many blocks. `exact_weights` (likewise,
+    and without a split): weights keep 16 bits of mantissa in the second product; `sinks`, `gates` and `out_scale` as in
+    `attention_prefill_bf16`, a negative window is a chunked mask and `out` may be a view into wider rows."""
+    _need(q, torch.bfloat16, "q")
+    if exact_weights:
+        _need_rows(out, torch.bfloat16, "out")
+        _sink_arguments(sinks, gates, q.shape[0], q_heads, "attention_tcgen05_prefill")
+    else:
+        _need(out, torch.bfloat16, "out")
     for name, t in (("block_table", block_table), ("cu_q", cu_q), ("ctx_len", ctx_len), ("tile_seq", tile_seq),
                     ("tile_q0", tile_q0)):
         _need(t, torch.int32, name)
@@ -1642,10 +1654,11 @@ def attention_tcgen05_prefill(q, pool, layer, out, block_table, cu_q, ctx_len, t
         partials = torch.empty(n_tiles * q_heads * splits * TCGEN05_TILE * (dim + 2), dtype=torch.float32, device=q.device)
     fn = _fn("attention_tcgen05", "lb_attention_tcgen05_prefill",
              [c_void_p, c_long, c_void_p, c_int, c_void_p, c_void_p, c_int] + [c_void_p] * 4 + [c_int] * 5 +
-             [c_float, c_int, c_int, c_void_p, c_void_p])
+             [c_float, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_float, c_long, c_void_p])
     _check(fn(_ptr(q), q.shape[0], ctypes.addressof(_pool_map(pool)), int(layer), _ptr(out), _ptr(block_table),
               block_table.shape[1], _ptr(cu_q), _ptr(ctx_len), _ptr(tile_seq), _ptr(tile_q0), n_tiles, q_heads, kv_heads,
-              dim, page_tokens, float(scale), int(window), int(splits), _ptr(partials), _stream()), "attention_tcgen05_prefill")
+              dim, page_tokens, float(scale), int(window), int(splits), _ptr(partials), int(bool(exact_weights)), _ptr(sinks), _ptr(gates),
+              float(out_scale), out.stride(0), _stream()), "attention_tcgen05_prefill")
     if splits > 1:
         global LAUNCHES
         LAUNCHES += 1          # the blocks' results are merged by a kernel of their own
@@ -1668,7 +1681,8 @@ def attention_bf16(q, cache, out, block_table, batch, q_heads, kv_heads, dim, pa
     """The bfloat16 path's attention for one step: prompt portions go through the tcgen05 tile kernel
     where it takes the sizes (head size 128, pages of 8..128 tokens), else through the mma.sync
     one; single tokens, alone or beside prompt portions, go through the split decode kernel. With
-    sinks, gates or exact weights the mma.sync kernels' variants for those run everywhere. `decode_share` > 1: the
+    sinks, gates or exact weights the kernels' variants for those run; the tcgen05 kernel's takes an even number of query heads
+    per key/value head and neither kept first keys nor a soft cap, which stay with the mma.sync one. `decode_share` > 1: the
     decode kernel takes the query heads of a key/value head as that many groups (each at most 16 heads)."""
     plain = sinks is None and gates is None and not exact_weights and not chunk and not keep_first and not softcap \
         and out_scale == 1.0 and out.is_contiguous()
@@ -1708,6 +1722,14 @@ def attention_bf16(q, cache, out, block_table, batch, q_heads, kv_heads, dim, pa
         attention_tcgen05_prefill(q, cache.pool, cache.layer, out, block_table, batch.cu_q, batch.ctx_len, tiles.tile_seq,
                                   tiles.tile_q0, tiles.count, q_heads, kv_heads, dim, page_tokens, scale, window,
                                   portion_splits(tiles.count, q_heads, kv_heads, seen(batch.max_ctx), sm_count(q.device)))
+        return
+    if (exact_weights and not keep_first and not softcap and TCGEN05_TILE in tiles_of and cache.pool is not None
+            and attention_tcgen05_exact_takes(q_heads, kv_heads, dim) and attention_tcgen05_supports(q_heads, kv_heads, dim, page_tokens)
+            and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0):
+        tiles = tiles_of[TCGEN05_TILE]
+        attention_tcgen05_prefill(q, cache.pool, cache.layer, out, block_table, batch.cu_q, batch.ctx_len, tiles.tile_seq,
+                                  tiles.tile_q0, tiles.count, q_heads, kv_heads, dim, page_tokens, scale, window, 1, True, sinks, gates,
+                                  out_scale)
         return
     tiles = tiles_of[attention_mma_block_queries()]
     attention_prefill_bf16(q, cache.k_pool, cache.v_pool, out, block_table, batch.cu_q, batch.ctx_len, tiles.tile_seq,

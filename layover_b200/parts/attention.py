@@ -188,12 +188,17 @@ class Attention(Part):
         return (self.general and dtype == torch.bfloat16 and self.q_heads // self.kv_heads <= 16 and max(self.dim, self.vdim) <= 256
                 and (self.rows32 or (self.dim % 16 == 0 and self.vdim % 16 == 0)))     # rows32: any size, padded to 16s
 
+    def _on_tcgen05(self) -> bool:
+        """Whether prompt portions of the general path may run on the tcgen05 kernel (see `ops.attention_bf16`)."""
+        room = -(-max(self.dim, self.vdim) // 16) * 16
+        return not self.softcap and not self.keep_first and ops.attention_tcgen05_exact_takes(self.q_heads, self.kv_heads, room)
+
     def parts(self):
         return [self.position] if self.position is not None else []
 
     def kernel_libraries(self, dtype):
         if self._on_tensor_cores(dtype):
-            return ("elementwise", "attention_mma")
+            return ("elementwise", "attention_mma") + (("attention_tcgen05",) if self._on_tcgen05() else ())
         if dtype == torch.float32 or self.general:
             return ("elementwise", "attention_simt")
         names = ["elementwise", "attention_mma"]
@@ -203,7 +208,7 @@ class Attention(Part):
 
     def tile_sizes(self, dtype):
         if self._on_tensor_cores(dtype):
-            return (ops.attention_mma_block_queries(),)
+            return (ops.attention_mma_block_queries(),) + ((ops.TCGEN05_TILE,) if self._on_tcgen05() else ())
         if dtype == torch.float32 or self.general:
             return (ops.attention_simt_block_queries(),)
         sizes = [ops.attention_mma_block_queries()]

@@ -93,3 +93,43 @@ def test_heads_of_a_projection_row_four_channels_at_a_time(flags):
         results.append((q, k_pool, v_pool))
     for a, b in zip(*results):
         assert not torch.isnan(a).any() and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("q_heads, kv_heads", [(2, 1), (12, 2)])
+@pytest.mark.parametrize("window", [0, 200, -96, -128, -1000])
+@pytest.mark.parametrize("extras", [False, True])
+def test_prompt_attention_with_exact_weights(q_heads, kv_heads, window, extras):
+    """Windows and chunks (negative) that begin inside, at and beyond a tile of 128 keys; sinks, gates, a factor and output rows
+    that are part of wider ones."""
+    o, dim, page = ops(), 128, 16
+    lengths, q_lens = [5, 129, 700, 1300, 513], [5, 129, 130, 1, 512]
+    k_pool, v_pool, table, ks, vs = paged_setup(torch.bfloat16, lengths, kv_heads, dim, page, 3)
+    pool = torch.stack((k_pool, v_pool))[None].contiguous()
+    gen, tokens = torch.Generator().manual_seed(4), sum(q_lens)
+    q = torch.randn(tokens, q_heads * dim, generator=gen).to(torch.bfloat16).cuda()
+    sinks = (2 * torch.randn(q_heads, generator=gen)).cuda() if extras else None
+    gates = torch.rand(tokens, q_heads, generator=gen).cuda() if extras else None
+    factor = 0.7 if extras else 1.0
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    starts = [sum(q_lens[:s]) for s in range(len(q_lens) + 1)]
+    tiles = [(s, q0) for s, n in enumerate(q_lens) for q0 in range(0, n, 128)]
+    wide = torch.full((tokens, q_heads * dim + (8 if extras else 0)), float("nan"), dtype=torch.bfloat16, device="cuda")
+    out = wide[:, : q_heads * dim]
+    o.attention_tcgen05_prefill(q, pool, 0, out, table, ints(starts), ints(lengths), ints([t[0] for t in tiles]), ints([t[1] for t in tiles]),
+                                len(tiles), q_heads, kv_heads, dim, page, dim ** -0.5, window, 1, True, sinks, gates, factor)
+    assert o.attention_tcgen05_status() == 0 and torch.isnan(wide[:, q_heads * dim:]).all()
+    for s, (length, n) in enumerate(zip(lengths, q_lens)):
+        i, j = torch.arange(length - n, length)[:, None], torch.arange(length)[None]
+        seen = (j <= i) & ((i - j < window) if window > 0 else (i // -window == j // -window) if window else (j >= 0))
+        for h in range(q_heads):
+            g = h // (q_heads // kv_heads)
+            rows = q[starts[s]: starts[s + 1]].view(n, q_heads, dim)[:, h].double().cpu()
+            scores = (rows @ ks[s][:, g].double().T * dim ** -0.5).masked_fill(~seen, -math.inf)
+            if extras:
+                scores = torch.cat((scores, sinks[h].double().cpu().expand(n, 1)), 1)
+            p = torch.softmax(scores, -1)[:, :length]
+            scale = factor * (gates[starts[s]: starts[s + 1], h, None].double().cpu() if extras else 1.0)
+            want, spread = p @ vs[s][:, g].double() * scale, p @ vs[s][:, g].double().abs() * scale
+            got = out[starts[s]: starts[s + 1]].view(n, q_heads, dim)[:, h].double().cpu()
+            # the output rounds to bfloat16 (2^-9), the weights keep 16 bits (2^-17) and their exponentials' 2^-22
+            assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -14 * spread + 1e-6).all()

@@ -22,15 +22,19 @@
 // memory into registers; the warps' partial sums are added in warp order at the end of the chunk.
 // RANGES and DPT depend on the head size only, never on the batch.
 //
-// A long portion of one sequence is a long chain for few blocks. Steps that hold one (the host
-// decides from the step's longest portion) run in three launches instead: every sequence's portion
-// is cut into segments of `seg_tokens`; MODE 1 scans every segment at once, a sequence's first
-// segment from the slot's state and the others from zero, and leaves each segment's end state in
-// `seg_state`; the combine kernel walks a sequence's segments in order, S_in(s+1) = decay^len(s)
-// S_in(s) + S_end(s), leaves S_in(s) where segment s finds it and the last one in the slot; MODE 2
-// adds what the incoming state contributes, o_t += decay^(t+1) S_in^T q_t for the t-th token of the
-// segment. The sums are the same numbers in another order: results agree with the single pass
-// within rounding, not bit for bit.
+// A long portion of one sequence is a long chain for few blocks. Steps that hold one (the host decides from the step's
+// longest portion) run in three launches instead: every sequence's portion is cut into segments of `seg_tokens`. With head
+// sizes of 33 to 128 what a segment of n tokens does is written as products of matrices, S_in the state that comes in:
+//
+//   E     = sum_j decay^(n-1-j) k_j v_j^T                                      `segment_state_kernel`
+//   S_in of the next segment = decay^n S_in + E, in order, the last one to the slot          `scan_combine_kernel`
+//   o_i   = decay^(i+1) S_in^T q_i + sum_(j<=i) decay^(i-j) (q_i . k_j) v_j     `segment_output_kernel`
+//
+// With other head sizes MODE 1 scans every segment at once, a sequence's first segment from the slot's state and the others
+// from zero, and leaves each segment's end state in `seg_state`; the combine kernel leaves S_in(s) where segment s finds
+// it (in the place of the segment before); MODE 2 adds decay^(t+1) S_in^T q_t. Either way everything is 32-bit on the FFMA
+// pipes and the sums are the same numbers in another order: results agree with the single pass within rounding, not bit
+// for bit.
 #include <math.h>
 
 #include "common.cuh"
@@ -176,8 +180,10 @@ decay_scan_kernel(const T* __restrict__ proj, long row_stride, int q_off, int k_
   }
 }
 
-// Per sequence, head and state element: the segments' end states become the states that come INTO the
-// segments (left in the place of the segment before), and the state after the last segment goes to the slot.
+// Per sequence, head and state element: the segments' end states become the states that come INTO the segments, and the
+// state after the last segment goes to the slot. FROM_ZERO: all segments started from zero, and what comes into segment s
+// is left in its own place; else the first one started from the slot, and it is left in the place of the segment before.
+template <bool FROM_ZERO>
 __global__ void scan_combine_kernel(float* __restrict__ seg_state, float* __restrict__ state, const int* __restrict__ cu_q,
                                     const int* __restrict__ state_slots, const float* __restrict__ decay, int heads,
                                     int per_head, int seg_tokens) {
@@ -191,13 +197,281 @@ __global__ void scan_combine_kernel(float* __restrict__ seg_state, float* __rest
   const int len = cu_q[seq + 1] - cu_q[seq], ns = max(1, (len + seg_tokens - 1) / seg_tokens);
   const float log2_lam = log2f(decay[i / per_head]);
   float* e = seg_state + (size_t)first_segment * per_segment + i;
-  float running = e[0];                              // the true state after the first segment
-  for (int sg = 1; sg < ns; ++sg) {
-    const float local = e[(size_t)sg * per_segment];
-    e[(size_t)(sg - 1) * per_segment] = running;     // what comes into segment sg
-    running = fmaf(exp2f((float)min(seg_tokens, len - sg * seg_tokens) * log2_lam), running, local);
+  float* slot = state + (size_t)state_slots[seq] * per_segment + i;
+  float running = FROM_ZERO ? *slot : e[0];          // what comes into segment 0, or the true state after it
+  constexpr int AHEAD = 4;                           // segments whose own parts are on their way at once
+  for (int s0 = FROM_ZERO ? 0 : 1; s0 < ns; s0 += AHEAD) {
+    float local[AHEAD];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) local[u] = s0 + u < ns ? e[(size_t)(s0 + u) * per_segment] : 0.f;
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int sg = s0 + u;
+      if (sg >= ns) break;
+      e[(size_t)(FROM_ZERO ? sg : sg - 1) * per_segment] = running;
+      running = fmaf(exp2f((float)min(seg_tokens, len - sg * seg_tokens) * log2_lam), running, local[u]);
+    }
   }
-  state[(size_t)state_slots[seq] * per_segment + i] = running;
+  *slot = running;
+}
+
+// ------------------------------------------------------------------ segments as matrix products (head sizes of 33 to 128)
+constexpr int SEG_THREADS = 256, SEG_ROWS = 64, SEG_PITCH = 132, SEG_STEP = 16;
+
+// Which tokens a block of the grid's z belongs to.
+struct Tokens { int seq, first, count; };
+__device__ __forceinline__ Tokens segment_tokens(const int* __restrict__ cu_q, int n_seqs, int seg_tokens, int g) {
+  Tokens k;
+  int segment, first_segment;
+  find_segment(cu_q, n_seqs, seg_tokens, g, k.seq, segment, first_segment);
+  k.first = cu_q[k.seq] + segment * seg_tokens;
+  k.count = max(0, min(seg_tokens, cu_q[k.seq + 1] - k.first));
+  return k;
+}
+
+// Four neighbouring activated channels c .. c + 3 of a token's head (zeros past `dim` and for a token that is not there).
+template <typename T, int ACT>
+__device__ __forceinline__ float4 load_quad(const T* __restrict__ head, int c, int dim, bool there, bool vec) {
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  if (there && vec && c + 4 <= dim) {
+    if (sizeof(T) == 2) {
+      const uint2 r = *reinterpret_cast<const uint2*>(head + c);
+      const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&r.x), hi = *reinterpret_cast<const __nv_bfloat162*>(&r.y);
+      v[0] = __low2float(lo); v[1] = __high2float(lo); v[2] = __low2float(hi); v[3] = __high2float(hi);
+    } else {
+      const float4 r = *reinterpret_cast<const float4*>(head + c);
+      v[0] = r.x; v[1] = r.y; v[2] = r.z; v[3] = r.w;
+    }
+  } else if (there) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (c + e < dim) v[e] = Elem<T>::load(head + c + e);
+  }
+  return make_float4(activate<ACT>(v[0]), activate<ACT>(v[1]), activate<ACT>(v[2]), activate<ACT>(v[3]));
+}
+__device__ __forceinline__ float decay_power(float log2_lam, int n) { return n == 0 ? 1.f : exp2f((float)n * log2_lam); }
+
+// E of one segment and head, 128 value columns a block: a 128 x 128 tile, 8 x 8 sums a thread, 16 tokens a step through two
+// buffers. The FFMA pipes bound it.
+template <typename T, int ACT>
+__global__ void __launch_bounds__(SEG_THREADS)
+segment_state_kernel(const T* __restrict__ proj, long row_stride, int k_off, int v_off, const int* __restrict__ cu_q,
+                     const float* __restrict__ decay, int heads, int dim, int vdim, float* __restrict__ seg_state, int seg_tokens,
+                     int n_seqs, bool vec) {
+  __shared__ __align__(16) float k_s[2][SEG_STEP][128], v_s[2][SEG_STEP][128];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int head = blockIdx.y, e0 = blockIdx.x * 128, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const Tokens seg = segment_tokens(cu_q, n_seqs, seg_tokens, blockIdx.z);
+  const float log2_lam = log2f(decay[head]);
+  float4 k_next[2], v_next[2];             // a thread stages two quads of k and of v a step
+  auto fetch = [&](int t0) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int t = t0 + (threadIdx.x >> 5) + 8 * u, c = (threadIdx.x & 31) * 4;
+      const T* row = proj + (size_t)(seg.first + t) * row_stride;
+      k_next[u] = load_quad<T, ACT>(row + k_off + head * dim, c, dim, t < seg.count, vec);
+      v_next[u] = load_quad<T, ACT>(row + v_off + head * vdim, e0 + c, vdim, t < seg.count, vec);
+      const float w = t < seg.count ? decay_power(log2_lam, seg.count - 1 - t) : 0.f;
+      k_next[u].x *= w; k_next[u].y *= w; k_next[u].z *= w; k_next[u].w *= w;
+    }
+  };
+  auto stage = [&](int buf) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int t = (threadIdx.x >> 5) + 8 * u, c = (threadIdx.x & 31) * 4;
+      *reinterpret_cast<float4*>(&k_s[buf][t][c]) = k_next[u];
+      *reinterpret_cast<float4*>(&v_s[buf][t][c]) = v_next[u];
+    }
+  };
+  float acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  fetch(0);
+  stage(0);
+  __syncthreads();
+  for (int t0 = 0, buf = 0; t0 < seg.count; t0 += SEG_STEP, buf ^= 1) {
+    const bool more = t0 + SEG_STEP < seg.count;
+    if (more) fetch(t0 + SEG_STEP);
+#pragma unroll 4
+    for (int t = 0; t < SEG_STEP; ++t) {
+      const float4 ka = *reinterpret_cast<const float4*>(&k_s[buf][t][4 * ty]), kb = *reinterpret_cast<const float4*>(&k_s[buf][t][64 + 4 * ty]);
+      const float4 va = *reinterpret_cast<const float4*>(&v_s[buf][t][4 * tx]), vb = *reinterpret_cast<const float4*>(&v_s[buf][t][64 + 4 * tx]);
+      const float k[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w}, v[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(k[i], v[j], acc[i][j]);
+    }
+    if (more) stage(buf ^ 1);
+    __syncthreads();
+  }
+  float* to = seg_state + ((size_t)blockIdx.z * heads + head) * dim * vdim;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int d = 64 * (i >> 2) + 4 * ty + (i & 3);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int e = e0 + 64 * (j >> 2) + 4 * tx + (j & 3);
+      if (d < dim && e < vdim) to[(size_t)d * vdim + e] = acc[i][j];
+    }
+  }
+}
+
+// The outputs of 64 tokens of one segment and head, 128 value columns a block. A thread has 4 tokens x 8 columns (8 x 8, half
+// as many threads, took 282 us where this takes 194): first
+// S_in^T q over slices of 64 rows of S_in, times decay^(i+1); then, for every block of 64 keys up to the tokens' own, the
+// 64 x 64 weights decay^(i-j) (q_i . k_j) through shared memory, and their product with the values. Rows of 132 floats keep
+// the 16-byte reads along a row free of bank conflicts. The FFMA pipes bound it.
+// Measured (one B200, one prompt of 1,500 tokens, 32 heads of 128 x 128, the three launches of a layer, states,
+// joining, outputs): 129 + 10 + 310 us when the segments walked their tokens one by one, now 90 + 24 + 193 us (the
+// outputs' 3.9 GFLOP at 0.27 of the nominal FFMA rate: 768 blocks are 2.6 waves, and the later 64 tokens of a segment have
+// twice the keys of the earlier ones)
+template <typename T, int ACT>
+__global__ void __launch_bounds__(SEG_THREADS, 2)
+segment_output_kernel(const T* __restrict__ proj, long row_stride, int q_off, int k_off, int v_off, float* __restrict__ out,
+                      const int* __restrict__ cu_q, const float* __restrict__ decay, int heads, int dim, int vdim,
+                      const float* __restrict__ seg_state, int seg_tokens, int n_seqs, int e_tiles, bool vec) {
+  extern __shared__ __align__(16) float scan_smem[];
+  float* q_s = scan_smem;                                   // [64][SEG_PITCH]
+  float* block_s = q_s + SEG_ROWS * SEG_PITCH;              // [64][SEG_PITCH]: a slice of S_in, keys, values
+  float* a_s = block_s + SEG_ROWS * SEG_PITCH;              // [64][68]
+  constexpr int A_PITCH = SEG_ROWS + 4;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int head = blockIdx.y, e0 = blockIdx.x % e_tiles * 128, i0 = blockIdx.x / e_tiles * SEG_ROWS;
+  const Tokens seg = segment_tokens(cu_q, n_seqs, seg_tokens, blockIdx.z);
+  if (i0 >= seg.count) return;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const float log2_lam = log2f(decay[head]);
+  // 64 tokens from t0 on, 128 channels each from column `off` of their rows
+  auto load_block = [&](float* dst, int t0, int off, int c0, int size) {
+#pragma unroll
+    for (int u = 0; u < SEG_ROWS * 32 / SEG_THREADS; ++u) {
+      const int t = (threadIdx.x >> 5) + 8 * u, c = (threadIdx.x & 31) * 4;
+      *reinterpret_cast<float4*>(dst + t * SEG_PITCH + c) =
+          load_quad<T, ACT>(proj + (size_t)(seg.first + t0 + t) * row_stride + off, c0 + c, size, t0 + t < seg.count, vec);
+    }
+  };
+  load_block(q_s, i0, q_off + head * dim, 0, dim);
+  float acc[4][8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  // acc += rows of `left` (4 ty ..; 64 columns from c0 on) times the 64 rows of block_s
+  auto multiply = [&](const float* left, int pitch, int c0) {
+#pragma unroll 2
+    for (int c = 0; c < SEG_ROWS; c += 4) {
+      float4 l[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) l[i] = *reinterpret_cast<const float4*>(left + (4 * ty + i) * pitch + c0 + c);
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const float4 ra = *reinterpret_cast<const float4*>(block_s + (c + s) * SEG_PITCH + 4 * tx);
+        const float4 rb = *reinterpret_cast<const float4*>(block_s + (c + s) * SEG_PITCH + 64 + 4 * tx);
+        const float r[8] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float x = s == 0 ? l[i].x : s == 1 ? l[i].y : s == 2 ? l[i].z : l[i].w;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x, r[j], acc[i][j]);
+        }
+      }
+    }
+  };
+  const float* from = seg_state + ((size_t)blockIdx.z * heads + head) * dim * vdim;
+  for (int d0 = 0; d0 < dim; d0 += SEG_ROWS) {
+    __syncthreads();                                        // the slice before is read
+#pragma unroll
+    for (int u = 0; u < SEG_ROWS * 32 / SEG_THREADS; ++u) {
+      const int d = d0 + (threadIdx.x >> 5) + 8 * u, c = (threadIdx.x & 31) * 4;
+      *reinterpret_cast<float4*>(block_s + (d - d0) * SEG_PITCH + c) =
+          load_quad<float, 0>(from + (size_t)d * vdim, e0 + c, vdim, d < dim, vdim % 4 == 0);
+    }
+    __syncthreads();
+    multiply(q_s, SEG_PITCH, d0);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float w = decay_power(log2_lam, i0 + 4 * ty + i + 1);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] *= w;
+  }
+  for (int j0 = 0; j0 <= i0; j0 += SEG_ROWS) {
+    __syncthreads();                                        // block_s and a_s are read
+    load_block(block_s, j0, k_off + head * dim, 0, dim);
+    __syncthreads();
+    float dot[4][4];                                        // tokens 4 ty + i, keys tx + 16 j
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) dot[i][j] = 0.f;
+#pragma unroll 2
+    for (int c = 0; c < dim; c += 4) {
+      float4 qv[4], kv[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) qv[i] = *reinterpret_cast<const float4*>(q_s + (4 * ty + i) * SEG_PITCH + c);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) kv[j] = *reinterpret_cast<const float4*>(block_s + (tx + 16 * j) * SEG_PITCH + c);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          dot[i][j] = fmaf(qv[i].x, kv[j].x, dot[i][j]);
+          dot[i][j] = fmaf(qv[i].y, kv[j].y, dot[i][j]);
+          dot[i][j] = fmaf(qv[i].z, kv[j].z, dot[i][j]);
+          dot[i][j] = fmaf(qv[i].w, kv[j].w, dot[i][j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int apart = i0 + 4 * ty + i - (j0 + tx + 16 * j);
+        a_s[(4 * ty + i) * A_PITCH + tx + 16 * j] = apart >= 0 ? decay_power(log2_lam, apart) * dot[i][j] : 0.f;
+      }
+    __syncthreads();                                        // the keys are read, the weights are there
+    load_block(block_s, j0, v_off + head * vdim, e0, vdim);
+    __syncthreads();
+    multiply(a_s, A_PITCH, 0);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = i0 + 4 * ty + i;
+    if (t >= seg.count) continue;
+    float* o = out + ((size_t)(seg.first + t) * heads + head) * vdim + e0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int e = 64 * (j >> 2) + 4 * tx + (j & 3);
+      if (e0 + e < vdim) o[e] = acc[i][j];
+    }
+  }
+}
+
+template <typename T, int ACT>
+int launch_segments(int n_seqs, int total_segments, int seg_tokens, float* seg_state, cudaStream_t stream, const void* proj,
+                    long row_stride, int q_off, int k_off, int v_off, float* out, float* state, const int* cu_q,
+                    const int* state_slots, const float* decay, int heads, int dim, int vdim) {
+  constexpr int smem = (2 * SEG_ROWS * SEG_PITCH + SEG_ROWS * (SEG_ROWS + 4)) * (int)sizeof(float);
+  static LbPerDeviceOnce once;
+  if (once.first() &&
+      cudaFuncSetAttribute(segment_output_kernel<T, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    return lb_last_error();
+  const int e_tiles = (vdim + 127) / 128, row_blocks = (seg_tokens + SEG_ROWS - 1) / SEG_ROWS, per_head = dim * vdim;
+  // four channels at a time where every head's rows start on four elements' boundaries
+  const bool vec = (uintptr_t)proj % (4 * sizeof(T)) == 0 && row_stride % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && v_off % 4 == 0 &&
+                   dim % 4 == 0 && vdim % 4 == 0;
+  lb_launch(segment_state_kernel<T, ACT>, dim3(e_tiles, heads, total_segments), SEG_THREADS, 0, stream, (const T*)proj, row_stride, k_off,
+            v_off, cu_q, decay, heads, dim, vdim, seg_state, seg_tokens, n_seqs, vec);
+  lb_launch(scan_combine_kernel<true>, dim3((unsigned)(((size_t)heads * per_head + 255) / 256), n_seqs), 256, 0, stream, seg_state, state,
+            cu_q, state_slots, decay, heads, per_head, seg_tokens);
+  lb_launch(segment_output_kernel<T, ACT>, dim3(row_blocks * e_tiles, heads, total_segments), SEG_THREADS, (size_t)smem, stream,
+            (const T*)proj, row_stride, q_off, k_off, v_off, out, cu_q, decay, heads, dim, vdim, (const float*)seg_state, seg_tokens, n_seqs,
+            e_tiles, vec);
+  return lb_last_error();
 }
 
 template <typename T, int RANGES, int DPT, int ACT, int MODE>
@@ -226,7 +500,7 @@ int launch_scan(int n_seqs, int total_segments, int seg_tokens, float* seg_state
   int code = LB_MODE(1, total_segments);
   if (code) return code;
   const int per_head = dim * vdim;
-  lb_launch(scan_combine_kernel, dim3((unsigned)(((size_t)heads * per_head + 255) / 256), n_seqs), 256, 0, stream, seg_state,
+  lb_launch(scan_combine_kernel<false>, dim3((unsigned)(((size_t)heads * per_head + 255) / 256), n_seqs), 256, 0, stream, seg_state,
             state, cu_q, state_slots, decay, heads, per_head, seg_tokens);
   if ((code = lb_last_error())) return code;
   return LB_MODE(2, total_segments);
@@ -242,6 +516,15 @@ int dispatch_scan(int act, int n_seqs, int total_segments, int seg_tokens, float
                                       v_off, out, state, cu_q, state_slots, decay, heads, dim, vdim)                         \
             : launch_scan<T, R, D, 0>(n_seqs, total_segments, seg_tokens, seg_state, stream, proj, row_stride, q_off, k_off, \
                                       v_off, out, state, cu_q, state_slots, decay, heads, dim, vdim))
+  // With heads of 33 to 128 the tiles of 128 x 128 of the segments' matrix products are mostly full; smaller heads would
+  // leave most of them empty, and larger ones do not fit a block's shared memory.
+  if (total_segments > 0 && dim > 32 && dim <= 128) {
+    if (act == 1)
+      return launch_segments<T, 1>(n_seqs, total_segments, seg_tokens, seg_state, stream, proj, row_stride, q_off, k_off, v_off, out, state,
+                                   cu_q, state_slots, decay, heads, dim, vdim);
+    return launch_segments<T, 0>(n_seqs, total_segments, seg_tokens, seg_state, stream, proj, row_stride, q_off, k_off, v_off, out, state,
+                                 cu_q, state_slots, decay, heads, dim, vdim);
+  }
   if (dim <= 32) return LB_SCAN(8, 4);          // the split of S over warps is a function of the head size alone
   if (dim <= 64) return LB_SCAN(16, 4);
   if (dim <= 128) return LB_SCAN(16, 8);

@@ -65,6 +65,39 @@ def test_prompt_attention_with_keys_dealt_to_several_blocks(q_heads, kv_heads, w
                 assert ((got - want).abs() <= 2.0 ** -8 * (spread + want.abs()) + 1e-6).all()
 
 
+@pytest.mark.parametrize("heads, dim, vdim, decay", [(2, 33, 7, [0.9, 0.0]), (1, 64, 130, [1.0]), (3, 128, 128, [0.999, 0.5, 0.97]), (2, 36, 4, [0.3, 0.99])])
+@pytest.mark.parametrize("lengths, segment", [([1], 128), ([127, 128, 129], 128), ([300, 2, 256], 128), ([70], 64), ([513, 100], 256)])
+def test_segments_as_matrix_products(heads, dim, vdim, decay, lengths, segment):
+    """Segments that end at, before and after blocks of 64 tokens, several sequences, heads whose rows allow four channels at a
+    time or not, states that are carried in and out."""
+    o, gen = ops(), torch.Generator().manual_seed(dim + sum(lengths))
+    tokens, n_seqs = sum(lengths), len(lengths)
+    qk, vv = heads * dim, heads * vdim
+    proj = torch.randn(tokens, 2 * qk + vv, generator=gen).cuda()
+    state = torch.randn(n_seqs + 1, heads, dim, vdim, generator=gen).cuda()
+    before, slots = state.double().clone(), list(range(n_seqs, 0, -1))
+    starts = [sum(lengths[:s]) for s in range(n_seqs + 1)]
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    lam = torch.tensor(decay, device="cuda")
+    segments = sum(max(1, -(-n // segment)) for n in lengths)
+    scratch = torch.full((segments, heads, dim, vdim), float("nan"), device="cuda")
+    out = torch.full((tokens, vv), float("nan"), device="cuda")
+    o.decay_scan(proj, 0, qk, 2 * qk, out, state, ints(starts), ints(slots), lam, n_seqs, heads, dim, vdim, None, segment, scratch)
+    assert torch.equal(state[0].double(), before[0])             # a slot of nobody's
+    x = proj.double()
+    q, k, v = x[:, :qk].view(-1, heads, dim), x[:, qk: 2 * qk].view(-1, heads, dim), x[:, 2 * qk:].view(-1, heads, vdim)
+    for s in range(n_seqs):
+        at, largest = before[slots[s]], before[slots[s]].abs()
+        for t in range(starts[s], starts[s + 1]):
+            at = lam.double()[:, None, None] * at + k[t][:, :, None] * v[t][:, None, :]
+            largest = lam.double()[:, None, None] * largest + (k[t][:, :, None] * v[t][:, None, :]).abs()
+            want = (q[t][:, :, None] * at).sum(1)
+            # every partial sum is below the sum of absolute values; a few hundred roundings of 2^-24, powers of the decay to 2^-21
+            bound = 2.0 ** -18 * (q[t].abs()[:, :, None] * largest).sum(1)
+            assert ((out[t].view(heads, vdim).double() - want).abs() <= bound + 1e-30).all()
+        assert ((state[slots[s]].double() - at).abs() <= 2.0 ** -18 * largest + 1e-30).all()
+
+
 @pytest.mark.parametrize("flags", [{}, {"neighbours": True}, {"whole_norm": True, "norms": True}, {"norms": True, "blend": 2}, {"values_from_keys": True}])
 def test_heads_of_a_projection_row_four_channels_at_a_time(flags):
     """Rows on 16-byte boundaries (four channels a thread) give the bits that rows off them (one a thread) give."""

@@ -9,6 +9,7 @@ that a kernel does not support is refused with a ValueError before or by the lau
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_float, c_int, c_long, c_void_p
 
 import torch
@@ -44,16 +45,18 @@ def _check(code: int, what: str) -> None:
     raise KernelError(f"{what}: CUDA error {code} at launch")
 
 
-def _ptr(t: torch.Tensor | None) -> c_void_p:
+def _ptr(t: torch.Tensor | None) -> int | None:
+    """The address of a tensor as a `c_void_p` argument takes it."""
     if t is None:
-        return c_void_p(0)
+        return None
     if not t.is_cuda:
         raise KernelError("layover_b200 kernels need CUDA tensors: there is no CPU path")
-    return c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
-def _stream() -> c_void_p:
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+def _stream() -> int:
+    """The handle of the current device's current stream (without the Stream object around it)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _need(t: torch.Tensor, dtype: torch.dtype | None, name: str) -> None:
@@ -71,17 +74,16 @@ def _need_rows(t: torch.Tensor, dtype: torch.dtype | None, name: str) -> None:
         raise ValueError(f"{name} must be 2-D with dense rows")
 
 
-_signatures_done: set[str] = set()
+# The libraries' functions that have been called, by name: a step of a short prompt is a few hundred launches of as many
+# microseconds as the host takes for each, so a wrapper looks its function up here before it describes the arguments.
+_FUNCTIONS: dict[str, object] = {}
 
 
 def _fn(lib_name: str, fn_name: str, argtypes, restype=c_int):
-    lib = build.load(lib_name)
-    fn = getattr(lib, fn_name)
-    key = lib_name + "." + fn_name
-    if key not in _signatures_done:
-        fn.argtypes = argtypes
-        fn.restype = restype
-        _signatures_done.add(key)
+    fn = getattr(build.load(lib_name), fn_name)
+    fn.argtypes = argtypes
+    fn.restype = restype
+    _FUNCTIONS[fn_name] = fn
     return fn
 
 
@@ -134,7 +136,7 @@ def add_rmsnorm(x: torch.Tensor, delta: torch.Tensor | None, weight: torch.Tenso
         _need(rows, torch.int32, "rows")
     if out.shape[0] < n_rows or out.shape[-1] != x.shape[-1] or weight.shape[0] != x.shape[-1]:
         raise ValueError("add_rmsnorm: shapes do not agree")
-    fn = _fn("elementwise", "lb_add_rmsnorm",
+    fn = _FUNCTIONS.get("lb_add_rmsnorm") or _fn("elementwise", "lb_add_rmsnorm",
              [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p])
     _check(fn(dtype_code(x.dtype), _ptr(x), _ptr(delta), _ptr(weight), _ptr(out), _ptr(rows), n_rows, x.shape[-1],
               float(eps), _stream()), "add_rmsnorm")
@@ -177,7 +179,7 @@ def residual_rmsnorm(x: torch.Tensor, delta: torch.Tensor | None, delta_weight: 
         raise ValueError("residual_rmsnorm: delta_scale scales a normed delta")
     if out is not None:
         _need(out, run, "out")
-    fn = _fn("elementwise", "lb_residual_rmsnorm",
+    fn = _FUNCTIONS.get("lb_residual_rmsnorm") or _fn("elementwise", "lb_residual_rmsnorm",
              [c_int, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float,
               c_float, c_void_p])
     _check(fn(dtype_code(run), _ptr(x), _ptr(delta), _ptr(delta_weight), float(delta_eps), _ptr(extra), _ptr(weight),
@@ -215,7 +217,7 @@ def qk_rownorm_kv(proj: torch.Tensor, q_out: torch.Tensor, k_pool: torch.Tensor,
         _need(gates, torch.float32, "gates")
         if tuple(gates.shape) != (tokens, q_heads):
             raise ValueError("qk_rownorm_kv: gates must be [tokens, q_heads]")
-    fn = _fn("elementwise", "lb_qk_rownorm_kv",
+    fn = _FUNCTIONS.get("lb_qk_rownorm_kv") or _fn("elementwise", "lb_qk_rownorm_kv",
              [c_int, c_void_p, c_long] + [c_void_p] * 7 + [c_int] * 6 + [c_float, c_int, c_int, c_int, c_void_p])
     _check(fn(dtype_code(proj.dtype), _ptr(proj), proj.stride(0), _ptr(q_out), _ptr(k_pool), _ptr(v_pool), _ptr(q_norm_w),
               _ptr(k_norm_w), _ptr(slot_map), _ptr(gates), tokens, q_heads, kv_heads, dim, vdim, page_tokens, float(eps),
@@ -228,7 +230,7 @@ def rope_table(positions: torch.Tensor, inv_freq: torch.Tensor, out: torch.Tenso
     tokens, n_freq = positions.shape[0], inv_freq.shape[0]
     if tuple(out.shape) != (tokens, 2, n_freq):
         raise ValueError("rope_table: out must be [tokens, 2, n_freq]")
-    fn = _fn("elementwise", "lb_rope_table", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p])
+    fn = _FUNCTIONS.get("lb_rope_table") or _fn("elementwise", "lb_rope_table", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p])
     _check(fn(_ptr(positions), _ptr(inv_freq), _ptr(out), tokens, n_freq, float(amplitude), _stream()), "rope_table")
     return out
 
@@ -255,7 +257,7 @@ def qk_norm_rope_kv(qkv: torch.Tensor, q_out: torch.Tensor | None, k_pool: torch
     if k_pool is not None:
         _need(k_pool, qkv.dtype, "k_pool"); _need(v_pool, qkv.dtype, "v_pool"); _need(slot_map, torch.int32, "slot_map")
     n_freq = 0 if table is None else table.shape[2]
-    fn = _fn("elementwise", "lb_qk_norm_rope_kv",
+    fn = _FUNCTIONS.get("lb_qk_norm_rope_kv") or _fn("elementwise", "lb_qk_norm_rope_kv",
              [c_int] + [c_void_p] * 8 + [c_int] * 6 + [c_float, c_void_p])
     _check(fn(dtype_code(qkv.dtype), _ptr(qkv), _ptr(q_out), _ptr(k_pool), _ptr(v_pool), _ptr(q_norm_w),
               _ptr(k_norm_w), _ptr(table), _ptr(slot_map), tokens, q_heads, kv_heads, dim, n_freq,
@@ -269,7 +271,7 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor, block: int = 0) -> torch.Te
     inter = gate_up.shape[1] // 2
     if gate_up.shape[1] != 2 * inter or out.shape[1] != inter or out.shape[0] != gate_up.shape[0]:
         raise ValueError("swiglu: shapes do not agree")
-    fn = _fn("elementwise", "lb_swiglu", [c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
+    fn = _FUNCTIONS.get("lb_swiglu") or _fn("elementwise", "lb_swiglu", [c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
     _check(fn(dtype_code(gate_up.dtype), _ptr(gate_up), _ptr(out), gate_up.shape[0], inter, int(block), _stream()),
            "swiglu")
     return out
@@ -288,7 +290,7 @@ def gated_act(gate_up: torch.Tensor, out: torch.Tensor, activation: str, block: 
         raise ValueError("gated_act: shapes do not agree")
     if activation not in GATE_ACTIVATIONS:
         raise ValueError(f"gated_act: unknown activation {activation!r}")
-    fn = _fn("elementwise", "lb_gated_act", [c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p])
+    fn = _FUNCTIONS.get("lb_gated_act") or _fn("elementwise", "lb_gated_act", [c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p])
     _check(fn(dtype_code(gate_up.dtype), _ptr(gate_up), _ptr(out), gate_up.shape[0], inter, int(block),
               GATE_ACTIVATIONS[activation], float(limit), float(slope), _stream()), "gated_act")
     return out
@@ -325,7 +327,7 @@ def residual_layernorm(x: torch.Tensor, delta_a: torch.Tensor | None, delta_b: t
         raise ValueError("residual_layernorm: weight and out come together, out [rows, H]")
     if out is not None:
         _need(out, run, "out")
-    fn = _fn("elementwise", "lb_residual_layernorm",
+    fn = _FUNCTIONS.get("lb_residual_layernorm") or _fn("elementwise", "lb_residual_layernorm",
              [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p])
     _check(fn(dtype_code(run), _ptr(x), _ptr(delta_a), _ptr(delta_b), _ptr(weight), _ptr(bias), _ptr(out), _ptr(rows),
               n_rows, hidden, float(eps), _stream()), "residual_layernorm")
@@ -398,7 +400,7 @@ def heads_bias_rope_kv(proj: torch.Tensor, q_out: torch.Tensor, k_pool: torch.Te
         _need(positions, torch.int32, "positions")
         if positions.shape[0] != tokens or every < 1:
             raise ValueError("heads_bias_rope_kv: a temperature needs every >= 1 and one position per token")
-    fn = _fn("elementwise", "lb_heads_bias_rope_kv",
+    fn = _FUNCTIONS.get("lb_heads_bias_rope_kv") or _fn("elementwise", "lb_heads_bias_rope_kv",
              [c_int, c_void_p, c_long] + [c_void_p] * 7 + [c_int, c_void_p, c_void_p, c_int, c_void_p] + [c_int] * 9
              + [c_void_p, c_void_p, c_float, c_int, c_void_p, c_float, c_int, c_void_p])
     _check(fn(dtype_code(q_out.dtype), _ptr(proj), proj.stride(0), _ptr(q_out), _ptr(k_pool), _ptr(v_pool), _ptr(q_bias),
@@ -416,7 +418,7 @@ def channel_gate(heads: torch.Tensor, logits: torch.Tensor, out: torch.Tensor, q
     if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride(1) != 1 or tuple(logits.shape) != (tokens, q_heads * vdim) \
             or tuple(out.shape) != (tokens, q_heads * vdim) or heads.shape[1] % q_heads or heads.shape[1] // q_heads < vdim:
         raise ValueError("channel_gate: shapes do not agree")
-    fn = _fn("elementwise", "lb_channel_gate", [c_int, c_void_p, c_void_p, c_long, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
+    fn = _FUNCTIONS.get("lb_channel_gate") or _fn("elementwise", "lb_channel_gate", [c_int, c_void_p, c_void_p, c_long, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
     _check(fn(dtype_code(heads.dtype), _ptr(heads), _ptr(logits), logits.stride(0), _ptr(out), tokens, q_heads, vdim,
               heads.shape[1] // q_heads, _stream()), "channel_gate")
     return out
@@ -430,7 +432,7 @@ def activation(x: torch.Tensor, out: torch.Tensor, kind: str) -> torch.Tensor:
     _need(x, None, "x"); _need(out, x.dtype, "out")
     if kind not in ACTIVATIONS or out.shape != x.shape:
         raise ValueError(f"activation: unknown kind {kind!r} or shapes that do not agree")
-    fn = _fn("elementwise", "lb_activation", [c_int, c_void_p, c_void_p, c_long, c_int, c_void_p])
+    fn = _FUNCTIONS.get("lb_activation") or _fn("elementwise", "lb_activation", [c_int, c_void_p, c_void_p, c_long, c_int, c_void_p])
     _check(fn(dtype_code(x.dtype), _ptr(x), _ptr(out), x.numel(), ACTIVATIONS[kind], _stream()), "activation")
     return out
 
@@ -440,7 +442,7 @@ def softcap(logits: torch.Tensor, cap: float) -> torch.Tensor:
     _need(logits, torch.float32, "logits")
     if not cap > 0:
         raise ValueError("softcap: the cap must be positive")
-    fn = _fn("elementwise", "lb_softcap", [c_void_p, c_long, c_float, c_void_p])
+    fn = _FUNCTIONS.get("lb_softcap") or _fn("elementwise", "lb_softcap", [c_void_p, c_long, c_float, c_void_p])
     _check(fn(_ptr(logits), logits.numel(), float(cap), _stream()), "softcap")
     return logits
 
@@ -494,7 +496,7 @@ def moe_route(h: torch.Tensor, router: torch.Tensor, top: int, ids: torch.Tensor
         if shared_w.numel() != hidden or shared_factor.numel() != tokens:
             raise ValueError("moe_route: shared_w [H] and shared_factor [T]")
     options = _route_options(experts, correction, groups, keep_groups, group_score, renormalize, route_scale, score, "moe_route")
-    fn = _fn("moe", "lb_moe_route", [c_int] + [c_void_p] * 6 + [c_int] * 4 + [c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p])
+    fn = _FUNCTIONS.get("lb_moe_route") or _fn("moe", "lb_moe_route", [c_int] + [c_void_p] * 6 + [c_int] * 4 + [c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p])
     _check(fn(dtype_code(h.dtype), _ptr(h), _ptr(router), _ptr(shared_w), _ptr(ids), _ptr(scores), _ptr(shared_factor), tokens,
               hidden, experts, int(top), *options, _stream()), "moe_route")
 
@@ -514,7 +516,7 @@ def moe_select(logits: torch.Tensor, experts: int, top: int, ids: torch.Tensor, 
     if shared_factor is not None:
         _need(shared_factor, torch.float32, "shared_factor")
     options = _route_options(experts, correction, groups, keep_groups, group_score, renormalize, route_scale, score, "moe_select")
-    fn = _fn("moe", "lb_moe_select", [c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+    fn = _FUNCTIONS.get("lb_moe_select") or _fn("moe", "lb_moe_select", [c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                       c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p])
     _check(fn(_ptr(logits), logits.stride(0), _ptr(ids), _ptr(scores), _ptr(shared_factor), tokens, int(experts), int(top),
               *options, _stream()), "moe_select")
@@ -526,7 +528,7 @@ def moe_group(ids: torch.Tensor, experts: int, offsets: torch.Tensor, order: tor
     _need(ids, torch.int32, "ids"); _need(offsets, torch.int32, "offsets"); _need(order, torch.int32, "order")
     if offsets.numel() != experts + 1 or order.numel() != ids.numel():
         raise ValueError("moe_group: offsets [experts + 1], order one entry per pair")
-    fn = _fn("moe", "lb_moe_group", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p])
+    fn = _FUNCTIONS.get("lb_moe_group") or _fn("moe", "lb_moe_group", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p])
     _check(fn(_ptr(ids), ids.numel(), int(experts), _ptr(offsets), _ptr(order), _stream()), "moe_group")
 
 
@@ -545,7 +547,7 @@ def moe_expert_up(h: torch.Tensor, order: torch.Tensor, offsets: torch.Tensor, s
     if hidden != h.shape[1] or (gated and rows % 2) or tuple(act.shape) != (pairs, inter) or pairs != h.shape[0] * top \
             or activation not in EXPERT_ACTIVATIONS or (not gated and (activation != "relu2" or interleaved or scores is not None)):
         raise ValueError("moe_expert_up: shapes do not agree")
-    fn = _fn("moe", "lb_moe_expert_up", [c_int, c_void_p, c_long] + [c_void_p] * 5 + [c_int] * 8 + [c_float, c_float, c_void_p])
+    fn = _FUNCTIONS.get("lb_moe_expert_up") or _fn("moe", "lb_moe_expert_up", [c_int, c_void_p, c_long] + [c_void_p] * 5 + [c_int] * 8 + [c_float, c_float, c_void_p])
     _check(fn(dtype_code(h.dtype), _ptr(h), h.stride(0), _ptr(order), _ptr(offsets), _ptr(scores), _ptr(gate_up), _ptr(act),
               pairs, int(top), experts, hidden, inter, EXPERT_ACTIVATIONS[activation], int(bool(interleaved)), int(bool(gated)),
               float(limit), float(slope), _stream()), "moe_expert_up")
@@ -559,7 +561,7 @@ def moe_expert_down(act: torch.Tensor, order: torch.Tensor, offsets: torch.Tenso
     pairs = order.numel()
     if tuple(act.shape) != (pairs, inter) or tuple(y.shape) != (pairs, hidden):
         raise ValueError("moe_expert_down: shapes do not agree")
-    fn = _fn("moe", "lb_moe_expert_down", [c_int] + [c_void_p] * 5 + [c_int] * 4 + [c_void_p])
+    fn = _FUNCTIONS.get("lb_moe_expert_down") or _fn("moe", "lb_moe_expert_down", [c_int] + [c_void_p] * 5 + [c_int] * 4 + [c_void_p])
     _check(fn(dtype_code(act.dtype), _ptr(act), _ptr(order), _ptr(offsets), _ptr(down), _ptr(y), pairs, experts, hidden, inter,
               _stream()), "moe_expert_down")
     return y
@@ -586,7 +588,7 @@ def moe_combine(y: torch.Tensor, out: torch.Tensor, top: int, pair_scale: torch.
     for name, t in (("pair_scale", pair_scale), ("shared_factor", shared_factor)):
         if t is not None:
             _need(t, torch.float32, name)
-    fn = _fn("moe", "lb_moe_combine", [c_int, c_void_p, c_int] + [c_void_p] * 4 + [c_int] * 3 + [c_void_p, c_void_p])
+    fn = _FUNCTIONS.get("lb_moe_combine") or _fn("moe", "lb_moe_combine", [c_int, c_void_p, c_int] + [c_void_p] * 4 + [c_int] * 3 + [c_void_p, c_void_p])
     _check(fn(dtype_code(out.dtype), _ptr(y), dtype_code(y.dtype), _ptr(pair_scale), _ptr(shared_out), _ptr(shared_factor), _ptr(out),
               tokens, hidden, int(top), _ptr(rows), _stream()), "moe_combine")
     return out
@@ -611,7 +613,7 @@ def moe_group_tiles(ids: torch.Tensor, experts: int, place_of: torch.Tensor, til
     if place_of.numel() != ids.numel() or tile_up.numel() != tile_down.numel() \
             or (tile_up.numel() - 1) * MOE_TILE_ROWS < moe_padded_rows(ids.numel(), experts):
         raise ValueError("moe_group_tiles: place_of one entry per pair, the tile lists one per tile of the padded buffers and one more")
-    fn = _fn("moe", "lb_moe_group_tiles", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
+    fn = _FUNCTIONS.get("lb_moe_group_tiles") or _fn("moe", "lb_moe_group_tiles", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
     _check(fn(_ptr(ids), ids.numel(), int(experts), _ptr(place_of), _ptr(tile_up), _ptr(tile_down), tile_up.numel() - 1, int(rows_up),
               int(rows_down), _stream()), "moe_group_tiles")
 
@@ -624,7 +626,7 @@ def moe_scatter_rows(h: torch.Tensor, place_of: torch.Tensor, scale: torch.Tenso
         raise ValueError("moe_scatter_rows: shapes do not agree")
     if scale is not None:
         _need(scale, torch.float32, "scale")
-    fn = _fn("moe", "lb_moe_scatter_rows", [c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
+    fn = _FUNCTIONS.get("lb_moe_scatter_rows") or _fn("moe", "lb_moe_scatter_rows", [c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
     _check(fn(dtype_code(h.dtype), _ptr(h), h.stride(0), _ptr(place_of), _ptr(scale), _ptr(rows), pairs, h.shape[1], int(top),
               _stream()), "moe_scatter_rows")
     return rows
@@ -655,7 +657,7 @@ def gemm_tcgen05_grouped(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ti
     if tuple(out.shape) != (m, out_cols) or out.stride(1) != 1 or tile_rows.numel() != m // MOE_TILE_ROWS + 1:
         raise ValueError("gemm_tcgen05_grouped: out [M, N], one tile entry per 128 rows and the count of tiles in use behind them")
     partials, counters, sms = gemm_scratch(a.device)
-    fn = _fn("gemm_tcgen05", "lb_gemm_tcgen05_grouped",
+    fn = _FUNCTIONS.get("lb_gemm_tcgen05_grouped") or _fn("gemm_tcgen05", "lb_gemm_tcgen05_grouped",
              [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_long, c_long, c_long, c_void_p, c_void_p, c_long,
               c_void_p, c_int, c_int, c_int, c_float, c_float, c_void_p])
     _check(fn(_ptr(a), _ptr(w), _ptr(out), dtype_code(out.dtype), m, n, k, int(groups), a.stride(0), w.stride(0), out.stride(0),
@@ -707,7 +709,7 @@ def stream_norm(x: torch.Tensor, update: tuple | None, read: torch.Tensor | None
         _need(mu, torch.float32, "mu"); _need(state, torch.float32, "state")
         if mu.numel() != width or state.dim() != 2 or state.shape[1] < width or rows is not None or batch.n_tokens != tokens:
             raise ValueError("stream_norm: the shift is mu [width], state [slots, >= width] and this batch, without picked rows")
-    fn = _fn("streams", "lb_stream_norm", [c_int, c_void_p, c_long, c_long] + [c_void_p] * 6 + [c_float, c_void_p, c_void_p, c_int, c_int, c_int,
+    fn = _FUNCTIONS.get("lb_stream_norm") or _fn("streams", "lb_stream_norm", [c_int, c_void_p, c_long, c_long] + [c_void_p] * 6 + [c_float, c_void_p, c_void_p, c_int, c_int, c_int,
                                            c_void_p, c_void_p, c_long, c_void_p, c_void_p, c_int, c_void_p])
     _check(fn(dtype_code(out.dtype), _ptr(x), x.stride(0), x.stride(1), _ptr(y), _ptr(mix), _ptr(gain), _ptr(read), _ptr(x_out),
               _ptr(weight), float(eps), _ptr(out), _ptr(rows), blocks, width, streams, _ptr(mu), _ptr(state),
@@ -751,7 +753,7 @@ def decay_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, out: torc
         raise ValueError("decay_scan: out, state or decay do not match the heads")
     if activation not in SCAN_ACTIVATIONS:
         raise ValueError(f"decay_scan: unknown activation {activation!r}")
-    fn = _fn("linear_attention", "lb_decay_scan",
+    fn = _FUNCTIONS.get("lb_decay_scan") or _fn("linear_attention", "lb_decay_scan",
              [c_int, c_void_p, c_long, c_int, c_int, c_int] + [c_void_p] * 5 + [c_int] * 5 + [c_void_p, c_int, c_int, c_void_p])
     _check(fn(dtype_code(proj.dtype), _ptr(proj), proj.stride(0), q_off, k_off, v_off, _ptr(out), _ptr(state), _ptr(cu_q),
               _ptr(state_slots), _ptr(decay), n_seqs, heads, dim, vdim, SCAN_ACTIVATIONS[activation],
@@ -788,7 +790,7 @@ def gated_rmsnorm(x: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, eps
     if gate.dim() != 2 or gate.stride(1) != 1 or tuple(gate.shape) != (tokens, n) or tuple(out.shape) != (tokens, n) \
             or weight.numel() != n:
         raise ValueError("gated_rmsnorm: shapes do not agree")
-    fn = _fn("linear_attention", "lb_gated_rmsnorm",
+    fn = _FUNCTIONS.get("lb_gated_rmsnorm") or _fn("linear_attention", "lb_gated_rmsnorm",
              [c_int, c_void_p, c_void_p, c_long, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p])
     _check(fn(dtype_code(gate.dtype), _ptr(x), _ptr(gate), gate.stride(0), _ptr(weight), _ptr(out), tokens, n, float(eps),
               _stream()), "gated_rmsnorm")
@@ -805,7 +807,7 @@ def add_position_rows(x: torch.Tensor, positions: torch.Tensor, table: torch.Ten
         _need(lowered, table.dtype, "lowered")
         if lowered.shape != x.shape:
             raise ValueError("add_position_rows: lowered must have x's shape")
-    fn = _fn("elementwise", "lb_add_position_rows", [c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p])
+    fn = _FUNCTIONS.get("lb_add_position_rows") or _fn("elementwise", "lb_add_position_rows", [c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p])
     _check(fn(dtype_code(table.dtype), _ptr(x), _ptr(positions), _ptr(table), table.shape[0], _ptr(lowered), x.shape[0],
               x.shape[1], _stream()), "add_position_rows")
     return x
@@ -816,7 +818,7 @@ def lower_rows(x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     _need(x, torch.float32, "x"); _need(out, None, "out")
     if out.shape != x.shape:
         raise ValueError("lower_rows: out must have x's shape")
-    fn = _fn("elementwise", "lb_lower_rows", [c_int, c_void_p, c_void_p, c_long, c_void_p])
+    fn = _FUNCTIONS.get("lb_lower_rows") or _fn("elementwise", "lb_lower_rows", [c_int, c_void_p, c_void_p, c_long, c_void_p])
     _check(fn(dtype_code(out.dtype), _ptr(x), _ptr(out), x.numel(), _stream()), "lower_rows")
     return out
 
@@ -845,7 +847,7 @@ def scaled_add_rmsnorm(x: torch.Tensor, a: torch.Tensor | None, a_weight: torch.
             _need(t, torch.float32, name)
             if t.numel() != hidden:
                 raise ValueError(f"scaled_add_rmsnorm: {name} must have one entry per channel")
-    fn = _fn("elementwise", "lb_scaled_add_rmsnorm",
+    fn = _FUNCTIONS.get("lb_scaled_add_rmsnorm") or _fn("elementwise", "lb_scaled_add_rmsnorm",
              [c_int] + [c_void_p] * 5 + [c_float, c_float, c_float, c_void_p, c_float, c_void_p, c_int, c_int, c_void_p])
     _check(fn(dtype_code(run), _ptr(x), _ptr(a), _ptr(a_weight), _ptr(b), _ptr(b_weight), float(part_eps), float(factor),
               float(alpha), _ptr(weight), float(eps), _ptr(out), x.shape[0], hidden, _stream()), "scaled_add_rmsnorm")
@@ -878,7 +880,7 @@ def latent_rows(proj: torch.Tensor, dkv_off: int, norm_w: torch.Tensor | None, e
         if cq_out.shape[0] != tokens or cq_norm_w.numel() != cq_rank or not 0 <= cq_off <= proj.shape[1] - cq_rank:
             raise ValueError("latent_rows: the projection row does not hold the queries' latent")
     dtype = (k_pool if dkv_off >= 0 else cq_out).dtype
-    fn = _fn("latent", "lb_latent_rows", [c_int, c_void_p, c_long, c_int, c_void_p, c_float, c_void_p, c_void_p, c_void_p] + [c_int] * 7
+    fn = _FUNCTIONS.get("lb_latent_rows") or _fn("latent", "lb_latent_rows", [c_int, c_void_p, c_long, c_int, c_void_p, c_float, c_void_p, c_void_p, c_void_p] + [c_int] * 7
              + [c_void_p, c_void_p, c_void_p])
     _check(fn(dtype_code(dtype), _ptr(proj), proj.stride(0), int(dkv_off), _ptr(norm_w), float(eps), _ptr(table), _ptr(slot_map),
               _ptr(k_pool), tokens, rot, rank, room, page_tokens, int(cq_off), cq_rank, _ptr(cq_norm_w), _ptr(cq_out), _stream()),
@@ -913,7 +915,7 @@ def heads_linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gate: torc
         if gate.dtype != torch.float32 or gate.dim() != 2 or gate.stride(1) != 1 or gate.shape[0] != tokens \
                 or gate.shape[1] not in (heads, heads * n_out):
             raise ValueError("heads_linear: gate must be [tokens, heads * N] or [tokens, heads]")
-    fn = _fn("latent", "lb_heads_linear", [c_int, c_int, c_void_p, c_long, c_long, c_void_p, c_void_p, c_long, c_long, c_void_p,
+    fn = _FUNCTIONS.get("lb_heads_linear") or _fn("latent", "lb_heads_linear", [c_int, c_int, c_void_p, c_long, c_long, c_void_p, c_void_p, c_long, c_long, c_void_p,
                                            c_long, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p])
     _check(fn(dtype_code(w.dtype), int(a.dtype == torch.float32), _ptr(a), a.stride(0), a.stride(1), _ptr(w), _ptr(out),
               out.stride(0), out.stride(1), _ptr(gate), gate.stride(0) if gate is not None else 0, int(per_head), tokens, heads, n_out,
@@ -946,7 +948,7 @@ def delta_prepare(proj: torch.Tensor, b_off: int, a_off: int, taps: torch.Tensor
             or state.shape[1] < conv_off + (n_taps - 1) * channels:
         raise ValueError("delta_prepare: shapes do not agree")
     tiles = batch.tiles[delta_prepare_tokens()]
-    fn = _fn("delta_rule", "lb_delta_prepare",
+    fn = _FUNCTIONS.get("lb_delta_prepare") or _fn("delta_rule", "lb_delta_prepare",
              [c_void_p, c_long, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_long, c_int, c_void_p, c_void_p,
               c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p])
     _check(fn(_ptr(proj), proj.stride(0), int(b_off), int(a_off), _ptr(taps), n_taps, _ptr(a_log), _ptr(dt_bias), _ptr(state),
@@ -965,7 +967,7 @@ def delta_scan(prepared: torch.Tensor, out: torch.Tensor, state: torch.Tensor, b
     if tuple(prepared.shape) != (out.shape[0], channels + 2 * heads) or out.shape[1] != heads * vdim or state.dim() != 2 \
             or state.shape[1] < heads * dim * vdim:
         raise ValueError("delta_scan: shapes do not agree")
-    fn = _fn("delta_rule", "lb_delta_scan", [c_void_p, c_void_p, c_void_p, c_long, c_void_p, c_void_p] + [c_int] * 5 + [c_void_p])
+    fn = _FUNCTIONS.get("lb_delta_scan") or _fn("delta_rule", "lb_delta_scan", [c_void_p, c_void_p, c_void_p, c_long, c_void_p, c_void_p] + [c_int] * 5 + [c_void_p])
     _check(fn(_ptr(prepared), _ptr(out), _ptr(state), state.stride(0), _ptr(batch.cu_q), _ptr(batch.state_slots), batch.n_seqs,
               heads, kv_heads, dim, vdim, _stream()), "delta_scan")
     return out
@@ -984,7 +986,7 @@ def head_gated_rmsnorm(o: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor
             or gate.stride(1) != 1 or tuple(gate.shape) != (tokens, heads * vdim) or weight.numel() not in (vdim, heads * vdim):
         raise ValueError("head_gated_rmsnorm: shapes do not agree")
     per_channel = weight.numel() == heads * vdim and heads > 1
-    fn = _fn("delta_rule", "lb_head_gated_rmsnorm", [c_int, c_void_p, c_void_p, c_long, c_void_p, c_void_p, c_int, c_int, c_int,
+    fn = _FUNCTIONS.get("lb_head_gated_rmsnorm") or _fn("delta_rule", "lb_head_gated_rmsnorm", [c_int, c_void_p, c_void_p, c_long, c_void_p, c_void_p, c_int, c_int, c_int,
                                                      c_float, c_int, c_long, c_void_p])
     _check(fn(dtype_code(out.dtype), _ptr(o), _ptr(gate), gate.stride(0), _ptr(weight), _ptr(out), tokens, heads, vdim, float(eps),
               vdim if per_channel else 0, out.stride(0), _stream()), "head_gated_rmsnorm")
@@ -1009,7 +1011,7 @@ def wkv_shift_mix(h: torch.Tensor, mu: torch.Tensor, state: torch.Tensor, shift_
             or state.shape[1] < shift_off + width:
         raise ValueError("wkv_shift_mix: shapes do not agree")
     tiles = batch.tiles[wkv_mix_tokens()]
-    fn = _fn("wkv", "lb_wkv_shift_mix", [c_int, c_void_p, c_void_p, c_void_p, c_long, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
+    fn = _FUNCTIONS.get("lb_wkv_shift_mix") or _fn("wkv", "lb_wkv_shift_mix", [c_int, c_void_p, c_void_p, c_void_p, c_long, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                          c_int, c_int, c_void_p, c_int, c_int, c_int, c_void_p])
     _check(fn(dtype_code(h.dtype), _ptr(h), _ptr(mu), _ptr(state), state.stride(0), int(shift_off), _ptr(batch.cu_q),
               _ptr(batch.state_slots), _ptr(tiles.tile_seq), _ptr(tiles.tile_q0), tiles.count, batch.n_seqs, _ptr(mixes), tokens,
@@ -1026,7 +1028,7 @@ def wkv_decay(a: torch.Tensor, w2: torch.Tensor, w0: torch.Tensor, decay: torch.
     if a.dtype != torch.float32 or a.dim() != 2 or a.stride(1) != 1 or a.shape[1] < rank or w0.numel() != channels \
             or tuple(decay.shape) != (tokens, channels):
         raise ValueError("wkv_decay: shapes do not agree")
-    fn = _fn("wkv", "lb_wkv_decay", [c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
+    fn = _FUNCTIONS.get("lb_wkv_decay") or _fn("wkv", "lb_wkv_decay", [c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
     _check(fn(dtype_code(w2.dtype), _ptr(a), a.stride(0), _ptr(w2), _ptr(w0), _ptr(decay), tokens, channels, rank, _stream()), "wkv_decay")
     return decay
 
@@ -1046,7 +1048,7 @@ def wkv_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, w: torch.Tensor,
     if channels != heads * dim or tuple(w.shape) != (tokens, channels) or u.numel() != channels or state.dim() != 2 \
             or state.shape[1] < heads * dim * dim:
         raise ValueError("wkv_scan: shapes do not agree")
-    fn = _fn("wkv", "lb_wkv_scan", [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_void_p,
+    fn = _FUNCTIONS.get("lb_wkv_scan") or _fn("wkv", "lb_wkv_scan", [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_void_p,
                                     c_long, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
     _check(fn(_ptr(r), r.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(w), _ptr(u), _ptr(out), _ptr(state),
               state.stride(0), _ptr(batch.cu_q), _ptr(batch.state_slots), batch.n_seqs, heads, dim, _stream()), "wkv_scan")
@@ -1061,7 +1063,7 @@ def gate_decay(a: torch.Tensor, w2: torch.Tensor, w0: torch.Tensor, tau: float, 
     if a.dtype != torch.float32 or a.dim() != 2 or a.stride(1) != 1 or a.shape[1] < rank or w0.numel() != channels \
             or tuple(decay.shape) != (tokens, channels) or not tau > 0:
         raise ValueError("gate_decay: shapes do not agree, or tau is not positive")
-    fn = _fn("wkv", "lb_gate_decay", [c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p])
+    fn = _FUNCTIONS.get("lb_gate_decay") or _fn("wkv", "lb_gate_decay", [c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p])
     _check(fn(dtype_code(w2.dtype), _ptr(a), a.stride(0), _ptr(w2), _ptr(w0), _ptr(decay), tokens, channels, rank, float(tau),
               _stream()), "gate_decay")
     return decay
@@ -1081,7 +1083,7 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, w: torch.Tenso
             raise ValueError(f"gated_scan: {name} must be float32 [tokens, {n}] with dense rows")
     if out.shape[1] != heads * vdim or tuple(w.shape) != (tokens, heads * dim) or tuple(state.shape[1:]) != (heads, dim, vdim):
         raise ValueError("gated_scan: shapes do not agree")
-    fn = _fn("wkv", "lb_gated_scan", [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_long,
+    fn = _FUNCTIONS.get("lb_gated_scan") or _fn("wkv", "lb_gated_scan", [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_long,
                                       c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p])
     _check(fn(_ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(w), _ptr(out), _ptr(state), state.stride(0),
               _ptr(batch.cu_q), _ptr(batch.state_slots), batch.n_seqs, heads, dim, vdim, float(scale), _stream()), "gated_scan")
@@ -1103,9 +1105,9 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tens
         raise ValueError("gemm: innermost dimension must be contiguous")
     scratch = None
     if a.dtype == torch.float32 and min(m, n, k) > 0:      # partial sums of this call alone, on its own stream
-        wanted = _fn("gemm_simt", "lb_gemm_simt_scratch", [c_int] * 4, c_long)(m, n, k, sm_count(a.device))
+        wanted = (_FUNCTIONS.get("lb_gemm_simt_scratch") or _fn("gemm_simt", "lb_gemm_simt_scratch", [c_int] * 4, c_long))(m, n, k, sm_count(a.device))
         scratch = torch.empty(wanted, dtype=torch.float32, device=a.device) if wanted else None
-    fn = _fn("gemm_simt", "lb_gemm_simt",
+    fn = _FUNCTIONS.get("lb_gemm_simt") or _fn("gemm_simt", "lb_gemm_simt",
              [c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_long, c_long, c_long, c_void_p, c_int, c_void_p])
     _check(fn(dtype_code(a.dtype), dtype_code(out.dtype), _ptr(a), _ptr(w), _ptr(out), m, n, k, a.stride(0),
               w.stride(0), out.stride(0), _ptr(scratch), sm_count(a.device), _stream()), "gemm_simt")
@@ -1163,7 +1165,7 @@ def attention_simt(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, 
     if splits > 1:          # of this call alone, on its own stream
         partials = torch.empty(_simt_rows(n_tiles, q_heads, kv_heads, vdim, max_q_len)[1] * chunk_room * (vdim + 2),
                                dtype=torch.float32, device=q.device)
-    fn = _fn("attention_simt", "lb_attention_simt",
+    fn = _FUNCTIONS.get("lb_attention_simt") or _fn("attention_simt", "lb_attention_simt",
              [c_int] + [c_void_p] * 5 + [c_int] + [c_void_p] * 4 + [c_int] * 5 + [c_float, c_int, c_int, c_void_p,
               c_void_p, c_int, c_int, c_float, c_float, c_long, c_int, c_int, c_void_p, c_int, c_void_p])
     _check(fn(dtype_code(q.dtype), _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(out), _ptr(block_table),
@@ -1180,19 +1182,20 @@ def attention_simt(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, 
 def _simt_rows(n_tiles: int, q_heads: int, kv_heads: int, vdim: int, max_q_len: int) -> tuple[int, int]:
     """(blocks, rows over all blocks) of the 32-bit attention kernel without a split."""
     rows = c_int(0)
-    blocks = _fn("attention_simt", "lb_attention_simt_plan", [c_int] * 5 + [c_void_p])(n_tiles, q_heads, kv_heads, vdim, max_q_len,
-                                                                                       ctypes.addressof(rows))
+    fn = _FUNCTIONS.get("lb_attention_simt_plan") or _fn("attention_simt", "lb_attention_simt_plan", [c_int] * 5 + [c_void_p])
+    blocks = fn(n_tiles, q_heads, kv_heads, vdim, max_q_len, ctypes.addressof(rows))
     return blocks, blocks * rows.value
 
 
 _SIMT_SCRATCH_FLOATS = 64 << 20     # the most that the chunks' results may take (256 MiB)
 
 
+@functools.lru_cache(maxsize=1024)      # of the sizes alone, asked for by every layer of a step
 def _simt_splits(n_tiles: int, q_heads: int, kv_heads: int, vdim: int, max_q_len: int, max_ctx: int, room_tokens: int,
                  device: torch.device) -> tuple[int, int]:
     """(blocks that share a row's keys, chunks there must be room for): three blocks an SM where the rows alone do not give
     them, as far as there are chunks to share."""
-    keys = _fn("attention_simt", "lb_attention_simt_chunk", [])()
+    keys = (_FUNCTIONS.get("lb_attention_simt_chunk") or _fn("attention_simt", "lb_attention_simt_chunk", []))()
     blocks, rows = _simt_rows(n_tiles, q_heads, kv_heads, vdim, max_q_len)
     room = -(-room_tokens // keys)
     splits = min(-(-max_ctx // keys), -(-3 * sm_count(device) // max(blocks, 1)), room)
@@ -1240,7 +1243,7 @@ def sample(logits: torch.Tensor, tokens: torch.Tensor, records: torch.Tensor | N
             _need(t, torch.int32, name)
     if status is not None:
         _need(status, torch.int64, "status")
-    fn = _fn("sampling", "lb_sample", [c_void_p, c_long, c_int, c_int] + [c_void_p] * 6 + [c_int, c_void_p])
+    fn = _FUNCTIONS.get("lb_sample") or _fn("sampling", "lb_sample", [c_void_p, c_long, c_int, c_int] + [c_void_p] * 6 + [c_int, c_void_p])
     _check(fn(_ptr(logits), logits.stride(0), rows, vocab, _ptr(records), _ptr(row_slots), _ptr(positions),
               _ptr(logit_rows), _ptr(tokens), _ptr(status), n_status, _stream()), "sample")
     return tokens
@@ -1364,7 +1367,7 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, max_splits
     if w.shape[1] != k or tuple(out.shape) != (m, out_cols) or out.stride(1) != 1:
         raise ValueError(f"gemm: shapes do not agree: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
     partials, counters, sms = gemm_scratch(a.device)
-    fn = _fn("gemm_tcgen05", "lb_gemm_tcgen05",
+    fn = _FUNCTIONS.get("lb_gemm_tcgen05") or _fn("gemm_tcgen05", "lb_gemm_tcgen05",
              [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_long, c_long, c_long, c_void_p, c_long,
               c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p])
     _check(fn(_ptr(a), _ptr(w), _ptr(out), dtype_code(out.dtype), m, n, k, a.stride(0), w.stride(0), out.stride(0),
@@ -1393,7 +1396,7 @@ def gemm_qkv_heads(h: torch.Tensor, w_qkv: torch.Tensor, q_out: torch.Tensor, k_
             or q_out.shape != (tokens, q_heads * dim) or not q_out.is_contiguous():
         raise ValueError("gemm_qkv_heads: shapes do not agree")
     sms = gemm_scratch(h.device)[2]
-    fn = _fn("gemm_tcgen05", "lb_gemm_qkv_heads",
+    fn = _FUNCTIONS.get("lb_gemm_qkv_heads") or _fn("gemm_tcgen05", "lb_gemm_qkv_heads",
              [c_void_p, c_void_p, c_int, c_int, c_long, c_long, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int,
               c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_float, c_int, c_void_p])
     code = fn(_ptr(h), _ptr(w_qkv), tokens, h.shape[1], h.stride(0), w_qkv.stride(0), q_heads, kv_heads, dim,
@@ -1482,7 +1485,7 @@ def attention_prefill_bf16(q, k_pool, v_pool, out, block_table, cu_q, ctx_len, t
     for name, t in (("block_table", block_table), ("cu_q", cu_q), ("ctx_len", ctx_len), ("tile_seq", tile_seq),
                     ("tile_q0", tile_q0)):
         _need(t, torch.int32, name)
-    fn = _fn("attention_mma", "lb_attention_prefill_bf16",
+    fn = _FUNCTIONS.get("lb_attention_prefill_bf16") or _fn("attention_mma", "lb_attention_prefill_bf16",
              [c_void_p] * 5 + [c_int] + [c_void_p] * 4 + [c_int] * 5 + [c_float, c_int, c_void_p, c_void_p, c_int, c_int, c_float, c_float,
                                                                               c_long, c_void_p])
     _check(fn(_ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(out), _ptr(block_table), block_table.shape[1], _ptr(cu_q),
@@ -1492,6 +1495,7 @@ def attention_prefill_bf16(q, k_pool, v_pool, out, block_table, cu_q, ctx_len, t
     return out
 
 
+@functools.lru_cache(maxsize=1024)      # of the sizes alone, asked for by every layer of a step
 def decode_plan(n_seqs: int, q_heads: int, kv_heads: int, dim: int, max_context: int, sm_count: int,
                 mean_context: int | None = None) -> tuple[int, int]:
     """(splits, stages): how many ways to split the context of a decode step, and which kernel variant.
@@ -1577,7 +1581,7 @@ def attention_decode_bf16(q, k_pool, v_pool, out, block_table, cu_q, ctx_len, se
     if seq_list is not None:
         _need(seq_list, torch.int32, "seq_list")
     partials, counters = attention_scratch(q.device)
-    fn = _fn("attention_mma", "lb_attention_decode_bf16",
+    fn = _FUNCTIONS.get("lb_attention_decode_bf16") or _fn("attention_mma", "lb_attention_decode_bf16",
              [c_void_p] * 5 + [c_int] + [c_void_p] * 3 + [c_int] * 5 + [c_float, c_int, c_int, c_void_p, c_long, c_void_p,
                                                                         c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float,
                                                                         c_float, c_long, c_void_p])
@@ -1617,7 +1621,7 @@ def _pool_map(pool: torch.Tensor):
         _need(pool, torch.bfloat16, "pool")
         layers, two, pages, kv_heads, page_tokens, dim = pool.shape
         blob = (ctypes.c_ubyte * 128)()
-        fn = _fn("attention_tcgen05", "lb_attention_tcgen05_pool_map", [c_void_p, c_void_p, c_long, c_long, c_int, c_int, c_int])
+        fn = _FUNCTIONS.get("lb_attention_tcgen05_pool_map") or _fn("attention_tcgen05", "lb_attention_tcgen05_pool_map", [c_void_p, c_void_p, c_long, c_long, c_int, c_int, c_int])
         code = fn(ctypes.addressof(blob), _ptr(pool), layers * two, pages, kv_heads, page_tokens, dim)
         if code:
             raise ValueError(f"attention_tcgen05: cannot describe the pool to TMA ({_REFUSALS.get(code, code)})")
@@ -1652,7 +1656,7 @@ def attention_tcgen05_prefill(q, pool, layer, out, block_table, cu_q, ctx_len, t
     partials = None
     if splits > 1:          # of this call alone, on its own stream
         partials = torch.empty(n_tiles * q_heads * splits * TCGEN05_TILE * (dim + 2), dtype=torch.float32, device=q.device)
-    fn = _fn("attention_tcgen05", "lb_attention_tcgen05_prefill",
+    fn = _FUNCTIONS.get("lb_attention_tcgen05_prefill") or _fn("attention_tcgen05", "lb_attention_tcgen05_prefill",
              [c_void_p, c_long, c_void_p, c_int, c_void_p, c_void_p, c_int] + [c_void_p] * 4 + [c_int] * 5 +
              [c_float, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_float, c_long, c_void_p])
     _check(fn(_ptr(q), q.shape[0], ctypes.addressof(_pool_map(pool)), int(layer), _ptr(out), _ptr(block_table),
@@ -1665,6 +1669,7 @@ def attention_tcgen05_prefill(q, pool, layer, out, block_table, cu_q, ctx_len, t
     return out
 
 
+@functools.lru_cache(maxsize=1024)      # of the sizes alone, asked for by every layer of a step
 def portion_splits(n_tiles: int, q_heads: int, kv_heads: int, keys: int, sms: int) -> int:
     """How many blocks share the keys of a prompt portion's rows: the number that ends first when a block holds an SM,
     takes its key tiles and two tiles' time to start and end, and a split costs four tiles' time (the partial results'

@@ -150,15 +150,14 @@ __device__ __forceinline__ void ldmatrix_x4_trans_at(uint32_t (&r)[4], uint32_t 
 // The 16 query rows of one warp against PAIRS * 16 keys of a tile in shared memory:
 // scores, mask, running maximum and sum, P V. `k_addr` / `v_addr` are shared-memory byte addresses
 // of the warp's first key row plus this lane's ldmatrix offset; with EXACT the head size equals
-// MAX_DIM and every address offset is a constant. UPPER false skips the softmax of rows 8..15
-// (decode with at most 8 query heads per KV head). `masked` false skips the comparisons for a
+// MAX_DIM and every address offset is a constant. `masked` false skips the comparisons for a
 // tile that every row sees completely. Scores stay unscaled; the scale enters the exponent.
 // SPLIT: a weight enters the second product as the sum of two bfloat16 numbers (its rounded value and
 // the rounded rest), each multiplied exactly and added in 32-bit: the weights keep 16 bits of
 // mantissa instead of 8, at one more MMA per step of P V. With `cap_in` != 0 (SPLIT only) a score s becomes
 // cap_out * tanh(cap_in s / (2 log2 e)) = cap_out - 2 cap_out / (1 + 2^(cap_in s)), already in the exponent's
 // base-2 units (c = 1): the absolute error is about cap_out times a float's rounding, whatever the score.
-template <int MAX_DIM, bool EXACT, int PAIRS, bool UPPER, bool SPLIT = false>
+template <int MAX_DIM, bool EXACT, int PAIRS, bool SPLIT = false>
 __device__ __forceinline__ void warp_tile(const uint32_t (&qf)[MAX_DIM / 16][4], uint32_t k_addr, uint32_t v_addr,
                                           int dim, float (&o)[MAX_DIM / 8][4], float (&m_run)[2], float (&l_run)[2],
                                           bool masked, int key0, int p0, int p1, int key_lo, int window, float c,
@@ -211,7 +210,6 @@ __device__ __forceinline__ void warp_tile(const uint32_t (&qf)[MAX_DIM / 16][4],
     for (int n = 0; n < NT_S; ++n) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        if (!UPPER && e >= 2) continue;
         s[n][e] = cap_out - __fdividef(2.f * cap_out, 1.f + fast_exp2(s[n][e] * cap_in));
       }
     }
@@ -221,7 +219,6 @@ __device__ __forceinline__ void warp_tile(const uint32_t (&qf)[MAX_DIM / 16][4],
     for (int n = 0; n < NT_S; ++n) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        if (!UPPER && e >= 2) continue;
         const int key = key0 + n * 8 + 2 * t + (e & 1);
         const int p = e < 2 ? p0 : p1;
         const bool seen = key <= p && (key < keep || (key >= key_lo && (window <= 0 || p - key < window))) &&
@@ -234,11 +231,11 @@ __device__ __forceinline__ void warp_tile(const uint32_t (&qf)[MAX_DIM / 16][4],
 #pragma unroll
   for (int n = 0; n < NT_S; ++n) {
     tile_max[0] = fmaxf(tile_max[0], fmaxf(s[n][0], s[n][1]));
-    if (UPPER) tile_max[1] = fmaxf(tile_max[1], fmaxf(s[n][2], s[n][3]));
+    tile_max[1] = fmaxf(tile_max[1], fmaxf(s[n][2], s[n][3]));
   }
   float alpha[2] = {1.f, 1.f}, neg_base[2] = {0.f, 0.f};
 #pragma unroll
-  for (int r = 0; r < (UPPER ? 2 : 1); ++r) {
+  for (int r = 0; r < 2; ++r) {
     tile_max[r] = fmaxf(tile_max[r], __shfl_xor_sync(0xffffffffu, tile_max[r], 1));
     tile_max[r] = fmaxf(tile_max[r], __shfl_xor_sync(0xffffffffu, tile_max[r], 2));
     const float m_new = fmaxf(m_run[r], tile_max[r]);
@@ -256,23 +253,20 @@ __device__ __forceinline__ void warp_tile(const uint32_t (&qf)[MAX_DIM / 16][4],
     tile_sum[0] += e0 + e1;
     pf[n >> 1][(n & 1) * 2] = pack_bf16(e0, e1);
     if (SPLIT) pl[n >> 1][(n & 1) * 2] = pack_bf16(e0 - Elem<bf16>::round(e0), e1 - Elem<bf16>::round(e1));
-    if (UPPER) {
+    {
       const float e2 = fast_exp2(fmaf(s[n][2], c, neg_base[1])), e3 = fast_exp2(fmaf(s[n][3], c, neg_base[1]));
       tile_sum[1] += e2 + e3;
       pf[n >> 1][(n & 1) * 2 + 1] = pack_bf16(e2, e3);
       if (SPLIT) pl[n >> 1][(n & 1) * 2 + 1] = pack_bf16(e2 - Elem<bf16>::round(e2), e3 - Elem<bf16>::round(e3));
-    } else {
-      pf[n >> 1][(n & 1) * 2 + 1] = 0u;
-      if (SPLIT) pl[n >> 1][(n & 1) * 2 + 1] = 0u;
     }
   }
   l_run[0] = l_run[0] * alpha[0] + tile_sum[0];
-  if (UPPER) l_run[1] = l_run[1] * alpha[1] + tile_sum[1];
+  l_run[1] = l_run[1] * alpha[1] + tile_sum[1];
 #pragma unroll
   for (int n = 0; n < NT_O; ++n) {
     if (EXACT || n * 8 < dim) {
       o[n][0] *= alpha[0]; o[n][1] *= alpha[0];
-      if (UPPER) { o[n][2] *= alpha[1]; o[n][3] *= alpha[1]; }
+      o[n][2] *= alpha[1]; o[n][3] *= alpha[1];
     }
   }
 #pragma unroll
@@ -392,7 +386,7 @@ attention_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_
       // every row of the warp sees the whole tile unless it reaches past the first row's position,
       // starts before the first visible key or a window cuts it
       const bool masked = tile * BKEYS + BKEYS - 1 > p_warp || tile * BKEYS < key_lo || window != 0;
-      warp_tile<MAX_DIM, EXACT, BKEYS / 16, true, SINK>(qf, k_base + buf * buf_bytes, v_base + buf * buf_bytes, dim, o, m_run,
+      warp_tile<MAX_DIM, EXACT, BKEYS / 16, SINK>(qf, k_base + buf * buf_bytes, v_base + buf * buf_bytes, dim, o, m_run,
                                                         l_run, masked, tile * BKEYS, p0, p1, key_lo, window, scale_log2, t,
                                                         keep_first, cap_in, cap_out);
     }
@@ -424,8 +418,128 @@ attention_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_
   }
 }
 
+// ------------------------------------------------------------------------------- decode, at most 8 query heads a key/value head
+// The products the other way round: a warp's 16 keys are the rows of the first one and the value channels those of the second,
+// the query heads (at most 8) the columns of both, so that no instruction multiplies rows that are not there and the outputs take
+// half the registers. A warp also loads its own keys, as many tiles ahead as the block has, and waits for nobody else until the
+// merge. Head size 128. With the heads as rows (16 of them, 12 empty at 4 heads a group) the loop was bound by its instructions,
+// about 760 a warp and tile at 12 warps an SM.
+// Measured (one B200, 32 heads over 8, bfloat16, before and now): 8 sequences of 3,072 keys 24.8 -> 18.9 us (5.3 TB/s), 64 of
+// 3,072 146 -> 131 us (6.2 TB/s), 64 of 350 .. 3,100 109 -> 80 us, one of 1,000 5.7 us both; with exact weights, 16 of 16 heads
+// over 4 and 230 .. 1,500 keys 24.1 -> 15.0 us
+__device__ __forceinline__ uint32_t transposed(uint32_t a) {       // an 8 x 8 matrix of 16-bit elements, one row a lane group of four
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+  return d;
+}
+
+// Copies keys [key0, key0 + 16) of one KV head (128 channels), key0 a multiple of 16, into shared memory rows of (128 + PAD);
+// what is not to be seen becomes zeros. All of one page, they are one run of 4 KB and the offsets are constants.
+__device__ __forceinline__ void load_warp_keys(bf16* k_s, bf16* v_s, const bf16* __restrict__ k_pool, const bf16* __restrict__ v_pool,
+                                               const TableSlice& pages, int key0, int key_lo, int key_hi, const TileShape& shape, int keep) {
+  constexpr int DIM = 128, STRIDE = DIM + PAD;
+  const int lane = threadIdx.x & 31, r0 = lane >> 4, c8 = (lane & 15) * 8;
+  bf16 *k_to = k_s + r0 * STRIDE + c8, *v_to = v_s + r0 * STRIDE + c8;
+  const bool values = v_s != k_s;
+  if (shape.page_shift >= 4 && key0 >= key_lo && key0 + 16 <= key_hi) {
+    const size_t at = (((size_t)pages.page(key0 >> shape.page_shift) * shape.kv_heads + shape.kv_head) * shape.page_tokens +
+                       (key0 & (shape.page_tokens - 1)) + r0) * DIM + c8;
+    const bf16 *k_from = k_pool + at, *v_from = v_pool + at;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) cp_async16(k_to + 2 * j * STRIDE, k_from + 2 * j * DIM, 16);
+    if (values) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) cp_async16(v_to + 2 * j * STRIDE, v_from + 2 * j * DIM, 16);
+    }
+    return;
+  }
+#pragma unroll 1
+  for (int j = 0; j < 8; ++j) {
+    const int key = key0 + 2 * j + r0;
+    const bool live = (key >= key_lo || key < keep) && key < key_hi;
+    size_t at = 0;
+    if (live) {
+      const int index = shape.page_shift >= 0 ? key >> shape.page_shift : key / shape.page_tokens;
+      at = (((size_t)pages.page(index) * shape.kv_heads + shape.kv_head) * shape.page_tokens + (key - index * shape.page_tokens)) * DIM + c8;
+    }
+    cp_async16(k_to + 2 * j * STRIDE, k_pool + at, live ? 16 : 0);
+    if (values) cp_async16(v_to + 2 * j * STRIDE, v_pool + at, live ? 16 : 0);
+  }
+}
+
+// A warp's 16 keys against up to 8 queries: `qf` holds the queries' 128 channels, lane (g, t) ends with channels 16 n + g (+ 8) of
+// queries 2 t and 2 t + 1 in `o`, their base `m_run` (the same for every g) and its keys' share of the sums. The base is a
+// maximum that may lag by `slack`, 8 in the exponent's units: weights stay below 2^8, their precision is relative, and the outputs
+// are rescaled only when a score rises above that. SPLIT and the cap as in `warp_tile`.
+template <bool SPLIT>
+__device__ __forceinline__ void warp_keys(const uint32_t (&qf)[4][4], uint32_t k_addr, uint32_t v_addr, float (&o)[8][4],
+                                          float (&m_run)[2], float (&l_run)[2], bool masked, int key, int p, int key_lo, int keep,
+                                          float c, float slack, float cap_in, float cap_out) {
+  float s[4] = {0.f, 0.f, 0.f, 0.f}, odd[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int k0 = 0; k0 < 8; k0 += 4) {
+    uint32_t a[4][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) ldmatrix_x4_at(a[u], k_addr + (k0 + u) * 32);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) mma_bf16(u & 1 ? odd : s, a[u], qf[(k0 + u) >> 1][2 * (u & 1)], qf[(k0 + u) >> 1][2 * (u & 1) + 1]);
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) s[e] += odd[e];
+  if (SPLIT && cap_in != 0.f) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[e] = cap_out - __fdividef(2.f * cap_out, 1.f + fast_exp2(s[e] * cap_in));
+  }
+  if (masked) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int j = key + 8 * (e >> 1);
+      if (!(j <= p && (j < keep || j >= key_lo))) s[e] = -INFINITY;
+    }
+  }
+  const float limit[2] = {m_run[0] + slack, m_run[1] + slack};
+  if (__any_sync(0xffffffffu, s[0] > limit[0] || s[1] > limit[1] || s[2] > limit[0] || s[3] > limit[1])) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      float top = fmaxf(s[r], s[r + 2]);
+#pragma unroll
+      for (int x = 4; x < 32; x <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
+      top = fmaxf(m_run[r], top);
+      const float alpha = fast_exp2((m_run[r] - (top == -INFINITY ? 0.f : top)) * c);      // exp2(-inf) = 0 on the first tile
+      m_run[r] = top;
+      l_run[r] *= alpha;
+#pragma unroll
+      for (int n = 0; n < 8; ++n) { o[n][r] *= alpha; o[n][r + 2] *= alpha; }
+    }
+  }
+  const float neg_base[2] = {m_run[0] == -INFINITY ? 0.f : -m_run[0] * c, m_run[1] == -INFINITY ? 0.f : -m_run[1] * c};
+  float w[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) w[e] = fast_exp2(fmaf(s[e], c, neg_base[e & 1]));
+  l_run[0] += w[0] + w[2];
+  l_run[1] += w[1] + w[3];
+  const uint32_t b0 = transposed(pack_bf16(w[0], w[1])), b1 = transposed(pack_bf16(w[2], w[3]));
+  uint32_t r0 = 0, r1 = 0;                          // the rests
+  if (SPLIT) {
+    r0 = transposed(pack_bf16(w[0] - Elem<bf16>::round(w[0]), w[1] - Elem<bf16>::round(w[1])));
+    r1 = transposed(pack_bf16(w[2] - Elem<bf16>::round(w[2]), w[3] - Elem<bf16>::round(w[3])));
+  }
+#pragma unroll
+  for (int n0 = 0; n0 < 8; n0 += 4) {
+    uint32_t a[4][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) ldmatrix_x4_trans_at(a[u], v_addr + (n0 + u) * 32);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      mma_bf16(o[n0 + u], a[u], b0, b1);
+      if (SPLIT) mma_bf16(o[n0 + u], a[u], r0, r1);
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------- decode
-// Rows 0..group-1 of the 16-row tile are the query heads of one KV head (group <= 16).
+// Rows 0..group-1 of the 16-row tile are the query heads of one KV head (group <= 16); with at most 8 of head size 128 they are
+// columns (NARROW, see `warp_keys`).
 // CLUSTER: the `splits` blocks of a (sequence, KV head) are one thread-block cluster (grid z =
 // cluster z = splits). Instead of writing partial results to scratch memory and leaving the merge
 // to the block that arrives last at a counter, every block owns a share of the group's outputs:
@@ -435,8 +549,8 @@ attention_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_
 // in split order and store them.
 // STAGES: K/V tiles of a block in shared memory. Three keep a block's own stream going (two loads in
 // flight); with two a block is slower but three blocks share an SM instead of two, which wins once a
-// launch has more blocks than two per SM can hold at once (12 warps an SM hide the MMAs' latency
-// better than 8; measured at 64 sequences of 3,072 keys: 148 us against 158 us).
+// launch has more blocks than two per SM can hold at once and the lengths differ (64 sequences of 350 .. 3,100 keys in 4 splits:
+// 80 us against 88 us; of 3,072 keys each 131 us, and 123 us unsplit with three stages).
 // SINK: as in the prefill kernel; the sink joins the denominator once, where the splits have been merged.
 template <int MAX_DIM, bool EXACT, bool UPPER, bool CLUSTER = false, int STAGES = 3, bool SINK = false>
 __global__ void __launch_bounds__(THREADS, STAGES == 2 ? 3 : 2)
@@ -449,6 +563,7 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_p
                         const float* __restrict__ sinks, const float* __restrict__ gates, int keep_first, int kv_share,
                         float cap_in, float cap_out, float out_scale, long out_stride) {
   constexpr int KSTEPS = MAX_DIM / 16, NT_O = MAX_DIM / 8;
+  constexpr bool NARROW = EXACT && MAX_DIM == 128 && !UPPER;
   extern __shared__ __align__(16) uint8_t smem_raw[];
   const int dim = EXACT ? MAX_DIM : dim_arg;
   const int stride = dim + PAD;
@@ -491,11 +606,17 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_p
   __syncthreads();
 
   const int newest_tile = p / BKEYS;
+  auto load_tile = [&](int buf, int tile) {       // all of it by the block, or a warp's own keys
+    if constexpr (NARROW) {
+      const int at = (buf * BKEYS + warp * 16) * stride;
+      load_warp_keys(k_s + at, v_s + at, k_pool, v_pool, pages, tile * BKEYS + warp * 16, key_lo, ctx, shape, keep);
+    } else {
+      load_kv_tile(k_s + buf * BKEYS * stride, v_s + buf * BKEYS * stride, k_pool, v_pool, pages, tile, key_lo, ctx, shape, keep);
+    }
+  };
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
-    if (tile_begin + s < tile_end && tile_of(tile_begin + s) != newest_tile)
-      load_kv_tile(k_s + s * BKEYS * stride, v_s + s * BKEYS * stride, k_pool, v_pool, pages, tile_of(tile_begin + s), key_lo, ctx,
-                   shape, keep);
+    if (tile_begin + s < tile_end && tile_of(tile_begin + s) != newest_tile) load_tile(s, tile_of(tile_begin + s));
     cp_async_commit();
   }
   pdl_wait();
@@ -510,65 +631,83 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_p
   }
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
-    if (tile_begin + s < tile_end && tile_of(tile_begin + s) == newest_tile)
-      load_kv_tile(k_s + s * BKEYS * stride, v_s + s * BKEYS * stride, k_pool, v_pool, pages, tile_of(tile_begin + s), key_lo, ctx,
-                   shape, keep);
+    if (tile_begin + s < tile_end && tile_of(tile_begin + s) == newest_tile) load_tile(s, tile_of(tile_begin + s));
   }
   cp_async_commit();     // the query and the held tile: one more group than the ring has stages
 
-  uint32_t qf[KSTEPS][4];
-  float o[NT_O][4];
+  uint32_t qf[NARROW ? 4 : KSTEPS][4];
+  float o[NARROW ? 8 : NT_O][4];
 #pragma unroll
-  for (int n = 0; n < NT_O; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+  for (int n = 0; n < (NARROW ? 8 : NT_O); ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
-  const uint32_t k_lane = (uint32_t)((warp * 16 + (lane >> 4) * 8 + (lane & 7)) * stride + ((lane >> 3) & 1) * 8) * 2;
-  const uint32_t v_lane = (uint32_t)((warp * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * stride + (lane >> 4) * 8) * 2;
+  // lane offsets of the ldmatrix rows: keys in the order of the operand they become
+  const int k_row = NARROW ? (lane & 7) + ((lane >> 3) & 1) * 8 : (lane >> 4) * 8 + (lane & 7);
+  const int k_col = NARROW ? (lane >> 4) * 8 : ((lane >> 3) & 1) * 8;
+  const uint32_t k_lane = (uint32_t)((warp * 16 + k_row) * stride + k_col) * 2;
+  const uint32_t v_lane = (uint32_t)((warp * 16 + (NARROW ? (lane >> 4) * 8 + (lane & 7) : ((lane >> 3) & 1) * 8 + (lane & 7))) * stride +
+                                     (NARROW ? ((lane >> 3) & 1) * 8 : (lane >> 4) * 8)) * 2;
   const uint32_t k_base = smem_u32(k_s) + k_lane, v_base = smem_u32(v_s) + v_lane;
   const uint32_t buf_bytes = (uint32_t)BKEYS * stride * 2;
+  const float slack = scale_log2 > 0.f ? 8.f / scale_log2 : 0.f;
 
   for (int walk = tile_begin; walk < tile_end; ++walk) {
     const int tile = tile_of(walk);
     const int i = walk - tile_begin, buf = i % STAGES;
-    if (walk + STAGES - 1 < tile_end) {
-      const int nb = (i + STAGES - 1) % STAGES;
-      load_kv_tile(k_s + nb * BKEYS * stride, v_s + nb * BKEYS * stride, k_pool, v_pool, pages, tile_of(walk + STAGES - 1), key_lo,
-                   ctx, shape, keep);
-    }
+    if (walk + STAGES - 1 < tile_end) load_tile((i + STAGES - 1) % STAGES, tile_of(walk + STAGES - 1));
     cp_async_commit();
     // the first tile also waits for the group of the query, which was committed after the ring's
     if (i == 0) cp_async_wait<1>(); else cp_async_wait<STAGES - 1>();
-    __syncthreads();
-    if (i == 0) {
-#pragma unroll
-      for (int k = 0; k < KSTEPS; ++k)
-        if (EXACT || k < dk) ldmatrix_x4(qf[k], q_s + (lane & 15) * stride + k * 16 + (lane >> 4) * 8);
-    }
+    if (!NARROW || i == 0) __syncthreads(); else __syncwarp();      // the queries are the block's, a warp's keys its own
     // only the tile that holds the last key, or the first visible one, needs the comparisons
     const bool masked = tile * BKEYS + BKEYS - 1 > p || tile * BKEYS < key_lo;
-    warp_tile<MAX_DIM, EXACT, 1, UPPER, SINK>(qf, k_base + buf * buf_bytes, v_base + buf * buf_bytes, dim, o, m_run, l_run,
-                                              masked, tile * BKEYS + warp * 16, p, p, key_lo, 0, scale_log2, t, keep, cap_in,
-                                              cap_out);
-    __syncthreads();
+    if constexpr (NARROW) {
+      if (i == 0) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) ldmatrix_x4(qf[k], q_s + (lane & 7) * stride + k * 32 + (lane >> 3) * 8);
+      }
+      warp_keys<SINK>(qf, k_base + buf * buf_bytes, v_base + buf * buf_bytes, o, m_run, l_run, masked, tile * BKEYS + warp * 16 + g, p,
+                      key_lo, keep, scale_log2, slack, cap_in, cap_out);
+      __syncwarp();
+    } else {
+      if (i == 0) {
+#pragma unroll
+        for (int k = 0; k < KSTEPS; ++k)
+          if (EXACT || k < dk) ldmatrix_x4(qf[k], q_s + (lane & 15) * stride + k * 16 + (lane >> 4) * 8);
+      }
+      warp_tile<MAX_DIM, EXACT, 1, SINK>(qf, k_base + buf * buf_bytes, v_base + buf * buf_bytes, dim, o, m_run, l_run, masked,
+                                         tile * BKEYS + warp * 16, p, p, key_lo, 0, scale_log2, t, keep, cap_in, cap_out);
+      __syncthreads();
+    }
   }
   cp_async_wait<0>();
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
-    l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 1);
-    l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 2);
+#pragma unroll
+    for (int x = NARROW ? 4 : 1; x < (NARROW ? 32 : 4); x <<= 1) l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], x);
   }
 
   // ---- merge the four warps through shared memory (the tile buffers are free now)
   __syncthreads();
   float* merge = reinterpret_cast<float*>(smem_raw);      // [WARPS][16][dim + 2]: output, then max, then sum
   const int mstride = dim + 2;
+  if constexpr (NARROW) {
 #pragma unroll
-  for (int r = 0; r < (UPPER ? 2 : 1); ++r) {
-    float* dst = merge + ((size_t)warp * 16 + g + 8 * r) * mstride;
+    for (int e = 0; e < 4; ++e) {
+      float* dst = merge + ((size_t)warp * 16 + 2 * t + (e & 1)) * mstride;
 #pragma unroll
-    for (int n = 0; n < NT_O; ++n) {
-      if (EXACT || n * 8 < dim) { dst[n * 8 + 2 * t] = o[n][2 * r]; dst[n * 8 + 2 * t + 1] = o[n][2 * r + 1]; }
+      for (int n = 0; n < 8; ++n) dst[n * 16 + g + 8 * (e >> 1)] = o[n][e];
+      if (g == 0 && e < 2) { dst[dim] = m_run[e]; dst[dim + 1] = l_run[e]; }
     }
-    if (t == 0) { dst[dim] = m_run[r]; dst[dim + 1] = l_run[r]; }
+  } else {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      float* dst = merge + ((size_t)warp * 16 + g + 8 * r) * mstride;
+#pragma unroll
+      for (int n = 0; n < NT_O; ++n) {
+        if (EXACT || n * 8 < dim) { dst[n * 8 + 2 * t] = o[n][2 * r]; dst[n * 8 + 2 * t + 1] = o[n][2 * r + 1]; }
+      }
+      if (t == 0) { dst[dim] = m_run[r]; dst[dim + 1] = l_run[r]; }
+    }
   }
   __syncthreads();
   const float c = scale_log2;

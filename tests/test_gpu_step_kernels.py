@@ -166,3 +166,35 @@ def test_prompt_attention_with_exact_weights(q_heads, kv_heads, window, extras):
             got = out[starts[s]: starts[s + 1]].view(n, q_heads, dim)[:, h].double().cpu()
             # the output rounds to bfloat16 (2^-9), the weights keep 16 bits (2^-17) and their exponentials' 2^-22
             assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -14 * spread + 1e-6).all()
+
+
+@pytest.mark.parametrize("group, page, splits, stages", [(1, 8, 1, 3), (4, 16, 4, 2), (8, 24, 3, 3), (7, 64, 8, 3), (2, 16, 1, 2)])
+@pytest.mark.parametrize("window, keep, extras", [(0, 0, False), (100, 0, False), (70, 30, True), (-96, 0, True)])
+@pytest.mark.parametrize("factor", [0.3, 4.0])
+def test_decode_attention_with_a_warps_own_keys(group, page, splits, stages, window, keep, extras, factor):
+    """Contexts that end at, before and after a warp's 16 keys and a tile's 64; scores that stay within a base and that outgrow it."""
+    o, dim, kv_heads = ops(), 128, 2
+    lengths = [1, 15, 16, 17, 64, 65, 200, 529, 1281]
+    k_pool, v_pool, table, ks, vs = paged_setup(torch.bfloat16, lengths, kv_heads, dim, page, 5)
+    gen, n, q_heads = torch.Generator().manual_seed(6), len(lengths), group * kv_heads
+    q = (factor * torch.randn(n, q_heads * dim, generator=gen)).to(torch.bfloat16).cuda()
+    sinks = torch.randn(q_heads, generator=gen).cuda() if extras else None
+    gates = torch.rand(n, q_heads, generator=gen).cuda() if extras else None
+    out = torch.full((n, q_heads * dim), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    o.attention_decode_bf16(q, k_pool, v_pool, out, table, ints(list(range(n + 1))), ints(lengths), None, n, q_heads, kv_heads, dim, page,
+                            dim ** -0.5, window, splits, stages, sinks=sinks, gates=gates, keep_first=keep)
+    for s, length in enumerate(lengths):
+        j, i = torch.arange(length), length - 1
+        seen = (i - j < window) | (j < keep) if window > 0 else (i // -window == j // -window) if window else (j >= 0)
+        for h in range(q_heads):
+            g = h // group
+            scores = (ks[s][:, g].double() @ q[s].view(q_heads, dim)[h].double().cpu() * dim ** -0.5).masked_fill(~seen, -math.inf)
+            if extras:
+                scores = torch.cat((scores, sinks[h, None].double().cpu()))
+            p = torch.softmax(scores, -1)[:length] * (gates[s, h].double().cpu() if extras else 1.0)
+            want, spread = p @ vs[s][:, g].double(), p @ vs[s][:, g].double().abs()
+            got = out[s].view(q_heads, dim)[h].double().cpu()
+            # the output rounds to bfloat16 (2^-9), a weight to bfloat16 (2^-9) or to 16 bits (2^-17, exponentials 2^-22); scores of
+            # up to 60 in 32-bit are off by 2^-18
+            assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + (2.0 ** -14 if extras else 2.0 ** -8) * spread + 1e-6).all()

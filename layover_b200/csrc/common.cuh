@@ -114,8 +114,8 @@ static inline bool lb_pdl_enabled() {
 }
 
 template <typename... KArgs, typename... Args>
-static inline int lb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                            Args... args) {
+static inline int lb_launch_as(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                               Args... args) {
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
   config.blockDim = block;
@@ -125,8 +125,20 @@ static inline int lb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
   attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute[0].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
-  config.numAttrs = lb_pdl_enabled() ? 1 : 0;
+  config.numAttrs = early && lb_pdl_enabled() ? 1 : 0;
   return (int)cudaLaunchKernelEx(&config, kernel, static_cast<KArgs>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+static inline int lb_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  return lb_launch_as(true, kernel, grid, block, smem, stream, args...);
+}
+
+// A launch whose blocks are placed when the kernels before it have ended. Blocks that come early go where the earlier kernels'
+// blocks leave room, which is uneven, and stay there: a stream of a few blocks an SM then has some SMs idle.
+template <typename... KArgs, typename... Args>
+static inline int lb_launch_settled(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  return lb_launch_as(false, kernel, grid, block, smem, stream, args...);
 }
 
 // One lane's share of a head's sum of squares: eight elements of each half, as the per-head norm

@@ -416,25 +416,33 @@ __global__ void moe_scatter_rows_kernel(const T* __restrict__ h, long h_stride, 
 }
 
 // Which expert's rows block `tile` of a products' launch owns, when every expert's group is cut into tiles of `rows_per_tile`
-// places: all threads read the group sizes at once (one round trip to memory), thread 0 walks the tiles' counts in shared
-// memory. found[0] = expert (-1: no such tile), found[1] = first place, found[2] = places. `counts`: `experts` ints.
+// places: all threads read the group sizes at once (one round trip to memory), warp 0 counts the tiles 32 experts at a
+// time. found[0] = expert (-1: no such tile), found[1] = first place, found[2] = places. `counts`: `experts` ints.
 __device__ __forceinline__ void find_tile(const int* __restrict__ offsets, int experts, int rows_per_tile, int tile,
                                           int* counts, int* found) {
   for (int e = threadIdx.x; e < experts; e += blockDim.x) counts[e] = offsets[e + 1] - offsets[e];
+  if (threadIdx.x == 0) found[0] = -1;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int left = tile, expert = -1, first = 0, rows = 0, begin = 0;
-    for (int e = 0; e < experts && expert < 0; ++e) {
-      const int count = counts[e], tiles = (count + rows_per_tile - 1) / rows_per_tile;
-      if (left < tiles) {
-        expert = e;
-        first = begin + left * rows_per_tile;
-        rows = min(rows_per_tile, count - left * rows_per_tile);
+  if (threadIdx.x < 32) {
+    int left = tile, begin = 0;                     // of the experts from e0 on
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+      const int e = e0 + threadIdx.x, count = e < experts ? counts[e] : 0, tiles = (count + rows_per_tile - 1) / rows_per_tile;
+      int upto_tiles = tiles, upto = count;         // sums over the lanes up to this one
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, upto_tiles, o), y = __shfl_up_sync(0xffffffffu, upto, o);
+        if ((int)threadIdx.x >= o) { upto_tiles += x; upto += y; }
       }
-      left -= tiles;
-      begin += count;
+      const int before = upto_tiles - tiles;
+      if (left >= before && left < upto_tiles) {    // one lane at most
+        const int skipped = (left - before) * rows_per_tile;
+        found[0] = e; found[1] = begin + upto - count + skipped; found[2] = min(rows_per_tile, count - skipped);
+      }
+      const int all_tiles = __shfl_sync(0xffffffffu, upto_tiles, 31);
+      if (left < all_tiles) break;                  // the same for the whole warp
+      left -= all_tiles;
+      begin += __shfl_sync(0xffffffffu, upto, 31);
     }
-    found[0] = expert; found[1] = first; found[2] = rows;
   }
   __syncthreads();
 }
@@ -647,6 +655,120 @@ moe_expert_rows_kernel(const T* __restrict__ a, long a_stride, const int* __rest
   }
 }
 
+// The same in a bfloat16 run on mma.sync: a weight then costs its load and a sixteenth of an instruction for up to 8 rows,
+// where the FFMA pipes need an unpacking and a multiply-add a row. A block owns 16 features (gated: 16 gate and 16 up rows) of
+// one expert and 8 places of its group; its warps share the channels, which gives a step of one token blocks enough. A lane
+// loads 16 neighbouring bytes of two weight rows and of one place's row: of a step of 32 channels lane t of a row has channels
+// 8 t .. 8 t + 7, and both operands name them alike, the first four to one instruction and the last four to the next, so that
+// no shuffle is needed (a sum does not mind the order of its channels; it is the same for every row and batch). AHEAD steps are
+// on their way: what bounds it is the stream. The tensor cores' own sums lose a little at every step (1e-6 of the result over
+// 1,024 channels), so an instruction adds its 16 channels alone and the rest is added here, AHEAD sums a warp, in a fixed order:
+// 6.9e-8 at 1,024 channels and 7.3e-8 at 1,536, where FFMA has 7.0e-8 and 7.5e-8 (against 64 bits).
+// Measured (one B200, 32 experts of 1,024 x 2,048, 4 a token), up and down product: 1 token 10.6 + 6.6 us on FFMA, 10.7 + 4.9 now;
+// 8 tokens 59 + 36, 33 + 21; 16 tokens in a captured decode step 104 + 54, 44 + 27 (5.3 and 4.4 TB/s; 90 + 38 with
+// blocks placed early: the launch is a settled one for that)
+constexpr int MMA_ROWS = 8, MMA_WARPS = 4, MMA_AHEAD = 4;     // four of each: the sums are written out so
+
+__device__ __forceinline__ uint4 load_weights(const bf16* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <typename OutT, bool GATED, int ACT>
+__global__ void __launch_bounds__(MMA_WARPS * 32)
+moe_expert_mma_kernel(const bf16* __restrict__ a, long a_stride, const int* __restrict__ a_rows, int a_div,
+                      const int* __restrict__ offsets, int experts, const bf16* __restrict__ w, long expert_stride,
+                      int n_out, int k_dim, OutT* __restrict__ out, long out_stride, const int* __restrict__ out_rows,
+                      const float* __restrict__ pair_scale, const int* __restrict__ order, int interleaved, LbClip clip) {
+  constexpr int Z = GATED ? 2 : 1, SUMS = GATED ? 2 : MMA_AHEAD;
+  __shared__ int found[3];
+  __shared__ float parts[MMA_WARPS][Z][4][32];   // the warps' sums
+  extern __shared__ int group_counts[];          // [experts]
+  pdl_launch_dependents();
+  pdl_wait();
+  find_tile(offsets, experts, MMA_ROWS, blockIdx.x, group_counts, found);
+  const int expert = found[0], first = found[1], rows = found[2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int f0 = blockIdx.y * 16;
+  if (expert < 0) return;                        // the whole block
+  const bf16* wg = w + (size_t)expert * expert_stride;
+  const bf16* wr[Z][2];                          // gate (and up) rows of features g and g + 8
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int n = min(f0 + g + 8 * h, n_out - 1);                // a feature past the end repeats the last one and is not stored
+    const size_t gate_row = (GATED && interleaved) ? (size_t)(n >> 6) * 128 + (n & 63) : (size_t)n;
+    wr[0][h] = wg + gate_row * k_dim;
+    if (GATED) wr[Z - 1][h] = wg + (interleaved ? gate_row + 64 : (size_t)n_out + n) * k_dim;
+  }
+  const bool live = g < rows;
+  const bf16* x_row = a + (live ? (long)(a_rows ? a_rows[first + g] / a_div : first + g) * a_stride : 0);
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  uint4 wq[MMA_AHEAD][Z][2], xq[MMA_AHEAD];
+  auto load = [&](int u, int step) {
+    const int k = 32 * step + 8 * t;             // a multiple of 8, as k_dim is
+    const bool inside = k < k_dim;
+#pragma unroll
+    for (int z = 0; z < Z; ++z)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) wq[u][z][h] = inside ? load_weights(wr[z][h] + k) : zero;
+    xq[u] = inside && live ? *reinterpret_cast<const uint4*>(x_row + k) : zero;
+  };
+  const int steps = (k_dim + 31) / 32;
+#pragma unroll
+  for (int u = 0; u < MMA_AHEAD; ++u) load(u, warp * MMA_AHEAD + u);
+  float acc[SUMS][Z][4];
+#pragma unroll
+  for (int u = 0; u < SUMS; ++u)
+#pragma unroll
+    for (int z = 0; z < Z; ++z)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[u][z][e] = 0.f;
+  for (int s0 = warp * MMA_AHEAD; s0 < steps; s0 += MMA_WARPS * MMA_AHEAD) {
+#pragma unroll
+    for (int u = 0; u < MMA_AHEAD; ++u) {
+#pragma unroll
+      for (int z = 0; z < Z; ++z) {
+        float lo[4] = {0.f, 0.f, 0.f, 0.f}, hi[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_16816(lo, wq[u][z][0].x, wq[u][z][1].x, wq[u][z][0].y, wq[u][z][1].y, xq[u].x, xq[u].y);
+        mma_16816(hi, wq[u][z][0].z, wq[u][z][1].z, wq[u][z][0].w, wq[u][z][1].w, xq[u].z, xq[u].w);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[u % SUMS][z][e] += lo[e] + hi[e];
+      }
+      load(u, s0 + u + MMA_WARPS * MMA_AHEAD);
+    }
+  }
+#pragma unroll
+  for (int z = 0; z < Z; ++z)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) parts[warp][z][e][lane] = SUMS == 2 ? acc[0][z][e] + acc[1][z][e] : (acc[0][z][e] + acc[1][z][e]) + (acc[SUMS - 2][z][e] + acc[SUMS - 1][z][e]);
+  __syncthreads();
+  if (warp) return;
+  float sum[Z][4];
+#pragma unroll
+  for (int z = 0; z < Z; ++z)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) sum[z][e] = (parts[0][z][e][lane] + parts[1][z][e][lane]) + (parts[2][z][e][lane] + parts[3][z][e][lane]);
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {                  // places 2 t and 2 t + 1
+    if (2 * t + c >= rows) continue;
+    const int place = first + 2 * t + c;
+    const long dst = out_rows ? out_rows[place] : place;
+    const float sc = (GATED && pair_scale) ? pair_scale[order[place]] : 1.f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int n = f0 + g + 8 * h;
+      if (n >= n_out) continue;
+      const float v = sum[0][2 * h + c], u = sum[Z - 1][2 * h + c];
+      Elem<OutT>::store(out + dst * out_stride + n, GATED ? expert_gate<ACT>(sc * v, sc * u, clip) : (ACT == 2 ? expert_activation<2>(v) : v));
+    }
+  }
+}
+
 template <typename T, typename YT>
 __global__ void moe_combine_kernel(const YT* __restrict__ y, const float* __restrict__ pair_scale,
                                    const T* __restrict__ shared_out, const float* __restrict__ shared_factor,
@@ -675,18 +797,35 @@ int launch_product(bool few, int act, const void* a, long a_stride, const int* a
                     (OutT*)out, out_stride, out_rows, pair_scale, order, interleaved, clip
   const bool aligned = (uintptr_t)a % 16 == 0 && (uintptr_t)w % 16 == 0 && k_dim % Piece<T>::N == 0 &&
                        (a_stride * sizeof(T)) % 16 == 0;
-  if (few && aligned) {     // a handful of rows per expert: a stream of the chosen experts' weight rows
-    // enough blocks to fill the GPU: the tiles are about the experts in use, the features are dealt over grid y
-    int tiles = (n_pairs + FEW_ROWS - 1) / FEW_ROWS + experts;
-    if (tiles > n_pairs) tiles = n_pairs;
-    int per_warp = 8;
-    while (per_warp > FEW_FEATURES && (long)tiles * ((n_out + FEW_WARPS * per_warp - 1) / (FEW_WARPS * per_warp)) < 4 * 148) per_warp >>= 1;
-    dim3 grid(tiles, (n_out + FEW_WARPS * per_warp - 1) / (FEW_WARPS * per_warp));
-    if (GATED && act == 3) lb_launch(moe_expert_rows_kernel<T, OutT, GATED, GATED ? 3 : 0>, grid, FEW_WARPS * 32, (size_t)experts * sizeof(int), stream, LB_MOE_ARGS, per_warp);
-    else if (act == 1) lb_launch(moe_expert_rows_kernel<T, OutT, GATED, 1>, grid, FEW_WARPS * 32, (size_t)experts * sizeof(int), stream, LB_MOE_ARGS, per_warp);
-    else if (act == 2) lb_launch(moe_expert_rows_kernel<T, OutT, GATED, 2>, grid, FEW_WARPS * 32, (size_t)experts * sizeof(int), stream, LB_MOE_ARGS, per_warp);
-    else lb_launch(moe_expert_rows_kernel<T, OutT, GATED, 0>, grid, FEW_WARPS * 32, (size_t)experts * sizeof(int), stream, LB_MOE_ARGS, per_warp);
-  } else if (few) {      // the same through tiles of 8 places, for sizes and addresses that cannot be read 16 bytes at a time
+  if constexpr (sizeof(T) == 2) {
+    if (few && aligned && n_out <= 16 * 65535) {   // a handful of rows per expert: a stream of the chosen experts' weight rows
+      int tiles = (n_pairs + MMA_ROWS - 1) / MMA_ROWS + experts;
+      if (tiles > n_pairs) tiles = n_pairs;
+      const dim3 grid(tiles, (n_out + 15) / 16);
+      const size_t smem = (size_t)experts * sizeof(int);
+      if (GATED && act == 3) lb_launch_settled(moe_expert_mma_kernel<OutT, GATED, GATED ? 3 : 0>, grid, MMA_WARPS * 32, smem, stream, LB_MOE_ARGS);
+      else if (act == 1) lb_launch_settled(moe_expert_mma_kernel<OutT, GATED, 1>, grid, MMA_WARPS * 32, smem, stream, LB_MOE_ARGS);
+      else if (act == 2) lb_launch_settled(moe_expert_mma_kernel<OutT, GATED, 2>, grid, MMA_WARPS * 32, smem, stream, LB_MOE_ARGS);
+      else lb_launch_settled(moe_expert_mma_kernel<OutT, GATED, 0>, grid, MMA_WARPS * 32, smem, stream, LB_MOE_ARGS);
+      return lb_last_error();
+    }
+  }
+  if constexpr (sizeof(T) == 4) {
+    if (few && aligned) {   // the same in 32-bit
+      // enough blocks to fill the GPU: the tiles are about the experts in use, the features are dealt over grid y
+      int tiles = (n_pairs + FEW_ROWS - 1) / FEW_ROWS + experts;
+      if (tiles > n_pairs) tiles = n_pairs;
+      int per_warp = 8;
+      while (per_warp > FEW_FEATURES && (long)tiles * ((n_out + FEW_WARPS * per_warp - 1) / (FEW_WARPS * per_warp)) < 4 * 148) per_warp >>= 1;
+      dim3 grid(tiles, (n_out + FEW_WARPS * per_warp - 1) / (FEW_WARPS * per_warp));
+      if (GATED && act == 3) lb_launch(moe_expert_rows_kernel<T, OutT, GATED, GATED ? 3 : 0>, grid, FEW_WARPS * 32, (size_t)experts * sizeof(int), stream, LB_MOE_ARGS, per_warp);
+      else if (act == 1) lb_launch(moe_expert_rows_kernel<T, OutT, GATED, 1>, grid, FEW_WARPS * 32, (size_t)experts * sizeof(int), stream, LB_MOE_ARGS, per_warp);
+      else if (act == 2) lb_launch(moe_expert_rows_kernel<T, OutT, GATED, 2>, grid, FEW_WARPS * 32, (size_t)experts * sizeof(int), stream, LB_MOE_ARGS, per_warp);
+      else lb_launch(moe_expert_rows_kernel<T, OutT, GATED, 0>, grid, FEW_WARPS * 32, (size_t)experts * sizeof(int), stream, LB_MOE_ARGS, per_warp);
+      return lb_last_error();
+    }
+  }
+  if (few) {      // the same through tiles of 8 places, for sizes and addresses that cannot be read 16 bytes at a time
     constexpr int BM = 8, BN = 128;
     dim3 grid((n_pairs + BM - 1) / BM + experts, (n_out + BN - 1) / BN);
     if (grid.x > (unsigned)n_pairs) grid.x = n_pairs;   // every tile holds a pair

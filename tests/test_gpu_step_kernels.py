@@ -10,6 +10,42 @@ from test_gpu_kernels import ops, paged_setup
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("gated, interleaved", [(True, True), (True, False), (False, False)])
+@pytest.mark.parametrize("hidden, inter", [(8, 64), (40, 128), (264, 192), (2048, 64)])
+def test_expert_products_on_few_rows(gated, interleaved, hidden, inter):
+    """Groups of 0, 1, 7, 8, 9 and 17 places beside 40 idle experts (the tiles are counted 32 experts at a time); channels that
+    end within a step of 32, features past the last warp's 16."""
+    o, gen = ops(), torch.Generator().manual_seed(hidden + inter)
+    groups = [0, 1, 7, 8, 9, 17] + [0] * 40 + [2]
+    experts, pairs = len(groups), sum(groups)
+    h = torch.randn(pairs, hidden, generator=gen).to(torch.bfloat16).cuda()       # top 1: a pair is a token
+    rows = 2 * inter if gated else inter
+    w = (torch.randn(experts, rows, hidden, generator=gen) / math.sqrt(hidden)).to(torch.bfloat16).cuda()
+    down = (torch.randn(experts, hidden, inter, generator=gen) / math.sqrt(inter)).to(torch.bfloat16).cuda()
+    scores = torch.rand(pairs, generator=gen).cuda() if gated else None
+    order = torch.randperm(pairs, generator=gen).to(torch.int32).cuda()
+    offsets = torch.tensor([sum(groups[:e]) for e in range(experts + 1)], dtype=torch.int32, device="cuda")
+    stacked = torch.stack([o.interleave_gate_up(x[:inter], x[inter:]) for x in w]) if interleaved else w
+    act = torch.full((pairs, inter), float("nan"), dtype=torch.bfloat16, device="cuda")
+    o.moe_expert_up(h, order, offsets, scores, stacked, act, 1, "silu" if gated else "relu2", interleaved, gated)
+    y = torch.full((pairs, hidden), float("nan"), device="cuda")
+    o.moe_expert_down(act, order, offsets, down, y)
+    expert_of = [e for e, n in enumerate(groups) for _ in range(n)]
+    for place, e in enumerate(expert_of):
+        pair = int(order[place])
+        z = w[e].double() @ h[pair].double()
+        if gated:
+            g, u = float(scores[pair]) * z[:inter], float(scores[pair]) * z[inter:]
+            want = torch.nn.functional.silu(g) * u
+        else:
+            want = torch.relu(z) ** 2
+        # sums of `hidden` terms of about 1 / sqrt(hidden), 32-bit: far below the rounding to bfloat16
+        assert ((act[place].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
+        want = down[e].double() @ act[place].double()
+        bound = inter * 2.0 ** -23 * (down[e].double().abs() @ act[place].double().abs())
+        assert ((y[pair].double() - want).abs() <= bound + 1e-30).all()
+
+
 @pytest.mark.parametrize("m", [1, 7, 16])
 @pytest.mark.parametrize("inter, k", [(64, 512), (64, 4096), (74 * 64, 520), (75 * 64, 512), (19 * 64, 1000)])
 def test_few_token_gated_product_split_over_a_cluster(m, inter, k):

@@ -662,7 +662,7 @@ moe_expert_rows_kernel(const T* __restrict__ a, long a_stride, const int* __rest
 // 8 t .. 8 t + 7, and both operands name them alike, the first four to one instruction and the last four to the next, so that
 // no shuffle is needed (a sum does not mind the order of its channels; it is the same for every row and batch). AHEAD steps are
 // on their way: what bounds it is the stream. The tensor cores' own sums lose a little at every step (1e-6 of the result over
-// 1,024 channels), so an instruction adds its 16 channels alone and the rest is added here, AHEAD sums a warp, in a fixed order:
+// 1,024 channels), so an instruction adds its 16 channels alone and the rest is added here, two or four sums a warp, in a fixed order:
 // 6.9e-8 at 1,024 channels and 7.3e-8 at 1,536, where FFMA has 7.0e-8 and 7.5e-8 (against 64 bits).
 // Measured (one B200, 32 experts of 1,024 x 2,048, 4 a token), up and down product: 1 token 10.6 + 6.6 us on FFMA, 10.7 + 4.9 now;
 // 8 tokens 59 + 36, 33 + 21; 16 tokens in a captured decode step 104 + 54, 44 + 27 (5.3 and 4.4 TB/s; 90 + 38 with

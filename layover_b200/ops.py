@@ -1518,7 +1518,12 @@ def decode_plan(n_seqs: int, q_heads: int, kv_heads: int, dim: int, max_context:
     others have finished, so the context is cut further, into about 7 blocks an SM (at least 12 tiles
     each), with three blocks an SM as soon as two do not hold them all. Measured with lengths spread
     evenly over 0.1..1 of 8,192 keys (us, the plan for equal lengths against this one): 8 sequences
-    54 -> 47, 16: 106 -> 80, 32: 219 -> 136; over 0.1..1 of 3,072 keys: 16: 41 -> 36, 32: 79 -> 56."""
+    54 -> 47, 16: 106 -> 80, 32: 219 -> 136; over 0.1..1 of 3,072 keys: 16: 41 -> 36, 32: 79 -> 56.
+    Where twelve tiles a block would cut the context less than for equal lengths, the plan for those stays: 8 sequences of
+    0.1..1 of 2,400 keys with 2 splits 18.1, with 4 12.2 us, of 1,500 keys 13.1 and 9.5.
+
+    The figures are those of the kernel that had the query heads as rows. With at most 8 heads a KV head it takes less since
+    (8 sequences of 3,072 keys: 24.8 -> 18.9, 64: 146 -> 131, which 123 us unsplit would beat now), and the plans are kept."""
     natural = n_seqs * kv_heads
     want = max(1, 2 * sm_count // natural)                    # all blocks resident at once, two per SM
     splits = min(want, 128, max(1, max_context // 192))       # at least three 64-key tiles per split
@@ -1545,7 +1550,7 @@ def decode_plan(n_seqs: int, q_heads: int, kv_heads: int, dim: int, max_context:
             count *= 2
         while count > 1 and tiles // count < 12:
             count //= 2
-        if count >= 2:
+        if count >= max(2, plan[0]):       # the twelve tiles are no reason to cut less than for equal lengths
             return (count, 3) if natural * count <= 2 * sm_count else (count, 2)
     if 10 * natural >= 17 * sm_count and natural <= 2 * sm_count and tiles >= 64 and q_heads // kv_heads <= 8:
         # just under two blocks an SM, long contexts: four splits with three blocks an SM measured

@@ -36,3 +36,11 @@ def test_decode_plan_cuts_further_when_the_longest_sequence_stands_out():
         for ctx in (130, 1000, 5000, 70000):
             splits, stages = plan(seqs, ctx, ctx // 3)
             assert splits >= 1 and stages in (2, 3)
+
+
+def test_decode_plan_for_unequal_lengths_cuts_at_least_as_far_as_for_equal_ones():
+    for seqs in range(5, 16):
+        for ctx in range(256, 3072, 128):
+            equal = ops.decode_plan(seqs, 32, 8, 128, ctx, SMS)
+            assert ops.decode_plan(seqs, 32, 8, 128, ctx, SMS, ctx // 2)[0] >= equal[0]
+    assert ops.decode_plan(8, 32, 8, 128, 2400, SMS, 1300) == (4, 3)

@@ -326,9 +326,9 @@ segment_state_kernel(const T* __restrict__ proj, long row_stride, int k_off, int
 // 64 x 64 weights decay^(i-j) (q_i . k_j) through shared memory, and their product with the values. Rows of 132 floats keep
 // the 16-byte reads along a row free of bank conflicts. The FFMA pipes bound it.
 // Measured (one B200, one prompt of 1,500 tokens, 32 heads of 128 x 128, the three launches of a layer, states,
-// joining, outputs): 129 + 10 + 310 us when the segments walked their tokens one by one, now 90 + 24 + 193 us (the
-// outputs' 3.9 GFLOP at 0.27 of the nominal FFMA rate: 768 blocks are 2.6 waves, and the later 64 tokens of a segment have
-// twice the keys of the earlier ones)
+// joining, outputs): 129 + 10 + 310 us when the segments walked their tokens one by one, then 90 + 24 + 193 us with
+// segments of 128, 283 in all with segments of 64, whose blocks have equal work. The next block's rows on their way while one is
+// multiplied changed nothing (305 against 306 us): the blocks beside it hide them
 template <typename T, int ACT>
 __global__ void __launch_bounds__(SEG_THREADS, 2)
 segment_output_kernel(const T* __restrict__ proj, long row_stride, int q_off, int k_off, int v_off, float* __restrict__ out,

@@ -77,7 +77,7 @@ class DecayLinearAttention(Part):
         tokens, qk, vv = h.shape[0], self.heads * self.dim, self.heads * self.vdim
         proj = self.runtime.linear(h, self.w_in)                    # [T, q | k | v | gate (| padding)]
         scanned = torch.empty((tokens, vv), dtype=torch.float32, device=h.device)
-        segment_tokens, segments = ops.scan_segments(batch.q_lens, 4 * self.heads * self.dim * self.vdim)
+        segment_tokens, segments = ops.scan_segments(batch.q_lens, 4 * self.heads * self.dim * self.vdim, self.dim)
         scratch = torch.empty((segments, self.heads, self.dim, self.vdim), dtype=torch.float32, device=h.device) if segments else None
         ops.decay_scan(proj, 0, qk, 2 * qk, scanned, cache.state, batch.cu_q, batch.state_slots, self.decay, batch.n_seqs,
                        self.heads, self.dim, self.vdim, self.activation, segment_tokens, scratch)

@@ -102,7 +102,7 @@ def test_prompt_attention_with_keys_dealt_to_several_blocks(q_heads, kv_heads, w
 
 
 @pytest.mark.parametrize("heads, dim, vdim, decay", [(2, 33, 7, [0.9, 0.0]), (1, 64, 130, [1.0]), (3, 128, 128, [0.999, 0.5, 0.97]), (2, 36, 4, [0.3, 0.99])])
-@pytest.mark.parametrize("lengths, segment", [([1], 128), ([127, 128, 129], 128), ([300, 2, 256], 128), ([70], 64), ([513, 100], 256)])
+@pytest.mark.parametrize("lengths, segment", [([1], 128), ([127, 128, 129], 128), ([300, 2, 256], 128), ([70], 64), ([300, 65, 128], 64), ([513, 100], 256)])
 def test_segments_as_matrix_products(heads, dim, vdim, decay, lengths, segment):
     """Segments that end at, before and after blocks of 64 tokens, several sequences, heads whose rows allow four channels at a
     time or not, states that are carried in and out."""

@@ -47,6 +47,9 @@ template <int ACT> __device__ __forceinline__ float activate(float z) {
   return ACT == 1 ? z / (1.0f + __expf(-z)) : z;      // 1: silu, 0: none
 }
 
+// decay^n; 1 for n = 0 also where the decay is 0 (its logarithm is -inf)
+__device__ __forceinline__ float decay_power(float log2_lam, int n) { return n == 0 ? 1.f : exp2f((float)n * log2_lam); }
+
 // the sequence and the segment of it that global segment `g` is; a sequence has at least one segment
 __device__ __forceinline__ void find_segment(const int* __restrict__ cu_q, int n_seqs, int seg_tokens, int g, int& seq,
                                              int& segment, int& first_segment) {
@@ -209,7 +212,7 @@ __global__ void scan_combine_kernel(float* __restrict__ seg_state, float* __rest
       const int sg = s0 + u;
       if (sg >= ns) break;
       e[(size_t)(FROM_ZERO ? sg : sg - 1) * per_segment] = running;
-      running = fmaf(exp2f((float)min(seg_tokens, len - sg * seg_tokens) * log2_lam), running, local[u]);
+      running = fmaf(decay_power(log2_lam, min(seg_tokens, len - sg * seg_tokens)), running, local[u]);
     }
   }
   *slot = running;
@@ -249,7 +252,6 @@ __device__ __forceinline__ float4 load_quad(const T* __restrict__ head, int c, i
   }
   return make_float4(activate<ACT>(v[0]), activate<ACT>(v[1]), activate<ACT>(v[2]), activate<ACT>(v[3]));
 }
-__device__ __forceinline__ float decay_power(float log2_lam, int n) { return n == 0 ? 1.f : exp2f((float)n * log2_lam); }
 
 // E of one segment and head, 128 value columns a block: a 128 x 128 tile, 8 x 8 sums a thread, 16 tokens a step through two
 // buffers. The FFMA pipes bound it.

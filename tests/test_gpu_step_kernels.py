@@ -234,3 +234,22 @@ def test_decode_attention_with_a_warps_own_keys(group, page, splits, stages, win
             # the output rounds to bfloat16 (2^-9), a weight to bfloat16 (2^-9) or to 16 bits (2^-17, exponentials 2^-22); scores of
             # up to 60 in 32-bit are off by 2^-18
             assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + (2.0 ** -14 if extras else 2.0 ** -8) * spread + 1e-6).all()
+
+
+@pytest.mark.parametrize("dim", [24, 64])       # segments that walk their tokens, and segments as matrix products
+@pytest.mark.parametrize("lengths", [[0], [130, 0, 70], [0, 300, 0]])
+def test_segments_of_a_sequence_without_tokens_leave_its_state(dim, lengths):
+    """A decay of 0 to the power 0 is 1: the state of a request that brings no tokens keeps its bits."""
+    o, heads, vdim, segment = ops(), 2, 20, 64
+    gen, tokens, n_seqs = torch.Generator().manual_seed(dim), sum(lengths), len(lengths)
+    proj = torch.randn(tokens, heads * (2 * dim + vdim), generator=gen).cuda()
+    state = torch.randn(n_seqs, heads, dim, vdim, generator=gen).cuda()
+    before = state.clone()
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    scratch = torch.full((sum(max(1, -(-n // segment)) for n in lengths), heads, dim, vdim), float("nan"), device="cuda")
+    out = torch.full((tokens, heads * vdim), float("nan"), device="cuda")
+    o.decay_scan(proj, 0, heads * dim, 2 * heads * dim, out, state, ints([sum(lengths[:s]) for s in range(n_seqs + 1)]), ints(list(range(n_seqs))),
+                 torch.tensor([0.0, 0.9], device="cuda"), n_seqs, heads, dim, vdim, None, segment, scratch)
+    assert not torch.isnan(out).any() and not torch.isnan(state).any()
+    for s, n in enumerate(lengths):
+        assert torch.equal(state[s], before[s]) == (n == 0)

@@ -37,6 +37,8 @@
 // for bit.
 #include <math.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace {
@@ -363,26 +365,29 @@ segment_output_kernel(const T* __restrict__ proj, long row_stride, int q_off, in
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-  // acc += rows of `left` (4 ty ..; 64 columns from c0 on) times the 64 rows of block_s
-  auto multiply = [&](const float* left, int pitch, int c0) {
-#pragma unroll 2
-    for (int c = 0; c < SEG_ROWS; c += 4) {
-      float4 l[4];
+  // acc += rows of `left` (4 ty ..; `columns` columns from c0 on) times the first `columns` rows of block_s; a CORNER leaves out
+  // what lies above the diagonal of its four columns
+  auto multiply_quad = [&](const float* left, int pitch, int c, auto corner) {
+    constexpr bool CORNER = decltype(corner)::value;
+    float4 l[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) l[i] = *reinterpret_cast<const float4*>(left + (4 * ty + i) * pitch + c0 + c);
+    for (int i = 0; i < 4; ++i) l[i] = *reinterpret_cast<const float4*>(left + (4 * ty + i) * pitch + c);
 #pragma unroll
-      for (int s = 0; s < 4; ++s) {
-        const float4 ra = *reinterpret_cast<const float4*>(block_s + (c + s) * SEG_PITCH + 4 * tx);
-        const float4 rb = *reinterpret_cast<const float4*>(block_s + (c + s) * SEG_PITCH + 64 + 4 * tx);
-        const float r[8] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
+    for (int s = 0; s < 4; ++s) {
+      const float* row = block_s + (c % SEG_ROWS + s) * SEG_PITCH;
+      const float4 ra = *reinterpret_cast<const float4*>(row + 4 * tx), rb = *reinterpret_cast<const float4*>(row + 64 + 4 * tx);
+      const float r[8] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float x = s == 0 ? l[i].x : s == 1 ? l[i].y : s == 2 ? l[i].z : l[i].w;
+      for (int i = CORNER ? s : 0; i < 4; ++i) {
+        const float x = s == 0 ? l[i].x : s == 1 ? l[i].y : s == 2 ? l[i].z : l[i].w;
 #pragma unroll
-          for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x, r[j], acc[i][j]);
-        }
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x, r[j], acc[i][j]);
       }
     }
+  };
+  auto multiply = [&](const float* left, int pitch, int c0, int columns) {
+#pragma unroll 2
+    for (int c = 0; c < columns; c += 4) multiply_quad(left, pitch, c0 + c, std::false_type());
   };
   const float* from = seg_state + ((size_t)blockIdx.z * heads + head) * dim * vdim;
   for (int d0 = 0; d0 < dim; d0 += SEG_ROWS) {
@@ -394,7 +399,7 @@ segment_output_kernel(const T* __restrict__ proj, long row_stride, int q_off, in
           load_quad<float, 0>(from + (size_t)d * vdim, e0 + c, vdim, d < dim, vdim % 4 == 0);
     }
     __syncthreads();
-    multiply(q_s, SEG_PITCH, d0);
+    multiply(q_s, SEG_PITCH, d0, SEG_ROWS);
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -438,7 +443,13 @@ segment_output_kernel(const T* __restrict__ proj, long row_stride, int q_off, in
     __syncthreads();                                        // the keys are read, the weights are there
     load_block(block_s, j0, v_off + head * vdim, e0, vdim);
     __syncthreads();
-    multiply(a_s, A_PITCH, 0);
+    // a token takes the values of its own and of earlier tokens alone: a weight of 0 does not keep out a value that is not finite
+    if (j0 < i0) {
+      multiply(a_s, A_PITCH, 0, SEG_ROWS);
+    } else {
+      multiply(a_s, A_PITCH, 0, 4 * ty);
+      multiply_quad(a_s, A_PITCH, 4 * ty, std::true_type());
+    }
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {

@@ -253,3 +253,29 @@ def test_segments_of_a_sequence_without_tokens_leave_its_state(dim, lengths):
     assert not torch.isnan(out).any() and not torch.isnan(state).any()
     for s, n in enumerate(lengths):
         assert torch.equal(state[s], before[s]) == (n == 0)
+
+
+@pytest.mark.parametrize("dim", [24, 128])      # segments that walk their tokens, and segments as matrix products
+@pytest.mark.parametrize("what", ["k", "v"])
+@pytest.mark.parametrize("value", [math.inf, -math.inf, math.nan])
+def test_segments_keep_a_value_that_is_not_finite_from_earlier_tokens(dim, what, value):
+    """The outputs of the tokens before it keep their bits, wherever it stands in a block of 64 tokens; its own is not finite."""
+    o, heads, vdim, tokens = ops(), 2, 128, 200
+    gen = torch.Generator().manual_seed(dim)
+    clean = torch.randn(tokens, heads * (2 * dim + vdim), generator=gen).cuda()
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    lam = torch.tensor([0.9, 0.99], device="cuda")
+
+    def run(proj):
+        state, out = torch.zeros(1, heads, dim, vdim, device="cuda"), torch.empty(tokens, heads * vdim, device="cuda")
+        scratch = torch.empty(2, heads, dim, vdim, device="cuda")
+        o.decay_scan(proj, 0, heads * dim, 2 * heads * dim, out, state, ints([0, tokens]), ints([0]), lam, 1, heads, dim, vdim, None, 128, scratch)
+        return out.view(tokens, heads, vdim)
+
+    want, column = run(clean), heads * dim + 5 if what == "k" else 2 * heads * dim + 5
+    for at in (1, 2, 30, 63, 64, 66, 127, 128, 131, 199):
+        proj = clean.clone()
+        proj[at, column] = value
+        got = run(proj)
+        assert torch.equal(got[:at], want[:at]) and torch.equal(got[:, 1], want[:, 1])
+        assert not torch.isfinite(got[at, 0]).all()

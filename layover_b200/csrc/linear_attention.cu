@@ -337,7 +337,7 @@ template <typename T, int ACT>
 __global__ void __launch_bounds__(SEG_THREADS, 2)
 segment_output_kernel(const T* __restrict__ proj, long row_stride, int q_off, int k_off, int v_off, float* __restrict__ out,
                       const int* __restrict__ cu_q, const float* __restrict__ decay, int heads, int dim, int vdim,
-                      const float* __restrict__ seg_state, int seg_tokens, int n_seqs, int e_tiles, bool vec) {
+                      const float* __restrict__ seg_state, int seg_tokens, int n_seqs, int e_tiles, bool vec, bool vec_state) {
   extern __shared__ __align__(16) float scan_smem[];
   float* q_s = scan_smem;                                   // [64][SEG_PITCH]
   float* block_s = q_s + SEG_ROWS * SEG_PITCH;              // [64][SEG_PITCH]: a slice of S_in, keys, values
@@ -396,7 +396,7 @@ segment_output_kernel(const T* __restrict__ proj, long row_stride, int q_off, in
     for (int u = 0; u < SEG_ROWS * 32 / SEG_THREADS; ++u) {
       const int d = d0 + (threadIdx.x >> 5) + 8 * u, c = (threadIdx.x & 31) * 4;
       *reinterpret_cast<float4*>(block_s + (d - d0) * SEG_PITCH + c) =
-          load_quad<float, 0>(from + (size_t)d * vdim, e0 + c, vdim, d < dim, vdim % 4 == 0);
+          load_quad<float, 0>(from + (size_t)d * vdim, e0 + c, vdim, d < dim, vec_state);
     }
     __syncthreads();
     multiply(q_s, SEG_PITCH, d0, SEG_ROWS);
@@ -477,13 +477,14 @@ int launch_segments(int n_seqs, int total_segments, int seg_tokens, float* seg_s
   // four channels at a time where every head's rows start on four elements' boundaries
   const bool vec = (uintptr_t)proj % (4 * sizeof(T)) == 0 && row_stride % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && v_off % 4 == 0 &&
                    dim % 4 == 0 && vdim % 4 == 0;
+  const bool vec_state = (uintptr_t)seg_state % 16 == 0 && vdim % 4 == 0;      // the caller's scratch may begin anywhere
   lb_launch(segment_state_kernel<T, ACT>, dim3(e_tiles, heads, total_segments), SEG_THREADS, 0, stream, (const T*)proj, row_stride, k_off,
             v_off, cu_q, decay, heads, dim, vdim, seg_state, seg_tokens, n_seqs, vec);
   lb_launch(scan_combine_kernel<true>, dim3((unsigned)(((size_t)heads * per_head + 255) / 256), n_seqs), 256, 0, stream, seg_state, state,
             cu_q, state_slots, decay, heads, per_head, seg_tokens);
   lb_launch(segment_output_kernel<T, ACT>, dim3(row_blocks * e_tiles, heads, total_segments), SEG_THREADS, (size_t)smem, stream,
             (const T*)proj, row_stride, q_off, k_off, v_off, out, cu_q, decay, heads, dim, vdim, (const float*)seg_state, seg_tokens, n_seqs,
-            e_tiles, vec);
+            e_tiles, vec, vec_state);
   return lb_last_error();
 }
 

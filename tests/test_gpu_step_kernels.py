@@ -279,3 +279,17 @@ def test_segments_keep_a_value_that_is_not_finite_from_earlier_tokens(dim, what,
         got = run(proj)
         assert torch.equal(got[:at], want[:at]) and torch.equal(got[:, 1], want[:, 1])
         assert not torch.isfinite(got[at, 0]).all()
+
+
+def test_segments_with_scratch_that_begins_anywhere():
+    """Scratch four bytes off a 16-byte boundary gives the bits that aligned scratch gives."""
+    o, heads, dim, vdim, tokens = ops(), 2, 64, 64, 150
+    proj = torch.randn(tokens, heads * (2 * dim + vdim), generator=torch.Generator().manual_seed(1)).cuda()
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    lam, floats, results = torch.tensor([0.9, 0.99], device="cuda"), 3 * heads * dim * vdim, []
+    for shift in (0, 1):
+        scratch = torch.empty(floats + 1, device="cuda")[shift: shift + floats].view(3, heads, dim, vdim)
+        state, out = torch.ones(1, heads, dim, vdim, device="cuda"), torch.empty(tokens, heads * vdim, device="cuda")
+        o.decay_scan(proj, 0, heads * dim, 2 * heads * dim, out, state, ints([0, tokens]), ints([0]), lam, 1, heads, dim, vdim, None, 64, scratch)
+        results.append((out, state))
+    assert all(torch.equal(a, b) for a, b in zip(*results))

@@ -1107,13 +1107,14 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tens
         raise ValueError(f"gemm: shapes do not agree: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
     if a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
         raise ValueError("gemm: innermost dimension must be contiguous")
+    a_ptr, w_ptr, out_ptr = _ptr(a), _ptr(w), _ptr(out)        # refuses other devices, before theirs is asked about
     scratch = None
     if a.dtype == torch.float32 and min(m, n, k) > 0:      # partial sums of this call alone, on its own stream
         wanted = (_FUNCTIONS.get("lb_gemm_simt_scratch") or _fn("gemm_simt", "lb_gemm_simt_scratch", [c_int] * 4, c_long))(m, n, k, sm_count(a.device))
         scratch = torch.empty(wanted, dtype=torch.float32, device=a.device) if wanted else None
     fn = _FUNCTIONS.get("lb_gemm_simt") or _fn("gemm_simt", "lb_gemm_simt",
              [c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_long, c_long, c_long, c_void_p, c_int, c_void_p])
-    _check(fn(dtype_code(a.dtype), dtype_code(out.dtype), _ptr(a), _ptr(w), _ptr(out), m, n, k, a.stride(0),
+    _check(fn(dtype_code(a.dtype), dtype_code(out.dtype), a_ptr, w_ptr, out_ptr, m, n, k, a.stride(0),
               w.stride(0), out.stride(0), _ptr(scratch), sm_count(a.device), _stream()), "gemm_simt")
     if scratch is not None:
         global LAUNCHES
@@ -1164,6 +1165,7 @@ def attention_simt(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, 
                     ("tile_q0", tile_q0)):
         _need(t, torch.int32, name)
     max_q_len = 1 << 30 if max_q_len is None else int(max_q_len)
+    q_ptr = _ptr(q)        # refuses other devices, before theirs is asked about
     splits, chunk_room = _simt_splits(n_tiles, q_heads, kv_heads, vdim, max_q_len, max_ctx, block_table.shape[1] * page_tokens, q.device)
     partials = None
     if splits > 1:          # of this call alone, on its own stream
@@ -1172,7 +1174,7 @@ def attention_simt(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, 
     fn = _FUNCTIONS.get("lb_attention_simt") or _fn("attention_simt", "lb_attention_simt",
              [c_int] + [c_void_p] * 5 + [c_int] + [c_void_p] * 4 + [c_int] * 5 + [c_float, c_int, c_int, c_void_p,
               c_void_p, c_int, c_int, c_float, c_float, c_long, c_int, c_int, c_void_p, c_int, c_void_p])
-    _check(fn(dtype_code(q.dtype), _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(out), _ptr(block_table),
+    _check(fn(dtype_code(q.dtype), q_ptr, _ptr(k_pool), _ptr(v_pool), _ptr(out), _ptr(block_table),
               block_table.shape[1], _ptr(cu_q), _ptr(ctx_len), _ptr(tile_seq), _ptr(tile_q0), n_tiles, q_heads,
               kv_heads, dim, page_tokens, float(scale), int(window), vdim, _ptr(sinks), _ptr(gates), int(chunk), int(keep_first),
               float(softcap), float(out_scale), out.stride(0), max_q_len, splits, _ptr(partials), chunk_room, _stream()),

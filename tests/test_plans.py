@@ -1,5 +1,8 @@
 """Launch plans that are plain functions of sizes (no device needed)."""
 
+import pytest
+import torch
+
 from layover_b200 import ops
 
 SMS = 148
@@ -44,3 +47,13 @@ def test_decode_plan_for_unequal_lengths_cuts_at_least_as_far_as_for_equal_ones(
             equal = ops.decode_plan(seqs, 32, 8, 128, ctx, SMS)
             assert ops.decode_plan(seqs, 32, 8, 128, ctx, SMS, ctx // 2)[0] >= equal[0]
     assert ops.decode_plan(8, 32, 8, 128, 2400, SMS, 1300) == (4, 3)
+
+
+def test_tensors_of_another_device_are_refused_before_the_device_is_asked_about():
+    a, w, out = torch.zeros(4, 64), torch.zeros(32, 64), torch.zeros(4, 32)
+    with pytest.raises(ops.KernelError):
+        ops.gemm_simt(a, w, out)
+    ints = lambda *values: torch.tensor(values, dtype=torch.int32)
+    q, pool, out = torch.zeros(1, 128), torch.zeros(4, 1, 16, 64), torch.zeros(1, 128)
+    with pytest.raises(ops.KernelError):
+        ops.attention_simt(q, pool, pool, out, ints(0, 1, 2)[None], ints(0, 1), ints(40), ints(0), ints(0), 1, 2, 1, 64, 16, 0.125, max_ctx=40)

@@ -83,6 +83,7 @@ class StepBatch:
     n_decode_seqs: int
     decode_max_ctx: int
     portion_tiles: dict[int, QueryTiles]
+    portion_max_ctx: int         # the longest context among the sequences of `portion_tiles`
     # host-side facts for planning launches
     q_lens: list[int]
     ctx_lens: list[int]
@@ -299,6 +300,7 @@ class BatchBuilder:
             decode_max_ctx=max((ctx_lens[s] for s in singles), default=0) if mixed else 0,
             portion_tiles={size: QueryTiles(get(f"ptile_seq{size}"), get(f"ptile_q0{size}"), len(tiles))
                            for size, tiles in portion_lists.items()},
+            portion_max_ctx=max((c for n, c in zip(q_lens, ctx_lens) if n > 1), default=0) if mixed else 0,
             q_lens=q_lens, ctx_lens=ctx_lens, max_q_len=max(q_lens), max_ctx=max(ctx_lens),
             all_decode=max(q_lens) == 1, real_seqs=real,
             plan_max_ctx=plan_ctx[0] if plan_ctx else max((ctx_lens[s] for s in singles), default=0),

@@ -1721,7 +1721,7 @@ def attention_bf16(q, cache, out, block_table, batch, q_heads, kv_heads, dim, pa
                               batch.n_seqs, q_heads, decode_groups, dim, page_tokens, scale, window, splits, stages,
                               kv_share=decode_share, **extras)
         return
-    tiles_of = batch.tiles
+    tiles_of, portion_ctx = batch.tiles, batch.max_ctx
     if batch.n_decode_seqs > 0 and q_heads // decode_groups <= 16:
         # a mixed step: the sequences with a single token go through the decode kernel (a tile kernel
         # would spend a whole tile of queries on each), the prompt portions through the tile kernel
@@ -1732,12 +1732,12 @@ def attention_bf16(q, cache, out, block_table, batch, q_heads, kv_heads, dim, pa
         attention_decode_bf16(q, cache.k_pool, cache.v_pool, out, block_table, batch.cu_q, batch.ctx_len, batch.decode_seqs,
                               batch.n_decode_seqs, q_heads, decode_groups, dim, page_tokens, scale, window, splits, stages,
                               kv_share=decode_share, **extras)
-        tiles_of = batch.portion_tiles
+        tiles_of, portion_ctx = batch.portion_tiles, batch.portion_max_ctx
     if plain and cache.pool is not None and attention_tcgen05_supports(q_heads, kv_heads, dim, page_tokens):
         tiles = tiles_of[TCGEN05_TILE]
         attention_tcgen05_prefill(q, cache.pool, cache.layer, out, block_table, batch.cu_q, batch.ctx_len, tiles.tile_seq,
                                   tiles.tile_q0, tiles.count, q_heads, kv_heads, dim, page_tokens, scale, window,
-                                  portion_splits(tiles.count, q_heads, kv_heads, seen(batch.max_ctx), sm_count(q.device)))
+                                  portion_splits(tiles.count, q_heads, kv_heads, seen(portion_ctx), sm_count(q.device)))
         return
     if (exact_weights and not keep_first and not softcap and TCGEN05_TILE in tiles_of and cache.pool is not None
             and attention_tcgen05_exact_takes(q_heads, kv_heads, dim) and attention_tcgen05_supports(q_heads, kv_heads, dim, page_tokens)

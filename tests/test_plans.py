@@ -4,6 +4,9 @@ import pytest
 import torch
 
 from layover_b200 import ops
+from layover_b200.cache import CacheManager
+from layover_b200.engine.batch import BatchBuilder, StepEntry
+from layover_b200.parts.base import PagedKVNeed
 
 SMS = 148
 
@@ -57,3 +60,46 @@ def test_tensors_of_another_device_are_refused_before_the_device_is_asked_about(
     q, pool, out = torch.zeros(1, 128), torch.zeros(4, 1, 16, 64), torch.zeros(1, 128)
     with pytest.raises(ops.KernelError):
         ops.attention_simt(q, pool, pool, out, ints(0, 1, 2)[None], ints(0, 1), ints(40), ints(0), ints(0), 1, 2, 1, 64, 16, 0.125, max_ctx=40)
+
+
+class _Recorder:
+    """`ops.attention_bf16` for a step of (tokens before, new tokens) requests on the CPU: which kernels it would launch, and how."""
+
+    def __init__(self, monkeypatch, q_heads=32, kv_heads=8):
+        self.heads, self.calls = (q_heads, kv_heads), []
+        monkeypatch.setattr(ops, "gemm_scratch", lambda device: (None, None, SMS))
+        monkeypatch.setattr(ops, "sm_count", lambda device: SMS)
+        monkeypatch.setattr(ops, "attention_mma_block_queries", lambda: 64)
+        names = ("q", "pool", "layer", "out", "table", "cu_q", "ctx_len", "tile_seq", "tile_q0", "n_tiles", "q_heads", "kv_heads", "dim", "page",
+                 "scale", "window", "splits", "exact_weights")
+        monkeypatch.setattr(ops, "attention_tcgen05_prefill", lambda *a: self.calls.append(("tcgen05", dict(zip(names, a)))))
+        monkeypatch.setattr(ops, "attention_prefill_bf16", lambda *a, **k: self.calls.append(("mma", k)))
+        monkeypatch.setattr(ops, "attention_decode_bf16", lambda *a, **k: self.calls.append(("decode", k)))
+
+    def run(self, requests, capacity=None, **options):
+        q_heads, kv_heads = self.heads
+        cache = CacheManager([(0, PagedKVNeed(kv_heads, 128, None), None)], 4096, 16, torch.bfloat16, "meta", 64)
+        entries = []
+        for i, (held, new) in enumerate(requests):
+            seq = cache.open(str(i))
+            cache.grow(seq, held + new)
+            cache.commit(seq, held)
+            entries.append(StepEntry(seq, [0] * new, []))
+        batch = BatchBuilder(cache, torch.device("cpu"), (64, 128)).build(entries, capacity)
+        q = torch.empty(batch.n_tokens, q_heads * 128, dtype=torch.bfloat16)
+        self.calls.clear()
+        ops.attention_bf16(q, cache.view(0), torch.empty_like(q), batch.groups[0].block_table, batch, q_heads, kv_heads, 128, 16, 128 ** -0.5,
+                           options.pop("window", 0), **options)
+        return self.calls
+
+
+def test_a_portions_split_is_planned_from_the_portions_own_contexts(monkeypatch):
+    """What other requests of the step hold changes nothing: not the launches of a portion, and not its rounding."""
+    step = _Recorder(monkeypatch)
+    split = lambda requests: next(call["splits"] for name, call in step.run(requests) if name == "tcgen05")
+    for portion in ((0, 64), (0, 256), (0, 512), (1000, 128), (8209, 512)):
+        alone = split([portion])
+        for decoding in ((200, 1), (4000, 1), (8192, 1)):
+            assert split([portion, decoding]) == alone and split([decoding, portion, decoding]) == alone
+    assert split([(0, 64), (8192, 1)]) == 1 and split([(8209, 512)]) > 1
+    assert split([(0, 64), (3000, 64), (8192, 1)]) == split([(3000, 64), (0, 64)])     # the longest of the portions counts

@@ -238,7 +238,7 @@ template <int TOKENS> struct Few {
 template <int TOKENS>
 __global__ void __launch_bounds__(32 * Few<TOKENS>::WARPS)
 gemm_f32_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, float* __restrict__ C,
-                    float* __restrict__ partials, int M, int N, int K, long ldc) {
+                    float* __restrict__ partials, int M, int N, int K, long ldc, bool early_weights) {
   using F = Few<TOKENS>;
   extern __shared__ uint8_t raw_smem[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~(uintptr_t)1023);
@@ -274,9 +274,14 @@ gemm_f32_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   };
   if (!partials) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   pdl_launch_dependents();
-  if (lane == 0)
-    for (int i = 0; i < FEW_STAGES && i < stages; ++i) copy_weights(i);      // weights are written by no kernel
+  // before the wait only what no kernel that may still run writes: the caller says whether the weights are that
+  auto first_weights = [&] {
+    if (lane == 0)
+      for (int i = 0; i < FEW_STAGES && i < stages; ++i) copy_weights(i);
+  };
+  if (early_weights) first_weights();
   pdl_wait();
+  if (!early_weights) first_weights();
   if (lane == 0)
     for (int i = 0; i < FEW_STAGES && i < stages; ++i) copy_tokens(i);
 
@@ -500,6 +505,7 @@ struct Product {
   int M, N, K;
   long lda, ldw, ldc;
   int sm_count;
+  bool early_weights;
   cudaStream_t stream;
   bool tma() const {      // 16-byte aligned addresses and row strides
     return (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0 && lda % 4 == 0 && ldw % 4 == 0 && lda >= K && ldw >= K;
@@ -526,10 +532,11 @@ int launch_few(const Product& p) {
   const dim3 grid((p.N + FEW_ROWS - 1) / FEW_ROWS, 1, Split(p.K).groups()), block(32 * F::WARPS);
   if (!p.partials) {
     lb_launch_cluster(gemm_f32_few_kernel<TOKENS>, grid, block, (size_t)F::SMEM, p.stream, grid.z, map_w, map_a, p.C, p.partials, p.M,
-                      p.N, p.K, p.ldc);
+                      p.N, p.K, p.ldc, p.early_weights);
     return lb_last_error();
   }
-  lb_launch(gemm_f32_few_kernel<TOKENS>, grid, block, (size_t)F::SMEM, p.stream, map_w, map_a, p.C, p.partials, p.M, p.N, p.K, p.ldc);
+  lb_launch(gemm_f32_few_kernel<TOKENS>, grid, block, (size_t)F::SMEM, p.stream, map_w, map_a, p.C, p.partials, p.M, p.N, p.K, p.ldc,
+            p.early_weights);
   return sum_groups(p);
 }
 
@@ -587,13 +594,14 @@ LB_EXPORT long lb_gemm_simt_scratch(int M, int N, int K, int sm_count) {
 }
 
 // in_dtype: type of A and W; out_dtype: type of C (bf16 inputs may write 32-bit floats). `scratch`: null, or as many floats as
-// `lb_gemm_simt_scratch` says, used by this call alone.
+// `lb_gemm_simt_scratch` says, used by this call alone. `early_weights`: no kernel that may still run when this one is launched
+// writes W, which is then read before that kernel has ended.
 LB_EXPORT int lb_gemm_simt(int in_dtype, int out_dtype, const void* A, const void* W, void* C, int M, int N, int K,
-                           long lda, long ldw, long ldc, float* scratch, int sm_count, cudaStream_t stream) {
+                           long lda, long ldw, long ldc, float* scratch, int sm_count, int early_weights, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return LB_ERR_SIZE;
   if (in_dtype == LB_F32 && out_dtype == LB_F32) {
-    const Product p{A, W, (float*)C, scratch, M, N, K, lda, ldw, ldc, sm_count < 1 ? 1 : sm_count, stream};
+    const Product p{A, W, (float*)C, scratch, M, N, K, lda, ldw, ldc, sm_count < 1 ? 1 : sm_count, early_weights != 0, stream};
     if (p.tma() && (scratch || lb_gemm_simt_scratch(M, N, K, p.sm_count) == 0 || M > FT_M)) {
       if (M <= 2) return launch_few<2>(p);
       if (M <= 4) return launch_few<4>(p);

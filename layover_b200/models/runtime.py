@@ -16,7 +16,7 @@ from ..parts.base import Runtime
 
 def _linear_f32(a: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch.Tensor:
     out = torch.empty((a.shape[0], w.shape[0]), dtype=torch.float32, device=a.device)
-    return ops.gemm_simt(a, w, out)
+    return ops.gemm_simt(a, w, out, early_weights=True)      # a model's weights: no kernel writes them
 
 
 def _linear_bf16(a: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch.Tensor:

@@ -1095,10 +1095,12 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, w: torch.Tenso
 
 
 # ------------------------------------------------------------------ matrix products
-def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, early_weights: bool = False) -> torch.Tensor:
     """out[M, N] = a[M, K] @ w[N, K]^T with 32-bit FFMA accumulation (no tensor cores).
 
-    a and w share a dtype (float32 or bfloat16); out has it too, or float32. Rows may be strided."""
+    a and w share a dtype (float32 or bfloat16); out has it too, or float32. Rows may be strided. `early_weights`: no
+    kernel that may still be running on this stream writes w (a model's weights), so that it may be read before that
+    kernel has ended."""
     if a.dtype != w.dtype or a.dim() != 2 or w.dim() != 2 or out.dim() != 2:
         raise ValueError("gemm: operands must be 2-D and share a dtype")
     m, k = a.shape
@@ -1113,9 +1115,9 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tens
         wanted = (_FUNCTIONS.get("lb_gemm_simt_scratch") or _fn("gemm_simt", "lb_gemm_simt_scratch", [c_int] * 4, c_long))(m, n, k, sm_count(a.device))
         scratch = torch.empty(wanted, dtype=torch.float32, device=a.device) if wanted else None
     fn = _FUNCTIONS.get("lb_gemm_simt") or _fn("gemm_simt", "lb_gemm_simt",
-             [c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_long, c_long, c_long, c_void_p, c_int, c_void_p])
+             [c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_long, c_long, c_long, c_void_p, c_int, c_int, c_void_p])
     _check(fn(dtype_code(a.dtype), dtype_code(out.dtype), a_ptr, w_ptr, out_ptr, m, n, k, a.stride(0),
-              w.stride(0), out.stride(0), _ptr(scratch), sm_count(a.device), _stream()), "gemm_simt")
+              w.stride(0), out.stride(0), _ptr(scratch), sm_count(a.device), int(early_weights), _stream()), "gemm_simt")
     if scratch is not None:
         global LAUNCHES
         LAUNCHES += 1          # the ranges' sums are added by a kernel of their own

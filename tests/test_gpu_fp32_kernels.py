@@ -69,3 +69,21 @@ def test_f32_attention_split_over_blocks_has_the_bits_of_one_block(dtype, q_head
                 # scores of dim / 4 + 4 sums of terms below 12 in all, weights and their sums within as much, values below 6
                 tolerance = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -24 * (dim / 4 + 16) * 12
                 assert ((got - expected).abs() <= 6 * tolerance).all()
+
+
+@pytest.mark.parametrize("tokens", [1, 4, 16, 40])
+def test_f32_product_of_weights_that_the_kernel_before_wrote(tokens):
+    """Without `early_weights` the weights may be another kernel's output, in the same stream and a moment ago."""
+    o, n, k = ops(), 256, 2048
+    gen = torch.Generator().manual_seed(tokens)
+    a, first, second = torch.randn(tokens, k, generator=gen).cuda(), *(torch.randn(n, k, generator=gen).cuda() for _ in range(2))
+    wants = []
+    for w in (first, second):
+        wants.append(torch.empty(tokens, n, device="cuda"))
+        o.gemm_simt(a, w, wants[-1])
+    w, outs = torch.empty_like(first), [torch.empty(tokens, n, device="cuda") for _ in range(40)]
+    torch.cuda.synchronize()
+    for i, out in enumerate(outs):
+        o.lower_rows((first, second)[i % 2], w)
+        o.gemm_simt(a, w, out)
+    assert all(torch.equal(out, wants[i % 2]) for i, out in enumerate(outs))

@@ -7,7 +7,7 @@
 // depend on K alone; a range is one sequential chain of fused multiply-adds from zero, the sums of four neighbouring ranges
 // are added in order, and then the sums of those groups are. Ranges may therefore run one after the other, in the lanes
 // of a warp or in different blocks, with the same bits. For bf16 operands there is one chain over the whole of K. Any M, N, K >= 1 is accepted: operands whose
-// address and stride TMA can take go through the streaming kernels, others through the plain tiles.
+// address and stride TMA can take go through the streaming kernels, others through the plain tiles, with the same bits.
 #include "common.cuh"
 #include "tcgen05.cuh"
 
@@ -51,53 +51,62 @@ __device__ __forceinline__ void load_slab(const T* __restrict__ base, long ld, i
   for (int j = 0; j < 4; ++j) dst[kk + j][r] = v[j];
 }
 
-template <typename TA, typename TC>
-__global__ void __launch_bounds__(THREADS)
+// RANGES: sums over the ranges of `Split` (of `range_length` k each); what a thread keeps between them lies in shared memory, where
+// it costs no registers: 261 tokens x 6,144 x 2,561 (rows that TMA does not take) 564 us, in registers 642, one chain of K 530.
+template <typename TA, typename TC, bool RANGES = false>
+__global__ void __launch_bounds__(THREADS, RANGES ? 5 : 0)
 gemm_simt_kernel(const TA* __restrict__ A, const TA* __restrict__ W, TC* __restrict__ C, int M, int N, int K,
-                 long lda, long ldw, long ldc, bool vec_a, bool vec_w, int range_steps) {
+                 long lda, long ldw, long ldc, bool vec_a, bool vec_w, int range_length) {
   __shared__ float As[TILE_K][TILE_M + 4];
   __shared__ float Ws[TILE_K][TILE_N + 4];
+  __shared__ float kept[RANGES ? 2 * TM * TN : 1][RANGES ? THREADS : 1];     // of the group's ranges before, of the groups before
   pdl_launch_dependents();
   pdl_wait();
   const int m0 = blockIdx.y * TILE_M, n0 = blockIdx.x * TILE_N;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  // of the current range of K (`range_steps` slabs; 0: one range), of the group's ranges before it, of the groups before
-  float acc[TM][TN], group[TM][TN], total[TM][TN];
+  float acc[TM][TN];                      // of the current range of K
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
 
-  int steps = 0, range = 0;
-  for (int k0 = 0; k0 < K; k0 += TILE_K) {
-    load_slab<TA>(A, lda, m0, M, k0, K, vec_a, As);
-    load_slab<TA>(W, ldw, n0, N, k0, K, vec_w, Ws);
-    __syncthreads();
+  int k0 = 0;
+  for (int range = 0; k0 < K; ++range) {
+    const int end = RANGES ? min(K, k0 + range_length) : K;
+    for (; k0 < end; k0 += TILE_K) {
+      load_slab<TA>(A, lda, m0, M, k0, K, vec_a, As);
+      load_slab<TA>(W, ldw, n0, N, k0, K, vec_w, Ws);
+      __syncthreads();
 #pragma unroll
-    for (int k = 0; k < TILE_K; ++k) {
-      float a[TM], w[TN];
+      for (int k = 0; k < TILE_K; ++k) {
+        float a[TM], w[TN];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = As[k][ty * TM + i];
+        for (int i = 0; i < TM; ++i) a[i] = As[k][ty * TM + i];
 #pragma unroll
-      for (int j = 0; j < TN; ++j) w[j] = Ws[k][tx * TN + j];
+        for (int j = 0; j < TN; ++j) w[j] = Ws[k][tx * TN + j];
 #pragma unroll
-      for (int i = 0; i < TM; ++i)
+        for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+          for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+      }
+      __syncthreads();
     }
-    __syncthreads();
-    if (++steps == range_steps || k0 + TILE_K >= K) {
+    if (!RANGES) break;
+    const bool last = k0 >= K;
 #pragma unroll
-      for (int i = 0; i < TM; ++i)
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) {
-          group[i][j] = range % 4 ? group[i][j] + acc[i][j] : acc[i][j];
-          if (range % 4 == 3 || k0 + TILE_K >= K) total[i][j] = range < 4 ? group[i][j] : total[i][j] + group[i][j];
-          acc[i][j] = 0.f;
+      for (int j = 0; j < TN; ++j) {
+        float *group = &kept[i * TN + j][threadIdx.x], *total = &kept[TM * TN + i * TN + j][threadIdx.x];
+        float sum = range % 4 ? *group + acc[i][j] : acc[i][j];
+        if (range % 4 == 3 || last) {
+          if (range >= 4) sum = *total + sum;
+          *total = sum;
+        } else {
+          *group = sum;
         }
-      steps = 0;
-      ++range;
-    }
+        acc[i][j] = last ? sum : 0.f;
+      }
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
@@ -106,7 +115,7 @@ gemm_simt_kernel(const TA* __restrict__ A, const TA* __restrict__ W, TC* __restr
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
       const int col = n0 + tx * TN + j;
-      if (col < N) Elem<TC>::store(C + (long)row * ldc + col, total[i][j]);
+      if (col < N) Elem<TC>::store(C + (long)row * ldc + col, acc[i][j]);
     }
   }
 }
@@ -191,7 +200,7 @@ template <typename T> bool vec_ok(const void* p, long ld) {
 // ------------------------------------------------------------------ 32-bit operands
 __device__ int g_gemm_simt_error = 0;   // 0 = ok; a wait for a copy ran out in 1 the few-token kernel, 2 the many-token kernel
 
-// The ranges of K: four to 32 of them, whole stages long. Four ranges are a group: the sums of a group's ranges are added in
+// The ranges of K: up to 32 of them, whole stages long. Four ranges are a group: the sums of a group's ranges are added in
 // order, and then the groups' sums are.
 constexpr int STAGE_K = 32;             // 128 bytes of a row
 constexpr int GROUP = 4;
@@ -208,6 +217,73 @@ struct Split {
 // The 16 bytes of k .. k + 3 in row `row` of a tile of 128-byte rows as TMA's 128-byte swizzle leaves them.
 __device__ __forceinline__ float4 swizzled(const float* tile, int row, int k) {
   return *reinterpret_cast<const float4*>(tile + row * STAGE_K + (((k >> 2) ^ (row & 7)) << 2));
+}
+
+// Up to 16 tokens without TMA (rows or addresses that it does not take) and for short K, where the few-token kernel's cluster and
+// rings cost more than they bring: tiles of 16 tokens x 16 weight rows, a thread owns one weight row and two tokens. Slabs of 32 k
+// come by 4-byte asynchronous copies, PLAIN_STAGES - 1 of them on their way; what bounds it are the reads of shared memory, three for
+// two multiply-adds.
+// Measured (one B200, 8 tokens, K 2,561, which TMA does not take): 1,024 rows 35 us, 2,560 50, 6,144 88; one slab in registers ahead of
+// the other 47, 55 and 85, the 64 x 64 tiles 192, 193 and 226.
+constexpr int PLAIN_STAGES = 4;
+__device__ __forceinline__ void copy_float(float* dst, const float* src, bool there) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(there ? 4 : 0) : "memory");
+}
+
+__global__ void __launch_bounds__(FT_THREADS)
+gemm_f32_plain_few_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K, long lda,
+                          long ldw, long ldc) {
+  __shared__ float As[PLAIN_STAGES][FT_K][FT_M + 1];
+  __shared__ float Ws[PLAIN_STAGES][FT_K][FT_N + 1];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int n0 = blockIdx.x * FT_N, slabs = (K + FT_K - 1) / FT_K, range_slabs = Split(K).length / FT_K;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;        // a warp copies four rows of a slab, a lane one k of each
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;           // weight row of the tile, pair of tokens
+  auto copy_slab = [&](int i) {                                     // what lies beyond K or the rows becomes zeros
+    if (i < slabs) {
+      const int buf = i % PLAIN_STAGES, k = i * FT_K + lane, k_at = min(k, K - 1);
+#pragma unroll
+      for (int j = 0; j < FT_M / 4; ++j) {
+        const int r = warp * (FT_M / 4) + j;
+        copy_float(&As[buf][lane][r], A + min(r, M - 1) * lda + k_at, r < M && k < K);
+        copy_float(&Ws[buf][lane][r], W + min(n0 + r, N - 1) * ldw + k_at, n0 + r < N && k < K);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < PLAIN_STAGES - 1; ++i) copy_slab(i);
+  float acc[2] = {0.f, 0.f}, group[2] = {0.f, 0.f}, total[2] = {0.f, 0.f};
+  int range = 0, left = range_slabs;
+  for (int i = 0; i < slabs; ++i) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(PLAIN_STAGES - 2) : "memory");
+    __syncthreads();                                                // the slab is there, and the one before is read
+    copy_slab(i + PLAIN_STAGES - 1);
+    const int buf = i % PLAIN_STAGES;
+#pragma unroll
+    for (int k = 0; k < FT_K; ++k) {
+      const float w = Ws[buf][k][tx];
+      acc[0] = fmaf(As[buf][k][2 * ty], w, acc[0]);
+      acc[1] = fmaf(As[buf][k][2 * ty + 1], w, acc[1]);
+    }
+    if (--left == 0 || i + 1 == slabs) {
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        group[t] = range % GROUP ? group[t] + acc[t] : acc[t];
+        if (range % GROUP == GROUP - 1 || i + 1 == slabs) total[t] = range < GROUP ? group[t] : total[t] + group[t];
+        acc[t] = 0.f;
+      }
+      left = range_slabs;
+      ++range;
+    }
+  }
+  const int col = n0 + tx;
+  if (col < N) {
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+      if (2 * ty + t < M) C[(2 * ty + t) * ldc + col] = total[t];
+  }
 }
 
 // After a wait that ran out: copies still in flight get time to land before the block's memory goes away.
@@ -510,6 +586,8 @@ struct Product {
   bool tma() const {      // 16-byte aligned addresses and row strides
     return (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0 && lda % 4 == 0 && ldw % 4 == 0 && lda >= K && ldw >= K;
   }
+  bool streams() const;   // whether the streaming kernels take it
+  long scratch() const;   // floats for the ranges' sums in their form of it
 };
 
 int sum_groups(const Product& p) {
@@ -554,6 +632,26 @@ int many_parts(int M, int N, int K, int sm_count) {
   return parts < groups ? (int)parts : groups;
 }
 
+constexpr long SCRATCH_FLOATS = 64L << 20;       // the most that the ranges' sums may take (256 MiB); beyond, a block walks all of K
+
+long Product::scratch() const {
+  const long floats = (long)Split(K).groups() * M * N;
+  if (M <= FT_M) return lb_cluster_reduce_enabled() ? 0 : floats;
+  return many_parts(M, N, K, sm_count) > 1 && floats <= SCRATCH_FLOATS ? floats : 0;
+}
+
+// Short products are the plain tiles': the streaming kernels' rings and clusters take 2.8 us (2 tokens) to 5.6 us (16) before they
+// bring anything, where the plain few-token kernel takes 1.6 us and as long again for every 2,560 x 64 weights. Where both take as
+// long (us, plain and streaming): 2 tokens, 1,024 x 128 2.6 and 3.4, 2,560 x 96 3.2 and 3.4, 9,728 x 32 3.0 and 3.7; 4 tokens,
+// 1,024 x 512 7.1 and 7.4, 2,560 x 256 5.9 and 5.4; 8 tokens, 1,024 x 1,024 13.1 and 16.9, 2,560 x 512 10.4 and 11.0, 9,728 x 128
+// 8.4 and 7.4. Beyond 16 tokens the streaming kernel is ahead from one stage on (2,560 x 32, 32 tokens: 3.8 and 2.8).
+bool Product::streams() const {
+  if (!tma()) return false;
+  if (M > FT_M) return K >= STAGE_K;
+  const long limit = M <= 2 ? 1L << 17 : (M <= 4 ? 1L << 19 : 1L << 20);
+  return (long)K * (N > 1024 ? N : 1024) > limit;
+}
+
 template <int TM>
 int launch_many(const Product& p) {
   using T = Many<TM>;
@@ -586,11 +684,12 @@ LB_EXPORT int lb_gemm_simt_status() {
   return code;
 }
 
-// Floats of scratch that a product of 32-bit operands wants (0: none), for the ranges' sums.
-LB_EXPORT long lb_gemm_simt_scratch(int M, int N, int K, int sm_count) {
+// Floats of scratch that a product of 32-bit operands wants for the ranges' sums in the form that it will take (0: none, one
+// launch; else a second one adds them up).
+LB_EXPORT long lb_gemm_simt_scratch(const void* A, const void* W, int M, int N, int K, long lda, long ldw, int sm_count) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const bool wanted = M <= FT_M ? !lb_cluster_reduce_enabled() : many_parts(M, N, K, sm_count) > 1;
-  return wanted ? (long)Split(K).groups() * M * N : 0;
+  const Product p{A, W, nullptr, nullptr, M, N, K, lda, ldw, N, sm_count < 1 ? 1 : sm_count, false, nullptr};
+  return p.streams() ? p.scratch() : 0;
 }
 
 // in_dtype: type of A and W; out_dtype: type of C (bf16 inputs may write 32-bit floats). `scratch`: null, or as many floats as
@@ -602,7 +701,7 @@ LB_EXPORT int lb_gemm_simt(int in_dtype, int out_dtype, const void* A, const voi
   if (K <= 0) return LB_ERR_SIZE;
   if (in_dtype == LB_F32 && out_dtype == LB_F32) {
     const Product p{A, W, (float*)C, scratch, M, N, K, lda, ldw, ldc, sm_count < 1 ? 1 : sm_count, early_weights != 0, stream};
-    if (p.tma() && (scratch || lb_gemm_simt_scratch(M, N, K, p.sm_count) == 0 || M > FT_M)) {
+    if (p.streams() && (scratch || M > FT_M || !p.scratch())) {
       if (M <= 2) return launch_few<2>(p);
       if (M <= 4) return launch_few<4>(p);
       if (M <= 8) return launch_few<8>(p);
@@ -610,12 +709,14 @@ LB_EXPORT int lb_gemm_simt(int in_dtype, int out_dtype, const void* A, const voi
       return wide_tiles(M) ? launch_many<8>(p) : launch_many<4>(p);
     }
   }
-  if (M <= FT_M && in_dtype == LB_BF16) {
+  if (M <= FT_M) {
     dim3 few((N + FT_N - 1) / FT_N, 1);
-    if (out_dtype == LB_BF16)
+    if (in_dtype == LB_F32 && out_dtype == LB_F32)
+      lb_launch(gemm_f32_plain_few_kernel, few, FT_THREADS, 0, stream, (const float*)A, (const float*)W, (float*)C, M, N, K, lda, ldw, ldc);
+    else if (in_dtype == LB_BF16 && out_dtype == LB_BF16)
       lb_launch(gemm_simt_fewtoken_kernel<bf16, bf16>, few, FT_THREADS, 0, stream, (const bf16*)A, (const bf16*)W, (bf16*)C, M, N,
                 K, lda, ldw, ldc, vec_ok<bf16>(A, lda), vec_ok<bf16>(W, ldw));
-    else if (out_dtype == LB_F32)
+    else if (in_dtype == LB_BF16 && out_dtype == LB_F32)
       lb_launch(gemm_simt_fewtoken_kernel<bf16, float>, few, FT_THREADS, 0, stream, (const bf16*)A, (const bf16*)W, (float*)C, M,
                 N, K, lda, ldw, ldc, vec_ok<bf16>(A, lda), vec_ok<bf16>(W, ldw));
     else
@@ -625,9 +726,9 @@ LB_EXPORT int lb_gemm_simt(int in_dtype, int out_dtype, const void* A, const voi
   dim3 grid((N + TILE_N - 1) / TILE_N, (M + TILE_M - 1) / TILE_M);
   if (grid.y > 65535) return LB_ERR_SIZE;
   if (in_dtype == LB_F32 && out_dtype == LB_F32)
-    lb_launch(gemm_simt_kernel<float, float>, grid, THREADS, 0, stream, (const float*)A, (const float*)W, (float*)C, M, N, K,
+    lb_launch(gemm_simt_kernel<float, float, true>, grid, THREADS, 0, stream, (const float*)A, (const float*)W, (float*)C, M, N, K,
                                                                  lda, ldw, ldc, vec_ok<float>(A, lda),
-                                                                 vec_ok<float>(W, ldw), Split(K).length / TILE_K);
+                                                                 vec_ok<float>(W, ldw), Split(K).length);
   else if (in_dtype == LB_BF16 && out_dtype == LB_BF16)
     lb_launch(gemm_simt_kernel<bf16, bf16>, grid, THREADS, 0, stream, (const bf16*)A, (const bf16*)W, (bf16*)C, M, N, K, lda,
                                                                ldw, ldc, vec_ok<bf16>(A, lda), vec_ok<bf16>(W, ldw), 0);

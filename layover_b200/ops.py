@@ -1112,7 +1112,9 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, early_weights
     a_ptr, w_ptr, out_ptr = _ptr(a), _ptr(w), _ptr(out)        # refuses other devices, before theirs is asked about
     scratch = None
     if a.dtype == torch.float32 and min(m, n, k) > 0:      # partial sums of this call alone, on its own stream
-        wanted = (_FUNCTIONS.get("lb_gemm_simt_scratch") or _fn("gemm_simt", "lb_gemm_simt_scratch", [c_int] * 4, c_long))(m, n, k, sm_count(a.device))
+        plan = _FUNCTIONS.get("lb_gemm_simt_scratch") or _fn("gemm_simt", "lb_gemm_simt_scratch",
+                                                             [c_void_p] * 2 + [c_int] * 3 + [c_long] * 2 + [c_int], c_long)
+        wanted = plan(_ptr(a), _ptr(w), m, n, k, a.stride(0), w.stride(0), sm_count(a.device))
         scratch = torch.empty(wanted, dtype=torch.float32, device=a.device) if wanted else None
     fn = _FUNCTIONS.get("lb_gemm_simt") or _fn("gemm_simt", "lb_gemm_simt",
              [c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_long, c_long, c_long, c_void_p, c_int, c_int, c_void_p])

@@ -87,3 +87,59 @@ def test_f32_product_of_weights_that_the_kernel_before_wrote(tokens):
         o.lower_rows((first, second)[i % 2], w)
         o.gemm_simt(a, w, out)
     assert all(torch.equal(out, wants[i % 2]) for i, out in enumerate(outs))
+
+
+@pytest.mark.parametrize("tokens", [1, 2, 3, 4, 5, 16])
+@pytest.mark.parametrize("n, k", [(1, 1), (15, 31), (17, 33), (33, 129), (40, 1028), (100, 4100), (16, 8200), (2600, 64), (2049, 512)])
+def test_f32_product_of_a_few_tokens_has_the_same_bits_with_and_without_tma(tokens, n, k):
+    """Rows that TMA takes and rows that begin one float further; K on both sides of where the streaming kernel takes over."""
+    gen = torch.Generator().manual_seed(n * 10007 + k)
+    wide_a, wide_w = torch.zeros(40, -(-k // 4) * 4 + 4, device="cuda"), torch.zeros(n, -(-k // 4) * 4 + 4, device="cuda")
+    a, w, outs = torch.randn(40, k, generator=gen).cuda(), torch.randn(n, k, generator=gen).cuda(), []
+    for shift in (0, 1):
+        x, y = wide_a[:, shift: shift + k], wide_w[:, shift: shift + k]
+        x.copy_(a); y.copy_(w)
+        for rows in (tokens, 40):              # 40: the tiles of many tokens
+            outs.append(torch.empty(rows, n, device="cuda"))
+            ops().gemm_simt(x[:rows], y, outs[-1])
+    assert all(torch.equal(outs[0], out[:tokens]) for out in outs[1:])
+    bound = (k / 4 + 44) * 2.0 ** -24 * (a[:tokens].abs().double() @ w.abs().double().T)      # as above
+    assert ((outs[0].double() - a[:tokens].double() @ w.double().T).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("m, n, k", [(1, 70, 9728), (16, 33, 2560), (40, 100, 4100), (600, 2400, 2500), (130, 2560, 9728), (513, 19456, 1100)])
+def test_f32_product_says_how_much_scratch_its_form_takes(m, n, k):
+    """Groups of ranges dealt out one, several or all to a block: the bits of row slices; scratch, and a second launch, only
+    where the form that runs has one."""
+    o, gen = ops(), torch.Generator().manual_seed(m + n)
+    launches = lambda x, out: (lambda before: (o.gemm_simt(x, w, out), o.LAUNCHES - before)[1])(o.LAUNCHES)
+    a, w = torch.randn(m, k, generator=gen).cuda(), torch.randn(n, k, generator=gen).cuda()
+    full, part, few = torch.empty(m, n, device="cuda"), torch.empty(17, n, device="cuda"), torch.empty(3, n, device="cuda")
+    plan = lambda rows, shift=0: o._FUNCTIONS["lb_gemm_simt_scratch"](a.data_ptr() + 4 * shift, w.data_ptr(), rows, n, k, k, k, 148)
+    assert launches(a, full) == (2 if plan(m) else 1) and plan(m, 1) == 0
+    assert plan(m) <= 64 << 20 and (m > 16 or plan(m) == 0)
+    if m >= 17:
+        o.gemm_simt(a[m - 17:], w, part)
+        assert torch.equal(part, full[m - 17:])
+    if m >= 3:
+        o.gemm_simt(a[:3], w, few)
+        assert torch.equal(few, full[:3])
+    rows = slice(0, min(m, 20))
+    bound = (k / 4 + 44) * 2.0 ** -24 * (a[rows].abs().double() @ w.abs().double().T)
+    assert ((full[rows].double() - a[rows].double() @ w.double().T).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("m", [1, 7, 16])
+def test_f32_product_sums_through_scratch_where_clusters_are_off(m):
+    """The form without clusters, asked for through the exported function with scratch of its size: the same bits."""
+    import ctypes
+
+    o, n, k = ops(), 100, 9728
+    gen = torch.Generator().manual_seed(m)
+    a, w = torch.randn(m, k, generator=gen).cuda(), torch.randn(n, k, generator=gen).cuda()
+    want, got = torch.empty(m, n, device="cuda"), torch.full((m, n), float("nan"), device="cuda")
+    o.gemm_simt(a, w, want)
+    scratch = torch.full((8 * m * n,), float("nan"), device="cuda")
+    code = o._FUNCTIONS["lb_gemm_simt"](0, 0, a.data_ptr(), w.data_ptr(), got.data_ptr(), m, n, k, k, k, n, scratch.data_ptr(), 148, 0,
+                                        torch.cuda.current_stream().cuda_stream)
+    assert code == 0 and torch.equal(got, want)

@@ -782,14 +782,14 @@ def topidra_kernels(pk: dict) -> dict:
         gated = torch.empty(tokens, n, device=dev, dtype=bf)
         wn = torch.ones(n, device=dev)
         name = f"decay_scan_{'prompt2048' if seqs == 1 else f'decode_b{seqs}'}"
-        seg_tokens, segments = ops.scan_segments([tokens // seqs] * seqs, 4 * heads * dim * dim, dim)     # as the mixer runs it
+        seg_tokens, segments, products = ops.scan_plan([tokens // seqs] * seqs, heads, dim, dim, proj[0].dtype)     # as the mixer runs it
         scratch = torch.empty(segments, heads, dim, dim, device=dev) if segments else None
         if segments:
             point(name + "_single_pass", lambda i: ops.decay_scan(proj[i % ROT], 0, n, 2 * n, scanned, state[i % ROT], cu, slots,
                                                                   decay, seqs, heads, dim, dim, "silu"), ROT,
                   flops=4.0 * tokens * heads * dim * dim, peak_flops=FP32_TFLOPS * 1e12)
         point(name, lambda i: ops.decay_scan(proj[i % ROT], 0, n, 2 * n, scanned, state[i % ROT], cu, slots, decay, seqs, heads,
-                                             dim, dim, "silu", seg_tokens, scratch), ROT,
+                                             dim, dim, "silu", seg_tokens, scratch, products), ROT,
               nbytes=tokens * n * (3 * 2 + 4) + 2 * seqs * heads * dim * dim * 4,
               flops=4.0 * tokens * heads * dim * dim, peak_flops=FP32_TFLOPS * 1e12)
         point(f"gated_rmsnorm_{tokens}", lambda i: ops.gated_rmsnorm(scanned, proj[i % ROT][:, 3 * n:], wn, 1e-6, gated), ROT,
@@ -1252,10 +1252,10 @@ def kirenex_kernels(pk: dict) -> dict:
         lstate = torch.zeros(ROT, seqs + 1, heads, dim, dim, device=dev)
         slots = torch.arange(seqs, dtype=torch.int32, device=dev)
         decay = torch.full((heads,), 0.99, device=dev)
-        seg_tokens, segments = ops.scan_segments([per] * seqs, 4 * heads * dim * dim, dim)
+        seg_tokens, segments, products = ops.scan_plan([per] * seqs, heads, dim, dim, projb[0].dtype)
         scratch = torch.empty(segments, heads, dim, dim, device=dev) if segments else None
         point(f"like:decay_scan_{tag}", lambda i: ops.decay_scan(projb[i % ROT], 0, n, 2 * n, scanned, lstate[i % ROT], cu, slots, decay,
-                                                               seqs, heads, dim, dim, "silu", seg_tokens, scratch), ROT,
+                                                               seqs, heads, dim, dim, "silu", seg_tokens, scratch, products), ROT,
               nbytes=tokens * n * (3 * 2 + 4) + 2 * seqs * floats * 4, flops=4.0 * tokens * heads * dim * dim,
               peak_flops=FP32_TFLOPS * 1e12)
         if segments:
@@ -1503,10 +1503,10 @@ def vopozen_kernels(pk: dict) -> dict:
         lstate = torch.zeros(ROT, seqs + 1, heads, dim, dim, device=dev)
         lslots = torch.arange(seqs, dtype=torch.int32, device=dev)
         ldecay = torch.full((heads,), 0.99, device=dev)
-        seg_tokens, segments = ops.scan_segments([per] * seqs, 4 * heads * dim * dim, dim)
+        seg_tokens, segments, products = ops.scan_plan([per] * seqs, heads, dim, dim, projb[0].dtype)
         scratch = torch.empty(segments, heads, dim, dim, device=dev) if segments else None
         point(f"like:decay_scan_{tag}", lambda i: ops.decay_scan(projb[i % ROT], 0, n, 2 * n, scanned, lstate[i % ROT], cu, lslots, ldecay,
-                                                               seqs, heads, dim, dim, "silu", seg_tokens, scratch), ROT,
+                                                               seqs, heads, dim, dim, "silu", seg_tokens, scratch, products), ROT,
               nbytes=tokens * n * (3 * 2 + 4) + 2 * seqs * floats * 4, flops=4.0 * tokens * heads * dim * dim,
               peak_flops=FP32_TFLOPS * 1e12)
         if segments:
@@ -1817,10 +1817,10 @@ def fimilix_kernels(pk: dict) -> dict:
               nbytes=tokens * (channels + n) * 4 + 2 * seqs * floats * 4, flops=6.0 * tokens * heads * dim * dim, peak_flops=FP32_TFLOPS * 1e12)
         projb = [torch.randn(tokens, 4 * n, device=dev, dtype=bf) for _ in range(ROT)]
         ldecay = torch.full((heads,), 0.99, device=dev)
-        seg_tokens, segments = ops.scan_segments([per] * seqs, 4 * floats, dim)
+        seg_tokens, segments, products = ops.scan_plan([per] * seqs, heads, dim, dim, projb[0].dtype)
         scratch = torch.empty(segments, heads, dim, dim, device=dev) if segments else None
         point(f"like:decay_scan_{tag}", lambda i: ops.decay_scan(projb[i % ROT], 0, n, 2 * n, scanned, state[i % ROT], cu, batch.state_slots, ldecay,
-                                                               seqs, heads, dim, dim, "silu", seg_tokens, scratch), ROT,
+                                                               seqs, heads, dim, dim, "silu", seg_tokens, scratch, products), ROT,
               nbytes=tokens * n * (3 * 2 + 4) + 2 * seqs * floats * 4, flops=4.0 * tokens * heads * dim * dim, peak_flops=FP32_TFLOPS * 1e12)
         del proj, projb, state, dstate, wstate, lora
 

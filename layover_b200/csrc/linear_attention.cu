@@ -23,14 +23,14 @@
 // RANGES and DPT depend on the head size only, never on the batch.
 //
 // A long portion of one sequence is a long chain for few blocks. Steps that hold one (the host decides from the step's
-// longest portion) run in three launches instead: every sequence's portion is cut into segments of `seg_tokens`. With head
-// sizes of 33 to 128 what a segment of n tokens does is written as products of matrices, S_in the state that comes in:
+// longest portion) run in three launches instead: every sequence's portion is cut into segments of `seg_tokens`. `products`:
+// what a segment of n tokens does is written as products of matrices, S_in the state that comes in:
 //
 //   E     = sum_j decay^(n-1-j) k_j v_j^T                                      `segment_state_kernel`
 //   S_in of the next segment = decay^n S_in + E, in order, the last one to the slot          `scan_combine_kernel`
 //   o_i   = decay^(i+1) S_in^T q_i + sum_(j<=i) decay^(i-j) (q_i . k_j) v_j     `segment_output_kernel`
 //
-// With other head sizes MODE 1 scans every segment at once, a sequence's first segment from the slot's state and the others
+// Else MODE 1 scans every segment at once, a sequence's first segment from the slot's state and the others
 // from zero, and leaves each segment's end state in `seg_state`; the combine kernel leaves S_in(s) where segment s finds
 // it (in the place of the segment before); MODE 2 adds decay^(t+1) S_in^T q_t. Either way everything is 32-bit on the FFMA
 // pipes and the sums are the same numbers in another order: results agree with the single pass within rounding, not bit
@@ -220,7 +220,7 @@ __global__ void scan_combine_kernel(float* __restrict__ seg_state, float* __rest
   *slot = running;
 }
 
-// ------------------------------------------------------------------ segments as matrix products (head sizes of 33 to 128)
+// ------------------------------------------------------------------ segments as matrix products (head sizes up to 128)
 constexpr int SEG_THREADS = 256, SEG_ROWS = 64, SEG_PITCH = 132, SEG_STEP = 16;
 
 // Which tokens a block of the grid's z belongs to.
@@ -524,15 +524,13 @@ int launch_scan(int n_seqs, int total_segments, int seg_tokens, float* seg_state
 template <typename T>
 int dispatch_scan(int act, int n_seqs, int total_segments, int seg_tokens, float* seg_state, cudaStream_t stream,
                   const void* proj, long row_stride, int q_off, int k_off, int v_off, float* out, float* state,
-                  const int* cu_q, const int* state_slots, const float* decay, int heads, int dim, int vdim) {
+                  const int* cu_q, const int* state_slots, const float* decay, int heads, int dim, int vdim, bool products) {
 #define LB_SCAN(R, D)                                                                                                        \
   (act == 1 ? launch_scan<T, R, D, 1>(n_seqs, total_segments, seg_tokens, seg_state, stream, proj, row_stride, q_off, k_off, \
                                       v_off, out, state, cu_q, state_slots, decay, heads, dim, vdim)                         \
             : launch_scan<T, R, D, 0>(n_seqs, total_segments, seg_tokens, seg_state, stream, proj, row_stride, q_off, k_off, \
                                       v_off, out, state, cu_q, state_slots, decay, heads, dim, vdim))
-  // With heads of 33 to 128 the tiles of 128 x 128 of the segments' matrix products are mostly full; smaller heads would
-  // leave most of them empty, and larger ones do not fit a block's shared memory.
-  if (total_segments > 0 && dim > 32 && dim <= 128) {
+  if (total_segments > 0 && products) {
     if (act == 1)
       return launch_segments<T, 1>(n_seqs, total_segments, seg_tokens, seg_state, stream, proj, row_stride, q_off, k_off, v_off, out, state,
                                    cu_q, state_slots, decay, heads, dim, vdim);
@@ -586,22 +584,24 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ x, const T* __res
 // proj [tokens, row_stride] holds q at q_off (heads * dim), k at k_off (heads * dim), v at v_off (heads * vdim);
 // out float [tokens, heads * vdim]; state float [slots, heads, dim, vdim]; decay float [heads]; act 0 none, 1 silu.
 // total_segments > 0: the three-launch form for steps with long portions; seg_state float
-// [total_segments, heads, dim, vdim], total_segments = sum over sequences of max(1, ceil(tokens / seg_tokens)).
+// [total_segments, heads, dim, vdim], total_segments = sum over sequences of max(1, ceil(tokens / seg_tokens)). products: the
+// segments as matrix products (head sizes up to 128), else they walk their tokens.
 LB_EXPORT int lb_decay_scan(int dtype, const void* proj, long row_stride, int q_off, int k_off, int v_off, float* out,
                             float* state, const int* cu_q, const int* state_slots, const float* decay, int n_seqs,
                             int heads, int dim, int vdim, int act, float* seg_state, int seg_tokens, int total_segments,
-                            cudaStream_t stream) {
+                            int products, cudaStream_t stream) {
   if (n_seqs <= 0) return 0;
+  if (products && dim > 128) return LB_ERR_SIZE;         // a block's shared memory holds 64 rows of 128 channels
   if (heads <= 0 || heads > 65535 || n_seqs > 65535 || dim <= 0 || dim > 256 || vdim <= 0 || act < 0 || act > 1)
     return LB_ERR_SIZE;
   if (total_segments > 0 && (!seg_state || seg_tokens <= 0 || total_segments < n_seqs || total_segments > 65535))
     return LB_ERR_SIZE;
   if (dtype == LB_F32)
     return dispatch_scan<float>(act, n_seqs, total_segments, seg_tokens, seg_state, stream, proj, row_stride, q_off, k_off,
-                                v_off, out, state, cu_q, state_slots, decay, heads, dim, vdim);
+                                v_off, out, state, cu_q, state_slots, decay, heads, dim, vdim, products != 0);
   if (dtype == LB_BF16)
     return dispatch_scan<bf16>(act, n_seqs, total_segments, seg_tokens, seg_state, stream, proj, row_stride, q_off, k_off,
-                               v_off, out, state, cu_q, state_slots, decay, heads, dim, vdim);
+                               v_off, out, state, cu_q, state_slots, decay, heads, dim, vdim, products != 0);
   return LB_ERR_DTYPE;
 }
 

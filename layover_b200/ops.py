@@ -725,7 +725,7 @@ SCAN_ACTIVATIONS = {None: 0, "none": 0, "silu": 1}
 def decay_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, out: torch.Tensor, state: torch.Tensor,
                cu_q: torch.Tensor, state_slots: torch.Tensor, decay: torch.Tensor, n_seqs: int, heads: int, dim: int,
                vdim: int, activation: str | None = None, segment_tokens: int = 0,
-               segment_state: torch.Tensor | None = None) -> torch.Tensor:
+               segment_state: torch.Tensor | None = None, products: bool | None = None) -> torch.Tensor:
     """Per sequence and head S_t = decay_h S_(t-1) + k_t v_t^T, o_t = S_t^T q_t over the step's tokens, from and
     to the requests' state slots.
 
@@ -736,7 +736,8 @@ def decay_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, out: torc
     With `segment_tokens` > 0 every sequence's tokens are cut into segments of that many that are scanned at once
     (three launches; for steps with long portions, where one chain per sequence and head would leave most of
     the device idle): `segment_state` is float32 scratch [sum over sequences of max(1, ceil(tokens / segment_tokens)),
-    heads, dim, vdim] (`scan_segments` counts them). The result agrees with the single pass within rounding."""
+    heads, dim, vdim] (`scan_segments` counts them). The result agrees with the single pass within rounding. `products`: whether
+    a segment's work is done as matrix products (heads of up to 128) or token by token (None: as `scan_as_products` says)."""
     _need(out, torch.float32, "out"); _need(state, torch.float32, "state"); _need(decay, torch.float32, "decay")
     total_segments = 0
     if segment_tokens:
@@ -754,10 +755,12 @@ def decay_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, out: torc
     if activation not in SCAN_ACTIVATIONS:
         raise ValueError(f"decay_scan: unknown activation {activation!r}")
     fn = _FUNCTIONS.get("lb_decay_scan") or _fn("linear_attention", "lb_decay_scan",
-             [c_int, c_void_p, c_long, c_int, c_int, c_int] + [c_void_p] * 5 + [c_int] * 5 + [c_void_p, c_int, c_int, c_void_p])
+             [c_int, c_void_p, c_long, c_int, c_int, c_int] + [c_void_p] * 5 + [c_int] * 5 + [c_void_p, c_int, c_int, c_int, c_void_p])
+    if total_segments and products is None:
+        products = scan_as_products(tokens, total_segments, segment_tokens, heads, dim, vdim, proj.dtype)
     _check(fn(dtype_code(proj.dtype), _ptr(proj), proj.stride(0), q_off, k_off, v_off, _ptr(out), _ptr(state), _ptr(cu_q),
               _ptr(state_slots), _ptr(decay), n_seqs, heads, dim, vdim, SCAN_ACTIVATIONS[activation],
-              _ptr(segment_state), int(segment_tokens), total_segments, _stream()), "decay_scan")
+              _ptr(segment_state), int(segment_tokens), total_segments, int(bool(products and total_segments)), _stream()), "decay_scan")
     if total_segments:
         global LAUNCHES
         LAUNCHES += 2          # the segmented form is three kernels
@@ -768,13 +771,35 @@ SCAN_SEGMENT_TOKENS = 128      # the shortest segment of the segmented scan, whe
 SCAN_SEGMENT_BYTES = 1 << 30   # the most scratch its segments' states may take; longer segments beyond
 
 
+def scan_as_products(tokens: int, segments: int, segment_tokens: int, heads: int, dim: int, vdim: int, dtype: torch.dtype) -> bool:
+    """Whether the segmented scan of `tokens` tokens does its segments' work as matrix products rather than token by token.
+
+    The products' tiles are 64 tokens x 128 value channels over 128 key channels, whatever is in them, and a block's own chain
+    of loads and products takes about 70 us; the walk takes as long per token as it has channels, and 50 us at least. So the
+    products are taken where the tiles are full (heads of 65 to 128 with values that fill 128 columns, segments that are not
+    mostly the end of a short portion), where the walk has more than two blocks an SM one after the other, and, for a 32-bit
+    row, where the segments' states stay in the L2 between the launches. Measured (one B200, us of a layer, walk and products,
+    bfloat16; 32-bit): 32 heads of 128 x 128, one prompt of 300 tokens 100 and 89; 90 and 92, of 1,500 433 and 278; 373 and 320, of
+    4,000 1,150 and 868; 960 and 958, four of 600 678 and 561; 569 and 636, 1,500 beside 4 single tokens 458 and 349; 389 and 396,
+    beside 16 563 and 623; 503 and 689; 16 of 128 x 96, 1,500 tokens 162 and 158; 151 and 171; 4 of 128 x 128, 600 tokens 62 and 78;
+    32 of 64 x 64, 1,500 tokens 145 and 241; 137 and 277."""
+    room = segments * segment_tokens
+    full_tiles = 64 < dim <= 128 and -(-vdim // 32) % 4 == 0
+    walk_blocks = heads * -(-vdim // 32) * -(-room // SCAN_SEGMENT_TOKENS)
+    if not full_tiles or walk_blocks < 300:
+        return False
+    if dtype == torch.float32:
+        return 20 * tokens >= 17 * room and 4 * segments * heads * dim * vdim <= 64 << 20
+    return 10 * tokens >= 7 * room
+
+
 def scan_segments(q_lens: list[int], state_bytes: int, dim: int = 0) -> tuple[int, int]:
     """(tokens per segment, number of segments) for a step whose sequences bring `q_lens` tokens, or (0, 0)
     when no portion is long enough for the segmented scan to pay (two segments or more).
 
-    Heads of `dim` 33 to 128 have their segments as matrix products: half as long ones then have half the weights between a
-    segment's own tokens, and blocks of equal work, for twice the states. 32 heads of 128 x 128, one prompt of 1,500
-    tokens: 306 -> 283 us a layer with 64, of 300 tokens 118 -> 89, two of 700 and 900: 322 -> 298."""
+    `dim` 33 to 128: heads of that size whose segments' work is done as matrix products. Half as long segments then have half the
+    weights between a segment's own tokens, and blocks of equal work, for twice the states: 32 heads of 128 x 128, one prompt of
+    1,500 tokens: 306 -> 283 us a layer with 64, of 300 tokens 118 -> 89, two of 700 and 900: 322 -> 298."""
     longest = max(q_lens)
     if longest < 2 * SCAN_SEGMENT_TOKENS:
         return 0, 0
@@ -784,6 +809,15 @@ def scan_segments(q_lens: list[int], state_bytes: int, dim: int = 0) -> tuple[in
         if total * state_bytes <= SCAN_SEGMENT_BYTES or 2 * tokens > longest:
             return tokens, total
         tokens *= 2
+
+
+def scan_plan(q_lens: list[int], heads: int, dim: int, vdim: int, dtype: torch.dtype) -> tuple[int, int, bool]:
+    """(tokens per segment, number of segments, whether their work is done as matrix products) for `decay_scan`."""
+    state_bytes = 4 * heads * dim * vdim
+    tokens, segments = scan_segments(q_lens, state_bytes, dim)
+    if segments and scan_as_products(sum(q_lens), segments, tokens, heads, dim, vdim, dtype):
+        return tokens, segments, True
+    return (*scan_segments(q_lens, state_bytes), False)
 
 
 def gated_rmsnorm(x: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor) -> torch.Tensor:

@@ -77,10 +77,10 @@ class DecayLinearAttention(Part):
         tokens, qk, vv = h.shape[0], self.heads * self.dim, self.heads * self.vdim
         proj = self.runtime.linear(h, self.w_in)                    # [T, q | k | v | gate (| padding)]
         scanned = torch.empty((tokens, vv), dtype=torch.float32, device=h.device)
-        segment_tokens, segments = ops.scan_segments(batch.q_lens, 4 * self.heads * self.dim * self.vdim, self.dim)
+        segment_tokens, segments, products = ops.scan_plan(batch.q_lens, self.heads, self.dim, self.vdim, proj.dtype)
         scratch = torch.empty((segments, self.heads, self.dim, self.vdim), dtype=torch.float32, device=h.device) if segments else None
         ops.decay_scan(proj, 0, qk, 2 * qk, scanned, cache.state, batch.cu_q, batch.state_slots, self.decay, batch.n_seqs,
-                       self.heads, self.dim, self.vdim, self.activation, segment_tokens, scratch)
+                       self.heads, self.dim, self.vdim, self.activation, segment_tokens, scratch, products)
         gated = torch.empty((tokens, vv), dtype=h.dtype, device=h.device)
         ops.gated_rmsnorm(scanned, proj[:, 2 * qk + vv: 2 * qk + 2 * vv], self.norm_w, self.norm_eps, gated)
         return self.runtime.linear(gated, self.w_o)

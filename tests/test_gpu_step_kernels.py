@@ -1,5 +1,6 @@
 """Kernels of whole steps at the edges of their tiles, groups, segments and splits, against float64."""
 
+import functools
 import math
 
 import pytest
@@ -236,9 +237,10 @@ def test_decode_attention_with_a_warps_own_keys(group, page, splits, stages, win
             assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + (2.0 ** -14 if extras else 2.0 ** -8) * spread + 1e-6).all()
 
 
-@pytest.mark.parametrize("dim", [24, 64])       # segments that walk their tokens, and segments as matrix products
+@pytest.mark.parametrize("dim", [24, 64])
+@pytest.mark.parametrize("products", [False, True])
 @pytest.mark.parametrize("lengths", [[0], [130, 0, 70], [0, 300, 0]])
-def test_segments_of_a_sequence_without_tokens_leave_its_state(dim, lengths):
+def test_segments_of_a_sequence_without_tokens_leave_its_state(dim, products, lengths):
     """A decay of 0 to the power 0 is 1: the state of a request that brings no tokens keeps its bits."""
     o, heads, vdim, segment = ops(), 2, 20, 64
     gen, tokens, n_seqs = torch.Generator().manual_seed(dim), sum(lengths), len(lengths)
@@ -249,16 +251,17 @@ def test_segments_of_a_sequence_without_tokens_leave_its_state(dim, lengths):
     scratch = torch.full((sum(max(1, -(-n // segment)) for n in lengths), heads, dim, vdim), float("nan"), device="cuda")
     out = torch.full((tokens, heads * vdim), float("nan"), device="cuda")
     o.decay_scan(proj, 0, heads * dim, 2 * heads * dim, out, state, ints([sum(lengths[:s]) for s in range(n_seqs + 1)]), ints(list(range(n_seqs))),
-                 torch.tensor([0.0, 0.9], device="cuda"), n_seqs, heads, dim, vdim, None, segment, scratch)
+                 torch.tensor([0.0, 0.9], device="cuda"), n_seqs, heads, dim, vdim, None, segment, scratch, products)
     assert not torch.isnan(out).any() and not torch.isnan(state).any()
     for s, n in enumerate(lengths):
         assert torch.equal(state[s], before[s]) == (n == 0)
 
 
-@pytest.mark.parametrize("dim", [24, 128])      # segments that walk their tokens, and segments as matrix products
+@pytest.mark.parametrize("dim", [24, 128])
+@pytest.mark.parametrize("products", [False, True])
 @pytest.mark.parametrize("what", ["k", "v"])
 @pytest.mark.parametrize("value", [math.inf, -math.inf, math.nan])
-def test_segments_keep_a_value_that_is_not_finite_from_earlier_tokens(dim, what, value):
+def test_segments_keep_a_value_that_is_not_finite_from_earlier_tokens(dim, products, what, value):
     """The outputs of the tokens before it keep their bits, wherever it stands in a block of 64 tokens; its own is not finite."""
     o, heads, vdim, tokens = ops(), 2, 128, 200
     gen = torch.Generator().manual_seed(dim)
@@ -269,7 +272,7 @@ def test_segments_keep_a_value_that_is_not_finite_from_earlier_tokens(dim, what,
     def run(proj):
         state, out = torch.zeros(1, heads, dim, vdim, device="cuda"), torch.empty(tokens, heads * vdim, device="cuda")
         scratch = torch.empty(2, heads, dim, vdim, device="cuda")
-        o.decay_scan(proj, 0, heads * dim, 2 * heads * dim, out, state, ints([0, tokens]), ints([0]), lam, 1, heads, dim, vdim, None, 128, scratch)
+        o.decay_scan(proj, 0, heads * dim, 2 * heads * dim, out, state, ints([0, tokens]), ints([0]), lam, 1, heads, dim, vdim, None, 128, scratch, products)
         return out.view(tokens, heads, vdim)
 
     want, column = run(clean), heads * dim + 5 if what == "k" else 2 * heads * dim + 5
@@ -290,6 +293,25 @@ def test_segments_with_scratch_that_begins_anywhere():
     for shift in (0, 1):
         scratch = torch.empty(floats + 1, device="cuda")[shift: shift + floats].view(3, heads, dim, vdim)
         state, out = torch.ones(1, heads, dim, vdim, device="cuda"), torch.empty(tokens, heads * vdim, device="cuda")
-        o.decay_scan(proj, 0, heads * dim, 2 * heads * dim, out, state, ints([0, tokens]), ints([0]), lam, 1, heads, dim, vdim, None, 64, scratch)
+        o.decay_scan(proj, 0, heads * dim, 2 * heads * dim, out, state, ints([0, tokens]), ints([0]), lam, 1, heads, dim, vdim, None, 64, scratch, True)
         results.append((out, state))
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("products", [False, True])
+@pytest.mark.parametrize("heads, dim, vdim, decay", [(2, 33, 7, [0.9, 0.0]), (1, 64, 130, [1.0]), (3, 128, 128, [0.999, 0.5, 0.97]), (2, 5, 4, [0.3, 0.99])])
+@pytest.mark.parametrize("lengths, segment", [([1], 128), ([127, 128, 129], 128), ([300, 65, 128], 64), ([513, 100], 256)])
+def test_segments_in_both_forms(monkeypatch, products, heads, dim, vdim, decay, lengths, segment):
+    """The form asked for, whatever the plan would take: walked token by token or as matrix products."""
+    o = ops()
+    monkeypatch.setattr(o, "decay_scan", functools.partial(o.decay_scan, products=products))
+    test_segments_as_matrix_products(heads, dim, vdim, decay, lengths, segment)
+
+
+def test_segments_as_products_refuse_heads_that_a_block_does_not_hold():
+    o = ops()
+    proj, state, out = torch.zeros(300, 3 * 192, device="cuda"), torch.zeros(1, 1, 192, 192, device="cuda"), torch.zeros(300, 192, device="cuda")
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    scratch = torch.zeros(5, 1, 192, 192, device="cuda")
+    with pytest.raises(ValueError):
+        o.decay_scan(proj, 0, 192, 384, out, state, ints([0, 300]), ints([0]), torch.ones(1, device="cuda"), 1, 1, 192, 192, None, 64, scratch, True)

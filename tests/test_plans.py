@@ -103,3 +103,26 @@ def test_a_portions_split_is_planned_from_the_portions_own_contexts(monkeypatch)
             assert split([portion, decoding]) == alone and split([decoding, portion, decoding]) == alone
     assert split([(0, 64), (8192, 1)]) == 1 and split([(8209, 512)]) > 1
     assert split([(0, 64), (3000, 64), (8192, 1)]) == split([(3000, 64), (0, 64)])     # the longest of the portions counts
+
+
+def test_scan_plan_takes_products_where_their_tiles_are_full():
+    plan = lambda q_lens, heads=32, dim=128, vdim=128, dtype=torch.bfloat16: ops.scan_plan(q_lens, heads, dim, vdim, dtype)
+    assert plan([1500]) == (64, 24, True) and plan([300]) == (64, 5, True)
+    assert plan([255]) == (0, 0, False) and plan([1] * 64) == (0, 0, False)
+    assert plan([1500], vdim=64) == (128, 12, False) and plan([1500], dim=64, vdim=64) == (128, 12, False)
+    assert plan([1500], vdim=96) == (128, 12, False) and plan([1500], dim=96)[2] and plan([1500], dim=256) == (128, 12, False)
+    assert plan([600], heads=4) == (128, 5, False) and plan([4000], heads=4)[2]             # few chains: the walk is not waited for
+    assert plan([1500] + [1] * 4)[2] and not plan([1500] + [1] * 16)[2]                     # segments of one token
+    f32 = torch.float32
+    assert plan([1500], dtype=f32)[2] and not plan([1500] + [1] * 4, dtype=f32)[2]
+    assert not plan([4000], dtype=f32)[2]                                                   # the states leave the L2
+    assert plan([256] * 300, heads=64, vdim=1024)[0] > 64                                   # scratch of 1 GiB at most
+
+
+def test_scan_form_of_a_call_is_that_of_its_plan():
+    for heads, dim, vdim in ((32, 128, 128), (4, 128, 128), (16, 96, 160), (8, 64, 64), (2, 128, 512)):
+        for dtype in (torch.float32, torch.bfloat16):
+            for q_lens in ([256], [300], [1500], [4000], [300] + [1] * 9, [700, 900], [600] * 4, [20, 260, 7]):
+                tokens, segments, products = ops.scan_plan(q_lens, heads, dim, vdim, dtype)
+                if products:
+                    assert ops.scan_as_products(sum(q_lens), segments, tokens, heads, dim, vdim, dtype)

@@ -84,6 +84,10 @@ class StepBatch:
     decode_max_ctx: int
     portion_tiles: dict[int, QueryTiles]
     portion_max_ctx: int         # the longest context among the sequences of `portion_tiles`
+    # (new tokens, context) of the sequences of `tiles` and of `portion_tiles`, as a portion's attention is to plan for them (a
+    # captured portion: the middle of the contexts that its class holds)
+    tile_lens: tuple[tuple[int, int], ...]
+    portion_lens: tuple[tuple[int, int], ...]
     # host-side facts for planning launches
     q_lens: list[int]
     ctx_lens: list[int]
@@ -288,6 +292,9 @@ class BatchBuilder:
                 count *= s
             return device[offset:offset + count].view(*shape)
 
+        lens = tuple(zip(q_lens, ctx_lens))
+        if portion and not entries:
+            lens = ((portion, (portion + width * page) // 2),)
         return StepBatch(
             n_tokens=n_tokens, n_seqs=n_seqs,
             token_ids=get("token_ids"), positions=get("positions"), cu_q=get("cu_q"), ctx_len=get("ctx_len"),
@@ -301,6 +308,7 @@ class BatchBuilder:
             portion_tiles={size: QueryTiles(get(f"ptile_seq{size}"), get(f"ptile_q0{size}"), len(tiles))
                            for size, tiles in portion_lists.items()},
             portion_max_ctx=max((c for n, c in zip(q_lens, ctx_lens) if n > 1), default=0) if mixed else 0,
+            tile_lens=lens, portion_lens=tuple(x for x in lens if x[0] > 1) if mixed else (),
             q_lens=q_lens, ctx_lens=ctx_lens, max_q_len=max(q_lens), max_ctx=max(ctx_lens),
             all_decode=max(q_lens) == 1, real_seqs=real,
             plan_max_ctx=plan_ctx[0] if plan_ctx else max((ctx_lens[s] for s in singles), default=0),

@@ -1730,13 +1730,39 @@ def portion_splits(n_tiles: int, q_heads: int, kv_heads: int, keys: int, sms: in
     return min(range(1, max(2, min(9, tiles // 4 + 1))), key=cost)
 
 
+@functools.lru_cache(maxsize=1024)      # of the sizes alone, asked for by every layer of a step
+def exact_on_tcgen05(lens: tuple[tuple[int, int], ...], q_heads: int, window: int, sms: int) -> bool:
+    """Whether portions of (new tokens, context) with exact weights are quicker on the tcgen05 kernel than on the mma.sync one.
+
+    A block of the first takes 128 queries of two heads over tiles of 128 keys, of the second 64 queries of one head over tiles of
+    64. Either takes its start, and then the longer of its longest block's tiles one after the other and all blocks' tiles
+    shared out over the SMs; a mask within the tiles (a window) makes a tile longer. The figures (us) fit 1,016 measurements on one
+    B200 (12 over 2, 16 over 4, 32 over 8 and 64 over 8 heads, 1 to 16 prompts of 20 to 900 tokens, portions of 2 to 1,000 tokens
+    after 300 to 6,000, windows of 0, 128, 512 and 1,024): what this rule takes is 0.3 % over the better of the two on average,
+    at most 6 % over the mma.sync kernel. 16 over 4 heads, tcgen05 and mma.sync: one prompt of 20 tokens 16.7 and 7.4, of 261
+    23.6 and 18.9, of 512 25 and 30, two of 611 29.9 and 44.1, one of 1,500 52 and 102; 64 tokens after 500 34 and 31, after 3,000
+    86 and 131."""
+    def cost(rows: int, heads: int, start: float, tile: float, shared: float, masked: float) -> float:
+        longest = total = 0
+        for new, ctx in lens:
+            for first in range(ctx - new, ctx, rows):
+                last = min(first + rows, ctx) - 1
+                low = max(0, first - window + 1) if window > 0 else (first // -window * -window if window else 0)
+                tiles = last // rows - low // rows + 1
+                longest, total = max(longest, tiles), total + tiles
+        return start + (masked if window else 1.0) * max(tile * longest, shared * total * heads / sms)
+
+    return cost(128, q_heads // 2, 8.5, 4.85, 8.1, 1.92) < cost(64, q_heads, 4.9, 3.07, 2.49, 1.76)
+
+
 def attention_bf16(q, cache, out, block_table, batch, q_heads, kv_heads, dim, page_tokens, scale, window, sinks=None,
                    gates=None, exact_weights=False, chunk=0, keep_first=0, decode_share=1, softcap=0.0, out_scale=1.0):
     """The bfloat16 path's attention for one step: prompt portions go through the tcgen05 tile kernel
     where it takes the sizes (head size 128, pages of 8..128 tokens), else through the mma.sync
     one; single tokens, alone or beside prompt portions, go through the split decode kernel. With
     sinks, gates or exact weights the kernels' variants for those run; the tcgen05 kernel's takes an even number of query heads
-    per key/value head and neither kept first keys nor a soft cap, which stay with the mma.sync one. `decode_share` > 1: the
+    per key/value head and neither kept first keys nor a soft cap, which stay with the mma.sync one, and so do short portions
+    (`exact_on_tcgen05`). `decode_share` > 1: the
     decode kernel takes the query heads of a key/value head as that many groups (each at most 16 heads)."""
     plain = sinks is None and gates is None and not exact_weights and not chunk and not keep_first and not softcap \
         and out_scale == 1.0 and out.is_contiguous()
@@ -1759,7 +1785,7 @@ def attention_bf16(q, cache, out, block_table, batch, q_heads, kv_heads, dim, pa
                               batch.n_seqs, q_heads, decode_groups, dim, page_tokens, scale, window, splits, stages,
                               kv_share=decode_share, **extras)
         return
-    tiles_of, portion_ctx = batch.tiles, batch.max_ctx
+    tiles_of, portion_ctx, lens = batch.tiles, batch.max_ctx, batch.tile_lens
     if batch.n_decode_seqs > 0 and q_heads // decode_groups <= 16:
         # a mixed step: the sequences with a single token go through the decode kernel (a tile kernel
         # would spend a whole tile of queries on each), the prompt portions through the tile kernel
@@ -1770,7 +1796,7 @@ def attention_bf16(q, cache, out, block_table, batch, q_heads, kv_heads, dim, pa
         attention_decode_bf16(q, cache.k_pool, cache.v_pool, out, block_table, batch.cu_q, batch.ctx_len, batch.decode_seqs,
                               batch.n_decode_seqs, q_heads, decode_groups, dim, page_tokens, scale, window, splits, stages,
                               kv_share=decode_share, **extras)
-        tiles_of, portion_ctx = batch.portion_tiles, batch.portion_max_ctx
+        tiles_of, portion_ctx, lens = batch.portion_tiles, batch.portion_max_ctx, batch.portion_lens
     if plain and cache.pool is not None and attention_tcgen05_supports(q_heads, kv_heads, dim, page_tokens):
         tiles = tiles_of[TCGEN05_TILE]
         attention_tcgen05_prefill(q, cache.pool, cache.layer, out, block_table, batch.cu_q, batch.ctx_len, tiles.tile_seq,
@@ -1779,7 +1805,7 @@ def attention_bf16(q, cache, out, block_table, batch, q_heads, kv_heads, dim, pa
         return
     if (exact_weights and not keep_first and not softcap and TCGEN05_TILE in tiles_of and cache.pool is not None
             and attention_tcgen05_exact_takes(q_heads, kv_heads, dim) and attention_tcgen05_supports(q_heads, kv_heads, dim, page_tokens)
-            and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0):
+            and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0 and exact_on_tcgen05(lens, q_heads, window, sm_count(q.device))):
         tiles = tiles_of[TCGEN05_TILE]
         attention_tcgen05_prefill(q, cache.pool, cache.layer, out, block_table, batch.cu_q, batch.ctx_len, tiles.tile_seq,
                                   tiles.tile_q0, tiles.count, q_heads, kv_heads, dim, page_tokens, scale, window, 1, True, sinks, gates,

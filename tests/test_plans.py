@@ -5,7 +5,7 @@ import torch
 
 from layover_b200 import ops
 from layover_b200.cache import CacheManager
-from layover_b200.engine.batch import BatchBuilder, StepEntry
+from layover_b200.engine.batch import BatchBuilder, BatchCapacity, StepEntry
 from layover_b200.parts.base import PagedKVNeed
 
 SMS = 148
@@ -126,3 +126,20 @@ def test_scan_form_of_a_call_is_that_of_its_plan():
                 tokens, segments, products = ops.scan_plan(q_lens, heads, dim, vdim, dtype)
                 if products:
                     assert ops.scan_as_products(sum(q_lens), segments, tokens, heads, dim, vdim, dtype)
+
+
+def test_exact_weights_stay_on_mma_sync_for_short_portions(monkeypatch):
+    step = _Recorder(monkeypatch, 16, 4)
+    kernel = lambda requests, **options: step.run(requests, exact_weights=True, **options)[-1][0]
+    assert kernel([(0, 20)]) == kernel([(0, 261)]) == kernel([(500, 40)]) == "mma"
+    assert kernel([(0, 611), (0, 611)]) == kernel([(0, 1500)]) == kernel([(3000, 64)]) == "tcgen05"
+    assert kernel([(0, 64), (8000, 1)]) == "mma"                     # what a decoding request holds is nothing to the portion
+    assert kernel([(0, 128)] * 16) == "tcgen05"                      # many short prompts fill the SMs
+    assert kernel([(0, 1500)], window=1024) == "tcgen05" and kernel([(2000, 100)], window=128) == "mma"
+    assert kernel([(0, 1500)], chunk=1024) == "tcgen05" and kernel([(8000, 8)], chunk=4096) == "tcgen05"
+
+
+def test_captured_portion_with_exact_weights_is_planned_for_its_class(monkeypatch):
+    step = _Recorder(monkeypatch, 16, 4)
+    run = lambda tokens, width: step.run([], BatchCapacity(1, width, tokens), exact_weights=True)[-1][0]
+    assert run(512, 64) == run(64, 256) == "tcgen05" and run(16, 8) == "mma"

@@ -562,6 +562,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid
 // (gridDim.z), each of which leaves its maximum, sum and output for `attention_merge_kernel`. Measured (one B200, 32 heads
 // over 8, 512 tokens after 8,209, 64 blocks on 148 SMs): the attention
 // of a layer 177 -> 105 us (two blocks a tile) and 6 us for the merge
+// SPLIT is that form: without it the kernel carries nothing of it (20 .. 1,222 tokens 0.3 us a layer).
 // EXACT: the variant for attention with weights that keep 16 bits of mantissa in the second product (and sinks, gates, a
 // factor on the outputs; a negative window is a chunked mask: a query sees the keys of its own chunk of -window positions). A
 // weight is the sum of two bfloat16 numbers, its rounded value and the rounded rest; the rests take the upper half of the
@@ -571,7 +572,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid
 constexpr int PAIR_THREADS = 320;   // warp 0 producer, warp 1 MMA issuer, warps 2-5 and 6-9 the softmax warpgroups
 constexpr int PAIR_SMEM = TILE_BYTES * (2 + 2 * KV_STAGES) + 1024 + 512 + TABLE_CACHE * 4;   // Q x2, K and V stages, slack, barriers, table
 
-template <bool EXACT>
+template <bool EXACT, bool SPLIT>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map,
                               const Args args) {
@@ -606,9 +607,14 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
   const int key_lo = args.window > 0 ? max(0, p_first - args.window + 1) : (chunk ? p_first / chunk * chunk : 0);
   const int first_tile = key_lo / KEYS, all_tiles = max(0, p_last / KEYS + 1 - first_tile);
   const int q_row = row0 + q0;
-  // this block's share of the key tiles: all of them, or one of gridDim.z ranges (empty where there are fewer tiles)
-  const int tile_begin = first_tile + (int)((long)all_tiles * blockIdx.z / gridDim.z);
-  const int n_tiles = first_tile + (int)((long)all_tiles * (blockIdx.z + 1) / gridDim.z) - tile_begin;
+  // this block's share of the key tiles: all of them, or one of gridDim.z ranges (empty where there are fewer tiles; at most 32
+  // ranges of 2^24 tiles, so that 32 bits hold the products, whose divisions every block waits for)
+  unsigned from = 0, upto = (unsigned)all_tiles;
+  if (SPLIT) {
+    from = (unsigned)all_tiles * blockIdx.z / gridDim.z;
+    upto = (unsigned)all_tiles * (blockIdx.z + 1) / gridDim.z;
+  }
+  const int tile_begin = first_tile + (int)from, n_tiles = (int)(upto - from);
   const int* table = args.block_table + (size_t)seq * args.table_width;
 
   if (threadIdx.x == 0) {
@@ -811,10 +817,10 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
       const size_t token = (size_t)(q_row + (valid ? row : 0));
       bf16* dst = EXACT ? args.out + token * args.out_stride + (head0 + u) * DIM : args.out + (token * args.q_heads + head0 + u) * DIM;
       // with the keys dealt to several blocks: maximum, sum and unnormalised output, for the merge kernel
-      float* left = args.partials ? args.partials + ((((size_t)tile_index * args.q_heads + head0 + u) * gridDim.z + blockIdx.z) * ROWS + row) * (DIM + 2)
-                                  : nullptr;
-      if (left) reinterpret_cast<float2*>(left + DIM)[0] = make_float2(m_ref, l_sum);
-      float inv = left ? 1.0f : 1.0f / l_sum;
+      float* left = SPLIT ? args.partials + ((((size_t)tile_index * args.q_heads + head0 + u) * gridDim.z + blockIdx.z) * ROWS + row) * (DIM + 2)
+                          : nullptr;
+      if (SPLIT) reinterpret_cast<float2*>(left + DIM)[0] = make_float2(m_ref, l_sum);
+      float inv = SPLIT ? 1.0f : 1.0f / l_sum;
       if (EXACT) {       // the row's maximum is finite (a query sees itself); scores are unscaled, the sink is not to be scaled
         if (args.sinks) inv = 1.0f / (l_sum + fast_exp2(args.sinks[head0 + u] * 1.4426950408889634f - m_ref * c));
         if (args.gates) inv *= args.gates[token * args.q_heads + head0 + u];
@@ -830,7 +836,7 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
           for (int e = 0; e < 16; ++e) v[e] = 0.f;
         }
         if (!valid) continue;
-        if (left) {
+        if (SPLIT) {
 #pragma unroll
           for (int e = 0; e < 8; ++e) reinterpret_cast<float2*>(left + ch * 16)[e] = make_float2(v[2 * e], v[2 * e + 1]);
           continue;
@@ -907,8 +913,9 @@ void configure_once() {      // once per device: the attribute belongs to the de
   static LbPerDeviceOnce once;
   if (!once.first()) return;
   cudaFuncSetAttribute(attention_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-  cudaFuncSetAttribute(attention_tcgen05_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
-  cudaFuncSetAttribute(attention_tcgen05_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
+  cudaFuncSetAttribute(attention_tcgen05_pair_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
+  cudaFuncSetAttribute(attention_tcgen05_pair_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
+  cudaFuncSetAttribute(attention_tcgen05_pair_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
 }
 
 // q as a 2-D bf16 matrix [rows, cols] with rows `stride` elements apart: box 64 columns x 128 rows
@@ -992,10 +999,13 @@ LB_EXPORT int lb_attention_tcgen05_prefill(const void* q, long q_rows, const voi
             2 * layer, scale * 1.4426950408889634f, splits > 1 ? partials : nullptr, sinks, gates, out_scale, out_stride};
   int code;
   if (exact)
-    code = lb_launch(attention_tcgen05_pair_kernel<true>, dim3(q_heads / 2, n_tiles), dim3(PAIR_THREADS), (size_t)PAIR_SMEM, stream,
+    code = lb_launch(attention_tcgen05_pair_kernel<true, false>, dim3(q_heads / 2, n_tiles), dim3(PAIR_THREADS), (size_t)PAIR_SMEM, stream,
                      q_map, kv_map, args);
+  else if (splits > 1)
+    code = lb_launch(attention_tcgen05_pair_kernel<false, true>, dim3(q_heads / 2, n_tiles, splits), dim3(PAIR_THREADS), (size_t)PAIR_SMEM,
+                     stream, q_map, kv_map, args);
   else if ((q_heads / kv_heads) % 2 == 0)    // two heads of a KV head per block
-    code = lb_launch(attention_tcgen05_pair_kernel<false>, dim3(q_heads / 2, n_tiles, splits), dim3(PAIR_THREADS), (size_t)PAIR_SMEM, stream,
+    code = lb_launch(attention_tcgen05_pair_kernel<false, false>, dim3(q_heads / 2, n_tiles), dim3(PAIR_THREADS), (size_t)PAIR_SMEM, stream,
                      q_map, kv_map, args);
   else
     code = lb_launch(attention_tcgen05_kernel, dim3(q_heads, n_tiles), dim3(THREADS), (size_t)SMEM_BYTES, stream,

@@ -83,7 +83,6 @@ class StepBatch:
     n_decode_seqs: int
     decode_max_ctx: int
     portion_tiles: dict[int, QueryTiles]
-    portion_max_ctx: int         # the longest context among the sequences of `portion_tiles`
     # (new tokens, context) of the sequences of `tiles` and of `portion_tiles`, as a portion's attention is to plan for them (a
     # captured portion: the middle of the contexts that its class holds)
     tile_lens: tuple[tuple[int, int], ...]
@@ -307,7 +306,6 @@ class BatchBuilder:
             decode_max_ctx=max((ctx_lens[s] for s in singles), default=0) if mixed else 0,
             portion_tiles={size: QueryTiles(get(f"ptile_seq{size}"), get(f"ptile_q0{size}"), len(tiles))
                            for size, tiles in portion_lists.items()},
-            portion_max_ctx=max((c for n, c in zip(q_lens, ctx_lens) if n > 1), default=0) if mixed else 0,
             tile_lens=lens, portion_lens=tuple(x for x in lens if x[0] > 1) if mixed else (),
             q_lens=q_lens, ctx_lens=ctx_lens, max_q_len=max(q_lens), max_ctx=max(ctx_lens),
             all_decode=max(q_lens) == 1, real_seqs=real,

@@ -1718,16 +1718,40 @@ def attention_tcgen05_prefill(q, pool, layer, out, block_table, cu_q, ctx_len, t
     return out
 
 
+_PORTION_SCRATCH_FLOATS = 32 << 20     # the most that the partial results of split portions may take (128 MiB)
+
+
 @functools.lru_cache(maxsize=1024)      # of the sizes alone, asked for by every layer of a step
-def portion_splits(n_tiles: int, q_heads: int, kv_heads: int, keys: int, sms: int) -> int:
-    """How many blocks share the keys of a prompt portion's rows: the number that ends first when a block holds an SM,
-    takes its key tiles and two tiles' time to start and end, and a split costs four tiles' time (the partial results'
-    way through the L2, and their merge)."""
-    blocks, tiles = n_tiles * q_heads // 2, -(-keys // TCGEN05_TILE)
+def portion_splits(lens: tuple[tuple[int, int], ...], q_heads: int, kv_heads: int, window: int, sms: int) -> int:
+    """How many blocks share the keys of the rows of portions of (new tokens, context): the number that ends first.
+
+    A block holds an SM, takes 9 us and 2.25 us for each of its tiles of 128 keys, and the blocks run in rounds of one an SM: of
+    equal blocks where the keys are split, while the few short ones of a fresh prompt end early and leave their SMs to the last. A
+    split costs 8.2 us, 0.2 us a block of a row, and 0.57 us for each MB of partial results (130 floats a row, head and
+    block) on their way to the merge. The figures fit 549 measurements on one B200 (4 over 2 to 64 over 8 heads, 8 to 2,048
+    new tokens of one or three requests after 0 to 30,000): what they pick is 0.4 % over the best of 1 to 8 on average, 7 % over no split at
+    most, and 0.64 of it on average. 32 over 8 heads, no split and 2 blocks: 512 tokens after 1,000 37.4 and 37.5 us, after 8,000
+    162 and 105; 1,280 tokens after 1,000 62 and 102, after 15,000 569, 502 and with 4 blocks 470."""
+    blocks = sum(-(-new // TCGEN05_TILE) for new, _ in lens) * q_heads // 2
     if (q_heads // kv_heads) % 2 or blocks >= 2 * sms:
         return 1
-    cost = lambda s: -(-blocks * s // sms) * (-(-tiles // s) + 2) + (4 + s if s > 1 else 0)
-    return min(range(1, max(2, min(9, tiles // 4 + 1))), key=cost)
+
+    def tiles(first: int, ctx: int) -> int:          # that the queries from `first` on walk
+        low = max(0, first - window + 1) if window > 0 else 0
+        return (min(first + TCGEN05_TILE, ctx) - 1) // TCGEN05_TILE - low // TCGEN05_TILE + 1
+
+    longest = max(tiles(ctx - new + (new - 1) // TCGEN05_TILE * TCGEN05_TILE, ctx) for new, ctx in lens)
+    shortest = min(tiles(ctx - new, ctx) for new, ctx in lens)
+    megabytes = sum(new for new, _ in lens) * q_heads * 520e-6
+
+    def cost(s: int) -> float:
+        rounds = -(-blocks * s // sms)
+        if s == 1:
+            return 2.25 * (longest + (rounds - 1) * shortest)
+        return 2.25 * rounds * -(-longest // s) + 8.2 + (0.2 + 0.57 * megabytes) * s
+
+    most = min(8, longest // 2, _PORTION_SCRATCH_FLOATS // (2 * blocks * TCGEN05_TILE * 130))
+    return min(range(1, max(2, most + 1)), key=cost)
 
 
 @functools.lru_cache(maxsize=1024)      # of the sizes alone, asked for by every layer of a step
@@ -1785,7 +1809,7 @@ def attention_bf16(q, cache, out, block_table, batch, q_heads, kv_heads, dim, pa
                               batch.n_seqs, q_heads, decode_groups, dim, page_tokens, scale, window, splits, stages,
                               kv_share=decode_share, **extras)
         return
-    tiles_of, portion_ctx, lens = batch.tiles, batch.max_ctx, batch.tile_lens
+    tiles_of, lens = batch.tiles, batch.tile_lens
     if batch.n_decode_seqs > 0 and q_heads // decode_groups <= 16:
         # a mixed step: the sequences with a single token go through the decode kernel (a tile kernel
         # would spend a whole tile of queries on each), the prompt portions through the tile kernel
@@ -1796,12 +1820,12 @@ def attention_bf16(q, cache, out, block_table, batch, q_heads, kv_heads, dim, pa
         attention_decode_bf16(q, cache.k_pool, cache.v_pool, out, block_table, batch.cu_q, batch.ctx_len, batch.decode_seqs,
                               batch.n_decode_seqs, q_heads, decode_groups, dim, page_tokens, scale, window, splits, stages,
                               kv_share=decode_share, **extras)
-        tiles_of, portion_ctx, lens = batch.portion_tiles, batch.portion_max_ctx, batch.portion_lens
+        tiles_of, lens = batch.portion_tiles, batch.portion_lens
     if plain and cache.pool is not None and attention_tcgen05_supports(q_heads, kv_heads, dim, page_tokens):
         tiles = tiles_of[TCGEN05_TILE]
         attention_tcgen05_prefill(q, cache.pool, cache.layer, out, block_table, batch.cu_q, batch.ctx_len, tiles.tile_seq,
                                   tiles.tile_q0, tiles.count, q_heads, kv_heads, dim, page_tokens, scale, window,
-                                  portion_splits(tiles.count, q_heads, kv_heads, seen(portion_ctx), sm_count(q.device)))
+                                  portion_splits(lens, q_heads, kv_heads, window, sm_count(q.device)))
         return
     if (exact_weights and not keep_first and not softcap and TCGEN05_TILE in tiles_of and cache.pool is not None
             and attention_tcgen05_exact_takes(q_heads, kv_heads, dim) and attention_tcgen05_supports(q_heads, kv_heads, dim, page_tokens)

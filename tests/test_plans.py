@@ -143,3 +143,21 @@ def test_captured_portion_with_exact_weights_is_planned_for_its_class(monkeypatc
     step = _Recorder(monkeypatch, 16, 4)
     run = lambda tokens, width: step.run([], BatchCapacity(1, width, tokens), exact_weights=True)[-1][0]
     assert run(512, 64) == run(64, 256) == "tcgen05" and run(16, 8) == "mma"
+
+
+def test_portion_splits_weigh_what_a_split_takes():
+    plan = lambda *lens, heads=(32, 8), window=0: ops.portion_splits(lens, *heads, window, SMS)
+    assert plan((512, 8721)) == 2 and plan((512, 8512), heads=(16, 4)) == 4            # one round of blocks
+    assert plan((512, 512)) == plan((1280, 2280)) == plan((2048, 4096)) == 1           # partial results that cost more than they bring
+    assert plan((1280, 16280)) in (3, 4) and plan((512, 1512)) == 1
+    assert plan((512, 30512), heads=(64, 8)) == 1 and plan((1024, 30000), heads=(64, 8)) == 1
+    assert plan((8, 8008)) == 8 and plan((1, 100)) == 1
+    assert plan((64, 16000), heads=(12, 4)) == 1                                       # an odd number of heads a group
+    assert plan((64, 16000), window=256) == 1 and plan((64, 16000), window=8192) > 1   # the keys that are seen count
+    for new in (1, 40, 128, 300, 700, 1500):
+        for ctx in (new, new + 900, new + 20000, new + 120000):
+            for heads in ((2, 1), (32, 8), (64, 8)):
+                for count in (1, 3, 9):
+                    splits = plan(*[(new, ctx)] * count, heads=heads)
+                    tiles = count * -(-new // 128)
+                    assert 1 <= splits <= 8 and (splits == 1 or tiles * heads[0] * splits * 128 * 130 <= 32 << 20)

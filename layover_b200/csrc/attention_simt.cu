@@ -70,6 +70,7 @@ template <typename T> struct Attention {
   float* partials;            // [item][row of the item][chunk][2 + vdim]; null: a block walks all of its rows' chunks
   int chunk_room;             // chunks there is room for: all that a block table can hold
   int table_width, q_heads, kv_heads, dim, key_pitch, vdim, page_tokens, window, mask_chunk, keep_first, row_groups, stages;
+  bool q_quads;               // q's rows begin where four elements can be read at once
   float scale, cap, out_scale;
   long out_stride;
 };
@@ -157,7 +158,11 @@ attention_rows_kernel(const Attention<T> a) {
   for (int r = warp; r < rows; r += WARPS) {
     const int row = item.first_row + r;
     const T* src = a.q + ((size_t)(item.row0 + row / item.group) * a.q_heads + item.kv_head * item.group + row % item.group) * dim;
-    for (int c = 4 * lane; c < dim; c += 128) *reinterpret_cast<float4*>(q_s + r * dim + c) = Quad<T>::load(src + c);
+    if (a.q_quads) {
+      for (int c = 4 * lane; c < dim; c += 128) *reinterpret_cast<float4*>(q_s + r * dim + c) = Quad<T>::load(src + c);
+    } else {
+      for (int c = lane; c < dim; c += 32) q_s[r * dim + c] = Elem<T>::load(src + c);
+    }
   }
   const int p_first = item.position(item.first_row), p_last = item.position(item.first_row + rows - 1);
   int key_lo = a.window > 0 ? max(0, p_first - a.window + 1) : 0;            // first key any row here may see
@@ -433,6 +438,8 @@ LB_EXPORT int lb_attention_simt(int dtype, const void* q, const void* k_pool, co
   if (dim <= 0 || dim > MAX_DIM || dim % 4 || kv_heads <= 0 || q_heads % kv_heads || q_heads > 65535) return LB_ERR_SIZE;
   if (vdim <= 0 || vdim > MAX_DIM || vdim % 4 || keep_first < 0 || (keep_first && mask_chunk)) return LB_ERR_SIZE;
   if (!(softcap >= 0.f) || out_stride < (long)q_heads * vdim || max_q_len < 1 || (splits > 1 && !partials)) return LB_ERR_SIZE;
+  const int element = dtype == LB_F32 ? 4 : 2;           // keys and values are read four elements at a time
+  if ((uintptr_t)k_pool % (4 * element) || (uintptr_t)v_pool % (4 * element)) return LB_ERR_ALIGN;
   const int max_rows = (max_q_len < BQ ? max_q_len : BQ) * (q_heads / kv_heads);
   // rows of a key tile: a pitch of 4 floats beyond a multiple of 32 keeps the 16-byte reads of 32 keys free of bank conflicts
   const int key_pitch = dim + (36 - dim % 32) % 32;
@@ -440,7 +447,8 @@ LB_EXPORT int lb_attention_simt(int dtype, const void* q, const void* k_pool, co
   do {                                                                                                                       \
     Attention<T> a{(const T*)q, (const T*)k_pool, (const T*)v_pool, (T*)out, block_table, cu_q, ctx_len, tile_seq, tile_q0,   \
                    sinks, gates, splits > 1 ? partials : nullptr, chunk_room, table_width, q_heads, kv_heads, dim, key_pitch, \
-                   vdim, page_tokens, window, mask_chunk, keep_first, 0, 0, scale, softcap, out_scale, out_stride};           \
+                   vdim, page_tokens, window, mask_chunk, keep_first, 0, 0, (uintptr_t)q % (4 * sizeof(T)) == 0, scale, softcap, out_scale,  \
+                   out_stride};                                                                                               \
     return launch_attention<T>(a, n_tiles, max_rows, splits, stream);                                                        \
   } while (0)
   if (dtype == LB_F32) LB_SIMT(float);

@@ -143,3 +143,31 @@ def test_f32_product_sums_through_scratch_where_clusters_are_off(m):
     code = o._FUNCTIONS["lb_gemm_simt"](0, 0, a.data_ptr(), w.data_ptr(), got.data_ptr(), m, n, k, k, k, n, scratch.data_ptr(), 148, 0,
                                         torch.cuda.current_stream().cuda_stream)
     assert code == 0 and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("dim", [16, 128, 300])
+def test_f32_attention_of_queries_that_begin_anywhere(dtype, dim):
+    """Queries one element off an aligned address give the bits of aligned ones; keys or values there are refused."""
+    o, page, q_heads, kv_heads, lengths, q_lens = ops(), 16, 4, 2, [1, 40, 200], [1, 5, 17]
+    k_pool, v_pool, table, _, _ = paged_setup(dtype, lengths, kv_heads, dim, page, 5)
+    tokens, ints = sum(q_lens), lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    q = torch.randn(tokens * q_heads * dim, generator=torch.Generator().manual_seed(2)).to(dtype).cuda()
+    tiles = [(s, q0) for s, n in enumerate(q_lens) for q0 in range(0, n, 16)]
+    outs = []
+
+    def run(x, k, v):
+        out = torch.full((tokens, q_heads * dim), float("nan"), dtype=dtype, device="cuda")
+        o.attention_simt(x, k, v, out, table, ints([0, 1, 6, 23]), ints(lengths), ints([t[0] for t in tiles]), ints([t[1] for t in tiles]),
+                         len(tiles), q_heads, kv_heads, dim, page, dim ** -0.5)
+        return out
+
+    def shifted(t):
+        wide = torch.empty(t.numel() + 1, dtype=dtype, device="cuda")[1:]
+        return wide.copy_(t.reshape(-1)).view(t.shape)
+
+    q = q.view(tokens, q_heads * dim)
+    assert torch.equal(run(q, k_pool, v_pool), run(shifted(q), k_pool, v_pool))
+    for k, v in ((shifted(k_pool), v_pool), (k_pool, shifted(v_pool))):
+        with pytest.raises(ValueError, match="alignment"):
+            run(q, k, v)

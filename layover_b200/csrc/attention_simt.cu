@@ -39,7 +39,7 @@ constexpr int BQ = 16;      // queries per tile
 constexpr int BKEYS = 32;   // keys per tile (one per lane)
 constexpr int CHUNK_TILES = 4;
 constexpr int WARPS = 4;
-constexpr int MAX_DIM = 640;      // value sizes up to 128 keep one quad of the output a lane, the largest five
+constexpr int MAX_DIM = 640, MAX_QUADS = MAX_DIM / 128;      // value sizes up to 128 keep one quad of the output a lane, the largest five
 
 // four neighbouring elements with one load (the head size is a multiple of 4 and rows are 16-byte aligned)
 template <typename T> struct Quad;
@@ -53,13 +53,35 @@ template <> struct Quad<bf16> {
     return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
   }
 };
-// a quad of a page into shared memory, or zeros: asynchronously where no conversion is needed
-__device__ __forceinline__ void fetch_quad(float* dst, const float* src, bool valid) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(valid ? 16 : 0)
-               : "memory");
+// a key's or value's row of `size` channels (a lane four of every 128) into shared memory, or zeros: asynchronously where no
+// conversion is needed, else with all its loads on their way before the first is stored
+template <int QUADS>
+__device__ __forceinline__ void fetch_row(float* dst, const float* src, int size, bool valid, int lane) {
+#pragma unroll
+  for (int n = 0; n < QUADS; ++n) {
+    const int c = 4 * (lane + 32 * n);
+    if (c >= size) break;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + c)), "l"(src + c),
+                 "r"(valid ? 16 : 0) : "memory");
+  }
 }
-__device__ __forceinline__ void fetch_quad(float* dst, const bf16* src, bool valid) {
-  *reinterpret_cast<float4*>(dst) = valid ? Quad<bf16>::load(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+template <int QUADS>
+__device__ __forceinline__ void load_row(uint2 (&row)[QUADS], const bf16* src, int size, bool valid, int lane) {
+#pragma unroll
+  for (int n = 0; n < QUADS; ++n) {
+    const int c = 4 * (lane + 32 * n);
+    row[n] = valid && c < size ? *reinterpret_cast<const uint2*>(src + c) : make_uint2(0, 0);
+  }
+}
+template <int QUADS>
+__device__ __forceinline__ void widen_row(float* dst, const uint2 (&row)[QUADS], int size, int lane) {
+#pragma unroll
+  for (int n = 0; n < QUADS; ++n) {
+    const int c = 4 * (lane + 32 * n);
+    if (c < size)
+      *reinterpret_cast<float4*>(dst + c) = make_float4(__uint_as_float(row[n].x << 16), __uint_as_float(row[n].x & 0xffff0000u),
+                                                        __uint_as_float(row[n].y << 16), __uint_as_float(row[n].y & 0xffff0000u));
+  }
 }
 
 template <typename T> struct Attention {
@@ -196,8 +218,18 @@ attention_rows_kernel(const Attention<T> a) {
       const int j = warp + i * WARPS, key = tile * BKEYS + j, page = __shfl_sync(0xffffffffu, my_page, i);
       const bool valid = page >= 0;
       const size_t at = valid ? ((size_t)page * a.kv_heads + item.kv_head) * a.page_tokens + key % a.page_tokens : 0;
-      for (int c = 4 * lane; c < dim; c += 128) fetch_quad(k_s + (stage * BKEYS + j) * pitch + c, a.k_pool + at * dim + c, valid);
-      for (int c = 4 * lane; c < vdim; c += 128) fetch_quad(v_s + (stage * BKEYS + j) * vdim + c, a.v_pool + at * vdim + c, valid);
+      const T *k_from = a.k_pool + at * dim, *v_from = a.v_pool + at * vdim;
+      float *k_to = k_s + (stage * BKEYS + j) * pitch, *v_to = v_s + (stage * BKEYS + j) * vdim;
+      if constexpr (sizeof(T) == 4) {
+        fetch_row<MAX_QUADS>(k_to, k_from, dim, valid, lane);
+        fetch_row<MAX_QUADS>(v_to, v_from, vdim, valid, lane);
+      } else {
+        uint2 k_row[MAX_QUADS], v_row[NV];
+        load_row(k_row, k_from, dim, valid, lane);
+        load_row(v_row, v_from, vdim, valid, lane);
+        widen_row(k_to, k_row, dim, lane);
+        widen_row(v_to, v_row, vdim, lane);
+      }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -388,7 +420,7 @@ int launch_rows(Attention<T> a, int n_tiles, int max_rows, int splits, cudaStrea
     return lb_last_error();
   a.row_groups = (max_rows + ROWS - 1) / ROWS;
   auto smem = [&](int stages) { return (size_t)(ROWS * (a.dim + BKEYS) + stages * BKEYS * (a.key_pitch + a.vdim)) * sizeof(float); };
-  a.stages = smem(2) <= 227 * 1024 ? 2 : 1;
+  a.stages = sizeof(T) == 4 && smem(2) <= 227 * 1024 ? 2 : 1;      // a copy that converts is not asynchronous: a second stage waits all the same
   if (smem(a.stages) > 227 * 1024 || (long)a.kv_heads * a.row_groups > 65535) return LB_ERR_SIZE;
   const dim3 grid(n_tiles, a.kv_heads * a.row_groups, a.partials ? splits : 1);
   lb_launch(attention_rows_kernel<T, NV, R>, grid, dim3(WARPS * 32), smem(a.stages), stream, a);

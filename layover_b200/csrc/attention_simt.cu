@@ -24,7 +24,7 @@
 // Work is a list of tiles made on the host: tile w covers queries [tile_q0[w], +BQ) of sequence
 // tile_seq[w]. Query t of sequence s is row cu_q[s] + t of q and out, at absolute position ctx_len[s] - q_len(s) + t. A
 // row is one query of one query head; the rows of a tile that share a key/value head share every load of its keys and
-// values: a block takes 4 R of them (R a warp), and with few blocks (a decode step) the chunks of a row are dealt to
+// values: a block takes 4 R of them (R a warp, `rows_per_warp`), and with few blocks (a decode step) the chunks of a row are dealt to
 // `splits` blocks, which leave each chunk's maximum, sum and output in scratch memory for a second kernel to merge.
 // What bounds it: a decode step the latency of a tile (scores, softmax, output: about a thousand cycles for its 32 KB), which
 // more blocks hide; a prompt the reads of shared memory, one of 16 bytes per 4 R fused multiply-adds.
@@ -411,6 +411,12 @@ merge_chunks_kernel(const Attention<T> a) {
   }
 }
 
+size_t block_smem(int rows, int stages, int dim, int key_pitch, int vdim) {
+  return (size_t)(rows * (dim + BKEYS) + stages * BKEYS * (key_pitch + vdim)) * sizeof(float);
+}
+// rows of a key tile: a pitch of 4 floats beyond a multiple of 32 keeps the 16-byte reads of 32 keys free of bank conflicts
+int pitch_of(int dim) { return dim + (36 - dim % 32) % 32; }
+
 template <typename T, int NV, int R>
 int launch_rows(Attention<T> a, int n_tiles, int max_rows, int splits, cudaStream_t stream) {
   constexpr int ROWS = WARPS * R;
@@ -419,7 +425,7 @@ int launch_rows(Attention<T> a, int n_tiles, int max_rows, int splits, cudaStrea
       cudaFuncSetAttribute(attention_rows_kernel<T, NV, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
     return lb_last_error();
   a.row_groups = (max_rows + ROWS - 1) / ROWS;
-  auto smem = [&](int stages) { return (size_t)(ROWS * (a.dim + BKEYS) + stages * BKEYS * (a.key_pitch + a.vdim)) * sizeof(float); };
+  auto smem = [&](int stages) { return block_smem(ROWS, stages, a.dim, a.key_pitch, a.vdim); };
   a.stages = sizeof(T) == 4 && smem(2) <= 227 * 1024 ? 2 : 1;      // a copy that converts is not asynchronous: a second stage waits all the same
   if (smem(a.stages) > 227 * 1024 || (long)a.kv_heads * a.row_groups > 65535) return LB_ERR_SIZE;
   const dim3 grid(n_tiles, a.kv_heads * a.row_groups, a.partials ? splits : 1);
@@ -428,44 +434,54 @@ int launch_rows(Attention<T> a, int n_tiles, int max_rows, int splits, cudaStrea
   return lb_last_error();
 }
 
-// Rows of a warp: enough for a block to hold a tile's rows of a key/value head at once, as far as registers go.
-int rows_per_warp(int max_rows, int vdim) {
+// Rows of a warp: several, as far as registers go, share every read of a key or value; but one where the launch's rows, one a
+// warp, and their chunks of keys find room on the SMs at once, where a tile takes a warp as long as it has rows. Results do not depend
+// on it. Measured (one B200, 32-bit, us with one and with four rows a warp): 32 heads over 8, a prompt of 20 tokens 7.4 and 13.2, of 261
+// 133 and 104, 64 decoding requests of 1,500 keys of 32 heads over 1 437 and 254, one of 900 21 and 44. Eight rows a warp were slower
+// than four nearly everywhere (the prompt of 261: 127).
+int rows_per_warp(int max_rows, int dim, int vdim, long blocks_of_tiles, int chunks, int sm_count) {
   if (max_rows <= WARPS) return 1;
-  return vdim <= 128 ? (max_rows <= 4 * WARPS ? 4 : 8) : (vdim <= 256 ? 4 : 2);
+  const size_t smem = block_smem(WARPS, 2, dim, pitch_of(dim), vdim);
+  const long resident = smem > 0 ? (long)(227 * 1024 / smem) : 1, room = sm_count * (resident < 1 ? 1 : (resident > 3 ? 3 : resident));
+  const long blocks = blocks_of_tiles * ((max_rows + WARPS - 1) / WARPS);
+  if (blocks * (chunks > 1 ? chunks : 1) <= room) return 1;
+  return vdim <= 256 ? 4 : 2;
 }
 
 template <typename T>
-int launch_attention(const Attention<T>& a, int n_tiles, int max_rows, int splits, cudaStream_t stream) {
-  const int r = rows_per_warp(max_rows, a.vdim);
-  if (a.vdim <= 128) {
-    if (r == 1) return launch_rows<T, 1, 1>(a, n_tiles, max_rows, splits, stream);
-    return r == 4 ? launch_rows<T, 1, 4>(a, n_tiles, max_rows, splits, stream) : launch_rows<T, 1, 8>(a, n_tiles, max_rows, splits, stream);
+int launch_attention(const Attention<T>& a, int n_tiles, int max_rows, int rows, int splits, cudaStream_t stream) {
+  if (rows == 1) {
+    if (a.vdim <= 128) return launch_rows<T, 1, 1>(a, n_tiles, max_rows, splits, stream);
+    return a.vdim <= 256 ? launch_rows<T, 2, 1>(a, n_tiles, max_rows, splits, stream) : launch_rows<T, 5, 1>(a, n_tiles, max_rows, splits, stream);
   }
-  if (a.vdim <= 256) return r == 1 ? launch_rows<T, 2, 1>(a, n_tiles, max_rows, splits, stream) : launch_rows<T, 2, 4>(a, n_tiles, max_rows, splits, stream);
-  return r == 1 ? launch_rows<T, 5, 1>(a, n_tiles, max_rows, splits, stream) : launch_rows<T, 5, 2>(a, n_tiles, max_rows, splits, stream);
+  if (a.vdim <= 128) return launch_rows<T, 1, 4>(a, n_tiles, max_rows, splits, stream);
+  return a.vdim <= 256 ? launch_rows<T, 2, 4>(a, n_tiles, max_rows, splits, stream) : launch_rows<T, 5, 2>(a, n_tiles, max_rows, splits, stream);
 }
 }  // namespace
 
 LB_EXPORT int lb_attention_simt_block_queries() { return BQ; }
 
-// Blocks that a launch has without a split, and the rows that each leaves results for: what a caller needs to size the
-// scratch (blocks * rows * chunks a block table can hold * (vdim + 2) floats) and to choose `splits`.
-LB_EXPORT int lb_attention_simt_plan(int n_tiles, int q_heads, int kv_heads, int vdim, int max_q_len, int* rows_of_block) {
-  if (kv_heads <= 0 || q_heads % kv_heads) return 0;
+// Blocks that a launch has without a split, and the rows of each: what a caller needs to size the scratch (blocks * rows *
+// chunks a block table can hold * (vdim + 2) floats) and to choose `splits`. `max_chunks`: chunks of the longest context (about;
+// 0: unknown).
+LB_EXPORT int lb_attention_simt_plan(int n_tiles, int q_heads, int kv_heads, int dim, int vdim, int max_q_len, int max_chunks, int sm_count,
+                                     int* rows_of_block) {
+  if (kv_heads <= 0 || q_heads % kv_heads || dim <= 0 || dim > MAX_DIM || vdim <= 0 || vdim > MAX_DIM) { *rows_of_block = 0; return 0; }
   const int max_rows = (max_q_len < BQ ? max_q_len : BQ) * (q_heads / kv_heads);
-  *rows_of_block = WARPS * rows_per_warp(max_rows, vdim);
+  *rows_of_block = WARPS * rows_per_warp(max_rows, dim, vdim, (long)n_tiles * kv_heads, max_chunks, sm_count);
   return n_tiles * kv_heads * ((max_rows + *rows_of_block - 1) / *rows_of_block);
 }
 LB_EXPORT int lb_attention_simt_chunk() { return BKEYS * CHUNK_TILES; }
 
-// `max_q_len`: no sequence has more queries in this step (BQ or more: any number). `splits` > 1: the keys of a row are dealt to
+// `max_q_len`: no sequence has more queries in this step (BQ or more: any number). `rows_of_block`: as `lb_attention_simt_plan`
+// says for these sizes (any of its values will do). `splits` > 1: the keys of a row are dealt to
 // that many blocks, `partials` has the room that `lb_attention_simt_plan` speaks of, `chunk_room` chunks a row.
 LB_EXPORT int lb_attention_simt(int dtype, const void* q, const void* k_pool, const void* v_pool, void* out,
                                 const int* block_table, int table_width, const int* cu_q, const int* ctx_len,
                                 const int* tile_seq, const int* tile_q0, int n_tiles, int q_heads, int kv_heads,
                                 int dim, int page_tokens, float scale, int window, int vdim, const float* sinks,
                                 const float* gates, int mask_chunk, int keep_first, float softcap, float out_scale,
-                                long out_stride, int max_q_len, int splits, float* partials, int chunk_room, cudaStream_t stream) {
+                                long out_stride, int max_q_len, int rows_of_block, int splits, float* partials, int chunk_room, cudaStream_t stream) {
   if (n_tiles <= 0) return 0;
   if (dim <= 0 || dim > MAX_DIM || dim % 4 || kv_heads <= 0 || q_heads % kv_heads || q_heads > 65535) return LB_ERR_SIZE;
   if (vdim <= 0 || vdim > MAX_DIM || vdim % 4 || keep_first < 0 || (keep_first && mask_chunk)) return LB_ERR_SIZE;
@@ -473,15 +489,15 @@ LB_EXPORT int lb_attention_simt(int dtype, const void* q, const void* k_pool, co
   const int element = dtype == LB_F32 ? 4 : 2;           // keys and values are read four elements at a time
   if ((uintptr_t)k_pool % (4 * element) || (uintptr_t)v_pool % (4 * element)) return LB_ERR_ALIGN;
   const int max_rows = (max_q_len < BQ ? max_q_len : BQ) * (q_heads / kv_heads);
-  // rows of a key tile: a pitch of 4 floats beyond a multiple of 32 keeps the 16-byte reads of 32 keys free of bank conflicts
-  const int key_pitch = dim + (36 - dim % 32) % 32;
+  const int key_pitch = pitch_of(dim), rows = rows_of_block / WARPS;
+  if (rows_of_block % WARPS || (rows != 1 && rows != (vdim <= 256 ? 4 : 2))) return LB_ERR_SIZE;
 #define LB_SIMT(T)                                                                                                           \
   do {                                                                                                                       \
     Attention<T> a{(const T*)q, (const T*)k_pool, (const T*)v_pool, (T*)out, block_table, cu_q, ctx_len, tile_seq, tile_q0,   \
                    sinks, gates, splits > 1 ? partials : nullptr, chunk_room, table_width, q_heads, kv_heads, dim, key_pitch, \
                    vdim, page_tokens, window, mask_chunk, keep_first, 0, 0, (uintptr_t)q % (4 * sizeof(T)) == 0, scale, softcap, out_scale,  \
                    out_stride};                                                                                               \
-    return launch_attention<T>(a, n_tiles, max_rows, splits, stream);                                                        \
+    return launch_attention<T>(a, n_tiles, max_rows, rows, splits, stream);                                                      \
   } while (0)
   if (dtype == LB_F32) LB_SIMT(float);
   if (dtype == LB_BF16) LB_SIMT(bf16);

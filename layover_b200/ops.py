@@ -1204,18 +1204,18 @@ def attention_simt(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, 
         _need(t, torch.int32, name)
     max_q_len = 1 << 30 if max_q_len is None else int(max_q_len)
     q_ptr = _ptr(q)        # refuses other devices, before theirs is asked about
-    splits, chunk_room = _simt_splits(n_tiles, q_heads, kv_heads, vdim, max_q_len, max_ctx, block_table.shape[1] * page_tokens, q.device)
+    splits, chunk_room, blocks, rows = _simt_plan(n_tiles, q_heads, kv_heads, dim, vdim, max_q_len, max_ctx, block_table.shape[1] * page_tokens,
+                                                  q.device)
     partials = None
     if splits > 1:          # of this call alone, on its own stream
-        partials = torch.empty(_simt_rows(n_tiles, q_heads, kv_heads, vdim, max_q_len)[1] * chunk_room * (vdim + 2),
-                               dtype=torch.float32, device=q.device)
+        partials = torch.empty(blocks * rows * chunk_room * (vdim + 2), dtype=torch.float32, device=q.device)
     fn = _FUNCTIONS.get("lb_attention_simt") or _fn("attention_simt", "lb_attention_simt",
              [c_int] + [c_void_p] * 5 + [c_int] + [c_void_p] * 4 + [c_int] * 5 + [c_float, c_int, c_int, c_void_p,
-              c_void_p, c_int, c_int, c_float, c_float, c_long, c_int, c_int, c_void_p, c_int, c_void_p])
+              c_void_p, c_int, c_int, c_float, c_float, c_long, c_int, c_int, c_int, c_void_p, c_int, c_void_p])
     _check(fn(dtype_code(q.dtype), q_ptr, _ptr(k_pool), _ptr(v_pool), _ptr(out), _ptr(block_table),
               block_table.shape[1], _ptr(cu_q), _ptr(ctx_len), _ptr(tile_seq), _ptr(tile_q0), n_tiles, q_heads,
               kv_heads, dim, page_tokens, float(scale), int(window), vdim, _ptr(sinks), _ptr(gates), int(chunk), int(keep_first),
-              float(softcap), float(out_scale), out.stride(0), max_q_len, splits, _ptr(partials), chunk_room, _stream()),
+              float(softcap), float(out_scale), out.stride(0), max_q_len, rows, splits, _ptr(partials), chunk_room, _stream()),
            "attention_simt")
     if splits > 1:
         global LAUNCHES
@@ -1223,29 +1223,23 @@ def attention_simt(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, 
     return out
 
 
-def _simt_rows(n_tiles: int, q_heads: int, kv_heads: int, vdim: int, max_q_len: int) -> tuple[int, int]:
-    """(blocks, rows over all blocks) of the 32-bit attention kernel without a split."""
-    rows = c_int(0)
-    fn = _FUNCTIONS.get("lb_attention_simt_plan") or _fn("attention_simt", "lb_attention_simt_plan", [c_int] * 5 + [c_void_p])
-    blocks = fn(n_tiles, q_heads, kv_heads, vdim, max_q_len, ctypes.addressof(rows))
-    return blocks, blocks * rows.value
-
-
 _SIMT_SCRATCH_FLOATS = 64 << 20     # the most that the chunks' results may take (256 MiB)
 
 
 @functools.lru_cache(maxsize=1024)      # of the sizes alone, asked for by every layer of a step
-def _simt_splits(n_tiles: int, q_heads: int, kv_heads: int, vdim: int, max_q_len: int, max_ctx: int, room_tokens: int,
-                 device: torch.device) -> tuple[int, int]:
-    """(blocks that share a row's keys, chunks there must be room for): three blocks an SM where the rows alone do not give
-    them, as far as there are chunks to share."""
+def _simt_plan(n_tiles: int, q_heads: int, kv_heads: int, dim: int, vdim: int, max_q_len: int, max_ctx: int, room_tokens: int,
+               device: torch.device) -> tuple[int, int, int, int]:
+    """(blocks that share a row's keys, chunks there must be room for, blocks without a split, rows of a block): three blocks an
+    SM where the rows alone do not give them, as far as there are chunks to share."""
     keys = (_FUNCTIONS.get("lb_attention_simt_chunk") or _fn("attention_simt", "lb_attention_simt_chunk", []))()
-    blocks, rows = _simt_rows(n_tiles, q_heads, kv_heads, vdim, max_q_len)
-    room = -(-room_tokens // keys)
-    splits = min(-(-max_ctx // keys), -(-3 * sm_count(device) // max(blocks, 1)), room)
-    if splits <= 1 or rows * room * (vdim + 2) > _SIMT_SCRATCH_FLOATS:
-        return 1, 0
-    return splits, room
+    plan = _FUNCTIONS.get("lb_attention_simt_plan") or _fn("attention_simt", "lb_attention_simt_plan", [c_int] * 8 + [c_void_p])
+    rows, sms, room = c_int(0), sm_count(device), -(-room_tokens // keys)
+    chunks = min(-(-max_ctx // keys), room)
+    blocks = plan(n_tiles, q_heads, kv_heads, dim, vdim, max_q_len, chunks, sms, ctypes.addressof(rows))
+    splits = min(chunks, -(-3 * sms // max(blocks, 1)))
+    if splits <= 1 or blocks * rows.value * room * (vdim + 2) > _SIMT_SCRATCH_FLOATS:
+        splits, room = 1, 0
+    return splits, room, blocks, rows.value
 
 
 def attention_f32(q, cache, out, block_table, batch, q_heads, kv_heads, dim, page_tokens, scale, window, vdim=None,

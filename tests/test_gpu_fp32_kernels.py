@@ -171,3 +171,29 @@ def test_f32_attention_of_queries_that_begin_anywhere(dtype, dim):
     for k, v in ((shifted(k_pool), v_pool), (k_pool, shifted(v_pool))):
         with pytest.raises(ValueError, match="alignment"):
             run(q, k, v)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("q_heads, kv_heads, dim, vdim", [(40, 2, 16, 16), (32, 1, 128, 128), (12, 1, 64, 200), (12, 1, 300, 512)])
+def test_f32_attention_has_the_same_bits_however_many_rows_share_a_warp(monkeypatch, dtype, q_heads, kv_heads, dim, vdim):
+    o, page, lengths, q_lens = ops(), 16, [1, 40, 300, 520], [1, 5, 1, 18]
+    k_pool, _, table, _, _ = paged_setup(dtype, lengths, kv_heads, dim, page, 5)
+    _, v_pool, _, _, _ = paged_setup(dtype, lengths, kv_heads, vdim, page, 5)
+    tokens, ints = sum(q_lens), lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    q = torch.randn(tokens, q_heads * dim, generator=torch.Generator().manual_seed(2)).to(dtype).cuda()
+    tiles = [(s, q0) for s, n in enumerate(q_lens) for q0 in range(0, n, 16)]
+    rows_seen, outs, plan = set(), [], o._simt_plan
+    for sms in (0, 1 << 20):          # a device with no room and one with room for everything
+        def planned(*args):
+            splits, room, _, _ = plan(*args)
+            rows = o.c_int(0)
+            blocks = o._FUNCTIONS["lb_attention_simt_plan"](len(tiles), q_heads, kv_heads, dim, vdim, 18, 5, sms, o.ctypes.addressof(rows))
+            rows_seen.add(rows.value)
+            return splits, room, blocks, rows.value
+        monkeypatch.setattr(o, "_simt_plan", planned)
+        for max_ctx in (0, 520):
+            out = torch.full((tokens, q_heads * vdim), float("nan"), dtype=dtype, device="cuda")
+            o.attention_simt(q, k_pool, v_pool, out, table, ints([0, 1, 6, 7, 25]), ints(lengths), ints([t[0] for t in tiles]),
+                             ints([t[1] for t in tiles]), len(tiles), q_heads, kv_heads, dim, page, dim ** -0.5, vdim=vdim, max_q_len=18, max_ctx=max_ctx)
+            outs.append(out)
+    assert len(rows_seen) == 2 and not torch.isnan(outs[0]).any() and all(torch.equal(outs[0], out) for out in outs[1:])

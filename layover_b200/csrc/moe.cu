@@ -856,16 +856,21 @@ static void launch_route(const void* h, const float* router, const float* shared
                    (uintptr_t)h % 16 == 0;
 #define LB_ROUTE_ARGS (const T*)h, router, shared_w, ids, scores, shared_factor, tokens, hidden, experts, top, opt
   const size_t per_token = (size_t)(experts + (opt.general() ? experts + opt.groups : 0)) * sizeof(float);
+  const int n_rows = experts + (shared_w ? 1 : 0);
   // few tokens: a block of 32 warps each (a warp an expert or two), so that the step's latency is about one dot product's;
-  // many: eight a block share every weight they read
+  // many: eight a block share every weight they read. A warp takes one row of the router where the block has a warp for
+  // each (us with one, with several, one B200): 2,048 channels, one token, 32-bit, 32 experts 6.3 and 8.0, bfloat16, 12 experts 4.8
+  // and 5.1 (24: 5.6 both); 65 tokens, 8 experts of 512 channels 5.6 and 8.3, but 1,222 tokens of 4,096 channels 19.2 and 17.4
   if (tokens <= 64) {
     const size_t smem = per_token;
-    if (vec) lb_launch(moe_route_kernel<T, 1, 32, 2, true>, tokens, 1024, smem, stream, LB_ROUTE_ARGS);
+    if (vec && n_rows <= (sizeof(T) == 4 ? 32 : 16)) lb_launch(moe_route_kernel<T, 1, 32, 1, true>, tokens, 1024, smem, stream, LB_ROUTE_ARGS);
+    else if (vec) lb_launch(moe_route_kernel<T, 1, 32, 2, true>, tokens, 1024, smem, stream, LB_ROUTE_ARGS);
     else lb_launch(moe_route_kernel<T, 1, 32, 2, false>, tokens, 1024, smem, stream, LB_ROUTE_ARGS);
   } else {
     const size_t smem = 8 * per_token;
     const int blocks = (tokens + 7) / 8;
-    if (vec) lb_launch(moe_route_kernel<T, 8, 8, 4, true>, blocks, 256, smem, stream, LB_ROUTE_ARGS);
+    if (vec && sizeof(T) == 2 && n_rows <= 8 && hidden < 4096) lb_launch(moe_route_kernel<T, 8, 8, 1, true>, blocks, 256, smem, stream, LB_ROUTE_ARGS);
+    else if (vec) lb_launch(moe_route_kernel<T, 8, 8, 4, true>, blocks, 256, smem, stream, LB_ROUTE_ARGS);
     else lb_launch(moe_route_kernel<T, 8, 8, 4, false>, blocks, 256, smem, stream, LB_ROUTE_ARGS);
   }
 #undef LB_ROUTE_ARGS

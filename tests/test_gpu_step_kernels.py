@@ -315,3 +315,26 @@ def test_segments_as_products_refuse_heads_that_a_block_does_not_hold():
     scratch = torch.zeros(5, 1, 192, 192, device="cuda")
     with pytest.raises(ValueError):
         o.decay_scan(proj, 0, 192, 384, out, state, ints([0, 300]), ints([0]), torch.ones(1, device="cuda"), 1, 1, 192, 192, None, 64, scratch, True)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("experts, shared", [(7, True), (8, False), (8, True), (15, True), (16, True), (31, True), (32, True), (40, False)])
+@pytest.mark.parametrize("hidden", [512, 4096, 1001])
+def test_router_gives_a_token_the_same_bits_in_every_batch(dtype, experts, shared, hidden):
+    """One, two and four rows of the router a warp: on both sides of where each is taken."""
+    o, gen = ops(), torch.Generator().manual_seed(experts + hidden)
+    h = torch.randn(70, hidden, generator=gen).to(dtype).cuda()
+    router = torch.randn(experts, hidden, generator=gen).cuda() / math.sqrt(hidden)
+    gate = torch.randn(hidden, generator=gen).cuda() / math.sqrt(hidden) if shared else None
+    results = []
+    for tokens in (70, 64, 1):
+        ids, scores = torch.empty(tokens, 3, dtype=torch.int32, device="cuda"), torch.empty(tokens, 3, device="cuda")
+        factor = torch.empty(tokens, device="cuda") if shared else None
+        o.moe_route(h[:tokens], router, 3, ids, scores, gate, factor)
+        results.append((ids, scores) + ((factor,) if shared else ()))
+    for got in results[1:]:
+        assert all(torch.equal(a[: b.shape[0]], b) for a, b in zip(results[0], got))
+    chosen = torch.gather(h.double() @ router.double().T, 1, results[0][0].long())
+    # a lane's chain of at most hidden / 32 + 8 products and five sums, each off by 2^-24 of the terms' absolute sum; a sigmoid's slope is 1/4
+    bound = (hidden / 32 + 13) * 2.0 ** -26 * torch.gather(h.double().abs() @ router.double().abs().T, 1, results[0][0].long()) + 2.0 ** -22
+    assert ((results[0][1].double() - torch.sigmoid(chosen)).abs() <= bound).all()

@@ -875,33 +875,35 @@ template <typename Kernel> void allow_smem(Kernel kernel, size_t bytes) {
 }
 void configure_once() {      // once per device: the attribute belongs to the device that is current
   static LbPerDeviceOnce once;
-  if (!once.first()) return;
-  allow_smem(attention_prefill_kernel<128, true>, prefill_smem(128));
-  allow_smem(attention_prefill_kernel<128, false>, prefill_smem(128));
-  allow_smem(attention_prefill_kernel<256, true>, prefill_smem(256));
-  allow_smem(attention_prefill_kernel<256, false>, prefill_smem(256));
-  allow_smem(attention_decode_kernel<128, true, false>, decode_smem(128));
-  allow_smem(attention_decode_kernel<128, true, true>, decode_smem(128));
-  allow_smem(attention_decode_kernel<128, false, true>, decode_smem(128));
-  allow_smem(attention_decode_kernel<256, true, true>, decode_smem(256));
-  allow_smem(attention_decode_kernel<256, false, true>, decode_smem(256));
-  allow_smem(attention_decode_kernel<128, true, false, true>, decode_smem(128));
-  allow_smem(attention_decode_kernel<128, true, true, true>, decode_smem(128));
-  // clusters of 16 blocks (one sequence's context cut 16 ways) are beyond the portable size of 8
-  cudaFuncSetAttribute(attention_decode_kernel<128, true, false, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  cudaFuncSetAttribute(attention_decode_kernel<128, true, true, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  cudaGetLastError();
-  allow_smem(attention_decode_kernel<128, true, false, false, 2>, decode_smem(128, 2));
-  allow_smem(attention_decode_kernel<128, true, false, true, 2>, decode_smem(128, 2));
-  allow_smem(attention_prefill_kernel<128, true, true>, prefill_smem(128));
-  allow_smem(attention_prefill_kernel<128, false, true>, prefill_smem(128));
-  allow_smem(attention_prefill_kernel<256, true, true>, prefill_smem(256));
-  allow_smem(attention_prefill_kernel<256, false, true>, prefill_smem(256));
-  allow_smem(attention_decode_kernel<128, true, true, false, 3, true>, decode_smem(128));
-  allow_smem(attention_decode_kernel<128, true, false, false, 3, true>, decode_smem(128));
-  allow_smem(attention_decode_kernel<128, false, true, false, 3, true>, decode_smem(128));
-  allow_smem(attention_decode_kernel<256, true, true, false, 3, true>, decode_smem(256));
-  allow_smem(attention_decode_kernel<256, false, true, false, 3, true>, decode_smem(256));
+  once.run([] {
+    allow_smem(attention_prefill_kernel<128, true>, prefill_smem(128));
+    allow_smem(attention_prefill_kernel<128, false>, prefill_smem(128));
+    allow_smem(attention_prefill_kernel<256, true>, prefill_smem(256));
+    allow_smem(attention_prefill_kernel<256, false>, prefill_smem(256));
+    allow_smem(attention_decode_kernel<128, true, false>, decode_smem(128));
+    allow_smem(attention_decode_kernel<128, true, true>, decode_smem(128));
+    allow_smem(attention_decode_kernel<128, false, true>, decode_smem(128));
+    allow_smem(attention_decode_kernel<256, true, true>, decode_smem(256));
+    allow_smem(attention_decode_kernel<256, false, true>, decode_smem(256));
+    allow_smem(attention_decode_kernel<128, true, false, true>, decode_smem(128));
+    allow_smem(attention_decode_kernel<128, true, true, true>, decode_smem(128));
+    // clusters of 16 blocks (one sequence's context cut 16 ways) are beyond the portable size of 8
+    cudaFuncSetAttribute(attention_decode_kernel<128, true, false, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaFuncSetAttribute(attention_decode_kernel<128, true, true, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaGetLastError();
+    allow_smem(attention_decode_kernel<128, true, false, false, 2>, decode_smem(128, 2));
+    allow_smem(attention_decode_kernel<128, true, false, true, 2>, decode_smem(128, 2));
+    allow_smem(attention_prefill_kernel<128, true, true>, prefill_smem(128));
+    allow_smem(attention_prefill_kernel<128, false, true>, prefill_smem(128));
+    allow_smem(attention_prefill_kernel<256, true, true>, prefill_smem(256));
+    allow_smem(attention_prefill_kernel<256, false, true>, prefill_smem(256));
+    allow_smem(attention_decode_kernel<128, true, true, false, 3, true>, decode_smem(128));
+    allow_smem(attention_decode_kernel<128, true, false, false, 3, true>, decode_smem(128));
+    allow_smem(attention_decode_kernel<128, false, true, false, 3, true>, decode_smem(128));
+    allow_smem(attention_decode_kernel<256, true, true, false, 3, true>, decode_smem(256));
+    allow_smem(attention_decode_kernel<256, false, true, false, 3, true>, decode_smem(256));
+    return true;      // a limit that was refused shows at the launch
+  });
 }
 
 // the variants with sinks, gates and split weights: three stages, merged through scratch memory

@@ -421,9 +421,8 @@ template <typename T, int NV, int R>
 int launch_rows(Attention<T> a, int n_tiles, int max_rows, int splits, cudaStream_t stream) {
   constexpr int ROWS = WARPS * R;
   static LbPerDeviceOnce configured;
-  if (configured.first() &&
-      cudaFuncSetAttribute(attention_rows_kernel<T, NV, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
-    return lb_last_error();
+  auto kernel = attention_rows_kernel<T, NV, R>;
+  if (!configured.run(LB_ALLOW_SMEM(kernel, 227 * 1024))) return lb_last_error();
   a.row_groups = (max_rows + ROWS - 1) / ROWS;
   auto smem = [&](int stages) { return block_smem(ROWS, stages, a.dim, a.key_pitch, a.vdim); };
   a.stages = sizeof(T) == 4 && smem(2) <= 227 * 1024 ? 2 : 1;      // a copy that converts is not asynchronous: a second stage waits all the same

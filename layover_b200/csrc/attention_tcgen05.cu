@@ -911,11 +911,13 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 
 void configure_once() {      // once per device: the attribute belongs to the device that is current
   static LbPerDeviceOnce once;
-  if (!once.first()) return;
-  cudaFuncSetAttribute(attention_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-  cudaFuncSetAttribute(attention_tcgen05_pair_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
-  cudaFuncSetAttribute(attention_tcgen05_pair_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
-  cudaFuncSetAttribute(attention_tcgen05_pair_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
+  once.run([] {
+    cudaFuncSetAttribute(attention_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    cudaFuncSetAttribute(attention_tcgen05_pair_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
+    cudaFuncSetAttribute(attention_tcgen05_pair_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
+    cudaFuncSetAttribute(attention_tcgen05_pair_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
+    return true;      // a limit that was refused shows at the launch
+  });
 }
 
 // q as a 2-D bf16 matrix [rows, cols] with rows `stride` elements apart: box 64 columns x 128 rows

@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "once.h"
+
 #define LB_EXPORT extern "C" __attribute__((visibility("default")))
 
 enum LbDtype { LB_F32 = 0, LB_BF16 = 1 };
@@ -75,24 +77,7 @@ __device__ __forceinline__ float block_sum(float v, float* scratch /* >= 33 floa
 
 static inline int lb_last_error() { return (int)cudaGetLastError(); }
 
-// Function attributes (the raised shared-memory limit of a kernel) belong to a device, not to the
-// process: `first()` is true once per device, for the device that is current at the call.
-struct LbPerDeviceOnce {
-  static constexpr int MAX_DEVICES = 64;
-  bool done[MAX_DEVICES] = {};
-  int current() const {
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= MAX_DEVICES) return -1;
-    return device;
-  }
-  bool first() {
-    const int device = current();
-    if (device < 0) return true;          // unknown device: configure again rather than not at all
-    if (done[device]) return false;
-    done[device] = true;
-    return true;
-  }
-};
+// Function attributes (the raised shared-memory limit of a kernel) belong to a device, not to the process: see once.h.
 
 // ---- programmatic dependent launch
 // Every kernel of this package is launched so that it may start while its predecessor in the

@@ -670,10 +670,9 @@ static int launch_residual_rmsnorm(float* x, const void* delta, const float* del
   static LbPerDeviceOnce once;
   const size_t smem = (size_t)(hidden + 33) * sizeof(float);
   if (smem > 200 * 1024) return LB_ERR_SIZE;
-  if (smem > 48 * 1024 && once.first()) {
-    cudaFuncSetAttribute(residual_rmsnorm_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(residual_rmsnorm_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  }
+  auto fast = residual_rmsnorm_kernel<T, true>, plain = residual_rmsnorm_kernel<T, false>;
+  if (smem > 48 * 1024 && !once.run([&] { return LB_ALLOW_SMEM(fast, 200 * 1024)() && LB_ALLOW_SMEM(plain, 200 * 1024)(); }))
+    return lb_last_error();
   // the form, like the block size, depends on the width and the buffers' alignment only, never on the batch
   const bool vec = hidden % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)delta % 16 == 0 && (uintptr_t)extra % 16 == 0 &&
                    (uintptr_t)out % 16 == 0 && (uintptr_t)delta_w % 16 == 0 && (uintptr_t)weight % 16 == 0;
@@ -873,10 +872,9 @@ static int launch_residual_layernorm(float* x, const void* delta_a, const void* 
   static LbPerDeviceOnce once;
   const size_t smem = (size_t)(hidden + 33) * sizeof(float);
   if (smem > 200 * 1024) return LB_ERR_SIZE;
-  if (smem > 48 * 1024 && once.first()) {
-    cudaFuncSetAttribute(residual_layernorm_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(residual_layernorm_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  }
+  auto fast = residual_layernorm_kernel<T, true>, plain = residual_layernorm_kernel<T, false>;
+  if (smem > 48 * 1024 && !once.run([&] { return LB_ALLOW_SMEM(fast, 200 * 1024)() && LB_ALLOW_SMEM(plain, 200 * 1024)(); }))
+    return lb_last_error();
   const bool vec = hidden % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)delta_a % 16 == 0 && (uintptr_t)delta_b % 16 == 0 &&
                    (uintptr_t)out % 16 == 0 && (uintptr_t)weight % 16 == 0 && (uintptr_t)bias % 16 == 0;
   const int threads = hidden >= 4096 ? 512 : (hidden >= 1024 ? 256 : 128);
@@ -1311,8 +1309,8 @@ static int launch_scaled_add_rmsnorm(float* x, const void* a, const float* a_w, 
   static LbPerDeviceOnce once;
   const size_t smem = (size_t)(hidden + 33) * sizeof(float);
   if (smem > 200 * 1024) return LB_ERR_SIZE;
-  if (smem > 48 * 1024 && once.first())
-    cudaFuncSetAttribute(scaled_add_rmsnorm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  auto kernel = scaled_add_rmsnorm_kernel<T>;
+  if (smem > 48 * 1024 && !once.run(LB_ALLOW_SMEM(kernel, 200 * 1024))) return lb_last_error();
   const int threads = hidden >= 4096 ? 512 : (hidden >= 1024 ? 256 : 128);
   lb_launch(scaled_add_rmsnorm_kernel<T>, n_rows, threads, smem, stream, x, (const T*)a, a_w, (const T*)b, b_w, part_eps, factor,
             alpha, weight, eps, (T*)out, hidden);

@@ -601,9 +601,8 @@ template <int TOKENS>
 int launch_few(const Product& p) {
   using F = Few<TOKENS>;
   static LbPerDeviceOnce configured;
-  if (configured.first() &&
-      cudaFuncSetAttribute(gemm_f32_few_kernel<TOKENS>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM) != cudaSuccess)
-    return lb_last_error();
+  auto kernel = gemm_f32_few_kernel<TOKENS>;
+  if (!configured.run(LB_ALLOW_SMEM(kernel, F::SMEM))) return lb_last_error();
   CUtensorMap map_w, map_a;
   if (!make_map_f32(&map_w, p.W, p.N, p.K, p.ldw, FEW_ROWS, true) || !make_map_f32(&map_a, p.A, p.M, p.K, p.lda, TOKENS, false))
     return LB_ERR_ALIGN;
@@ -656,9 +655,8 @@ template <int TM>
 int launch_many(const Product& p) {
   using T = Many<TM>;
   static LbPerDeviceOnce configured;
-  if (configured.first() &&
-      cudaFuncSetAttribute(gemm_f32_many_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM) != cudaSuccess)
-    return lb_last_error();
+  auto kernel = gemm_f32_many_kernel<TM>;
+  if (!configured.run(LB_ALLOW_SMEM(kernel, T::SMEM))) return lb_last_error();
   CUtensorMap map_w, map_a;
   if (!make_map_f32(&map_w, p.W, p.N, p.K, p.ldw, MANY_COLS, true) || !make_map_f32(&map_a, p.A, p.M, p.K, p.lda, T::ROWS, true))
     return LB_ERR_ALIGN;

@@ -973,13 +973,17 @@ int launch(const CUtensorMap& map_a, const CUtensorMap& map_b, void* C, long ldc
   auto kernel = gemm_tcgen05_kernel<BN, SWAP, OutT, EPI>;
   static int blocks_per_sm = 0;      // how many blocks of this kernel an SM really holds (the same on every B200)
   static LbPerDeviceOnce configured;
-  if (configured.first()) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM) != cudaSuccess)
-      return lb_last_error();
+  const bool ready = configured.run([&] {
     int fit = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, PERSISTENT_THREADS, T::SMEM) != cudaSuccess || fit < 1)
-      return lb_last_error() ? lb_last_error() : LB_ERR_SIZE;
+    if (!LB_ALLOW_SMEM(kernel, T::SMEM)() ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, PERSISTENT_THREADS, T::SMEM) != cudaSuccess || fit < 1)
+      return false;
     blocks_per_sm = fit < T::BLOCKS_PER_SM ? fit : T::BLOCKS_PER_SM;
+    return true;
+  });
+  if (!ready) {
+    const int code = lb_last_error();
+    return code ? code : LB_ERR_SIZE;
   }
   // Blocks that split a tile wait for one another, so a launch never has more blocks than the GPU
   // holds at once.
@@ -1047,9 +1051,8 @@ int launch_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, void* C, lon
   auto kernel = gemm_tcgen05_kernel<BN, false, OutT, EPI, true>;
   static int pairs_resident = 0;      // clusters of two that the GPU holds at once (the same on every B200)
   static LbPerDeviceOnce configured;
-  if (configured.first()) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM) != cudaSuccess)
-      return lb_last_error();
+  const bool ready = configured.run([&] {
+    if (!LB_ALLOW_SMEM(kernel, T::SMEM)()) return false;
     cudaLaunchConfig_t probe = {};
     probe.gridDim = dim3(2 * pb.sm_count);
     probe.blockDim = dim3(persistent_threads(EPI));
@@ -1064,7 +1067,9 @@ int launch_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, void* C, lon
     int fit = 0;
     if (cudaOccupancyMaxActiveClusters(&fit, kernel, &probe) != cudaSuccess) { cudaGetLastError(); fit = 0; }
     pairs_resident = fit;
-  }
+    return true;
+  });
+  if (!ready) return lb_last_error();
   // Blocks that split a tile wait for one another, so a launch never has more pairs than the GPU
   // holds at once.
   const int slots = pairs_resident < pb.sm_count / 2 ? pairs_resident : pb.sm_count / 2;
@@ -1111,10 +1116,7 @@ int launch_fewtoken(const CUtensorMap& map_a, const CUtensorMap& map_b, void* C,
   using T = SmallTile<BN>;
   auto kernel = gemm_fewtoken_kernel<BN, OutT, EPI>;
   static LbPerDeviceOnce configured;
-  if (configured.first()) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM) != cudaSuccess)
-      return lb_last_error();
-  }
+  if (!configured.run(LB_ALLOW_SMEM(kernel, T::SMEM))) return lb_last_error();
   const int tiles = (pb.rows_a + BM - 1) / BM, total_kb = (pb.K + BK - 1) / BK;
   int splits = 1;
   if (EPI == 0 && pb.scratch && pb.counters && tiles <= pb.n_counters && tiles < pb.sm_count) {
@@ -1142,10 +1144,7 @@ int launch_fewtoken(const CUtensorMap& map_a, const CUtensorMap& map_b, void* C,
       // the K ranges of a tile as one cluster: partial sums travel through distributed shared memory
       auto cluster_kernel = gemm_fewtoken_kernel<BN, OutT, EPI, true>;
       static LbPerDeviceOnce cluster_configured;
-      if (cluster_configured.first()) {
-        if (cudaFuncSetAttribute(cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM_CLUSTER) != cudaSuccess)
-          return lb_last_error();
-      }
+      if (!cluster_configured.run(LB_ALLOW_SMEM(cluster_kernel, T::SMEM_CLUSTER))) return lb_last_error();
       const int code = lb_launch_cluster(cluster_kernel, grid, dim3(SMALL_THREADS), (size_t)T::SMEM_CLUSTER, stream,
                                          (unsigned)splits, map_a, map_b, (OutT*)C, ldc, pb.rows_a, pb.rows_b, pb.K,
                                          splits, (float*)nullptr, (unsigned*)nullptr, HeadsEpilogue{}, clip);
@@ -1172,10 +1171,7 @@ int launch_heads(const CUtensorMap& map_a, const CUtensorMap& map_b, const Probl
   if (splits < 2 || !lb_cluster_reduce_enabled()) return 1;
   auto kernel = gemm_fewtoken_kernel<BN, bf16, 2, true>;
   static LbPerDeviceOnce configured;
-  if (configured.first()) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM_CLUSTER) != cudaSuccess)
-      return lb_last_error();
-  }
+  if (!configured.run(LB_ALLOW_SMEM(kernel, T::SMEM_CLUSTER))) return lb_last_error();
   dim3 grid(tiles, 1, splits);
   const int code = lb_launch_cluster(kernel, grid, dim3(SMALL_THREADS), (size_t)T::SMEM_CLUSTER, stream, (unsigned)splits,
                                      map_a, map_b, (bf16*)nullptr, 0L, pb.rows_a, pb.rows_b, pb.K, splits, (float*)nullptr,

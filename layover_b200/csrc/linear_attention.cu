@@ -470,9 +470,8 @@ int launch_segments(int n_seqs, int total_segments, int seg_tokens, float* seg_s
                     const int* state_slots, const float* decay, int heads, int dim, int vdim) {
   constexpr int smem = (2 * SEG_ROWS * SEG_PITCH + SEG_ROWS * (SEG_ROWS + 4)) * (int)sizeof(float);
   static LbPerDeviceOnce once;
-  if (once.first() &&
-      cudaFuncSetAttribute(segment_output_kernel<T, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-    return lb_last_error();
+  auto kernel = segment_output_kernel<T, ACT>;
+  if (!once.run(LB_ALLOW_SMEM(kernel, smem))) return lb_last_error();
   const int e_tiles = (vdim + 127) / 128, row_blocks = (seg_tokens + SEG_ROWS - 1) / SEG_ROWS, per_head = dim * vdim;
   // four channels at a time where every head's rows start on four elements' boundaries
   const bool vec = (uintptr_t)proj % (4 * sizeof(T)) == 0 && row_stride % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && v_off % 4 == 0 &&
@@ -495,8 +494,8 @@ int launch_scan_mode(dim3 grid, cudaStream_t stream, const void* proj, long row_
   // q and k twice (two buffers), v twice, the warps' partial sums
   constexpr size_t smem = (size_t)(4 * CHUNK * RANGES * DPT + 2 * CHUNK * COLS + CHUNK * RANGES * COLS) * sizeof(float);
   static LbPerDeviceOnce once;
-  if (smem > 48 * 1024 && once.first())
-    cudaFuncSetAttribute(decay_scan_kernel<T, RANGES, DPT, ACT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto kernel = decay_scan_kernel<T, RANGES, DPT, ACT, MODE>;
+  if (smem > 48 * 1024 && !once.run(LB_ALLOW_SMEM(kernel, smem))) return lb_last_error();
   lb_launch(decay_scan_kernel<T, RANGES, DPT, ACT, MODE>, grid, RANGES * COLS, smem, stream, (const T*)proj, row_stride, q_off,
             k_off, v_off, out, state, cu_q, state_slots, decay, heads, dim, vdim, seg_state, seg_tokens, n_seqs);
   return lb_last_error();

@@ -305,10 +305,8 @@ int launch_scan(const float* r, long r_stride, const float* k, long k_stride, co
   constexpr int GROUPS = RANGES * (32 / COLS);
   constexpr size_t smem = (size_t)(2 * 3 * CHUNK * GROUPS * DPT + 2 * CHUNK * COLS + CHUNK * GROUPS * COLS) * sizeof(float);
   static LbPerDeviceOnce once;
-  if (smem > 48 * 1024 && once.first()) {
-    cudaFuncSetAttribute(wkv_scan_kernel<DPT, COLS, true, AFTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(wkv_scan_kernel<DPT, COLS, false, AFTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  }
+  auto fast = wkv_scan_kernel<DPT, COLS, true, AFTER>, plain = wkv_scan_kernel<DPT, COLS, false, AFTER>;
+  if (smem > 48 * 1024 && !once.run([&] { return LB_ALLOW_SMEM(fast, smem)() && LB_ALLOW_SMEM(plain, smem)(); })) return lb_last_error();
   const bool vec = dim % 4 == 0 && r_stride % 4 == 0 && k_stride % 4 == 0 && (uintptr_t)r % 16 == 0 && (uintptr_t)k % 16 == 0 &&
                    (uintptr_t)w % 16 == 0;
   if (vec) lb_launch(wkv_scan_kernel<DPT, COLS, true, AFTER>, grid, SCAN_THREADS, smem, stream, r, r_stride, k, k_stride, v, v_stride, w, u, out, state,

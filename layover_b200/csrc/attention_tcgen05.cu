@@ -990,7 +990,7 @@ LB_EXPORT int lb_attention_tcgen05_prefill(const void* q, long q_rows, const voi
   if (n_tiles <= 0) return 0;
   if (!lb_attention_tcgen05_supports(q_heads, kv_heads, dim, page_tokens) || n_tiles > 65535) return LB_ERR_SIZE;
   if (splits < 1 || splits > 32 || (splits > 1 && (!partials || exact || (q_heads / kv_heads) % 2))) return LB_ERR_SIZE;
-  if (exact ? (q_heads / kv_heads) % 2 || out_stride < (long)q_heads * dim : sinks || gates || window < 0 || out_scale != 1.f) return LB_ERR_SIZE;
+  if (exact ? (q_heads / kv_heads) % 2 || out_stride < (long)q_heads * dim : sinks || gates || out_scale != 1.f) return LB_ERR_SIZE;
   if (exact && (out_stride % 8 || (uintptr_t)out % 16)) return LB_ERR_ALIGN;
   if ((uintptr_t)q % 16) return LB_ERR_ALIGN;
   configure_once();

@@ -338,3 +338,19 @@ def test_router_gives_a_token_the_same_bits_in_every_batch(dtype, experts, share
     # a lane's chain of at most hidden / 32 + 8 products and five sums, each off by 2^-24 of the terms' absolute sum; a sigmoid's slope is 1/4
     bound = (hidden / 32 + 13) * 2.0 ** -26 * torch.gather(h.double().abs() @ router.double().abs().T, 1, results[0][0].long()) + 2.0 ** -22
     assert ((results[0][1].double() - torch.sigmoid(chosen)).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("q_heads, kv_heads", [(4, 2), (3, 1)])
+def test_plain_prompt_attention_takes_a_negative_window_as_none(q_heads, kv_heads):
+    """A chunked mask is the exact variant's; without it a window that is not positive masks nothing."""
+    o, dim, page, lengths, q_lens = ops(), 128, 16, [40, 300], [40, 130]
+    k_pool, v_pool, table, _, _ = paged_setup(torch.bfloat16, lengths, kv_heads, dim, page, 3)
+    pool = torch.stack((k_pool, v_pool))[None].contiguous()
+    q = torch.randn(170, q_heads * dim, generator=torch.Generator().manual_seed(4)).to(torch.bfloat16).cuda()
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    outs = []
+    for window in (0, -64):
+        outs.append(torch.full_like(q, float("nan")))
+        o.attention_tcgen05_prefill(q, pool, 0, outs[-1], table, ints([0, 40, 170]), ints(lengths), ints([0, 1, 1]), ints([0, 0, 128]), 3,
+                                    q_heads, kv_heads, dim, page, dim ** -0.5, window)
+    assert not torch.isnan(outs[0]).any() and torch.equal(*outs)

@@ -549,8 +549,8 @@ __device__ __forceinline__ void warp_keys(const uint32_t (&qf)[4][4], uint32_t k
 // in split order and store them.
 // STAGES: K/V tiles of a block in shared memory. Three keep a block's own stream going (two loads in
 // flight); with two a block is slower but three blocks share an SM instead of two, which wins once a
-// launch has more blocks than two per SM can hold at once and the lengths differ (64 sequences of 350 .. 3,100 keys in 4 splits:
-// 80 us against 88 us; of 3,072 keys each 131 us, and 123 us unsplit with three stages).
+// launch has more blocks than two per SM can hold at once and the lengths differ (40 sequences of 0.1 .. 1 of 8,192 keys in 4
+// splits 122 us, unsplit with three stages 147; 64 equally long ones of 3,072 keys 131 us, and 123 unsplit with three).
 // SINK: as in the prefill kernel; the sink joins the denominator once, where the splits have been merged.
 template <int MAX_DIM, bool EXACT, bool UPPER, bool CLUSTER = false, int STAGES = 3, bool SINK = false>
 __global__ void __launch_bounds__(THREADS, STAGES == 2 ? 3 : 2)

@@ -80,9 +80,9 @@ static inline int lb_last_error() { return (int)cudaGetLastError(); }
 // Function attributes (the raised shared-memory limit of a kernel) belong to a device, not to the process: see once.h.
 
 // ---- programmatic dependent launch
-// Every kernel of this package is launched so that it may start while its predecessor in the
-// stream is still running: its blocks set themselves up (and a matrix product already streams
-// weights, which no kernel writes) and then wait in `pdl_wait()` until the predecessor has
+// A kernel of this package is launched so that it may start while its predecessor in the
+// stream is still running (but for those of `lb_launch_settled`): its blocks set themselves up (and
+// a matrix product already streams weights that no kernel is writing) and then wait in `pdl_wait()` until the predecessor has
 // finished and its writes are visible. Every kernel calls `pdl_wait()` before it touches memory
 // that an earlier kernel wrote or that a later kernel may still read, so completion is
 // transitive along the stream. LAYOVER_B200_PDL=0 launches the plain way.

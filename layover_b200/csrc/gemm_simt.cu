@@ -6,7 +6,8 @@
 // token's result does not depend on how a batch was cut. For 32-bit operands K is cut into the ranges of `Split`, which
 // depend on K alone; a range is one sequential chain of fused multiply-adds from zero, the sums of four neighbouring ranges
 // are added in order, and then the sums of those groups are. Ranges may therefore run one after the other, in the lanes
-// of a warp or in different blocks, with the same bits. For bf16 operands there is one chain over the whole of K. Any M, N, K >= 1 is accepted: operands whose
+// of a warp or in different blocks, with the same bits. For bf16 operands there is one chain over the whole of K. Any
+// M, N, K >= 1 is accepted: operands whose
 // address and stride TMA can take go through the streaming kernels, others through the plain tiles, with the same bits.
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -440,13 +441,16 @@ gemm_f32_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 }
 
 // More tokens: tiles of 8 TM tokens x 64 weight rows, 128 threads with TM x 4 sums each, a ring of stages of 32 k filled with
-// TMA by one thread. A thread reads four k of TM + 4 rows and does 16 TM fused multiply-adds with them. The FFMA pipes and
-// what the register file can feed them are the bound (a loop of nothing but three-register FFMAs reaches 55 TFLOP/s);
-// three blocks an SM of 32 sums a thread run at the rate of two of 64, and leave fewer rows and SMs idle. `partials` null: a block walks all groups of ranges and adds each group's sums to its
-// elements of C, which nobody else touches. Else the grid's z deals the groups out, and each group's sums go to
-// partials[group] for `sum_groups_kernel`: for products whose tiles are too few to keep every SM at work to the end.
+// TMA by one thread. A thread reads four k of TM + 4 rows and does 16 TM fused multiply-adds with them. What bounds it is
+// the way from shared memory and the register file to the FFMA pipes: 73 % of the shared-memory rate, 49 % of the pipes' cycles, a
+// dispatch stall for every instruction issued (261 tokens x 19,456 x 2,560; a loop of nothing but three-register FFMAs reaches
+// 55 TFLOP/s);
+// three blocks an SM of 32 sums a thread run at the rate of two of 64, and leave fewer rows and SMs idle. `partials` null: a block
+// walks all groups of ranges and adds each group's sums to its elements of C, which nobody else touches. Else the grid's z deals
+// the groups out, and each group's sums go to partials[group] for `sum_groups_kernel`: for products whose tiles are too few to keep
+// every SM at work to the end.
 // Measured (one B200, the four products of the same layer together): 1.98 ms for 261 tokens (26 TFLOP/s; 3.54 ms with 64 x 64
-// tiles filled by plain loads), 5.99 ms for 1,024 (34 TFLOP/s).
+// tiles filled by plain loads), 5.99 ms for 1,024 (34 TFLOP/s). cuBLAS in 32-bit, without TF32: 1.38 and 4.01 ms.
 constexpr int MANY_COLS = 64, MANY_TN = 4, MANY_STAGES = 3, MANY_THREADS = 128;
 template <int TM> struct Many {
   static constexpr int ROWS = 8 * TM, STAGE_FLOATS = (ROWS + MANY_COLS) * STAGE_K;
@@ -465,7 +469,7 @@ gemm_f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   const int m0 = (int)(blockIdx.x % tiles_m) * T::ROWS, n0 = (int)(blockIdx.x / tiles_m) * MANY_COLS;
   const int tn = threadIdx.x & 15, tm = threadIdx.x >> 4;      // weight rows tn + 16 j, tokens tm + 8 i
   const Split split(K);
-  const int first_group = (int)((long)split.groups() * blockIdx.z / gridDim.z), end_group = (int)((long)split.groups() * (blockIdx.z + 1) / gridDim.z);
+  const int first_group = (int)(split.groups() * blockIdx.z / gridDim.z), end_group = (int)(split.groups() * (blockIdx.z + 1) / gridDim.z);
   const int k_begin = first_group * GROUP * split.length, k_end = min(K, end_group * GROUP * split.length);
   const int stages = (k_end - k_begin + STAGE_K - 1) / STAGE_K, per_range = split.length / STAGE_K;
 

@@ -256,7 +256,9 @@ __device__ __forceinline__ float4 load_quad(const T* __restrict__ head, int c, i
 }
 
 // E of one segment and head, 128 value columns a block: a 128 x 128 tile, 8 x 8 sums a thread, 16 tokens a step through two
-// buffers. The FFMA pipes bound it.
+// buffers. What bounds it is the latency of its few warps: 128 registers a thread leave two blocks an SM, 22 % of its warps, which
+// wait for the next step's rows and their stores (one prompt of 1,500 tokens, 32 heads of 128 x 128, 87 us: FFMA pipes 33 % and issue
+// slots 45 % busy, 27 % of the memory system's rate).
 template <typename T, int ACT>
 __global__ void __launch_bounds__(SEG_THREADS)
 segment_state_kernel(const T* __restrict__ proj, long row_stride, int k_off, int v_off, const int* __restrict__ cu_q,
@@ -328,11 +330,13 @@ segment_state_kernel(const T* __restrict__ proj, long row_stride, int k_off, int
 // as many threads, took 282 us where this takes 194): first
 // S_in^T q over slices of 64 rows of S_in, times decay^(i+1); then, for every block of 64 keys up to the tokens' own, the
 // 64 x 64 weights decay^(i-j) (q_i . k_j) through shared memory, and their product with the values. Rows of 132 floats keep
-// the 16-byte reads along a row free of bank conflicts. The FFMA pipes bound it.
+// the 16-byte reads along a row free of bank conflicts. What bounds it is the latency of a block's chain, load, barrier,
+// multiply, with two blocks an SM (registers and shared memory) to hide it: FFMA pipes 32 % and issue slots 45 % busy, shared-memory
+// reads 43 % (165 us at the size below).
 // Measured (one B200, one prompt of 1,500 tokens, 32 heads of 128 x 128, the three launches of a layer, states,
 // joining, outputs): 129 + 10 + 310 us when the segments walked their tokens one by one, then 90 + 24 + 193 us with
 // segments of 128, 283 in all with segments of 64, whose blocks have equal work. The next block's rows on their way while one is
-// multiplied changed nothing (305 against 306 us): the blocks beside it hide them
+// multiplied changed nothing (305 against 306 us).
 template <typename T, int ACT>
 __global__ void __launch_bounds__(SEG_THREADS, 2)
 segment_output_kernel(const T* __restrict__ proj, long row_stride, int q_off, int k_off, int v_off, float* __restrict__ out,
@@ -611,7 +615,8 @@ LB_EXPORT int lb_gated_rmsnorm(int dtype, const float* x, const void* gate, long
   const int threads = n >= 1024 ? 256 : 128;
   const bool vec = n % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)weight % 16 == 0;
   if (dtype == LB_F32) {
-    if (vec) lb_launch(gated_rmsnorm_kernel<float, true>, tokens, threads, 0, stream, x, (const float*)gate, gate_stride, weight, (float*)out, n, eps);
+    if (vec)
+      lb_launch(gated_rmsnorm_kernel<float, true>, tokens, threads, 0, stream, x, (const float*)gate, gate_stride, weight, (float*)out, n, eps);
     else lb_launch(gated_rmsnorm_kernel<float, false>, tokens, threads, 0, stream, x, (const float*)gate, gate_stride, weight, (float*)out, n, eps);
   } else if (dtype == LB_BF16) {
     if (vec) lb_launch(gated_rmsnorm_kernel<bf16, true>, tokens, threads, 0, stream, x, (const bf16*)gate, gate_stride, weight, (bf16*)out, n, eps);

@@ -116,8 +116,8 @@ def embed(ids: torch.Tensor, table: torch.Tensor, out: torch.Tensor, token_src: 
         _need(token_src, torch.int32, "token_src"); _need(records, torch.int32, "records")
         if records.dim() != 2 or records.shape[1] != RECORD_WORDS or token_src.shape[0] != ids.shape[0]:
             raise ValueError("embed: records must be [slots, RECORD_WORDS] and token_src one entry per token")
-    fn = _fn("elementwise", "lb_embed_wide" if wide else "lb_embed",
-             [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
+    name = "lb_embed_wide" if wide else "lb_embed"
+    fn = _FUNCTIONS.get(name) or _fn("elementwise", name, [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
     _check(fn(dtype_code(table.dtype), _ptr(ids), _ptr(token_src), _ptr(records), _ptr(table), _ptr(out), ids.shape[0],
               table.shape[1], table.shape[0], _stream()), "embed")
     return out
@@ -290,7 +290,8 @@ def gated_act(gate_up: torch.Tensor, out: torch.Tensor, activation: str, block: 
         raise ValueError("gated_act: shapes do not agree")
     if activation not in GATE_ACTIVATIONS:
         raise ValueError(f"gated_act: unknown activation {activation!r}")
-    fn = _FUNCTIONS.get("lb_gated_act") or _fn("elementwise", "lb_gated_act", [c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p])
+    fn = _FUNCTIONS.get("lb_gated_act") or _fn(
+             "elementwise", "lb_gated_act", [c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p])
     _check(fn(dtype_code(gate_up.dtype), _ptr(gate_up), _ptr(out), gate_up.shape[0], inter, int(block),
               GATE_ACTIVATIONS[activation], float(limit), float(slope), _stream()), "gated_act")
     return out
@@ -418,7 +419,8 @@ def channel_gate(heads: torch.Tensor, logits: torch.Tensor, out: torch.Tensor, q
     if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride(1) != 1 or tuple(logits.shape) != (tokens, q_heads * vdim) \
             or tuple(out.shape) != (tokens, q_heads * vdim) or heads.shape[1] % q_heads or heads.shape[1] // q_heads < vdim:
         raise ValueError("channel_gate: shapes do not agree")
-    fn = _FUNCTIONS.get("lb_channel_gate") or _fn("elementwise", "lb_channel_gate", [c_int, c_void_p, c_void_p, c_long, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
+    fn = _FUNCTIONS.get("lb_channel_gate") or _fn(
+             "elementwise", "lb_channel_gate", [c_int, c_void_p, c_void_p, c_long, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
     _check(fn(dtype_code(heads.dtype), _ptr(heads), _ptr(logits), logits.stride(0), _ptr(out), tokens, q_heads, vdim,
               heads.shape[1] // q_heads, _stream()), "channel_gate")
     return out
@@ -496,7 +498,8 @@ def moe_route(h: torch.Tensor, router: torch.Tensor, top: int, ids: torch.Tensor
         if shared_w.numel() != hidden or shared_factor.numel() != tokens:
             raise ValueError("moe_route: shared_w [H] and shared_factor [T]")
     options = _route_options(experts, correction, groups, keep_groups, group_score, renormalize, route_scale, score, "moe_route")
-    fn = _FUNCTIONS.get("lb_moe_route") or _fn("moe", "lb_moe_route", [c_int] + [c_void_p] * 6 + [c_int] * 4 + [c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p])
+    fn = _FUNCTIONS.get("lb_moe_route") or _fn(
+             "moe", "lb_moe_route", [c_int] + [c_void_p] * 6 + [c_int] * 4 + [c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p])
     _check(fn(dtype_code(h.dtype), _ptr(h), _ptr(router), _ptr(shared_w), _ptr(ids), _ptr(scores), _ptr(shared_factor), tokens,
               hidden, experts, int(top), *options, _stream()), "moe_route")
 
@@ -547,7 +550,8 @@ def moe_expert_up(h: torch.Tensor, order: torch.Tensor, offsets: torch.Tensor, s
     if hidden != h.shape[1] or (gated and rows % 2) or tuple(act.shape) != (pairs, inter) or pairs != h.shape[0] * top \
             or activation not in EXPERT_ACTIVATIONS or (not gated and (activation != "relu2" or interleaved or scores is not None)):
         raise ValueError("moe_expert_up: shapes do not agree")
-    fn = _FUNCTIONS.get("lb_moe_expert_up") or _fn("moe", "lb_moe_expert_up", [c_int, c_void_p, c_long] + [c_void_p] * 5 + [c_int] * 8 + [c_float, c_float, c_void_p])
+    fn = _FUNCTIONS.get("lb_moe_expert_up") or _fn(
+             "moe", "lb_moe_expert_up", [c_int, c_void_p, c_long] + [c_void_p] * 5 + [c_int] * 8 + [c_float, c_float, c_void_p])
     _check(fn(dtype_code(h.dtype), _ptr(h), h.stride(0), _ptr(order), _ptr(offsets), _ptr(scores), _ptr(gate_up), _ptr(act),
               pairs, int(top), experts, hidden, inter, EXPERT_ACTIVATIONS[activation], int(bool(interleaved)), int(bool(gated)),
               float(limit), float(slope), _stream()), "moe_expert_up")
@@ -588,7 +592,8 @@ def moe_combine(y: torch.Tensor, out: torch.Tensor, top: int, pair_scale: torch.
     for name, t in (("pair_scale", pair_scale), ("shared_factor", shared_factor)):
         if t is not None:
             _need(t, torch.float32, name)
-    fn = _FUNCTIONS.get("lb_moe_combine") or _fn("moe", "lb_moe_combine", [c_int, c_void_p, c_int] + [c_void_p] * 4 + [c_int] * 3 + [c_void_p, c_void_p])
+    fn = _FUNCTIONS.get("lb_moe_combine") or _fn(
+             "moe", "lb_moe_combine", [c_int, c_void_p, c_int] + [c_void_p] * 4 + [c_int] * 3 + [c_void_p, c_void_p])
     _check(fn(dtype_code(out.dtype), _ptr(y), dtype_code(y.dtype), _ptr(pair_scale), _ptr(shared_out), _ptr(shared_factor), _ptr(out),
               tokens, hidden, int(top), _ptr(rows), _stream()), "moe_combine")
     return out
@@ -613,7 +618,8 @@ def moe_group_tiles(ids: torch.Tensor, experts: int, place_of: torch.Tensor, til
     if place_of.numel() != ids.numel() or tile_up.numel() != tile_down.numel() \
             or (tile_up.numel() - 1) * MOE_TILE_ROWS < moe_padded_rows(ids.numel(), experts):
         raise ValueError("moe_group_tiles: place_of one entry per pair, the tile lists one per tile of the padded buffers and one more")
-    fn = _FUNCTIONS.get("lb_moe_group_tiles") or _fn("moe", "lb_moe_group_tiles", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
+    fn = _FUNCTIONS.get("lb_moe_group_tiles") or _fn(
+             "moe", "lb_moe_group_tiles", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
     _check(fn(_ptr(ids), ids.numel(), int(experts), _ptr(place_of), _ptr(tile_up), _ptr(tile_down), tile_up.numel() - 1, int(rows_up),
               int(rows_down), _stream()), "moe_group_tiles")
 
@@ -626,7 +632,8 @@ def moe_scatter_rows(h: torch.Tensor, place_of: torch.Tensor, scale: torch.Tenso
         raise ValueError("moe_scatter_rows: shapes do not agree")
     if scale is not None:
         _need(scale, torch.float32, "scale")
-    fn = _FUNCTIONS.get("lb_moe_scatter_rows") or _fn("moe", "lb_moe_scatter_rows", [c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
+    fn = _FUNCTIONS.get("lb_moe_scatter_rows") or _fn(
+             "moe", "lb_moe_scatter_rows", [c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
     _check(fn(dtype_code(h.dtype), _ptr(h), h.stride(0), _ptr(place_of), _ptr(scale), _ptr(rows), pairs, h.shape[1], int(top),
               _stream()), "moe_scatter_rows")
     return rows
@@ -709,7 +716,8 @@ def stream_norm(x: torch.Tensor, update: tuple | None, read: torch.Tensor | None
         _need(mu, torch.float32, "mu"); _need(state, torch.float32, "state")
         if mu.numel() != width or state.dim() != 2 or state.shape[1] < width or rows is not None or batch.n_tokens != tokens:
             raise ValueError("stream_norm: the shift is mu [width], state [slots, >= width] and this batch, without picked rows")
-    fn = _FUNCTIONS.get("lb_stream_norm") or _fn("streams", "lb_stream_norm", [c_int, c_void_p, c_long, c_long] + [c_void_p] * 6 + [c_float, c_void_p, c_void_p, c_int, c_int, c_int,
+    fn = _FUNCTIONS.get("lb_stream_norm") or _fn(
+             "streams", "lb_stream_norm", [c_int, c_void_p, c_long, c_long] + [c_void_p] * 6 + [c_float, c_void_p, c_void_p, c_int, c_int, c_int,
                                            c_void_p, c_void_p, c_long, c_void_p, c_void_p, c_int, c_void_p])
     _check(fn(dtype_code(out.dtype), _ptr(x), x.stride(0), x.stride(1), _ptr(y), _ptr(mix), _ptr(gain), _ptr(read), _ptr(x_out),
               _ptr(weight), float(eps), _ptr(out), _ptr(rows), blocks, width, streams, _ptr(mu), _ptr(state),
@@ -845,7 +853,8 @@ def add_position_rows(x: torch.Tensor, positions: torch.Tensor, table: torch.Ten
         _need(lowered, table.dtype, "lowered")
         if lowered.shape != x.shape:
             raise ValueError("add_position_rows: lowered must have x's shape")
-    fn = _FUNCTIONS.get("lb_add_position_rows") or _fn("elementwise", "lb_add_position_rows", [c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p])
+    fn = _FUNCTIONS.get("lb_add_position_rows") or _fn(
+             "elementwise", "lb_add_position_rows", [c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p])
     _check(fn(dtype_code(table.dtype), _ptr(x), _ptr(positions), _ptr(table), table.shape[0], _ptr(lowered), x.shape[0],
               x.shape[1], _stream()), "add_position_rows")
     return x
@@ -918,7 +927,8 @@ def latent_rows(proj: torch.Tensor, dkv_off: int, norm_w: torch.Tensor | None, e
         if cq_out.shape[0] != tokens or cq_norm_w.numel() != cq_rank or not 0 <= cq_off <= proj.shape[1] - cq_rank:
             raise ValueError("latent_rows: the projection row does not hold the queries' latent")
     dtype = (k_pool if dkv_off >= 0 else cq_out).dtype
-    fn = _FUNCTIONS.get("lb_latent_rows") or _fn("latent", "lb_latent_rows", [c_int, c_void_p, c_long, c_int, c_void_p, c_float, c_void_p, c_void_p, c_void_p] + [c_int] * 7
+    fn = _FUNCTIONS.get("lb_latent_rows") or _fn(
+             "latent", "lb_latent_rows", [c_int, c_void_p, c_long, c_int, c_void_p, c_float, c_void_p, c_void_p, c_void_p] + [c_int] * 7
              + [c_void_p, c_void_p, c_void_p])
     _check(fn(dtype_code(dtype), _ptr(proj), proj.stride(0), int(dkv_off), _ptr(norm_w), float(eps), _ptr(table), _ptr(slot_map),
               _ptr(k_pool), tokens, rot, rank, room, page_tokens, int(cq_off), cq_rank, _ptr(cq_norm_w), _ptr(cq_out), _stream()),
@@ -953,7 +963,8 @@ def heads_linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gate: torc
         if gate.dtype != torch.float32 or gate.dim() != 2 or gate.stride(1) != 1 or gate.shape[0] != tokens \
                 or gate.shape[1] not in (heads, heads * n_out):
             raise ValueError("heads_linear: gate must be [tokens, heads * N] or [tokens, heads]")
-    fn = _FUNCTIONS.get("lb_heads_linear") or _fn("latent", "lb_heads_linear", [c_int, c_int, c_void_p, c_long, c_long, c_void_p, c_void_p, c_long, c_long, c_void_p,
+    fn = _FUNCTIONS.get("lb_heads_linear") or _fn(
+             "latent", "lb_heads_linear", [c_int, c_int, c_void_p, c_long, c_long, c_void_p, c_void_p, c_long, c_long, c_void_p,
                                            c_long, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p])
     _check(fn(dtype_code(w.dtype), int(a.dtype == torch.float32), _ptr(a), a.stride(0), a.stride(1), _ptr(w), _ptr(out),
               out.stride(0), out.stride(1), _ptr(gate), gate.stride(0) if gate is not None else 0, int(per_head), tokens, heads, n_out,
@@ -1005,7 +1016,8 @@ def delta_scan(prepared: torch.Tensor, out: torch.Tensor, state: torch.Tensor, b
     if tuple(prepared.shape) != (out.shape[0], channels + 2 * heads) or out.shape[1] != heads * vdim or state.dim() != 2 \
             or state.shape[1] < heads * dim * vdim:
         raise ValueError("delta_scan: shapes do not agree")
-    fn = _FUNCTIONS.get("lb_delta_scan") or _fn("delta_rule", "lb_delta_scan", [c_void_p, c_void_p, c_void_p, c_long, c_void_p, c_void_p] + [c_int] * 5 + [c_void_p])
+    fn = _FUNCTIONS.get("lb_delta_scan") or _fn(
+             "delta_rule", "lb_delta_scan", [c_void_p, c_void_p, c_void_p, c_long, c_void_p, c_void_p] + [c_int] * 5 + [c_void_p])
     _check(fn(_ptr(prepared), _ptr(out), _ptr(state), state.stride(0), _ptr(batch.cu_q), _ptr(batch.state_slots), batch.n_seqs,
               heads, kv_heads, dim, vdim, _stream()), "delta_scan")
     return out
@@ -1024,7 +1036,8 @@ def head_gated_rmsnorm(o: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor
             or gate.stride(1) != 1 or tuple(gate.shape) != (tokens, heads * vdim) or weight.numel() not in (vdim, heads * vdim):
         raise ValueError("head_gated_rmsnorm: shapes do not agree")
     per_channel = weight.numel() == heads * vdim and heads > 1
-    fn = _FUNCTIONS.get("lb_head_gated_rmsnorm") or _fn("delta_rule", "lb_head_gated_rmsnorm", [c_int, c_void_p, c_void_p, c_long, c_void_p, c_void_p, c_int, c_int, c_int,
+    fn = _FUNCTIONS.get("lb_head_gated_rmsnorm") or _fn(
+             "delta_rule", "lb_head_gated_rmsnorm", [c_int, c_void_p, c_void_p, c_long, c_void_p, c_void_p, c_int, c_int, c_int,
                                                      c_float, c_int, c_long, c_void_p])
     _check(fn(dtype_code(out.dtype), _ptr(o), _ptr(gate), gate.stride(0), _ptr(weight), _ptr(out), tokens, heads, vdim, float(eps),
               vdim if per_channel else 0, out.stride(0), _stream()), "head_gated_rmsnorm")
@@ -1049,7 +1062,8 @@ def wkv_shift_mix(h: torch.Tensor, mu: torch.Tensor, state: torch.Tensor, shift_
             or state.shape[1] < shift_off + width:
         raise ValueError("wkv_shift_mix: shapes do not agree")
     tiles = batch.tiles[wkv_mix_tokens()]
-    fn = _FUNCTIONS.get("lb_wkv_shift_mix") or _fn("wkv", "lb_wkv_shift_mix", [c_int, c_void_p, c_void_p, c_void_p, c_long, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
+    fn = _FUNCTIONS.get("lb_wkv_shift_mix") or _fn(
+             "wkv", "lb_wkv_shift_mix", [c_int, c_void_p, c_void_p, c_void_p, c_long, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                          c_int, c_int, c_void_p, c_int, c_int, c_int, c_void_p])
     _check(fn(dtype_code(h.dtype), _ptr(h), _ptr(mu), _ptr(state), state.stride(0), int(shift_off), _ptr(batch.cu_q),
               _ptr(batch.state_slots), _ptr(tiles.tile_seq), _ptr(tiles.tile_q0), tiles.count, batch.n_seqs, _ptr(mixes), tokens,
@@ -1066,7 +1080,8 @@ def wkv_decay(a: torch.Tensor, w2: torch.Tensor, w0: torch.Tensor, decay: torch.
     if a.dtype != torch.float32 or a.dim() != 2 or a.stride(1) != 1 or a.shape[1] < rank or w0.numel() != channels \
             or tuple(decay.shape) != (tokens, channels):
         raise ValueError("wkv_decay: shapes do not agree")
-    fn = _FUNCTIONS.get("lb_wkv_decay") or _fn("wkv", "lb_wkv_decay", [c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
+    fn = _FUNCTIONS.get("lb_wkv_decay") or _fn(
+             "wkv", "lb_wkv_decay", [c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
     _check(fn(dtype_code(w2.dtype), _ptr(a), a.stride(0), _ptr(w2), _ptr(w0), _ptr(decay), tokens, channels, rank, _stream()), "wkv_decay")
     return decay
 
@@ -1086,7 +1101,8 @@ def wkv_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, w: torch.Tensor,
     if channels != heads * dim or tuple(w.shape) != (tokens, channels) or u.numel() != channels or state.dim() != 2 \
             or state.shape[1] < heads * dim * dim:
         raise ValueError("wkv_scan: shapes do not agree")
-    fn = _FUNCTIONS.get("lb_wkv_scan") or _fn("wkv", "lb_wkv_scan", [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_void_p,
+    fn = _FUNCTIONS.get("lb_wkv_scan") or _fn(
+             "wkv", "lb_wkv_scan", [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_void_p,
                                     c_long, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
     _check(fn(_ptr(r), r.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(w), _ptr(u), _ptr(out), _ptr(state),
               state.stride(0), _ptr(batch.cu_q), _ptr(batch.state_slots), batch.n_seqs, heads, dim, _stream()), "wkv_scan")
@@ -1101,7 +1117,8 @@ def gate_decay(a: torch.Tensor, w2: torch.Tensor, w0: torch.Tensor, tau: float, 
     if a.dtype != torch.float32 or a.dim() != 2 or a.stride(1) != 1 or a.shape[1] < rank or w0.numel() != channels \
             or tuple(decay.shape) != (tokens, channels) or not tau > 0:
         raise ValueError("gate_decay: shapes do not agree, or tau is not positive")
-    fn = _FUNCTIONS.get("lb_gate_decay") or _fn("wkv", "lb_gate_decay", [c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p])
+    fn = _FUNCTIONS.get("lb_gate_decay") or _fn(
+             "wkv", "lb_gate_decay", [c_int, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p])
     _check(fn(dtype_code(w2.dtype), _ptr(a), a.stride(0), _ptr(w2), _ptr(w0), _ptr(decay), tokens, channels, rank, float(tau),
               _stream()), "gate_decay")
     return decay
@@ -1121,7 +1138,8 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, w: torch.Tenso
             raise ValueError(f"gated_scan: {name} must be float32 [tokens, {n}] with dense rows")
     if out.shape[1] != heads * vdim or tuple(w.shape) != (tokens, heads * dim) or tuple(state.shape[1:]) != (heads, dim, vdim):
         raise ValueError("gated_scan: shapes do not agree")
-    fn = _FUNCTIONS.get("lb_gated_scan") or _fn("wkv", "lb_gated_scan", [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_long,
+    fn = _FUNCTIONS.get("lb_gated_scan") or _fn(
+             "wkv", "lb_gated_scan", [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_long,
                                       c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p])
     _check(fn(_ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(w), _ptr(out), _ptr(state), state.stride(0),
               _ptr(batch.cu_q), _ptr(batch.state_slots), batch.n_seqs, heads, dim, vdim, float(scale), _stream()), "gated_scan")
@@ -1542,26 +1560,24 @@ def decode_plan(n_seqs: int, q_heads: int, kv_heads: int, dim: int, max_context:
     SM; the variant with two tiles fits three (head size 128, at most 8 heads per KV head) but each
     block is slower (about 1.15x per tile). Blocks run in rounds of blocks-per-SM x SMs. With head size
     128 the kernel runs 2, 4 or 8 splits as a thread-block cluster that merges through distributed
-    shared memory (16 where all the launch's blocks still fit one per SM: a single sequence, 8.7
-    against 10.6 us at 3,072 keys; two sequences 16.5 against 12.1 us, so not there); more splits merge
+    shared memory (16 where all the launch's blocks still fit one per SM: a single sequence, 7.4
+    us against 7.6 with 8 at 3,072 keys; two sequences 14.1 against 9.0 us, so not there); more splits merge
     through scratch memory, which costs more. The plan is the one
     with the lowest estimate rounds x (64-key tiles per split + overhead in tiles): 4 for a cluster,
-    10 for the scratch merge. That fits what was measured at 3,072 keys (sequences: best splits)
-    1: 8, 4: 8, 8: 4, 16: 2, 24: 4, 32: 1, 40: 4, 48: 2, 128: 2, one sequence of 32,768 keys: 32 or
-    more through scratch memory, and 64 sequences: 4 splits with three blocks an SM (148 us against
-    158 us unsplit with two).
+    10 for the scratch merge.
 
     `mean_context`: the sequences' mean length where it is known to be well below the longest (more
     than 1.5 times). The longest sequence's blocks then run on alone at a lone block's rate after the
     others have finished, so the context is cut further, into about 7 blocks an SM (at least 12 tiles
-    each), with three blocks an SM as soon as two do not hold them all. Measured with lengths spread
-    evenly over 0.1..1 of 8,192 keys (us, the plan for equal lengths against this one): 8 sequences
-    54 -> 47, 16: 106 -> 80, 32: 219 -> 136; over 0.1..1 of 3,072 keys: 16: 41 -> 36, 32: 79 -> 56.
-    Where twelve tiles a block would cut the context less than for equal lengths, the plan for those stays: 8 sequences of
-    0.1..1 of 2,400 keys with 2 splits 18.1, with 4 12.2 us, of 1,500 keys 13.1 and 9.5.
+    each), with three blocks an SM as soon as two do not hold them all. Where twelve tiles a block would cut the context
+    less than for equal lengths, the plan for those stays.
 
-    The figures are those of the kernel that had the query heads as rows. With at most 8 heads a KV head it takes less since
-    (8 sequences of 3,072 keys: 24.8 -> 18.9, 64: 146 -> 131, which 123 us unsplit would beat now), and the plans are kept."""
+    Measured on one B200, 32 heads over 8 (us; the plan, and no split): equal lengths of 3,072 keys, 1 sequence 7.4 and 28.9, 8: 15.8
+    and 32.9, 16: 35.5 and 40.4, 40: 85.6 and 96.5; one of 32,768 31.1 and 345; lengths spread evenly over 0.1..1 of 8,192 keys, 8: 32.8
+    and 81.4, 16: 55.7 and 96.0, 32: 101 and 128, 64: 187 and 219. Over 115 such shapes (1 to 128 sequences, 700 to 32,768 keys) the
+    plan takes 2 % more than the best of 1, 2, 4, 8 and 16 splits with either kernel. The constants fit the kernel that had the query
+    heads as rows, and where few blocks an SM share keys as columns now they are off by more: 64 equal sequences of 1,500 keys
+    72.3 (unsplit with three stages 63.6), of 3,072 131 (123), 32 of 0.1..1 of 1,500 keys 26.7 (22.2)."""
     natural = n_seqs * kv_heads
     want = max(1, 2 * sm_count // natural)                    # all blocks resident at once, two per SM
     splits = min(want, 128, max(1, max_context // 192))       # at least three 64-key tiles per split
@@ -1592,7 +1608,7 @@ def decode_plan(n_seqs: int, q_heads: int, kv_heads: int, dim: int, max_context:
             return (count, 3) if natural * count <= 2 * sm_count else (count, 2)
     if 10 * natural >= 17 * sm_count and natural <= 2 * sm_count and tiles >= 64 and q_heads // kv_heads <= 8:
         # just under two blocks an SM, long contexts: four splits with three blocks an SM measured
-        # 200 against 225 us (32 sequences of 8,192 keys; at 3,072 keys the two are equal)
+        # 170 against 182 us (32 sequences of 8,192 keys)
         return 4, 2
     if natural > 2 * sm_count and q_heads // kv_heads <= 8:
         # more blocks than two per SM hold at once: three slower blocks an SM may finish sooner
@@ -1664,7 +1680,8 @@ def _pool_map(pool: torch.Tensor):
         _need(pool, torch.bfloat16, "pool")
         layers, two, pages, kv_heads, page_tokens, dim = pool.shape
         blob = (ctypes.c_ubyte * 128)()
-        fn = _FUNCTIONS.get("lb_attention_tcgen05_pool_map") or _fn("attention_tcgen05", "lb_attention_tcgen05_pool_map", [c_void_p, c_void_p, c_long, c_long, c_int, c_int, c_int])
+        fn = _FUNCTIONS.get("lb_attention_tcgen05_pool_map") or _fn(
+                 "attention_tcgen05", "lb_attention_tcgen05_pool_map", [c_void_p, c_void_p, c_long, c_long, c_int, c_int, c_int])
         code = fn(ctypes.addressof(blob), _ptr(pool), layers * two, pages, kv_heads, page_tokens, dim)
         if code:
             raise ValueError(f"attention_tcgen05: cannot describe the pool to TMA ({_REFUSALS.get(code, code)})")

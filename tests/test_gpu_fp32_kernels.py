@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("n, k", [(1, 4), (31, 32), (33, 36), (64, 1024), (65, 1028), (257, 2560), (100, 4100), (70, 9728), (33, 8200), (5, 37)])
 def test_f32_product_has_the_same_bits_in_every_batch(n, k):
-    """Up to 2, 4, 8 and 16 tokens, tiles of 32 and of 64, split over blocks or not, K that TMA takes or not (37)."""
+    """Up to 2, 4, 8 and 16 tokens, tiles of 32 and of 64, every group of ranges a block of its own, K that TMA takes or not (37)."""
     gen = torch.Generator().manual_seed(n * 10007 + k)
     tokens = 257
     a, w = torch.randn(tokens, k, generator=gen).cuda(), torch.randn(n, k, generator=gen).cuda()
@@ -107,7 +107,7 @@ def test_f32_product_of_a_few_tokens_has_the_same_bits_with_and_without_tma(toke
     assert ((outs[0].double() - a[:tokens].double() @ w.double().T).abs() <= bound).all()
 
 
-@pytest.mark.parametrize("m, n, k", [(1, 70, 9728), (16, 33, 2560), (40, 100, 4100), (600, 2400, 2500), (130, 2560, 9728), (513, 19456, 1100)])
+@pytest.mark.parametrize("m, n, k", [(1, 70, 9728), (16, 33, 2560), (40, 100, 4100), (600, 2400, 2500), (130, 2560, 9728), (520, 9728, 2500), (513, 19456, 1100)])
 def test_f32_product_says_how_much_scratch_its_form_takes(m, n, k):
     """Groups of ranges dealt out one, several or all to a block: the bits of row slices; scratch, and a second launch, only
     where the form that runs has one."""

@@ -96,7 +96,7 @@ gemm_fewtoken_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_full + 1);
   uint32_t* flag = tmem_slot + 1;   // [0] failed, [1] this block is the last of its tile
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN, split = blockIdx.z;
   const int total_kb = (K + BK - 1) / BK;
   const int kb_begin = (int)((long)total_kb * split / splits), kb_end = (int)((long)total_kb * (split + 1) / splits);
@@ -136,14 +136,15 @@ gemm_fewtoken_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       tma_load_2d(tiles_a + s * T::A_BYTES, &map_a, &full[s], (kb_begin + i) * BK, m0);
       tma_load_2d(tiles_b + s * T::B_BYTES, &map_b, &full[s], (kb_begin + i) * BK, n0);
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
     // ---------------- MMA issuer
     constexpr uint32_t idesc = instr_desc(BN);
     bool ok = true;
-    for (int i = 0; i < n_kb && ok; ++i) {
+    const int kb_count = warp_uniform(n_kb);
+    for (int i = 0; i < kb_count && ok; ++i) {
       const int s = i % T::STAGES;
       const uint32_t phase = (i / T::STAGES) & 1;
-      if (!mbar_wait(&full[s], phase)) { atomicCAS(&g_gemm_error, 0, 2); flag[0] = 1; ok = false; break; }
+      if (!warp_wait(&full[s], phase)) { atomicCAS(&g_gemm_error, 0, 2); flag[0] = 1; ok = false; break; }
       fence_after_sync();
       const uint64_t a_desc = smem_desc(tiles_a + s * T::A_BYTES), b_desc = smem_desc(tiles_b + s * T::B_BYTES);
 #pragma unroll
@@ -512,7 +513,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   volatile uint32_t* flag = tmem_slot + 1;    // [0] a wait ran out, [1] this block is the last of its tile
   float* norm_w = reinterpret_cast<float*>(smem + T::STAGES * T::STAGE_BYTES + 256);   // EPI 2: [2][128] q and k norm weights
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int rank = PAIR ? (int)lb_cluster_rank() : 0;                // 0: the block that issues the MMAs
   const int block = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
   const int blocks = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
@@ -619,7 +620,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (!PAIR || (blockIdx.x & 1) == 0) {       // a pair's leader
       // ---------------- MMA issuer
       constexpr uint32_t idesc = instr_desc(BN, TILE_ROWS);
       int it = 0, live = 0, live_tiles = sch.tiles;
@@ -627,29 +628,34 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         pdl_wait();
         live_tiles = max(1, min(tile_b_rows[sch.tiles_m], sch.tiles_m)) * (sch.tiles / sch.tiles_m);
       }
-      for (int j = 0; j < n_segments && !flag[0]; ++j) {
+      live_tiles = warp_uniform(live_tiles);
+      bool ok = true;
+      for (int j = 0; j < n_segments && ok; ++j) {
         const Segment seg = segment_at(sch, block, blocks, j);
-        if (seg.tile >= live_tiles) continue;
+        if (warp_uniform(seg.tile) >= live_tiles) continue;
         const int buf = live & 1;
-        if (!mbar_wait(&acc_empty[buf], ((live >> 1) & 1) ^ 1)) { atomicCAS(&g_gemm_error, 0, 2); flag[0] = 1; break; }
+        ok = warp_wait(&acc_empty[buf], ((live >> 1) & 1) ^ 1);
+        if (!ok) { atomicCAS(&g_gemm_error, 0, 2); flag[0] = 1; break; }
         ++live;
         fence_after_sync();
         const uint32_t acc = tmem_base + buf * T::ACC_COLS;
-        for (int kb = seg.kb_begin; kb < seg.kb_end; ++kb, ++it) {
+        const int kb_count = warp_uniform(seg.kb_end - seg.kb_begin);
+        for (int kb = 0; kb < kb_count; ++kb, ++it) {
           const int s = it % T::STAGES;
           const uint32_t phase = (it / T::STAGES) & 1;
-          if (!mbar_wait(&full[s], phase)) { atomicCAS(&g_gemm_error, 0, 2); flag[0] = 1; break; }
+          ok = warp_wait(&full[s], phase);
+          if (!ok) { atomicCAS(&g_gemm_error, 0, 2); flag[0] = 1; break; }
           fence_after_sync();
           const uint64_t a_desc = smem_desc(tiles_a + s * T::A_BYTES), b_desc = smem_desc(tiles_b + s * T::B_BYTES);
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {  // +32 bytes per K step inside the swizzled row
-            if (PAIR) umma_bf16_pair(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > seg.kb_begin || k > 0) ? 1u : 0u);
-            else umma_bf16(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > seg.kb_begin || k > 0) ? 1u : 0u);
+            if (PAIR) umma_bf16_pair(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+            else umma_bf16(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
           }
           if (PAIR) umma_commit_pair(&empty[s], 3);
           else umma_commit(&empty[s]);
         }
-        if (flag[0]) break;
+        if (!ok) break;
         if (PAIR) umma_commit_pair(&acc_full[buf], 3);
         else umma_commit(&acc_full[buf]);
       }

@@ -66,7 +66,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }   // a whole warp
-__device__ __forceinline__ int warp_uniform(int x) { return __reduce_max_sync(0xffffffffu, x); }    // of a value that all lanes have alike
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {   // one look, never suspends
   uint32_t done;
   asm volatile(
@@ -76,6 +75,13 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {   //
       : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
   return done != 0;
 }
+// the same for what is about to happen: some looks without being suspended, whose end is seen a few hundred cycles later
+__device__ __forceinline__ bool warp_spin(uint64_t* bar, uint32_t parity) {
+  for (int n = 0; n < 256; ++n)
+    if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+  return warp_wait(bar, parity);
+}
+__device__ __forceinline__ int warp_uniform(int x) { return __reduce_max_sync(0xffffffffu, x); }    // of a value that all lanes have alike
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -429,7 +435,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid
       fence_after_sync();
       // the tile needs the comparisons if it reaches past the block's first position, starts before
       // the first visible key, or a window cuts it
-      const bool masked = key0 + KEYS - 1 > p_first || key0 < key_lo || args.window > 0;
+      const bool masked = key0 + KEYS - 1 > p_first || key0 < key_lo || (args.window > 0 && key0 <= p_last - args.window);
       float s[KEYS];
 #pragma unroll
       for (int ch = 0; ch < KEYS / 16; ++ch) {
@@ -567,22 +573,26 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid
 // accumulators in tensor memory and its own softmax warpgroup, and both read the same K and V
 // tiles. The MMA thread alternates between the heads (O_a += P_a V, S_a = Q_a K^T of the next
 // tile, then the same for b), so that the tensor cores work for one head while the other's
-// softmax runs. The probabilities never touch shared memory: each thread overwrites the scores of
+// softmax runs; the part of a second product that the first 96 keys make is issued under the
+// exponentials of the last 32. The probabilities never touch shared memory: each thread overwrites the scores of
 // its own row in tensor memory with them (bf16, two per column) and the second product reads its
 // A operand from there; products issued by one thread run in order, so the next tile's scores
 // land on those columns only after the product that read them.
 // A portion far into its context has few tiles of queries and many of keys: its keys are then dealt to several blocks
 // (gridDim.z), each of which leaves its maximum, sum and output for `attention_merge_kernel`. Measured (one B200, 32 heads
-// over 8, 512 tokens after 8,209, 64 blocks on 148 SMs): the attention
-// of a layer 177 -> 105 us (two blocks a tile) and 6 us for the merge
+// over 8, 512 tokens after 8,209, 64 blocks on 148 SMs): the attention of a layer 139 -> 85 us (two blocks a tile) and 6 us for the merge.
+// What bounds a tile of two heads, 3,450 cycles: one head's chain of softmax (2,050, of which the special-function unit takes 1,024),
+// the last quarter of P V, Q K^T and their hand-overs; the tensor cores work 2,100 of them (51.9 -> 45.5 us for a prompt of 2,048 tokens
+// with the issuing warp uniform, 96 keys ahead and looks at what is about to arrive instead of suspended waits)
 // SPLIT is that form: without it the kernel carries nothing of it (20 .. 1,222 tokens 0.3 us a layer).
 // EXACT: the variant for attention with weights that keep 16 bits of mantissa in the second product (and sinks, gates, a
 // factor on the outputs; a negative window is a chunked mask: a query sees the keys of its own chunk of -window positions). A
 // weight is the sum of two bfloat16 numbers, its rounded value and the rounded rest; the rests take the upper half of the
 // columns that the scores leave free, and the second product runs over them as well. Measured (one B200, 1,500 tokens of 32
-// heads over 8 behind a window of 1,024; two prompts of 611, 16 over 4): 224 -> 96 us and 87 -> 35 us
-// (on mma.sync before)
-constexpr int PAIR_THREADS = 320;   // warp 0 producer, warp 1 MMA issuer, warps 2-5 and 6-9 the softmax warpgroups
+// heads over 8 behind a window of 1,024; two prompts of 611, 16 over 4): 45 us and 26 us (on mma.sync 224 and 87; 96 and 35 with
+// comparisons in every tile of a window and one lane issuing)
+constexpr int PAIR_THREADS = 320;   // warp 0 producer, warps 1 and 10 the heads' MMA issuers, warps 2-5 and 6-9 the softmax warpgroups
+constexpr int MOST_KEYS = 96;       // keys of a tile whose part of the second product does not wait for the last exponentials
 constexpr int PAIR_SMEM = TILE_BYTES * (2 + 2 * KV_STAGES) + 1024 + 512 + TABLE_CACHE * 4;   // Q x2, K and V stages, slack, barriers, table
 
 template <bool EXACT, bool SPLIT>
@@ -601,9 +611,10 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
   uint64_t* v_full = bars + 5;        // [2]
   uint64_t* v_empty = bars + 7;       // [2]
   uint64_t* s_full = bars + 9;        // [2 heads] the scores of a tile are in tensor memory
-  uint64_t* p_full = bars + 11;       // [2 heads] the probabilities are, and the output is rescaled
-  uint64_t* pv_done = bars + 13;      // [2 heads] the second product of a tile is finished
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint64_t* p_most = bars + 11;       // [2 heads] the probabilities of the first 96 keys are, and the output is rescaled
+  uint64_t* p_full = bars + 13;       // [2 heads] all of them are
+  uint64_t* pv_done = bars + 15;      // [2 heads] the second product of a tile is finished
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile uint32_t* flag = tmem_slot + 1;   // [0] a wait ran out
   int* page_cache = reinterpret_cast<int*>(bars) + 128;
 
@@ -633,8 +644,8 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); mbar_init(&pv_done[i], 1);
+      mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);      // both heads' products
+      mbar_init(&s_full[i], 1); mbar_init(&p_most[i], 4); mbar_init(&p_full[i], 4); mbar_init(&pv_done[i], 1);
     }
     flag[0] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -664,11 +675,11 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
                             n_tiles, kv_head, flag, 21, lane);
     }
   } else if (warp == 1) {
+    // ---------------- the products: one warp for both heads, whose softmaxes then stay half a tile apart (with a warp for each head
+    // they drift together and the tensor cores idle: 123 against 95 us at 512 tokens after 8,209)
     const int count = warp_uniform(n_tiles);
     if (count > 0) {
       constexpr uint32_t idesc_s = instr_desc(false), idesc_o = instr_desc(true);
-      bool ok = warp_wait(q_full, 0);
-      if (!ok) { atomicCAS(&g_attn_error, 0, 22); flag[0] = 1; }
       auto issue_s = [&](int i, int u) {          // S_u = Q_u K(i)^T; K(i) has been waited for
         const int stage = i % KV_STAGES;
         const uint32_t q_addr = smem_u32(q_s + u * TILE_BYTES), k_addr = smem_u32(k_s + stage * TILE_BYTES);
@@ -680,44 +691,41 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
         umma_commit(&s_full[u]);
         if (u == 1) umma_commit(&k_empty[stage]);
       };
-      if (ok) {
-        ok = warp_wait(&k_full[0], 0);
-        if (!ok) { atomicCAS(&g_attn_error, 0, 23); flag[0] = 1; }
-      }
-      if (ok) {
-        fence_after_sync();
-        issue_s(0, 0);
-        issue_s(0, 1);
-      }
+      bool ok = warp_wait(q_full, 0) && warp_wait(&k_full[0], 0);
+      if (ok) { fence_after_sync(); issue_s(0, 0); issue_s(0, 1); }
       for (int i = 0; i < count && ok; ++i) {
         const int stage = i % KV_STAGES;
+        const uint32_t v_addr = smem_u32(v_s + stage * TILE_BYTES);
 #pragma unroll
-        for (int u = 0; u < 2 && ok; ++u) {
-          if (!warp_wait(&p_full[u], i & 1) || (u == 0 && !warp_wait(&v_full[stage], (i / KV_STAGES) & 1))) {
-            atomicCAS(&g_attn_error, 0, 24); flag[0] = 1; ok = false; break;
+        for (int u = 0; u < 2; ++u) {
+          if (u == 0) {      // the tiles first: the probabilities are what comes last
+            ok = warp_wait(&v_full[stage], (i / KV_STAGES) & 1);
+            if (ok && i + 1 < count) ok = warp_wait(&k_full[(i + 1) % KV_STAGES], ((i + 1) / KV_STAGES) & 1);
           }
+          ok = ok && warp_spin(&p_most[u], i & 1);
+          if (!ok) break;
           fence_after_sync();
-          const uint32_t v_addr = smem_u32(v_s + stage * TILE_BYTES);
+          // 16 keys a step: 8 columns of packed probabilities, 16 rows of V; the first 96 keys under the others' exponentials
 #pragma unroll
-          for (int ks = 0; ks < KEYS / 16; ++ks)       // 16 keys: 8 columns of packed probabilities, 16 rows of V
-            umma_bf16_ts(tmem_o + u * 128, tmem_s + u * 128 + ks * 8, desc_mn_major(v_addr + ks * 16 * 128), idesc_o,
-                         (i > 0 || ks > 0) ? 1u : 0u);
+          for (int ks = 0; ks < MOST_KEYS / 16; ++ks)
+            umma_bf16_ts(tmem_o + u * 128, tmem_s + u * 128 + ks * 8, desc_mn_major(v_addr + ks * 16 * 128), idesc_o, (i > 0 || ks > 0) ? 1u : 0u);
+          ok = warp_spin(&p_full[u], i & 1);
+          if (!ok) break;
+          fence_after_sync();
+#pragma unroll
+          for (int ks = MOST_KEYS / 16; ks < KEYS / 16; ++ks)
+            umma_bf16_ts(tmem_o + u * 128, tmem_s + u * 128 + ks * 8, desc_mn_major(v_addr + ks * 16 * 128), idesc_o, 1u);
           if (EXACT) {
 #pragma unroll
             for (int ks = 0; ks < KEYS / 16; ++ks)
               umma_bf16_ts(tmem_o + u * 128, tmem_s + u * 128 + 64 + ks * 8, desc_mn_major(v_addr + ks * 16 * 128), idesc_o, 1u);
           }
+          if (i + 1 < count) issue_s(i + 1, u);
           umma_commit(&pv_done[u]);
           if (u == 1) umma_commit(&v_empty[stage]);
-          if (i + 1 < count) {
-            if (u == 0 && !warp_wait(&k_full[(i + 1) % KV_STAGES], ((i + 1) / KV_STAGES) & 1)) {
-              atomicCAS(&g_attn_error, 0, 25); flag[0] = 1; ok = false; break;
-            }
-            fence_after_sync();
-            issue_s(i + 1, u);
-          }
         }
       }
+      if (!ok) { atomicCAS(&g_attn_error, 0, 22); flag[0] = 1; }
     }
   } else {
     // ---------------- softmax and epilogue: warpgroup u owns head u, one query row per thread
@@ -735,7 +743,7 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
       const int key0 = tile * KEYS;
       if (!mbar_wait(&s_full[u], i & 1)) { atomicCAS(&g_attn_error, 0, 26); flag[0] = 1; ok = false; break; }
       fence_after_sync();
-      const bool masked = key0 + KEYS - 1 > p_first || key0 < key_lo || args.window > 0 || (chunk && key0 < last_chunk);
+      const bool masked = key0 + KEYS - 1 > p_first || key0 < key_lo || (args.window > 0 && key0 <= p_last - args.window) || (chunk && key0 < last_chunk);
       float s[KEYS];
       {
         uint32_t raw[64];
@@ -782,39 +790,45 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
         }
         tmem_st16_nowait(my_s + ch * 16, w);
         if constexpr (EXACT) tmem_st16_nowait(my_s + 64 + ch * 16, rest);
+        if (ch == MOST_KEYS / 32 - 1) {           // what the first products need; few scores are still in registers
+          if (any_grow && i > 0) {
+            // the previous product of this head must be finished before its accumulator is touched
+            if (!mbar_wait(&pv_done[u], (i - 1) & 1)) { atomicCAS(&g_attn_error, 0, 27); flag[0] = 1; ok = false; break; }
+            fence_after_sync();
+#pragma unroll
+            for (int part = 0; part < DIM / 16; ++part) {
+              float v[16];
+              tmem_ld16(my_o + part * 16, v);
+#pragma unroll
+              for (int e = 0; e < 16; ++e) v[e] *= factor;
+              tmem_st16(my_o + part * 16, v);
+            }
+          }
+          // V rows of keys outside the context may hold anything: zero them (0 x NaN would be NaN).
+          // Both warpgroups do it, each before its own product is released.
+          const int limit = p_last + 1;
+          if (key0 + KEYS > limit || key0 < key_lo) {
+            if (!mbar_wait(&v_full[stage], (i / KV_STAGES) & 1)) { atomicCAS(&g_attn_error, 0, 28); flag[0] = 1; ok = false; break; }
+            const int key = key0 + row;
+            if (key >= limit || key < key_lo) {
+              uint8_t* vrow = v_s + stage * TILE_BYTES + row * 128;
+#pragma unroll
+              for (int chunk = 0; chunk < 8; ++chunk) {
+                *reinterpret_cast<uint4*>(vrow + chunk * 16) = make_uint4(0, 0, 0, 0);
+                *reinterpret_cast<uint4*>(vrow + HALF_BYTES + chunk * 16) = make_uint4(0, 0, 0, 0);
+              }
+            }
+            fence_async_smem();
+          }
+          tmem_wait_st();
+          fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&p_most[u]);
+        }
       }
       const float tile_sum = (part_sum[0] + part_sum[1]) + (part_sum[2] + part_sum[3]);
       l_sum = l_sum * factor + tile_sum;
       m_ref = m_new;
-      if (any_grow && i > 0) {
-        // the previous product of this head must be finished before its accumulator is touched
-        if (!mbar_wait(&pv_done[u], (i - 1) & 1)) { atomicCAS(&g_attn_error, 0, 27); flag[0] = 1; ok = false; break; }
-        fence_after_sync();
-#pragma unroll
-        for (int ch = 0; ch < DIM / 16; ++ch) {
-          float v[16];
-          tmem_ld16(my_o + ch * 16, v);
-#pragma unroll
-          for (int e = 0; e < 16; ++e) v[e] *= factor;
-          tmem_st16(my_o + ch * 16, v);
-        }
-      }
-      // V rows of keys outside the context may hold anything: zero them (0 x NaN would be NaN).
-      // Both warpgroups do it, each before its own product is released.
-      const int limit = p_last + 1;
-      if (key0 + KEYS > limit || key0 < key_lo) {
-        if (!mbar_wait(&v_full[stage], (i / KV_STAGES) & 1)) { atomicCAS(&g_attn_error, 0, 28); flag[0] = 1; ok = false; break; }
-        const int key = key0 + row;
-        if (key >= limit || key < key_lo) {
-          uint8_t* vrow = v_s + stage * TILE_BYTES + row * 128;
-#pragma unroll
-          for (int chunk = 0; chunk < 8; ++chunk) {
-            *reinterpret_cast<uint4*>(vrow + chunk * 16) = make_uint4(0, 0, 0, 0);
-            *reinterpret_cast<uint4*>(vrow + HALF_BYTES + chunk * 16) = make_uint4(0, 0, 0, 0);
-          }
-        }
-        fence_async_smem();
-      }
       tmem_wait_st();
       fence_before_sync();
       __syncwarp();

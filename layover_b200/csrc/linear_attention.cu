@@ -188,36 +188,59 @@ decay_scan_kernel(const T* __restrict__ proj, long row_stride, int q_off, int k_
 // Per sequence, head and state element: the segments' end states become the states that come INTO the segments, and the
 // state after the last segment goes to the slot. FROM_ZERO: all segments started from zero, and what comes into segment s
 // is left in its own place; else the first one started from the slot, and it is left in the place of the segment before.
-template <bool FROM_ZERO>
-__global__ void scan_combine_kernel(float* __restrict__ seg_state, float* __restrict__ state, const int* __restrict__ cu_q,
-                                    const int* __restrict__ state_slots, const float* __restrict__ decay, int heads,
-                                    int per_head, int seg_tokens) {
-  pdl_launch_dependents();
+// WIDTH 4: four elements a thread, where all rows begin on 16 bytes and a head's size is a multiple of 4. What bounds it is the
+// memory system, with eight segments' loads on their way at once (one B200, 24 segments of 32 heads of 128 x 128, 100 MB:
+// 47 -> 20 us inside a step; one element a thread and four segments before).
+// The walk over the segments starts when the joining has ended: its blocks, had they come early, would be placed around the
+// joining's and share SMs (4 heads of 128 x 128, 600 tokens, the whole layer: 84 us, 61 so; 16 heads, 300 tokens 88 and 74).
+template <bool FROM_ZERO, int WIDTH>
+__global__ void __launch_bounds__(256)
+scan_combine_kernel(float* __restrict__ seg_state, float* __restrict__ state, const int* __restrict__ cu_q,
+                    const int* __restrict__ state_slots, const float* __restrict__ decay, int heads,
+                    int per_head, int seg_tokens) {
+  struct __align__(4 * WIDTH) Part { float v[WIDTH]; };
+  if (FROM_ZERO) pdl_launch_dependents();
   pdl_wait();
   const int seq = blockIdx.y;
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, per_segment = (size_t)heads * per_head;
+  const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * WIDTH, per_segment = (size_t)heads * per_head;
   if (i >= per_segment) return;
   int first_segment = 0;
   for (int q = 0; q < seq; ++q) first_segment += max(1, (cu_q[q + 1] - cu_q[q] + seg_tokens - 1) / seg_tokens);
   const int len = cu_q[seq + 1] - cu_q[seq], ns = max(1, (len + seg_tokens - 1) / seg_tokens);
   const float log2_lam = log2f(decay[i / per_head]);
   float* e = seg_state + (size_t)first_segment * per_segment + i;
-  float* slot = state + (size_t)state_slots[seq] * per_segment + i;
-  float running = FROM_ZERO ? *slot : e[0];          // what comes into segment 0, or the true state after it
-  constexpr int AHEAD = 4;                           // segments whose own parts are on their way at once
+  auto at = [&](int s) { return reinterpret_cast<Part*>(e + (size_t)s * per_segment); };
+  Part* slot = reinterpret_cast<Part*>(state + (size_t)state_slots[seq] * per_segment + i);
+  Part running = FROM_ZERO ? *slot : *at(0);         // what comes into segment 0, or the true state after it
+  constexpr int AHEAD = 8;                           // segments whose own parts are on their way at once
   for (int s0 = FROM_ZERO ? 0 : 1; s0 < ns; s0 += AHEAD) {
-    float local[AHEAD];
+    Part local[AHEAD];
 #pragma unroll
-    for (int u = 0; u < AHEAD; ++u) local[u] = s0 + u < ns ? e[(size_t)(s0 + u) * per_segment] : 0.f;
+    for (int u = 0; u < AHEAD; ++u)
+      if (s0 + u < ns) local[u] = *at(s0 + u);
 #pragma unroll
     for (int u = 0; u < AHEAD; ++u) {
       const int sg = s0 + u;
       if (sg >= ns) break;
-      e[(size_t)(FROM_ZERO ? sg : sg - 1) * per_segment] = running;
-      running = fmaf(decay_power(log2_lam, min(seg_tokens, len - sg * seg_tokens)), running, local[u]);
+      *at(FROM_ZERO ? sg : sg - 1) = running;
+      const float w = decay_power(log2_lam, min(seg_tokens, len - sg * seg_tokens));
+#pragma unroll
+      for (int x = 0; x < WIDTH; ++x) running.v[x] = fmaf(w, running.v[x], local[u].v[x]);
     }
   }
   *slot = running;
+}
+
+template <bool FROM_ZERO>
+void launch_combine(int n_seqs, float* seg_state, float* state, const int* cu_q, const int* state_slots, const float* decay, int heads,
+                    int per_head, int seg_tokens, cudaStream_t stream) {
+  const bool wide = per_head % 4 == 0 && (uintptr_t)seg_state % 16 == 0 && (uintptr_t)state % 16 == 0;
+  const size_t threads = (size_t)heads * per_head / (wide ? 4 : 1);
+  const dim3 grid((unsigned)((threads + 255) / 256), n_seqs);
+  if (wide)
+    lb_launch(scan_combine_kernel<FROM_ZERO, 4>, grid, 256, 0, stream, seg_state, state, cu_q, state_slots, decay, heads, per_head, seg_tokens);
+  else
+    lb_launch(scan_combine_kernel<FROM_ZERO, 1>, grid, 256, 0, stream, seg_state, state, cu_q, state_slots, decay, heads, per_head, seg_tokens);
 }
 
 // ------------------------------------------------------------------ segments as matrix products (head sizes up to 128)
@@ -255,12 +278,20 @@ __device__ __forceinline__ float4 load_quad(const T* __restrict__ head, int c, i
   return make_float4(activate<ACT>(v[0]), activate<ACT>(v[1]), activate<ACT>(v[2]), activate<ACT>(v[3]));
 }
 
+// Two neighbouring sums at once: c = (x, x) * r + c, each the fused multiply-add that fmaf is.
+__device__ __forceinline__ void multiply_add_pair(float2& c, float x, float2 r) {
+  unsigned long long xx, rr = *reinterpret_cast<const unsigned long long*>(&r), cc = *reinterpret_cast<const unsigned long long*>(&c);
+  asm("mov.b64 %0, {%1, %1};" : "=l"(xx) : "f"(x));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(cc) : "l"(xx), "l"(rr));
+  c = *reinterpret_cast<float2*>(&cc);
+}
+
 // E of one segment and head, 128 value columns a block: a 128 x 128 tile, 8 x 8 sums a thread, 16 tokens a step through two
 // buffers. What bounds it is the latency of its few warps: 128 registers a thread leave two blocks an SM, 22 % of its warps, which
-// wait for the next step's rows and their stores (one prompt of 1,500 tokens, 32 heads of 128 x 128, 87 us: FFMA pipes 33 % and issue
-// slots 45 % busy, 27 % of the memory system's rate).
+// wait for the next step's rows and their stores (one prompt of 1,500 tokens, 32 heads of 128 x 128: FFMA pipes 33 % and issue slots
+// 45 % busy, 27 % of the memory system's rate, with one sum an instruction: 84 us inside a step, 77 with two).
 template <typename T, int ACT>
-__global__ void __launch_bounds__(SEG_THREADS)
+__global__ void __launch_bounds__(SEG_THREADS, 2)
 segment_state_kernel(const T* __restrict__ proj, long row_stride, int k_off, int v_off, const int* __restrict__ cu_q,
                      const float* __restrict__ decay, int heads, int dim, int vdim, float* __restrict__ seg_state, int seg_tokens,
                      int n_seqs, bool vec) {
@@ -290,11 +321,11 @@ segment_state_kernel(const T* __restrict__ proj, long row_stride, int k_off, int
       *reinterpret_cast<float4*>(&v_s[buf][t][c]) = v_next[u];
     }
   };
-  float acc[8][8];
+  float2 acc[8][4];                        // sums of columns 2 j, 2 j + 1
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
   fetch(0);
   stage(0);
   __syncthreads();
@@ -305,11 +336,12 @@ segment_state_kernel(const T* __restrict__ proj, long row_stride, int k_off, int
     for (int t = 0; t < SEG_STEP; ++t) {
       const float4 ka = *reinterpret_cast<const float4*>(&k_s[buf][t][4 * ty]), kb = *reinterpret_cast<const float4*>(&k_s[buf][t][64 + 4 * ty]);
       const float4 va = *reinterpret_cast<const float4*>(&v_s[buf][t][4 * tx]), vb = *reinterpret_cast<const float4*>(&v_s[buf][t][64 + 4 * tx]);
-      const float k[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w}, v[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
+      const float k[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
+      const float2 v[4] = {make_float2(va.x, va.y), make_float2(va.z, va.w), make_float2(vb.x, vb.y), make_float2(vb.z, vb.w)};
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(k[i], v[j], acc[i][j]);
+        for (int j = 0; j < 4; ++j) multiply_add_pair(acc[i][j], k[i], v[j]);
     }
     if (more) stage(buf ^ 1);
     __syncthreads();
@@ -321,7 +353,7 @@ segment_state_kernel(const T* __restrict__ proj, long row_stride, int k_off, int
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int e = e0 + 64 * (j >> 2) + 4 * tx + (j & 3);
-      if (d < dim && e < vdim) to[(size_t)d * vdim + e] = acc[i][j];
+      if (d < dim && e < vdim) to[(size_t)d * vdim + e] = j & 1 ? acc[i][j >> 1].y : acc[i][j >> 1].x;
     }
   }
 }
@@ -332,10 +364,11 @@ segment_state_kernel(const T* __restrict__ proj, long row_stride, int k_off, int
 // 64 x 64 weights decay^(i-j) (q_i . k_j) through shared memory, and their product with the values. Rows of 132 floats keep
 // the 16-byte reads along a row free of bank conflicts. What bounds it is the latency of a block's chain, load, barrier,
 // multiply, with two blocks an SM (registers and shared memory) to hide it: FFMA pipes 32 % and issue slots 45 % busy, shared-memory
-// reads 43 % (165 us at the size below).
+// reads 43 %, with one sum an instruction: 150 us at the size below inside a step, 138 with two.
 // Measured (one B200, one prompt of 1,500 tokens, 32 heads of 128 x 128, the three launches of a layer, states,
 // joining, outputs): 129 + 10 + 310 us when the segments walked their tokens one by one, then 90 + 24 + 193 us with
-// segments of 128, 283 in all with segments of 64, whose blocks have equal work. The next block's rows on their way while one is
+// segments of 128, 283 in all with segments of 64, whose blocks have equal work, 237 with two sums an instruction and the joining
+// in 20. The next block's rows on their way while one is
 // multiplied changed nothing (305 against 306 us).
 template <typename T, int ACT>
 __global__ void __launch_bounds__(SEG_THREADS, 2)
@@ -364,11 +397,11 @@ segment_output_kernel(const T* __restrict__ proj, long row_stride, int q_off, in
     }
   };
   load_block(q_s, i0, q_off + head * dim, 0, dim);
-  float acc[4][8];
+  float2 acc[4][4];                                         // sums of columns 2 j, 2 j + 1
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
   // acc += rows of `left` (4 ty ..; `columns` columns from c0 on) times the first `columns` rows of block_s; a CORNER leaves out
   // what lies above the diagonal of its four columns
   auto multiply_quad = [&](const float* left, int pitch, int c, auto corner) {
@@ -380,12 +413,12 @@ segment_output_kernel(const T* __restrict__ proj, long row_stride, int q_off, in
     for (int s = 0; s < 4; ++s) {
       const float* row = block_s + (c % SEG_ROWS + s) * SEG_PITCH;
       const float4 ra = *reinterpret_cast<const float4*>(row + 4 * tx), rb = *reinterpret_cast<const float4*>(row + 64 + 4 * tx);
-      const float r[8] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
+      const float2 r[4] = {make_float2(ra.x, ra.y), make_float2(ra.z, ra.w), make_float2(rb.x, rb.y), make_float2(rb.z, rb.w)};
 #pragma unroll
       for (int i = CORNER ? s : 0; i < 4; ++i) {
         const float x = s == 0 ? l[i].x : s == 1 ? l[i].y : s == 2 ? l[i].z : l[i].w;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x, r[j], acc[i][j]);
+        for (int j = 0; j < 4; ++j) multiply_add_pair(acc[i][j], x, r[j]);
       }
     }
   };
@@ -409,7 +442,7 @@ segment_output_kernel(const T* __restrict__ proj, long row_stride, int q_off, in
   for (int i = 0; i < 4; ++i) {
     const float w = decay_power(log2_lam, i0 + 4 * ty + i + 1);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] *= w;
+    for (int j = 0; j < 4; ++j) { acc[i][j].x *= w; acc[i][j].y *= w; }
   }
   for (int j0 = 0; j0 <= i0; j0 += SEG_ROWS) {
     __syncthreads();                                        // block_s and a_s are read
@@ -463,7 +496,7 @@ segment_output_kernel(const T* __restrict__ proj, long row_stride, int q_off, in
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int e = 64 * (j >> 2) + 4 * tx + (j & 3);
-      if (e0 + e < vdim) o[e] = acc[i][j];
+      if (e0 + e < vdim) o[e] = j & 1 ? acc[i][j >> 1].y : acc[i][j >> 1].x;
     }
   }
 }
@@ -483,8 +516,7 @@ int launch_segments(int n_seqs, int total_segments, int seg_tokens, float* seg_s
   const bool vec_state = (uintptr_t)seg_state % 16 == 0 && vdim % 4 == 0;      // the caller's scratch may begin anywhere
   lb_launch(segment_state_kernel<T, ACT>, dim3(e_tiles, heads, total_segments), SEG_THREADS, 0, stream, (const T*)proj, row_stride, k_off,
             v_off, cu_q, decay, heads, dim, vdim, seg_state, seg_tokens, n_seqs, vec);
-  lb_launch(scan_combine_kernel<true>, dim3((unsigned)(((size_t)heads * per_head + 255) / 256), n_seqs), 256, 0, stream, seg_state, state,
-            cu_q, state_slots, decay, heads, per_head, seg_tokens);
+  launch_combine<true>(n_seqs, seg_state, state, cu_q, state_slots, decay, heads, per_head, seg_tokens, stream);
   lb_launch(segment_output_kernel<T, ACT>, dim3(row_blocks * e_tiles, heads, total_segments), SEG_THREADS, (size_t)smem, stream,
             (const T*)proj, row_stride, q_off, k_off, v_off, out, cu_q, decay, heads, dim, vdim, (const float*)seg_state, seg_tokens, n_seqs,
             e_tiles, vec, vec_state);
@@ -517,8 +549,7 @@ int launch_scan(int n_seqs, int total_segments, int seg_tokens, float* seg_state
   int code = LB_MODE(1, total_segments);
   if (code) return code;
   const int per_head = dim * vdim;
-  lb_launch(scan_combine_kernel<false>, dim3((unsigned)(((size_t)heads * per_head + 255) / 256), n_seqs), 256, 0, stream, seg_state,
-            state, cu_q, state_slots, decay, heads, per_head, seg_tokens);
+  launch_combine<false>(n_seqs, seg_state, state, cu_q, state_slots, decay, heads, per_head, seg_tokens, stream);
   if ((code = lb_last_error())) return code;
   return LB_MODE(2, total_segments);
 #undef LB_MODE

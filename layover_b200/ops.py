@@ -787,10 +787,11 @@ def scan_as_products(tokens: int, segments: int, segment_tokens: int, heads: int
     products are taken where the tiles are full (heads of 65 to 128 with values that fill 128 columns, segments that are not
     mostly the end of a short portion), where the walk has more than two blocks an SM one after the other, and, for a 32-bit
     row, where the segments' states stay in the L2 between the launches. Measured (one B200, us of a layer, walk and products,
-    bfloat16; 32-bit): 32 heads of 128 x 128, one prompt of 300 tokens 100 and 89; 90 and 92, of 1,500 433 and 278; 373 and 320, of
-    4,000 1,150 and 868; 960 and 958, four of 600 678 and 561; 569 and 636, 1,500 beside 4 single tokens 458 and 349; 389 and 396,
-    beside 16 563 and 623; 503 and 689; 16 of 128 x 96, 1,500 tokens 162 and 158; 151 and 171; 4 of 128 x 128, 600 tokens 62 and 78;
-    32 of 64 x 64, 1,500 tokens 145 and 241; 137 and 277."""
+    bfloat16; 32-bit): 32 heads of 128 x 128, one prompt of 300 tokens 92 and 74; 82 and 74, of 1,500 443 and 237; 372 and 236, of
+    4,000 1,150 and 640; 952 and 634, four of 600 672 and 420; 561 and 429, 1,500 beside 16 single tokens 509 and 490; 440 and 490;
+    16 of 128 x 96, 1,500 tokens 166 and 145; 151 and 146; 4 of 128 x 128, 600 tokens 61 and 59; 52 and 58; 32 of 64 x 64, 1,500
+    tokens 151 and 230; 146 and 227. The lines were drawn with slower products (878 us for the 4,000 tokens, 642 beside the 16 single
+    ones): the form decides how a prompt's outputs are rounded, so a call keeps the one it has had, also where that now costs time."""
     room = segments * segment_tokens
     full_tiles = 64 < dim <= 128 and -(-vdim // 32) % 4 == 0
     walk_blocks = heads * -(-vdim // 32) * -(-room // SCAN_SEGMENT_TOKENS)

@@ -257,6 +257,25 @@ def test_qk_norm_rope_kv(dtype, q_heads, kv_heads, dim, page):
     assert float(untouched.abs().sum()) == 0.0          # nothing outside the given slots was written
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("q_heads, kv_heads, dim", [(4, 2, 16), (3, 1, 80), (2, 2, 256)])
+def test_qk_norm_weights_that_begin_anywhere(dtype, q_heads, kv_heads, dim):
+    """The norms' weights are read 16 bytes at a time where both begin on 16, one by one elsewhere: the same bits either way."""
+    o = ops()
+    rows = torch.randn(7, (q_heads + 2 * kv_heads) * dim, generator=torch.Generator().manual_seed(dim)).to(dtype)
+    room = 1 + 0.2 * torch.randn(2, dim + 4, device="cuda")
+    slots = torch.arange(7, dtype=torch.int32, device="cuda")
+    seen = []
+    for q_off, k_off in ((0, 0), (1, 0), (0, 1), (3, 2)):
+        q_w, k_w = (torch.empty(dim + 4, device="cuda")[off:off + dim].copy_(w[:dim]) for w, off in zip(room, (q_off, k_off)))
+        q_out = torch.empty(7, q_heads * dim, dtype=dtype, device="cuda")
+        pools = [torch.zeros(2, kv_heads, 4, dim, dtype=dtype, device="cuda") for _ in range(2)]
+        o.qk_norm_rope_kv(rows.cuda(), q_out, *pools, q_w, k_w, None, slots, q_heads, kv_heads, dim, 4, 1e-5)
+        seen.append((q_out, *pools))
+    for other in seen[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(seen[0], other))
+
+
 def test_qk_norm_rope_small_positions_are_tight():
     o = ops()
     dim, theta = 64, 10000.0

@@ -698,10 +698,7 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
         const uint32_t v_addr = smem_u32(v_s + stage * TILE_BYTES);
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-          if (u == 0) {      // the tiles first: the probabilities are what comes last
-            ok = warp_wait(&v_full[stage], (i / KV_STAGES) & 1);
-            if (ok && i + 1 < count) ok = warp_wait(&k_full[(i + 1) % KV_STAGES], ((i + 1) / KV_STAGES) & 1);
-          }
+          if (u == 0) ok = warp_wait(&v_full[stage], (i / KV_STAGES) & 1);      // the tile first: the probabilities come last
           ok = ok && warp_spin(&p_most[u], i & 1);
           if (!ok) break;
           fence_after_sync();
@@ -709,7 +706,8 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
 #pragma unroll
           for (int ks = 0; ks < MOST_KEYS / 16; ++ks)
             umma_bf16_ts(tmem_o + u * 128, tmem_s + u * 128 + ks * 8, desc_mn_major(v_addr + ks * 16 * 128), idesc_o, (i > 0 || ks > 0) ? 1u : 0u);
-          ok = warp_spin(&p_full[u], i & 1);
+          if (u == 0 && i + 1 < count) ok = warp_wait(&k_full[(i + 1) % KV_STAGES], ((i + 1) / KV_STAGES) & 1);
+          ok = ok && warp_spin(&p_full[u], i & 1);
           if (!ok) break;
           fence_after_sync();
 #pragma unroll

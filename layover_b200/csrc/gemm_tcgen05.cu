@@ -33,6 +33,8 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "tcgen05.cuh"
 
@@ -417,8 +419,9 @@ gemm_fewtoken_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 
 
 // ------------------------------------------------------------------ the persistent kernel
-// The few-token orientation asks for two blocks per SM (half the shared memory each): a weight
-// matrix with about as many tiles as SMs then still runs in one round.
+// One block an SM: a launch never counted on two of half the ring each (their tensor memory), and half a ring of weights in flight was
+// slower in the few-token orientation (one B200, q/k/v of 6144 rows, o and down of a 2560-wide model: 64 tokens 13.6 / 10.6 / 16.5
+// -> 12.5 / 10.1 / 15.0 us, 128 tokens 16.5 / 14.0 / 20.3 -> 14.6 / 12.2 / 17.0, the sum of the splits below included).
 // PAIR: two blocks of a cluster work as one MMA unit on a tile of 256 rows x BN columns; each block
 // stages its own 128 rows and its own half of the BN columns' operand, a third fewer bytes into
 // each SM per product than a block on its own, and so more stages in the same memory.
@@ -426,8 +429,7 @@ template <int BN, bool SWAP, bool PAIR = false> struct Tile {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int BLOCKS_PER_SM = SWAP ? 2 : 1;
-  static constexpr int BUDGET = SMEM_BUDGET / BLOCKS_PER_SM;   // a pair's seventh stage fits in 227 KB, and measured no faster
+  static constexpr int BUDGET = SMEM_BUDGET;                  // a pair's seventh stage fits in 227 KB, and measured no faster
   static constexpr int STAGES = (BUDGET / STAGE_BYTES) > 8 ? 8 : (BUDGET / STAGE_BYTES);
   static constexpr int ACC_COLS = BN < 16 ? 16 : BN;          // columns of one accumulator
   static constexpr int TMEM_COLS = 2 * ACC_COLS < 32 ? 32 : 2 * ACC_COLS;
@@ -483,7 +485,7 @@ __device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, 128;
 // epilogue handles its own 128 rows like a tile of its own (with a scratch slot of its own when K
 // is split).
 template <int BN, bool SWAP, typename OutT, int EPI, bool PAIR = false>
-__global__ void __launch_bounds__(persistent_threads(EPI), Tile<BN, SWAP, PAIR>::BLOCKS_PER_SM)
+__global__ void __launch_bounds__(persistent_threads(EPI), 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     OutT* __restrict__ C, long ldc, int rows_a, int rows_b, const Schedule sch,
                     float* __restrict__ partials, unsigned* __restrict__ counters, bool vector_ok, const HeadsEpilogue he,
@@ -875,54 +877,61 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
               }
             }
           } else if (m0 + row < rows_a) {
-            for (int q0 = q_begin; q0 < q_end; q0 += 4) {
-              float4 sum[4];
+            // All splits of a block's usual share on their way at once (one trip to the L2, two before: 333 tokens, left-over
+            // tiles in 3 to 8 splits, q/k/v 24.2 -> 23.2 us); every element is still summed in split order
+            auto add_up = [&](auto quads_at_once, auto splits_at_once) {
+              constexpr int QUADS = decltype(quads_at_once)::value, SPLITS = decltype(splits_at_once)::value;
+              for (int q0 = q_begin; q0 < q_end; q0 += QUADS) {
+                float4 sum[QUADS];
 #pragma unroll
-              for (int u = 0; u < 4; ++u) sum[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-              for (int s0 = 0; s0 < seg.splits; s0 += 4) {
-                float4 part[4][4];
+                for (int u = 0; u < QUADS; ++u) sum[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int s0 = 0; s0 < seg.splits; s0 += SPLITS) {
+                  float4 part[SPLITS][QUADS];
 #pragma unroll
-                for (int ds = 0; ds < 4; ++ds)
+                  for (int ds = 0; ds < SPLITS; ++ds)
 #pragma unroll
-                  for (int u = 0; u < 4; ++u)
-                    part[ds][u] = (s0 + ds < seg.splits && q0 + u < q_end)
-                                      ? tile_partials[((size_t)(s0 + ds) * (BN / 4) + q0 + u) * BM + row]
-                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int u = 0; u < QUADS; ++u)
+                      part[ds][u] = (s0 + ds < seg.splits && q0 + u < q_end)
+                                        ? tile_partials[((size_t)(s0 + ds) * (BN / 4) + q0 + u) * BM + row]
+                                        : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int ds = 0; ds < 4; ++ds)
+                  for (int ds = 0; ds < SPLITS; ++ds)
 #pragma unroll
-                  for (int u = 0; u < 4; ++u) {
-                    sum[u].x += part[ds][u].x; sum[u].y += part[ds][u].y;
-                    sum[u].z += part[ds][u].z; sum[u].w += part[ds][u].w;
-                  }
-              }
+                    for (int u = 0; u < QUADS; ++u) {
+                      sum[u].x += part[ds][u].x; sum[u].y += part[ds][u].y;
+                      sum[u].z += part[ds][u].z; sum[u].w += part[ds][u].w;
+                    }
+                }
 #pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                if (q0 + u >= q_end) continue;
-                const int col = (q0 + u) * 4;
-                const float vals[4] = {sum[u].x, sum[u].y, sum[u].z, sum[u].w};
-                if (!SWAP && vector_ok && col + 4 <= valid_cols) {
-                  OutT* dst = C + (size_t)(m0 + row) * ldc + n0 + col;
-                  if (sizeof(OutT) == 2) {
-                    const __nv_bfloat162 lo = __floats2bfloat162_rn(vals[0], vals[1]), hi = __floats2bfloat162_rn(vals[2], vals[3]);
-                    uint2 w;
-                    w.x = *reinterpret_cast<const uint32_t*>(&lo);
-                    w.y = *reinterpret_cast<const uint32_t*>(&hi);
-                    *reinterpret_cast<uint2*>(dst) = w;
+                for (int u = 0; u < QUADS; ++u) {
+                  if (q0 + u >= q_end) continue;
+                  const int col = (q0 + u) * 4;
+                  const float vals[4] = {sum[u].x, sum[u].y, sum[u].z, sum[u].w};
+                  if (!SWAP && vector_ok && col + 4 <= valid_cols) {
+                    OutT* dst = C + (size_t)(m0 + row) * ldc + n0 + col;
+                    if (sizeof(OutT) == 2) {
+                      const __nv_bfloat162 lo = __floats2bfloat162_rn(vals[0], vals[1]), hi = __floats2bfloat162_rn(vals[2], vals[3]);
+                      uint2 w;
+                      w.x = *reinterpret_cast<const uint32_t*>(&lo);
+                      w.y = *reinterpret_cast<const uint32_t*>(&hi);
+                      *reinterpret_cast<uint2*>(dst) = w;
+                    } else {
+                      *reinterpret_cast<float4*>(dst) = sum[u];
+                    }
                   } else {
-                    *reinterpret_cast<float4*>(dst) = sum[u];
-                  }
-                } else {
 #pragma unroll
-                  for (int e = 0; e < 4; ++e) {
-                    if (col + e < valid_cols) {
-                      if (SWAP) store_one<OutT>(C + (size_t)(n0 + col + e) * ldc + m0 + row, vals[e]);
-                      else store_one<OutT>(C + (size_t)(m0 + row) * ldc + n0 + col + e, vals[e]);
+                    for (int e = 0; e < 4; ++e) {
+                      if (col + e < valid_cols) {
+                        if (SWAP) store_one<OutT>(C + (size_t)(n0 + col + e) * ldc + m0 + row, vals[e]);
+                        else store_one<OutT>(C + (size_t)(m0 + row) * ldc + n0 + col + e, vals[e]);
+                      }
                     }
                   }
                 }
               }
-            }
+            };
+            if (seg.splits > 4) add_up(std::integral_constant<int, 3>{}, std::integral_constant<int, 8>{});
+            else add_up(std::integral_constant<int, 6>{}, std::integral_constant<int, 4>{});
           }
         }
         epilogue_sync();
@@ -977,15 +986,13 @@ int launch(const CUtensorMap& map_a, const CUtensorMap& map_b, void* C, long ldc
            cudaStream_t stream, const int* tile_b_rows = nullptr, LbClip clip = LbClip{}) {
   using T = Tile<BN, SWAP>;
   auto kernel = gemm_tcgen05_kernel<BN, SWAP, OutT, EPI>;
-  static int blocks_per_sm = 0;      // how many blocks of this kernel an SM really holds (the same on every B200)
   static LbPerDeviceOnce configured;
   const bool ready = configured.run([&] {
     int fit = 0;
     if (!LB_ALLOW_SMEM(kernel, T::SMEM)() ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, PERSISTENT_THREADS, T::SMEM) != cudaSuccess || fit < 1)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, PERSISTENT_THREADS, T::SMEM) != cudaSuccess)
       return false;
-    blocks_per_sm = fit < T::BLOCKS_PER_SM ? fit : T::BLOCKS_PER_SM;
-    return true;
+    return fit >= 1;
   });
   if (!ready) {
     const int code = lb_last_error();
@@ -993,7 +1000,7 @@ int launch(const CUtensorMap& map_a, const CUtensorMap& map_b, void* C, long ldc
   }
   // Blocks that split a tile wait for one another, so a launch never has more blocks than the GPU
   // holds at once.
-  const int slots = pb.sm_count * blocks_per_sm;
+  const int slots = pb.sm_count;
   Schedule sch;
   sch.tiles_m = (pb.rows_a + BM - 1) / BM;
   sch.tiles = sch.tiles_m * ((pb.rows_b + BN - 1) / BN);

@@ -59,7 +59,7 @@ class GatedMLP(Part):
     def activated(self, h: torch.Tensor) -> torch.Tensor:
         """act(h Wg^T) * (h Wu^T) over the interleaved weights. Many tokens, or at most 16: one
         product with the activation in its epilogue. In between: product, then the activation kernel,
-        which is faster there (a whole feed-forward at 64 tokens: 41.7 us against 43.5 us fused)."""
+        which is as fast there or faster (a whole feed-forward at 32 tokens: 35.6 us against 35.7 us fused, at 64: 39.0 against 39.7)."""
         tokens = h.shape[0]
         out = torch.empty((tokens, self.inter), dtype=torch.bfloat16, device=h.device)
         epilogue = FUSED_ACTIVATIONS.get(self.activation)

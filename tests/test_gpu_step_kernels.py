@@ -68,6 +68,28 @@ def test_few_token_gated_product_split_over_a_cluster(m, inter, k):
         assert ((out.double() - want).abs() <= 4 * 2.0 ** -8 * (want.abs() + u.abs() + 0.1)).all()
 
 
+@pytest.mark.parametrize("m", [1, 8, 9, 16, 17, 32, 33, 64, 65, 128])
+def test_few_token_gated_product_of_whole_tiles(m):
+    """Columns that the two halves of a tile compute for one another: none, one, all of a half. SwiGLU: the bits of product and activation."""
+    o, gen, inter, k = ops(), torch.Generator().manual_seed(m), 3 * 64, 200
+    a = torch.randn(m, k, generator=gen).to(torch.bfloat16).cuda()
+    w = (2 * torch.randn(2 * inter, k, generator=gen) / math.sqrt(k)).to(torch.bfloat16).cuda()      # interleaved already
+    rows, out = torch.empty(m, 2 * inter, dtype=torch.bfloat16, device="cuda"), torch.full((m, inter), float("nan"), dtype=torch.bfloat16, device="cuda")
+    want = torch.empty_like(out)
+    o.gemm_tcgen05(a, w, out, epilogue="swiglu")
+    o.gemm_tcgen05(a, w, rows, max_splits=1)
+    o.swiglu(rows, want, block=o.SWIGLU_BLOCK)
+    assert o.gemm_status() == 0 and torch.equal(out, want)
+    if m <= 16:
+        o.gemm_tcgen05(a, w, out.fill_(float("nan")), epilogue="clipped_swiglu", limit=1.0, slope=1.7)
+        g, u = (a.double() @ part.double().T for part in w.view(-1, 2, o.SWIGLU_BLOCK, k).transpose(0, 1).reshape(2, inter, k))
+        g, u = g.clamp(max=1.0), u.clamp(-1.0, 1.0)
+        clipped = g * torch.sigmoid(1.7 * g) * (u + 1)
+        # gate, up, activation and product each round to bfloat16 at most, as in the split product's test above
+        assert o.gemm_status() == 0
+        assert ((out.double() - clipped).abs() <= 4 * 2.0 ** -8 * (clipped.abs() + u.abs() + 0.1)).all()
+
+
 @pytest.mark.parametrize("q_heads, kv_heads", [(4, 2), (32, 8)])
 @pytest.mark.parametrize("window", [0, 200])
 def test_prompt_attention_with_keys_dealt_to_several_blocks(q_heads, kv_heads, window):

@@ -1737,13 +1737,13 @@ _PORTION_SCRATCH_FLOATS = 32 << 20     # the most that the partial results of sp
 def portion_splits(lens: tuple[tuple[int, int], ...], q_heads: int, kv_heads: int, window: int, sms: int) -> int:
     """How many blocks share the keys of the rows of portions of (new tokens, context): the number that ends first.
 
-    A block holds an SM, takes 9 us and 1.82 us for each of its tiles of 128 keys, and the blocks run in rounds of one an SM: of
+    A block holds an SM, takes 9 us and 2.25 us for each of its tiles of 128 keys, and the blocks run in rounds of one an SM: of
     equal blocks where the keys are split, while the few short ones of a fresh prompt end early and leave their SMs to the last. A
-    split costs 7 us, 0.1 us a block of a row, and 0.4 us for each MB of partial results (130 floats a row, head and
-    block) on their way to the merge. The figures fit 380 measurements on one B200 (8 over 2 to 64 over 8 heads, 40 to 2,048
-    new tokens after 0 to 20,000): what they pick is 0.15 % over the best of 1 to 8 on average, and nowhere over no split at
-    all. 32 over 8 heads, no split and 2 blocks: 512 tokens after 8,209 139 and 91 us; 16 over 2: 1,280 tokens after 1,000 45 and 56,
-    1,024 after 12,000 196 and 121."""
+    split costs 8.2 us, 0.2 us a block of a row, and 0.57 us for each MB of partial results (130 floats a row, head and
+    block) on their way to the merge. The figures fitted 549 measurements on one B200 (4 over 2 to 64 over 8 heads, 8 to 2,048
+    new tokens of one or three requests after 0 to 30,000) while a tile took that long; it takes 1.82 us since, and a split 7 us. The number
+    decides how a row's outputs are rounded, so a call keeps the one it has had. 32 over 8 heads, no split and 2 blocks: 512 tokens
+    after 8,209 139 and 91 us; 16 over 2: 1,280 tokens after 1,000 45 and 56, 1,024 after 12,000 196 and 121."""
     blocks = sum(-(-new // TCGEN05_TILE) for new, _ in lens) * q_heads // 2
     if (q_heads // kv_heads) % 2 or blocks >= 2 * sms:
         return 1
@@ -1759,8 +1759,8 @@ def portion_splits(lens: tuple[tuple[int, int], ...], q_heads: int, kv_heads: in
     def cost(s: int) -> float:
         rounds = -(-blocks * s // sms)
         if s == 1:
-            return 1.82 * (longest + (rounds - 1) * shortest)
-        return 1.82 * rounds * -(-longest // s) + 7.0 + (0.1 + 0.4 * megabytes) * s
+            return 2.25 * (longest + (rounds - 1) * shortest)
+        return 2.25 * rounds * -(-longest // s) + 8.2 + (0.2 + 0.57 * megabytes) * s
 
     most = min(8, longest // 2, _PORTION_SCRATCH_FLOATS // (2 * blocks * TCGEN05_TILE * 130))
     return min(range(1, max(2, most + 1)), key=cost)
@@ -1771,14 +1771,13 @@ def exact_on_tcgen05(lens: tuple[tuple[int, int], ...], q_heads: int, window: in
     """Whether portions of (new tokens, context) with exact weights are quicker on the tcgen05 kernel than on the mma.sync one.
 
     A block of the first takes 128 queries of two heads over tiles of 128 keys, of the second 64 queries of one head over tiles of
-    64. Either takes its start, the first 7 us more where pages are held, and then the longer of its longest block's tiles one after
-    the other and all blocks' tiles shared out over the SMs. A window makes every tile of the second longer, and of the first the tiles that it cuts, up to three a
-    block. The figures (us) fit 230 measurements on one B200 (12 over 2, 16 over 4, 32 over 8 and 64 over 8 heads, 1 to 8 prompts of 20
-    to 1,500 tokens, portions of 10 to 1,000 tokens after 500 to 6,000, windows of 0, 128 and 1,024, chunks of 1,024): what this rule
-    takes is 0.2 % over the better of the two on average, and nowhere over the mma.sync kernel. 16 over 4 heads, tcgen05 and mma.sync: one prompt of 20 tokens 16 and 9, of 261
-    22 and 19, of 512 24 and 28, two of 611 27 and 46, one of 1,500 44 and 104, behind a window of 1,024 44 and 137; 64 tokens after
-    500 32 and 32, after 3,000 69 and 132."""
-    def shape(rows: int) -> tuple[int, int]:          # tiles of the longest block, and of all blocks of one head or pair
+    64. Either takes its start, and then the longer of its longest block's tiles one after the other and all blocks' tiles
+    shared out over the SMs; a mask within the tiles (a window) makes a tile longer. The figures (us) fitted 1,016 measurements on one
+    B200 (12 over 2, 16 over 4, 32 over 8 and 64 over 8 heads, 1 to 16 prompts of 20 to 900 tokens, portions of 2 to 1,000 tokens
+    after 300 to 6,000, windows of 0, 128, 512 and 1,024) of a slower tcgen05 kernel. The two kernels round differently, so a call keeps
+    the one it has had. 16 over 4 heads, tcgen05 and mma.sync: one prompt of 20 tokens 16 and 9, of 261 22 and 19, of 512 24 and 28, two of
+    611 27 and 46, one of 1,500 44 and 104, behind a window of 1,024 44 and 137; 64 tokens after 500 32 and 32, after 3,000 69 and 132."""
+    def cost(rows: int, heads: int, start: float, tile: float, shared: float, masked: float) -> float:
         longest = total = 0
         for new, ctx in lens:
             for first in range(ctx - new, ctx, rows):
@@ -1786,13 +1785,9 @@ def exact_on_tcgen05(lens: tuple[tuple[int, int], ...], q_heads: int, window: in
                 low = max(0, first - window + 1) if window > 0 else (first // -window * -window if window else 0)
                 tiles = last // rows - low // rows + 1
                 longest, total = max(longest, tiles), total + tiles
-        return longest, total
+        return start + (masked if window else 1.0) * max(tile * longest, shared * total * heads / sms)
 
-    longest, total = shape(128)
-    start = 20.0 if any(ctx > new for new, ctx in lens) else 13.0
-    tcgen05 = start + max(2.6 * longest + 6.0 * min(longest, 3 if window > 0 else 0), 4.5 * total * (q_heads // 2) / sms)
-    longest, total = shape(64)
-    return tcgen05 < 4.9 + (1.76 if window else 1.0) * max(3.07 * longest, 2.49 * total * q_heads / sms)
+    return cost(128, q_heads // 2, 8.5, 4.85, 8.1, 1.92) < cost(64, q_heads, 4.9, 3.07, 2.49, 1.76)
 
 
 def attention_bf16(q, cache, out, block_table, batch, q_heads, kv_heads, dim, page_tokens, scale, window, sinks=None,

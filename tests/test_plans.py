@@ -161,3 +161,18 @@ def test_portion_splits_weigh_what_a_split_takes():
                     splits = plan(*[(new, ctx)] * count, heads=heads)
                     tiles = count * -(-new // 128)
                     assert 1 <= splits <= 8 and (splits == 1 or tiles * heads[0] * splits * 128 * 130 <= 32 << 20)
+
+
+@pytest.mark.parametrize("new, context, splits", [(128, 768, 1), (128, 897, 1), (128, 1024, 1), (256, 1400, 1), (256, 2600, 3), (512, 2100, 1),
+                                                  (512, 2200, 2), (777, 12100, 1), (5, 827, 3), (2, 749, 3)])
+def test_a_portion_keeps_its_number_of_blocks(new, context, splits):
+    """How many blocks share a row's keys decides how its outputs are rounded."""
+    assert ops.portion_splits(((new, context),), 32, 8, 0, SMS) == splits
+
+
+@pytest.mark.parametrize("window", [0, 1024, -1024])
+@pytest.mark.parametrize("heads", [16, 32])
+def test_prompts_with_exact_weights_keep_their_kernel(window, heads):
+    """The two kernels add a row's keys in tiles of different sizes and round differently."""
+    kernel = lambda new: ops.exact_on_tcgen05(((new, new),), heads, window, SMS)
+    assert not any(kernel(new) for new in (65, 97, 261, 320, 396, 404, 435)) and all(kernel(new) for new in (321, 371, 384, 512, 611, 1500))

@@ -39,7 +39,9 @@ constexpr int THREADS = 192;
 constexpr uint32_t SPIN_LIMIT = 1u << 20;
 constexpr float RESCALE_THRESHOLD = 8.0f;       // in log2 units
 
-__device__ int g_attn_error = 0;   // 0 = ok; which wait ran out otherwise
+// 0 = ok; which wait ran out otherwise. The kernel of one head: 1 to 8; of pairs: 21 producer, 22 queries, 23 first keys, 24 values or
+// probabilities, 25 next keys, 26 scores, 27 and 29 the second product, 28 values to be zeroed
+__device__ int g_attn_error = 0;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -691,23 +693,24 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
         umma_commit(&s_full[u]);
         if (u == 1) umma_commit(&k_empty[stage]);
       };
-      bool ok = warp_wait(q_full, 0) && warp_wait(&k_full[0], 0);
+      auto ran_out = [&](int code) { atomicCAS(&g_attn_error, 0, code); flag[0] = 1; return false; };
+      bool ok = (warp_wait(q_full, 0) || ran_out(22)) && (warp_wait(&k_full[0], 0) || ran_out(23));
       if (ok) { fence_after_sync(); issue_s(0, 0); issue_s(0, 1); }
       for (int i = 0; i < count && ok; ++i) {
         const int stage = i % KV_STAGES;
         const uint32_t v_addr = smem_u32(v_s + stage * TILE_BYTES);
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-          if (u == 0) ok = warp_wait(&v_full[stage], (i / KV_STAGES) & 1);      // the tile first: the probabilities come last
-          ok = ok && warp_spin(&p_most[u], i & 1);
+          if (u == 0) ok = warp_wait(&v_full[stage], (i / KV_STAGES) & 1) || ran_out(24);      // the tile first: the probabilities come last
+          ok = ok && (warp_spin(&p_most[u], i & 1) || ran_out(24));
           if (!ok) break;
           fence_after_sync();
           // 16 keys a step: 8 columns of packed probabilities, 16 rows of V; the first 96 keys under the others' exponentials
 #pragma unroll
           for (int ks = 0; ks < MOST_KEYS / 16; ++ks)
             umma_bf16_ts(tmem_o + u * 128, tmem_s + u * 128 + ks * 8, desc_mn_major(v_addr + ks * 16 * 128), idesc_o, (i > 0 || ks > 0) ? 1u : 0u);
-          if (u == 0 && i + 1 < count) ok = warp_wait(&k_full[(i + 1) % KV_STAGES], ((i + 1) / KV_STAGES) & 1);
-          ok = ok && warp_spin(&p_full[u], i & 1);
+          if (u == 0 && i + 1 < count) ok = warp_wait(&k_full[(i + 1) % KV_STAGES], ((i + 1) / KV_STAGES) & 1) || ran_out(25);
+          ok = ok && (warp_spin(&p_full[u], i & 1) || ran_out(24));
           if (!ok) break;
           fence_after_sync();
 #pragma unroll
@@ -723,7 +726,6 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
           if (u == 1) umma_commit(&v_empty[stage]);
         }
       }
-      if (!ok) { atomicCAS(&g_attn_error, 0, 22); flag[0] = 1; }
     }
   } else {
     // ---------------- softmax and epilogue: warpgroup u owns head u, one query row per thread

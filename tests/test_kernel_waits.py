@@ -1,0 +1,16 @@
+"""What a kernel does when one of its bounded waits runs out, read from the sources: nothing here lets a GPU wait for what never comes."""
+
+import re
+
+from layover_b200.csrc.build import HERE
+
+
+def _prompt_attention_of_pairs():
+    source = (HERE / "attention_tcgen05.cu").read_text()
+    return source[source.index("attention_tcgen05_pair_kernel(const"): source.index("attention_merge_kernel(const")]
+
+
+def test_prompt_attention_tells_which_wait_ran_out():
+    kernel = _prompt_attention_of_pairs()
+    codes = [int(code) for code in re.findall(r"g_attn_error, 0, (\d+)|ran_out\((\d+)\)|flag, (\d+), lane", kernel) for code in code if code]
+    assert set(codes) == set(range(21, 30))

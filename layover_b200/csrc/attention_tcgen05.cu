@@ -826,6 +826,7 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
           if (lane == 0) mbar_arrive(&p_most[u]);
         }
       }
+      if (!ok) break;         // a wait above ran out: nothing of this tile is announced
       const float tile_sum = (part_sum[0] + part_sum[1]) + (part_sum[2] + part_sum[3]);
       l_sum = l_sum * factor + tile_sum;
       m_ref = m_new;

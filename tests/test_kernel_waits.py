@@ -14,3 +14,9 @@ def test_prompt_attention_tells_which_wait_ran_out():
     kernel = _prompt_attention_of_pairs()
     codes = [int(code) for code in re.findall(r"g_attn_error, 0, (\d+)|ran_out\((\d+)\)|flag, (\d+), lane", kernel) for code in code if code]
     assert set(codes) == set(range(21, 30))
+
+
+def test_prompt_attention_announces_nothing_of_a_tile_whose_wait_ran_out():
+    kernel = _prompt_attention_of_pairs()
+    between = kernel[kernel.index("mbar_arrive(&p_most[u])"): kernel.index("mbar_arrive(&p_full[u])")]
+    assert "if (!ok) break;" in between          # the waits before stand in an inner loop, whose break leaves only that one

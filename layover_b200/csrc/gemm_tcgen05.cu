@@ -646,6 +646,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       live_tiles = warp_uniform(live_tiles);
       bool ok = true;
       for (int j = 0; j < n_segments && ok; ++j) {
+        if (j > 0 && warp_uniform((int)flag[0])) break;          // another warp's wait ran out
         const Segment seg = segment_at(sch, block, blocks, j);
         if (warp_uniform(seg.tile) >= live_tiles) continue;
         const int buf = live & 1;

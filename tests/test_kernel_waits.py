@@ -20,3 +20,10 @@ def test_prompt_attention_announces_nothing_of_a_tile_whose_wait_ran_out():
     kernel = _prompt_attention_of_pairs()
     between = kernel[kernel.index("mbar_arrive(&p_most[u])"): kernel.index("mbar_arrive(&p_full[u])")]
     assert "if (!ok) break;" in between          # the waits before stand in an inner loop, whose break leaves only that one
+
+
+def test_persistent_product_issues_no_tile_after_another_warps_wait_ran_out():
+    source = (HERE / "gemm_tcgen05.cu").read_text()
+    kernel = source[source.index("gemm_tcgen05_kernel(const"): source.index("// ---------------- teardown", source.index("gemm_tcgen05_kernel(const"))]
+    loops = re.findall(r"for \(int j = 0; j < n_segments(.*?)const Segment seg", kernel, re.S)
+    assert len(loops) == 4 and all("flag[0]" in loop for loop in loops[:3])        # two forms of the producer, the issuing warp; the epilogue is last

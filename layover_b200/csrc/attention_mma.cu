@@ -383,8 +383,8 @@ attention_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_
     }
     // a warp whose rows all lie before this tile has nothing to do in it
     if (tile * BKEYS <= p_warp + 15) {
-      // every row of the warp sees the whole tile unless it reaches past the first row's position,
-      // starts before the first visible key or a window cuts it
+      // every row of the warp sees the whole tile unless it reaches past the first row's position or starts before the
+      // first visible key; behind a window or a chunked mask every tile is compared, also one that no row's window cuts
       const bool masked = tile * BKEYS + BKEYS - 1 > p_warp || tile * BKEYS < key_lo || window != 0;
       warp_tile<MAX_DIM, EXACT, BKEYS / 16, SINK>(qf, k_base + buf * buf_bytes, v_base + buf * buf_bytes, dim, o, m_run,
                                                         l_run, masked, tile * BKEYS, p0, p1, key_lo, window, scale_log2, t,

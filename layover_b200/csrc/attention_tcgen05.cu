@@ -11,7 +11,7 @@
 //
 // Common to both: warp 0 walks the block table and issues one 5-D TMA copy per page and half of the
 // head, one copy per lane (the whole cache group's pool is ONE tensor map: dim, slot, KV head, page,
-// layer x {K, V}); warp 1 lane 0 issues the MMAs; the softmax warps own one query row per thread:
+// layer x {K, V}); warp 1 walks the products as a whole warp, one elected lane issuing them; the softmax warps own one query row per thread:
 // they read the row's 128 scores from tensor memory, keep the running maximum and sum, write the
 // probabilities as the bf16 A operand of the second product and rescale the output only when the
 // maximum has grown by more than 2^8 (the accumulated values stay exact relative to a reference
@@ -573,12 +573,12 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid
 // The kernel for prompt portions where an even number of query heads shares a KV head. A block
 // takes the same 128 tokens of TWO such heads: each head has its own query tile, score and output
 // accumulators in tensor memory and its own softmax warpgroup, and both read the same K and V
-// tiles. The MMA thread alternates between the heads (O_a += P_a V, S_a = Q_a K^T of the next
+// tiles. The issuing warp alternates between the heads (O_a += P_a V, S_a = Q_a K^T of the next
 // tile, then the same for b), so that the tensor cores work for one head while the other's
 // softmax runs; the part of a second product that the first 96 keys make is issued under the
 // exponentials of the last 32. The probabilities never touch shared memory: each thread overwrites the scores of
 // its own row in tensor memory with them (bf16, two per column) and the second product reads its
-// A operand from there; products issued by one thread run in order, so the next tile's scores
+// A operand from there; products issued by one lane run in order, so the next tile's scores
 // land on those columns only after the product that read them.
 // A portion far into its context has few tiles of queries and many of keys: its keys are then dealt to several blocks
 // (gridDim.z), each of which leaves its maximum, sum and output for `attention_merge_kernel`. Measured (one B200, 32 heads
@@ -593,7 +593,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid
 // columns that the scores leave free, and the second product runs over them as well. Measured (one B200, 1,500 tokens of 32
 // heads over 8 behind a window of 1,024; two prompts of 611, 16 over 4): 45 us and 26 us (on mma.sync 224 and 87; 96 and 35 with
 // comparisons in every tile of a window and one lane issuing)
-constexpr int PAIR_THREADS = 320;   // warp 0 producer, warps 1 and 10 the heads' MMA issuers, warps 2-5 and 6-9 the softmax warpgroups
+constexpr int PAIR_THREADS = 320;   // warp 0 producer, warp 1 MMA issuer, warps 2-5 and 6-9 the softmax warpgroups
 constexpr int MOST_KEYS = 96;       // keys of a tile whose part of the second product does not wait for the last exponentials
 constexpr int PAIR_SMEM = TILE_BYTES * (2 + 2 * KV_STAGES) + 1024 + 512 + TABLE_CACHE * 4;   // Q x2, K and V stages, slack, barriers, table
 
@@ -646,7 +646,7 @@ attention_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);      // both heads' products
+      mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
       mbar_init(&s_full[i], 1); mbar_init(&p_most[i], 4); mbar_init(&p_full[i], 4); mbar_init(&pv_done[i], 1);
     }
     flag[0] = 0;

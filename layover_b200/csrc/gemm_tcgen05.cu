@@ -16,8 +16,8 @@
 //
 // Two kernels share the PTX wrappers, descriptors and epilogue stores:
 //   many tokens: persistent blocks of six warps, one per SM. Warp 0 lane 0 issues TMA loads through
-//     a ring of stages, warp 1 lane 0 issues the MMAs into one of two accumulators in tensor memory
-//     and frees stages with tcgen05.commit, warps 2-5 run the epilogue of the other accumulator.
+//     a ring of stages, warp 1 (all of it, one elected lane issuing) the MMAs into one of two accumulators in
+//     tensor memory and frees stages with tcgen05.commit, warps 2-5 run the epilogue of the other accumulator.
 //     Whole rounds of tiles are dealt one tile per block; the tiles left over are split along K so
 //     that the last round keeps every SM busy, and the blocks of a tile then add up the partial
 //     tiles together, each its share of the columns, in split order.
@@ -1294,6 +1294,8 @@ LB_EXPORT int lb_gemm_tcgen05(const void* A, const void* W, void* C, int out_dty
   if (epilogue == 1) {
     if (swap) {
       if (bn == 16) return launch_fewtoken<16, bf16, 1>(map_a, map_b, C, ldc, pb, stream);
+      // 17 to 128 tokens are taken from whoever asks; the package's own feed-forward has product and activation as two kernels there,
+      // which is as fast or faster (2560 x 9728, 64 tokens: 39.0 against 39.7 us)
       if (bn == 32) return launch_fewtoken<32, bf16, 1>(map_a, map_b, C, ldc, pb, stream);
       if (bn == 64) return launch_fewtoken<64, bf16, 1>(map_a, map_b, C, ldc, pb, stream);
       return launch_fewtoken<128, bf16, 1>(map_a, map_b, C, ldc, pb, stream);

@@ -808,7 +808,8 @@ def scan_segments(q_lens: list[int], state_bytes: int, dim: int = 0) -> tuple[in
 
     `dim` 33 to 128: heads of that size whose segments' work is done as matrix products. Half as long segments then have half the
     weights between a segment's own tokens, and blocks of equal work, for twice the states: 32 heads of 128 x 128, one prompt of
-    1,500 tokens: 306 -> 283 us a layer with 64, of 300 tokens 118 -> 89, two of 700 and 900: 322 -> 298."""
+    1,500 tokens: 306 -> 283 us a layer with 64, of 300 tokens 118 -> 89, two of 700 and 900: 322 -> 298 (with one sum an instruction;
+    `scan_as_products` has the products' times as they are)."""
     longest = max(q_lens)
     if longest < 2 * SCAN_SEGMENT_TOKENS:
         return 0, 0

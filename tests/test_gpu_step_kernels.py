@@ -74,12 +74,13 @@ def test_few_token_gated_product_of_whole_tiles(m):
     o, gen, inter, k = ops(), torch.Generator().manual_seed(m), 3 * 64, 200
     a = torch.randn(m, k, generator=gen).to(torch.bfloat16).cuda()
     w = (2 * torch.randn(2 * inter, k, generator=gen) / math.sqrt(k)).to(torch.bfloat16).cuda()      # interleaved already
-    rows, out = torch.empty(m, 2 * inter, dtype=torch.bfloat16, device="cuda"), torch.full((m, inter), float("nan"), dtype=torch.bfloat16, device="cuda")
+    rows, room = torch.empty(m, 2 * inter, dtype=torch.bfloat16, device="cuda"), torch.full((m + 128, inter), float("nan"), dtype=torch.bfloat16, device="cuda")
+    out = room[:m]                              # columns are padded to 16, 32, 64 or 128 tokens: none of the padding is stored
     want = torch.empty_like(out)
     o.gemm_tcgen05(a, w, out, epilogue="swiglu")
     o.gemm_tcgen05(a, w, rows, max_splits=1)
     o.swiglu(rows, want, block=o.SWIGLU_BLOCK)
-    assert o.gemm_status() == 0 and torch.equal(out, want)
+    assert o.gemm_status() == 0 and torch.equal(out, want) and torch.isnan(room[m:]).all()
     if m <= 16:
         o.gemm_tcgen05(a, w, out.fill_(float("nan")), epilogue="clipped_swiglu", limit=1.0, slope=1.7)
         g, u = (a.double() @ part.double().T for part in w.view(-1, 2, o.SWIGLU_BLOCK, k).transpose(0, 1).reshape(2, inter, k))
@@ -88,6 +89,7 @@ def test_few_token_gated_product_of_whole_tiles(m):
         # gate, up, activation and product each round to bfloat16 at most, as in the split product's test above
         assert o.gemm_status() == 0
         assert ((out.double() - clipped).abs() <= 4 * 2.0 ** -8 * (clipped.abs() + u.abs() + 0.1)).all()
+        assert torch.isnan(room[m:]).all()
 
 
 @pytest.mark.parametrize("q_heads, kv_heads", [(4, 2), (32, 8)])
@@ -376,3 +378,35 @@ def test_plain_prompt_attention_takes_a_negative_window_as_none(q_heads, kv_head
         o.attention_tcgen05_prefill(q, pool, 0, outs[-1], table, ints([0, 40, 170]), ints(lengths), ints([0, 1, 1]), ints([0, 0, 128]), 3,
                                     q_heads, kv_heads, dim, page, dim ** -0.5, window)
     assert not torch.isnan(outs[0]).any() and torch.equal(*outs)
+
+
+@pytest.mark.parametrize("products", [False, True])
+@pytest.mark.parametrize("heads, dim, vdim, decay", [(2, 33, 7, [0.9, 0.0]), (3, 128, 128, [0.999, 0.5, 0.97])])
+@pytest.mark.parametrize("lengths, segment", [([512], 64), ([513], 64), ([1024, 70], 64), ([1500], 64), ([1025, 1153], 128)])
+def test_segments_that_are_joined_in_several_trips(monkeypatch, products, heads, dim, vdim, decay, lengths, segment):
+    """The joining takes eight segments a trip: 8, 9, 10, 16 and 24 of a sequence, a head's size that allows 16 bytes a load and one that
+    does not, in both forms (a first segment from the slot, all from zero)."""
+    o = ops()
+    monkeypatch.setattr(o, "decay_scan", functools.partial(o.decay_scan, products=products))
+    test_segments_as_matrix_products(heads, dim, vdim, decay, lengths, segment)
+
+
+@pytest.mark.parametrize("products", [False, True])
+@pytest.mark.parametrize("what", ["scratch", "state"])
+def test_joining_of_many_segments_gives_the_same_bits_from_anywhere(products, what):
+    """Scratch or states four bytes off a 16-byte boundary, 8, 9 and 17 segments a sequence."""
+    o, heads, dim, vdim, lengths, segment = ops(), 2, 64, 64, [512, 1088, 513], 64
+    tokens, n_seqs = sum(lengths), len(lengths)
+    gen = torch.Generator().manual_seed(2)
+    proj, start = torch.randn(tokens, heads * (2 * dim + vdim), generator=gen).cuda(), torch.randn(n_seqs, heads, dim, vdim, generator=gen).cuda()
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device="cuda")
+    lam, segments, results = torch.tensor([0.9, 0.999], device="cuda"), sum(-(-n // segment) for n in lengths), []
+    room = lambda count, shift: torch.full((count * heads * dim * vdim + 1,), float("nan"), device="cuda")[shift: shift + count * heads * dim * vdim] \
+        .view(count, heads, dim, vdim)
+    for shift in (0, 1):
+        scratch, state = room(segments, shift if what == "scratch" else 0), room(n_seqs, shift if what == "state" else 0).copy_(start)
+        out = torch.full((tokens, heads * vdim), float("nan"), device="cuda")
+        o.decay_scan(proj, 0, heads * dim, 2 * heads * dim, out, state, ints([sum(lengths[:s]) for s in range(n_seqs + 1)]), ints([2, 0, 1]), lam, n_seqs,
+                     heads, dim, vdim, None, segment, scratch, products)
+        results.append((out, state))
+    assert not any(torch.isnan(x).any() for x in results[0]) and all(torch.equal(a, b) for a, b in zip(*results))

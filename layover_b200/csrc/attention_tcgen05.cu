@@ -108,7 +108,8 @@ __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.a
 
 // The instructions of the tensor cores are called by a whole warp, whose branches and operands are the same for every lane, and issued
 // by one lane of it (always the same one): their operands then lie in uniform registers. From inside a branch of one lane an MMA
-// goes out every 52 cycles at best, and a commit or a wait costs as much again; a whole warp issues one every 12.
+// goes out every 53 cycles at best, and a commit or a wait costs as much again; from a whole warp as fast as the tensor cores take
+// them (1,024 products of 128 x 16 x 16 in a row: 54.6 and 39.0 cycles each).
 // Measured (one B200, 32 heads over 8): 512 tokens after 8,209 110.5 -> 95.6 us, a prompt of 2,048 51.9 -> 47.5: that warp was what a
 // tile took its 4,300 cycles for, of which the tensor cores worked 2,100 and either softmax 1,820.
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
@@ -591,7 +592,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid
 // factor on the outputs; a negative window is a chunked mask: a query sees the keys of its own chunk of -window positions). A
 // weight is the sum of two bfloat16 numbers, its rounded value and the rounded rest; the rests take the upper half of the
 // columns that the scores leave free, and the second product runs over them as well. Measured (one B200, 1,500 tokens of 32
-// heads over 8 behind a window of 1,024; two prompts of 611, 16 over 4): 45 us and 26 us (on mma.sync 224 and 87; 96 and 35 with
+// heads over 8 behind a window of 1,024; two prompts of 611, 16 over 4): 45 to 50 us and 26 us (on mma.sync 221 and 87; 96 and 35 with
 // comparisons in every tile of a window and one lane issuing)
 constexpr int PAIR_THREADS = 320;   // warp 0 producer, warp 1 MMA issuer, warps 2-5 and 6-9 the softmax warpgroups
 constexpr int MOST_KEYS = 96;       // keys of a tile whose part of the second product does not wait for the last exponentials

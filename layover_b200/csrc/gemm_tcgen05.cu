@@ -432,7 +432,8 @@ gemm_fewtoken_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 
 
 // ------------------------------------------------------------------ the persistent kernel
-// One block an SM: a launch never counted on two of half the ring each (their tensor memory), and half a ring of weights in flight was
+// One block an SM: of blocks with half the ring each, whose shared memory (99,584 bytes) and registers (121 x 192 threads) two would
+// share an SM, the occupancy query counted one all the same, and half a ring of weights in flight was
 // slower in the few-token orientation (one B200, q/k/v of 6144 rows, o and down of a 2560-wide model: 64 tokens 13.6 / 10.6 / 16.5
 // -> 12.5 / 10.1 / 15.0 us, 128 tokens 16.5 / 14.0 / 20.3 -> 14.6 / 12.2 / 17.0, the sum of the splits below included).
 // PAIR: two blocks of a cluster work as one MMA unit on a tile of 256 rows x BN columns; each block

@@ -1743,8 +1743,9 @@ def portion_splits(lens: tuple[tuple[int, int], ...], q_heads: int, kv_heads: in
     split costs 8.2 us, 0.2 us a block of a row, and 0.57 us for each MB of partial results (130 floats a row, head and
     block) on their way to the merge. The figures fitted 549 measurements on one B200 (4 over 2 to 64 over 8 heads, 8 to 2,048
     new tokens of one or three requests after 0 to 30,000) while a tile took that long; it takes 1.82 us since, and a split 7 us. The number
-    decides how a row's outputs are rounded, so a call keeps the one it has had. 32 over 8 heads, no split and 2 blocks: 512 tokens
-    after 8,209 139 and 91 us; 16 over 2: 1,280 tokens after 1,000 45 and 56, 1,024 after 12,000 196 and 121."""
+    decides how a row's outputs are rounded, so a call keeps the one it has had. 32 over 8 heads, one to five blocks: 512 tokens
+    after 8,209 137, 91, 123, 107 and 131 us (2 are taken), 128 after 769 26.9, 29.9, 28.9, 27.2 and 27.8 (1), 256 after 2,344 49, 43, 36.7,
+    35.3 and 52 (3), 5 after 822 20.4, 17.7, 16.5, 14.2 and 14.8 (3), 777 after 11,323 189, 211, 223, 233 and 214 (1)."""
     blocks = sum(-(-new // TCGEN05_TILE) for new, _ in lens) * q_heads // 2
     if (q_heads // kv_heads) % 2 or blocks >= 2 * sms:
         return 1
@@ -1776,8 +1777,9 @@ def exact_on_tcgen05(lens: tuple[tuple[int, int], ...], q_heads: int, window: in
     shared out over the SMs; a mask within the tiles (a window) makes a tile longer. The figures (us) fitted 1,016 measurements on one
     B200 (12 over 2, 16 over 4, 32 over 8 and 64 over 8 heads, 1 to 16 prompts of 20 to 900 tokens, portions of 2 to 1,000 tokens
     after 300 to 6,000, windows of 0, 128, 512 and 1,024) of a slower tcgen05 kernel. The two kernels round differently, so a call keeps
-    the one it has had. 16 over 4 heads, tcgen05 and mma.sync: one prompt of 20 tokens 16 and 9, of 261 22 and 19, of 512 24 and 28, two of
-    611 27 and 46, one of 1,500 44 and 104, behind a window of 1,024 44 and 137; 64 tokens after 500 32 and 32, after 3,000 69 and 132."""
+    the one it has had. 16 over 4 heads, tcgen05 and mma.sync: one prompt of 20 tokens 15.5 and 7.7, of 261 21.4 and 20.2, of 512 23 and 32,
+    of 1,500 46 and 104, behind a window of 1,024 45 and 136; 64 tokens after 500 32 and 31, after 3,000 71 and 131. Where the line is
+    off now: chunks of 1,024, 128 tokens 15.0 and 16.5, 261 21 and 38, 404 24 and 54, 568 27 and 68, mma.sync taken in all four."""
     def cost(rows: int, heads: int, start: float, tile: float, shared: float, masked: float) -> float:
         longest = total = 0
         for new, ctx in lens:

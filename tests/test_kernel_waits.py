@@ -17,9 +17,9 @@ def test_prompt_attention_tells_which_wait_ran_out():
 
 
 def test_prompt_attention_announces_nothing_of_a_tile_whose_wait_ran_out():
-    kernel = _prompt_attention_of_pairs()
-    between = kernel[kernel.index("mbar_arrive(&p_most[u])"): kernel.index("mbar_arrive(&p_full[u])")]
-    assert "if (!ok) break;" in between          # the waits before stand in an inner loop, whose break leaves only that one
+    # the waits before stand in an inner loop, whose break leaves only that one
+    announced = re.findall(r"if \((.*?)\) mbar_arrive\(&p_full\[u\]\)", _prompt_attention_of_pairs())
+    assert announced == ["ok && lane == 0"]
 
 
 def test_persistent_product_issues_no_tile_after_another_warps_wait_ran_out():
